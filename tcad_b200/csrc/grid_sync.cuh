@@ -1,0 +1,131 @@
+// Grid barrier that carries the dot products, for the single-launch solves
+// whose CTAs are all resident (cooperative launch, at most kSyncMaxCtas).
+//
+// A CTA stores its partial sums, one thread adds an arrival to a monotonic
+// counter (acquire-release) and polls it without backing off, and every CTA
+// then reads all partials: each thread takes one, so the totals are in every
+// thread after one block reduction.  Measured per step on 16 to 148 CTAs: 1.06
+// to 1.14 us without sums, 1.6 to 1.7 with one, 1.8 with three.  Tried and
+// slower at 148 CTAs: every CTA polling every other CTA's word with the sums
+// in it (one trip instead of two, but 148 x 148 polls contend: 4.1 / 5.3 /
+// 7.4 us), the same with private inboxes (2.3 / 2.6 / 6.4), a reduction
+// instead of the returning atomic (1.24 / 1.82 / 1.98).
+//
+// The sums are taken in the order of block_sum / Reduce::total, so a solve
+// gives the per-step kernels' bits.  Partials alternate between two buffers
+// by step parity: a CTA stores step k + 2 only after all have arrived at
+// k + 1, i.e. after all have read step k.
+//
+// Every wait is bounded (kBarrierNs of device time, or another CTA's give-up
+// flag); sum() then returns false in every thread of the CTA and the kernel
+// returns.
+#pragma once
+
+namespace tcad {
+
+constexpr unsigned long long kBarrierNs = 1000000000ull;   // 1 s
+constexpr int kSyncMaxCtas = kFlatThreads;                 // one partial per thread
+constexpr int kSyncSums = 3;                               // sums per step, at most
+
+// doubles of the partials' two buffers
+constexpr size_t sync_doubles() { return 2 * kSyncSums * (size_t)kSyncMaxCtas; }
+
+__device__ __forceinline__ unsigned long long globaltimer_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+__device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
+  unsigned old;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
+               : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+struct GridSync {
+  double* partial;   // sync_doubles()
+  unsigned* bar;     // [0]: arrivals; [2]: a CTA gave up; [3]: the give-up test
+                     // hook, an arrival to wait for that never comes
+  unsigned round;
+
+  __device__ __forceinline__ void init(double* part, unsigned* b) {
+    partial = part;
+    bar = b;
+    round = 0;
+  }
+
+  // tot = the sums over the grid of every thread's v, valid in every thread;
+  // NQ = 0: a barrier alone.  Orders all global writes before it, of any
+  // thread of the grid, before all reads after it.
+  template <int NQ>
+  __device__ __forceinline__ bool sum(const double* v, double* tot) {
+    static_assert(NQ <= kSyncSums, "sums per step");
+    constexpr int NT = kFlatThreads, NW = NT / 32, NS = NQ > 0 ? NQ : 1;
+    __shared__ double sa[NS][NW], sb[NS][NW];
+    __shared__ int ok;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned G = gridDim.x;
+    // the last tree of block_sum: 8 warp sums, halves added pairwise
+    const auto tree = [](const double* w) {
+      const double a = w[0] + w[4], b = w[1] + w[5], c = w[2] + w[6], d = w[3] + w[7];
+      return (a + c) + (b + d);
+    };
+    const auto warps = [&](double (*dst)[NW], double* r) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r[q] += __shfl_down_sync(0xffffffffu, r[q], o);
+        if (lane == 0) dst[q][warp] = r[q];
+      }
+    };
+    ++round;
+    double* const buf = partial + (round & 1u) * (size_t)(kSyncSums * kSyncMaxCtas);
+    double r[NS];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) r[q] = v[q];
+    warps(sa, r);
+    __syncthreads();   // the CTA's sums are in sa, its global writes are issued
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) buf[q * kSyncMaxCtas + blockIdx.x] = tree(sa[q]);
+      int good = 1;
+      const unsigned target = round * G + ld_acquire(&bar[3]);
+      if (atom_add_acq_rel(&bar[0], 1u) + 1u != target) {
+        unsigned long long t0 = 0;
+        for (unsigned it = 1; (int)(ld_acquire(&bar[0]) - target) < 0; ++it) {
+          if ((it & 255u) != 0u) continue;
+          const unsigned long long now = globaltimer_ns();
+          if (t0 == 0) t0 = now;
+          if (ld_acquire(&bar[2]) != 0u) { good = 0; break; }
+          if (now - t0 > kBarrierNs || it > (1u << 30)) {
+            atomicExch(&bar[2], 1u);
+            good = 0;
+            break;
+          }
+        }
+      }
+      ok = good;
+    }
+    __syncthreads();
+    if (!ok) return false;
+    if constexpr (NQ > 0) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        r[q] = 0.0 + (threadIdx.x < G ? __ldcg(&buf[q * kSyncMaxCtas + threadIdx.x]) : 0.0);
+      warps(sb, r);
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) tot[q] = tree(sb[q]);
+    }
+    return true;
+  }
+};
+
+}  // namespace tcad

@@ -667,6 +667,8 @@ k_true_resid(const tcad_pack_t pk, const TJ* __restrict__ J, const T* __restrict
 
 }  // namespace tcad
 #include "redblack.cuh"
+#include "grid_sync.cuh"
+#include "rb_resident.cuh"
 namespace tcad {
 
 // ---- the whole solve in one cooperative launch (single-instance packs whose
@@ -682,27 +684,6 @@ namespace tcad {
 // target: 0 always, except under the give-up test hook
 // (tcad_set_krylov_fused_test), which sets it to 1 so that the first barrier
 // waits for an arrival that never comes and its time limit runs out.
-constexpr unsigned long long kBarrierNs = 1000000000ull;   // 1 s
-
-__device__ __forceinline__ unsigned long long globaltimer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
-               : "=r"(old) : "l"(p), "r"(v) : "memory");
-  return old;
-}
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, unsigned& round) {
   __shared__ int ok;
   __syncthreads();
@@ -1555,17 +1536,28 @@ struct WorkRb {
   int64_t* flat_off;
   int32_t* flat_inst;
   int32_t* blk;  // compact list of the slot pack's flat blocks still iterating
+  double* partial;    // 8 per flat block of the slot pack: block partial sums
+  double* sync;       // the resident solve's step sums (grid_sync.cuh)
   size_t bytes;
 };
 
 // Slot-pack flat blocks hold pk->flat_nodes slots (measured, 200-iteration
 // solves on the two-lane 983k-node tri-gate: 419 us per iteration at 512
 // slots and 5 CTAs per SM, 450 at 256 slots, 511 at 256 slots and 4 CTAs,
-// 774 at 128).  The count is bounded by slots / rb_flat + n_inst <=
-// n_nodes / rb_flat + n_inst.
-static int64_t rb_flat(const tcad_pack_t* pk) { return pk->flat_nodes; }
+// 774 at 128).  A single instance that the resident solve takes (at most
+// kRbResidentCtas blocks of kRbResidentMaxSlots) is split over all SMs
+// instead: whole warps of slots, at most one block per SM.
+constexpr int64_t kRbResidentCtas = 148;
+static int64_t rb_flat(const tcad_pack_t* pk, int64_t slots) {
+  if (pk->n_inst != 1) return pk->flat_nodes;
+  const int64_t fn = ((slots + kRbResidentCtas - 1) / kRbResidentCtas + 31) / 32 * 32;
+  return fn <= kRbResidentMaxSlots ? fn : pk->flat_nodes;
+}
+// slots / rb_flat + n_inst <= n_nodes / flat_nodes + n_inst, or the resident
+// solve's blocks
 static size_t rb_flat_cap(const tcad_pack_t* pk) {
-  return (size_t)(pk->n_nodes / rb_flat(pk)) + (size_t)pk->n_inst + 1;
+  return (size_t)(pk->n_nodes / pk->flat_nodes) + (size_t)pk->n_inst + 1 +
+         (size_t)(pk->n_inst == 1 ? kRbResidentCtas : 0);
 }
 
 static WorkRb carve_rb(const tcad_pack_t* pk, void* base) {
@@ -1586,6 +1578,8 @@ static WorkRb carve_rb(const tcad_pack_t* pk, void* base) {
   w.flat_off = c.take<int64_t>((size_t)pk->n_inst + 1);
   w.flat_inst = c.take<int32_t>(rb_flat_cap(pk));
   w.blk = c.take<int32_t>(rb_flat_cap(pk));
+  w.partial = c.take<double>(8 * rb_flat_cap(pk));
+  w.sync = c.take<double>(sync_doubles());
   w.bytes = c.used;
   return w;
 }
@@ -1626,7 +1620,7 @@ static WorkEq carve_eq(const tcad_pack_t* pk, void* base) {
 }
 
 // The slot pack of a pack (host tables; see redblack.cuh): per instance
-// (ceil(Nx/2), Ny Nz, 1) slots of each colour, flat blocks of pk->flat_nodes
+// (ceil(Nx/2), Ny Nz, 1) slots of each colour, flat blocks of rb_flat slots
 struct RbLayout {
   tcad_pack_t pkb;
   RbMap mp;
@@ -1634,7 +1628,8 @@ struct RbLayout {
 };
 
 template <class W>   // WorkRb or WorkEq: the slot pack's table arrays
-static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream_t s) {
+static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream_t s,
+                     bool resident) {
   const int ni = pk->n_inst;
   std::vector<int32_t> shp(3 * (size_t)ni), sb(3 * (size_t)ni), fi;
   TCAD_CUDA_CHECK(cudaMemcpyAsync(shp.data(), pk->shape, sizeof(int32_t) * shp.size(),
@@ -1642,7 +1637,9 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
   std::vector<int64_t> noff(ni + 1), foff(ni + 1);
   noff[0] = 0; foff[0] = 0;
-  const int64_t fn = rb_flat(pk);
+  int64_t fn = pk->flat_nodes;
+  if (resident && ni == 1)
+    fn = rb_flat(pk, (int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2]);
   for (int i = 0; i < ni; ++i) {
     const int64_t hx = (shp[3 * i] + 1) / 2, rows = (int64_t)shp[3 * i + 1] * shp[3 * i + 2];
     sb[3 * i] = (int32_t)hx; sb[3 * i + 1] = (int32_t)rows; sb[3 * i + 2] = 1;
@@ -1651,10 +1648,10 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
     foff[i + 1] = foff[i] + nf;
     for (int64_t b = 0; b < nf; ++b) fi.push_back(i);
   }
-  // (the Krylov partials hold 8 n_flat doubles: 4 per slot block fit, as
-  // n_flat >= max(n_inst, n_nodes / flat_nodes))
+  // (without the resident blocks the Krylov partials, 8 n_flat doubles, hold
+  // 4 per slot block, as n_flat >= max(n_inst, n_nodes / flat_nodes))
   if (noff[ni] > pk->n_nodes || (size_t)foff[ni] > rb_flat_cap(pk) ||
-      4 * foff[ni] > 8 * pk->n_flat)
+      (!resident && 4 * foff[ni] > 8 * pk->n_flat))
     return TCAD_ERR_ARG;
   TCAD_CUDA_CHECK(cudaMemcpyAsync(wr.shape, sb.data(), sizeof(int32_t) * sb.size(),
                                   cudaMemcpyHostToDevice, s));
@@ -1969,6 +1966,97 @@ static bool rb_fused_fits(unsigned nb) {
   return nb >= 1 && (long long)nb <= (long long)per * sms;
 }
 
+// Launch configuration of a cooperative single-launch solve, its barrier
+// flags cleared (and the give-up test hook set)
+struct CoopLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+};
+static int coop_launch(CoopLaunch& c, unsigned blocks, size_t smem, unsigned* flags,
+                       cudaStream_t s) {
+  TCAD_CUDA_CHECK(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned), s));
+  if (g_fused_test_hold.load()) {
+    static const unsigned kPhantom = 1u;
+    TCAD_CUDA_CHECK(cudaMemcpyAsync(flags + 3, &kPhantom, sizeof(unsigned),
+                                    cudaMemcpyHostToDevice, s));
+  }
+  c.cfg.gridDim = dim3(blocks);
+  c.cfg.blockDim = dim3(NT);
+  c.cfg.dynamicSmemBytes = smem;
+  c.cfg.stream = s;
+  c.at[0].id = cudaLaunchAttributeCooperative;
+  c.at[0].val.cooperative = 1;
+  c.cfg.attrs = c.at;
+  c.cfg.numAttrs = 1;
+  return TCAD_OK;
+}
+
+// Waits for a single-launch solve and reads its result: 1 when a grid
+// barrier gave up (the caller then solves with one launch per step)
+static int coop_result(const Work& w, std::vector<KState>& hks, cudaStream_t s) {
+  hks.resize(1);
+  unsigned hbar[4] = {0u, 0u, 0u, 0u};
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState), cudaMemcpyDeviceToHost, s));
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(hbar, w.bar, sizeof(hbar), cudaMemcpyDeviceToHost, s));
+  TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+  if (hbar[2] != 0u) {
+    g_fused_gave_up.fetch_add(1);
+    return 1;
+  }
+  return TCAD_OK;
+}
+
+// k_bicgstab_rb_resident over the slot pack's blocks.  Returns TCAD_OK with
+// hks[0] filled, or 1 when the launch was refused or a wait gave up.
+template <int DIM, int K, bool JS>
+static int launch_rb_resident_t(const tcad_pack_t* pk, const RbLayout& L, const WorkRb& wr,
+                                const double* b, double* x, double rtol, int maxiter,
+                                const Work& w, const int32_t* pre_status,
+                                std::vector<KState>& hks, cudaStream_t s,
+                                const double* rtol_inst) {
+  const auto kern = k_bicgstab_rb_resident<DIM, K, JS>;
+  const size_t smem = JS ? (size_t)L.pkb.flat_nodes * Stencil<DIM>::NE * 16 : 0;
+  if (JS && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  CoopLaunch c;
+  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, smem, w.bar, s)) return rc;
+  const BiVec& bi = w.bi;
+  const int rechecks = 8;
+  // (a cooperative launch that does not fit is refused, not run)
+  if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, (const double*)wr.JR, (const double*)wr.JB,
+                         b, x, wr.bR, wr.tR, wr.xb, wr.rhs, bi.r, bi.p, bi.v, w.ks, wr.sync,
+                         w.bar, rtol, maxiter, pre_status, rtol_inst, rechecks) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  note_launch();
+  return coop_result(w, hks, s);
+}
+
+static int launch_bicgstab_rb_resident(const tcad_pack_t* pk, const RbLayout& L,
+                                       const WorkRb& wr, const double* b, double* x,
+                                       double rtol, int maxiter, const Work& w,
+                                       const int32_t* pre_status, std::vector<KState>& hks,
+                                       cudaStream_t s, const double* rtol_inst) {
+  const int fn = L.pkb.flat_nodes;
+  if (fn > kRbResidentMaxSlots || fn % 32) return 1;
+  const bool d2 = pk->dim == 2;
+  const bool js = fn <= rb_resident_js_slots(d2 ? TCAD_NE2 : TCAD_NE3);
+  auto go = [&](auto fnc) {
+    return fnc(pk, L, wr, b, x, rtol, maxiter, w, pre_status, hks, s, rtol_inst);
+  };
+  if (d2)
+    return fn <= NT ? go(launch_rb_resident_t<2, 1, true>)
+           : js     ? go(launch_rb_resident_t<2, 2, true>)
+                    : go(launch_rb_resident_t<2, 2, false>);
+  return fn <= NT ? go(launch_rb_resident_t<3, 1, true>)
+         : js     ? go(launch_rb_resident_t<3, 2, true>)
+                  : go(launch_rb_resident_t<3, 2, false>);
+}
+
 // The whole red-black solve of a single-instance pack in one launch (same
 // arithmetic as launch_bicgstab_rb's per-step loop).  Returns TCAD_OK with
 // hks[0] filled, or 1 when the launch was refused or a grid barrier gave up
@@ -1999,11 +2087,11 @@ static int launch_bicgstab_rb_fused(const tcad_pack_t* pk, const RbLayout& L,
       pk->dim == 2
           ? cudaLaunchKernelEx(&cfg, k_bicgstab_rb_fused<2>, L.pkb, L.mp, (const double*)wr.JR,
                                (const double*)wr.JB, b, x, wr.bR, wr.bB, wr.tR, wr.xb, wr.rhs,
-                               bi, w.ks, w.partial, w.bar, rtol, maxiter, pre_status,
+                               bi, w.ks, wr.partial, w.bar, rtol, maxiter, pre_status,
                                rtol_inst, rechecks)
           : cudaLaunchKernelEx(&cfg, k_bicgstab_rb_fused<3>, L.pkb, L.mp, (const double*)wr.JR,
                                (const double*)wr.JB, b, x, wr.bR, wr.bB, wr.tR, wr.xb, wr.rhs,
-                               bi, w.ks, w.partial, w.bar, rtol, maxiter, pre_status,
+                               bi, w.ks, wr.partial, w.bar, rtol, maxiter, pre_status,
                                rtol_inst, rechecks);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
@@ -2039,22 +2127,27 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
   BiVec bi = w.bi;   // black vectors (stride: the slot count)
   bi.ph = bi.p;
   bi.sh = bi.s;
-  if (g_fused_mode.load() && ni == 1 &&
-      (d2 ? rb_fused_fits<2>(nbb) : rb_fused_fits<3>(nbb)) &&
-      launch_bicgstab_rb_fused(pk, L, wr, b, x, rtol, maxiter, bi, w, pre_status, hks, s,
-                               rtol_inst) == TCAD_OK)
-    return TCAD_OK;
+  if (g_fused_mode.load() && ni == 1) {
+    const int rc = (int64_t)nbb <= kRbResidentCtas
+                       ? launch_bicgstab_rb_resident(pk, L, wr, b, x, rtol, maxiter, w,
+                                                     pre_status, hks, s, rtol_inst)
+                   : (d2 ? rb_fused_fits<2>(nbb) : rb_fused_fits<3>(nbb))
+                       ? launch_bicgstab_rb_fused(pk, L, wr, b, x, rtol, maxiter, bi, w,
+                                                  pre_status, hks, s, rtol_inst)
+                       : 1;
+    if (rc == TCAD_OK) return TCAD_OK;
+  }
   TCAD_CUDA_CHECK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned) * ni, s));
-  if (d2) k_rb_split<2><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, w.partial, w.ticket);
-  else    k_rb_split<3><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, w.partial, w.ticket);
+  if (d2) k_rb_split<2><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, wr.partial, w.ticket);
+  else    k_rb_split<3><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, wr.partial, w.ticket);
   note_launch();
   if (d2)
     k_rb_init<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.bR, wr.bB, wr.rhs, wr.xb, bi, wr.bbf,
-                                    w.ks, w.partial, w.ticket, rtol, maxiter, pre_status,
+                                    w.ks, wr.partial, w.ticket, rtol, maxiter, pre_status,
                                     rtol_inst);
   else
     k_rb_init<3><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.bR, wr.bB, wr.rhs, wr.xb, bi, wr.bbf,
-                                    w.ks, w.partial, w.ticket, rtol, maxiter, pre_status,
+                                    w.ks, wr.partial, w.ticket, rtol, maxiter, pre_status,
                                     rtol_inst);
   note_launch();
   TCAD_LAUNCH_CHECK();
@@ -2069,24 +2162,24 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
       k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist);
       if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.p, wr.tR, w.ks, dlist);
-        k_rb_v<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, w.partial, w.ticket,
+        k_rb_v<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
       } else {
         k_rb_red<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.p, wr.tR, w.ks, dlist);
-        k_rb_v<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, w.partial, w.ticket,
+        k_rb_v<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
       }
-      k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, w.partial, w.ticket, dlist);
+      k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist);
       if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.s, wr.tR, w.ks, dlist);
-        k_rb_t<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, w.partial, w.ticket,
+        k_rb_t<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
       } else {
         k_rb_red<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.s, wr.tR, w.ks, dlist);
-        k_rb_t<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, w.partial, w.ticket,
+        k_rb_t<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
       }
-      k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, w.partial, w.ticket, dlist);
+      k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, wr.partial, w.ticket, dlist);
       for (int l = 0; l < 7; ++l) note_launch();
     }
     TCAD_LAUNCH_CHECK();
@@ -2104,11 +2197,11 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
       if (d2) {
         k_rb_red<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JR, wr.xb, wr.tR, nullptr, nullptr);
         k_rb_true<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, wr.rhs, wr.xb, bi.r, w.ks,
-                                        w.partial, w.ticket, rearm);
+                                        wr.partial, w.ticket, rearm);
       } else {
         k_rb_red<3><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JR, wr.xb, wr.tR, nullptr, nullptr);
         k_rb_true<3><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, wr.rhs, wr.xb, bi.r, w.ks,
-                                        w.partial, w.ticket, rearm);
+                                        wr.partial, w.ticket, rearm);
       }
       note_launch();
       note_launch();
@@ -2505,7 +2598,7 @@ extern "C" int tcad_block_krylov(const tcad_pack_t* pk, const double* J, const d
     if (work_bytes < tcad_block_workspace_bytes(pk, 2, 0)) return TCAD_ERR_ARG;
     const WorkRb wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
     RbLayout rbl;
-    if ((rc = rb_layout(pk, wrb, rbl, s)) != TCAD_OK) return rc;
+    if ((rc = rb_layout(pk, wrb, rbl, s, true)) != TCAD_OK) return rc;
     const unsigned nbb = (unsigned)rbl.pkb.n_flat;
     if (pk->dim == 2)
       k_rb_pack<2><<<nbb, NT, 0, s>>>(rbl.pkb, rbl.mp, J, wrb.JR, wrb.JB);
@@ -2601,7 +2694,7 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
   RbLayout rbl;
   if (use_rb) {
     wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
-    if (int rc = rb_layout(pk, wrb, rbl, s)) return rc;
+    if (int rc = rb_layout(pk, wrb, rbl, s, true)) return rc;
   }
   std::vector<int32_t> mix_it(ni), mix_st(ni), mix_grew(ni, 0), mix_steps(ni, 0);
   std::vector<double> mix_rr(ni), mix_prev(ni, -1.0);
@@ -2936,7 +3029,7 @@ extern "C" int tcad_equilibrium_solve(const tcad_pack_t* pk, double* psi, double
   RbLayout rbl;
   if (use_rb) {
     we = carve_eq(pk, reinterpret_cast<char*>(work) + off_eq(pk));
-    if (int rc = rb_layout(pk, we, rbl, s)) return rc;
+    if (int rc = rb_layout(pk, we, rbl, s, false)) return rc;
   }
   for (int it = 0; it < opts->max_iter; ++it) {
     TCAD_CUDA_CHECK(cudaMemcpyAsync(dact, hact.data(), ni, cudaMemcpyHostToDevice, s));
