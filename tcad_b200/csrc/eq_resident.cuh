@@ -1,0 +1,185 @@
+// The equilibrium red-black PCG (k_eqrb_*) of a single-instance pack in one
+// cooperative launch with everything resident: one CTA per SM (and per flat
+// block of the slot pack, K * 256 slots at most), the CTA's rows of both
+// colours in shared memory, taken straight from the node-order J, its slots'
+// vectors in registers; z, p, x and Tr also in global memory for the
+// neighbours.
+//
+// The scalar rows are small (112 bytes a slot pair in 3D), so up to 303k slots
+// (600k nodes) stay resident and an iteration is bound by the latency of its
+// three steps -- red(p), q (alpha), x (beta) -- instead of four launches and
+// two last-block reductions.  240 x 120 MOSFET: 24 -> 6.5 us per iteration.
+// Expressions and the order of the sums are the per-step kernels', so the
+// update is bit-identical to launch_cg_rb's loop.
+#pragma once
+
+namespace tcad {
+
+constexpr int kEqResidentMaxSlots = 8 * NT;
+
+template <int DIM, int K>
+__global__ void __launch_bounds__(NT, 1)
+k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ J,
+                const double* __restrict__ F, double* __restrict__ d, double* zg, double* pg,
+                double* xg, double* Tr, KState* ks, double* part, unsigned* bar, double rtol,
+                int maxit, const uint8_t* __restrict__ active,
+                const double* __restrict__ rtol_inst) {
+  constexpr int NE = 1 + 2 * DIM, ND = 2 * DIM;
+  extern __shared__ __align__(16) double s_rows[];   // [2][NE][flat_nodes]
+  GridSync gs;
+  gs.init(part, bar);
+  const FlatBlock fb = flat_block(pkb, blockIdx.x);
+  const int inst = fb.inst;
+  const RbGeo g = rb_geo(pkb, mp, inst);
+  const int64_t NN = mp.n_full;
+  const int nloc = (int)(fb.end - fb.begin), fn = pkb.flat_nodes;
+  double* const sR = s_rows;
+  double* const sB = s_rows + (int64_t)NE * fn;
+  const int64_t q0 = fb.begin + threadIdx.x;   // slot k of the thread: q0 + k NT
+  int mr[K][ND], mb[K][ND];
+  bool own[K], realr[K], realb[K];
+  double x[K], r[K], z[K], p[K], q[K], si[K];
+  double sum[2], tot[2];
+  KState S;
+
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int l = threadIdx.x + k * NT;
+    own[k] = l < nloc;
+    const int64_t slot = own[k] ? q0 + k * NT : fb.begin;
+    const RbNode nr = rb_node(g, slot, 0), nk = rb_node(g, slot, 1);
+    realr[k] = own[k] && nr.real;
+    realb[k] = own[k] && nk.real;
+    int m[6];
+    rb_nbrs<DIM>(g, nr, (int)(slot - g.soff), m);
+#pragma unroll
+    for (int a = 0; a < ND; ++a) mr[k][a] = m[a];
+    rb_nbrs<DIM>(g, nk, (int)(slot - g.soff), m);
+#pragma unroll
+    for (int a = 0; a < ND; ++a) mb[k][a] = m[a];
+    r[k] = realr[k] ? F[nr.node] : 0.0;   // F_r here and F_b in q until the start
+    q[k] = realb[k] ? F[nk.node] : 0.0;
+    if (own[k])
+#pragma unroll
+      for (int e = 0; e < NE; ++e) {
+        sR[e * fn + l] = realr[k] ? J[(int64_t)e * NN + nr.node] : 0.0;
+        sB[e * fn + l] = realb[k] ? J[(int64_t)e * NN + nk.node] : 0.0;
+      }
+    // Sinv = 1 / diag(S), as k_eqrb_diag; a neighbour's row is J at its node
+    double sd = 0.0;
+    if (realb[k]) {
+      const int64_t sxy = (int64_t)g.nx * g.ny;
+      const int64_t step[6] = {-1, 1, -(int64_t)g.nx, g.nx, -sxy, sxy};
+      sd = -J[nk.node];
+#pragma unroll
+      for (int a = 0; a < ND; ++a) {
+        const double jbd = J[(int64_t)(1 + a) * NN + nk.node];
+        if (jbd != 0.0) {
+          const int64_t n = nk.node + step[a];
+          const double jrb = J[(int64_t)(1 + (a ^ 1)) * NN + n];
+          sd -= (jbd * jrb) / (-J[n]);
+        }
+      }
+    }
+    si[k] = (realb[k] && sd != 0.0) ? 1.0 / sd : 0.0;
+  }
+
+  // red pass: t = A_rr^-1 (vr - A_rb X) at the thread's red slots
+  auto red = [&](int k, const auto& X, double vr) {
+    double t = 0.0;
+    if (realr[k]) {
+      const int l = threadIdx.x + k * NT;
+      double a = 0.0;
+#pragma unroll
+      for (int e = 0; e < ND; ++e) a += sR[(1 + e) * fn + l] * X(mr[k][e]);
+      const double arr = -sR[l];
+      t = (vr + a) / arr;
+    }
+    return t;
+  };
+  // black coupling: -sum_d J_bd Tr(m_d)
+  auto black = [&](int k) {
+    const int l = threadIdx.x + k * NT;
+    const double* const ti = Tr + g.soff;
+    double a = 0.0;
+#pragma unroll
+    for (int e = 0; e < ND; ++e) a += sB[(1 + e) * fn + l] * __ldcg(ti + mb[k][e]);
+    return -a;
+  };
+
+  // start: Tr = A_rr^-1 F_r, rhs = F_b - A_br Tr; x = 0, r = rhs, z = p = Sinv r
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (own[k]) Tr[q0 + k * NT] = red(k, [](int) { return 0.0; }, r[k]);
+  if (!gs.sum<0>(nullptr, nullptr)) return;
+  sum[0] = 0.0; sum[1] = 0.0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    x[k] = 0.0; r[k] = 0.0; z[k] = 0.0; p[k] = 0.0;
+    if (!own[k]) continue;
+    const double bv = realb[k] ? q[k] - black(k) : 0.0;
+    z[k] = bv * si[k];
+    r[k] = bv;
+    zg[q0 + k * NT] = z[k];
+    pg[q0 + k * NT] = 0.0;
+    sum[0] += bv * z[k];
+    sum[1] += bv * bv;
+  }
+  if (!gs.sum<2>(sum, tot)) return;
+  fin_cg_init(S, tot[0], tot[1], rtol_inst ? rtol_inst[inst] : rtol, maxit,
+              !active || active[inst]);
+  S.beta = 0.0;   // the first direction is z: p = z + 0 * 0
+  while (S.active) {
+    const double beta = S.beta;
+    const double* const zi = zg + g.soff;
+    const double* const pi = pg + g.soff;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (own[k])
+        Tr[q0 + k * NT] =
+            red(k, [&](int m) { return __ldcg(zi + m) + beta * __ldcg(pi + m); }, 0.0);
+    if (!gs.sum<0>(nullptr, nullptr)) return;
+    sum[0] = 0.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (!own[k]) continue;
+      const double pv = z[k] + beta * p[k];
+      p[k] = pv;
+      pg[q0 + k * NT] = pv;
+      q[k] = realb[k] ? -sB[threadIdx.x + k * NT] * pv + black(k) : 0.0;
+      sum[0] += pv * q[k];
+    }
+    if (!gs.sum<1>(sum, tot)) return;
+    fin_cg_q(S, tot[0]);
+    if (!S.active) break;
+    sum[0] = 0.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (!own[k]) continue;
+      x[k] = x[k] + S.alpha * p[k];
+      const double rn = r[k] - S.alpha * q[k];
+      r[k] = rn;
+      z[k] = rn * si[k];
+      zg[q0 + k * NT] = z[k];
+      sum[0] += rn * z[k];
+    }
+    if (!gs.sum<1>(sum, tot)) return;
+    fin_cg_x(S, tot[0]);
+  }
+  // d_r = A_rr^-1 (F_r - A_rb d_b), d_b = x
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (own[k]) xg[q0 + k * NT] = x[k];
+  if (!gs.sum<0>(nullptr, nullptr)) return;
+  const double* const xi = xg + g.soff;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (!own[k]) continue;
+    const RbNode nr = rb_node(g, q0 + k * NT, 0), nk = rb_node(g, q0 + k * NT, 1);
+    if (realr[k]) d[nr.node] = red(k, [&](int m) { return __ldcg(xi + m); }, F[nr.node]);
+    if (realb[k]) d[nk.node] = x[k];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) ks[inst] = S;
+}
+
+}  // namespace tcad

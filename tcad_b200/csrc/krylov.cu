@@ -954,6 +954,44 @@ struct CgVec {
   double *r, *z, *p, *q;
 };
 
+// scalar updates of one instance from its totals, for the per-step kernels
+// and the resident solve
+__device__ __forceinline__ void fin_cg_init(KState& s, double rz, double rr, double rt,
+                                            int maxit, bool on) {
+  s.bb = rz; s.rho = rz; s.rr = rz;
+  s.tol2 = rt * rt * rz;
+  s.it = 0; s.maxit = maxit; s.status = TCAD_OK; s.restart = 0; s.early = 0;
+  if (!isfinite(rz) || !isfinite(rr)) s.status = TCAD_ERR_NONFINITE;
+  s.active = (s.status == TCAD_OK && rz > 0.0 && on) ? 1 : 0;
+}
+
+__device__ __forceinline__ void fin_cg_q(KState& s, double pq) {
+  if (!(pq > 0.0) || !isfinite(pq)) {
+    s.status = TCAD_ERR_BREAKDOWN;
+    s.active = 0;
+  } else {
+    s.alpha = s.rho / pq;
+  }
+}
+
+__device__ __forceinline__ void fin_cg_x(KState& s, double rz) {
+  s.it += 1;
+  s.rho_prev = s.rho;
+  s.rho = rz;
+  s.rr = rz;
+  if (!isfinite(rz)) {
+    s.status = TCAD_ERR_NONFINITE;
+    s.active = 0;
+  } else if (rz <= s.tol2) {
+    s.active = 0;
+  } else if (s.it >= s.maxit) {
+    s.status = TCAD_ERR_NOCONV;
+    s.active = 0;
+  } else {
+    s.beta = s.rho / s.rho_prev;
+  }
+}
+
 template <int DIM>
 __device__ __forceinline__ double pspmv(const double* __restrict__ J,
                                         const double* __restrict__ x, int64_t k, int64_t NN,
@@ -984,15 +1022,9 @@ k_cg_init(const tcad_pack_t pk, const double* __restrict__ J, const double* __re
   }
   (void)NN;
   double tot[2];
-  if (Reduce<2>::run(pk, blockIdx.x, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0) {
-    KState& s = ks[fb.inst];
-    s.bb = tot[0]; s.rho = tot[0]; s.rr = tot[0];
-    const double rt = rtol_inst ? rtol_inst[fb.inst] : rtol;
-    s.tol2 = rt * rt * tot[0];
-    s.it = 0; s.maxit = maxit; s.status = TCAD_OK; s.restart = 0; s.early = 0;
-    if (!isfinite(tot[0]) || !isfinite(tot[1])) s.status = TCAD_ERR_NONFINITE;
-    s.active = (s.status == TCAD_OK && tot[0] > 0.0 && (!active || active[fb.inst])) ? 1 : 0;
-  }
+  if (Reduce<2>::run(pk, blockIdx.x, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0)
+    fin_cg_init(ks[fb.inst], tot[0], tot[1], rtol_inst ? rtol_inst[fb.inst] : rtol, maxit,
+                !active || active[fb.inst]);
 }
 
 template <int DIM>
@@ -1013,15 +1045,8 @@ k_cg_q(const tcad_pack_t pk, const double* __restrict__ J, CgVec w, KState* ks,
     v[0] += w.p[k] * q;
   }
   double tot[1];
-  if (Reduce<1>::run(pk, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0) {
-    KState& s = ks[fb.inst];
-    if (!(tot[0] > 0.0) || !isfinite(tot[0])) {
-      s.status = TCAD_ERR_BREAKDOWN;
-      s.active = 0;
-    } else {
-      s.alpha = s.rho / tot[0];
-    }
-  }
+  if (Reduce<1>::run(pk, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0)
+    fin_cg_q(ks[fb.inst], tot[0]);
 }
 
 __global__ void __launch_bounds__(NT)
@@ -1041,24 +1066,8 @@ k_cg_x(const tcad_pack_t pk, const double* __restrict__ J, double* __restrict__ 
     v[0] += r * z;
   }
   double tot[1];
-  if (Reduce<1>::run(pk, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0) {
-    KState& s = ks[fb.inst];
-    s.it += 1;
-    s.rho_prev = s.rho;
-    s.rho = tot[0];
-    s.rr = tot[0];
-    if (!isfinite(tot[0])) {
-      s.status = TCAD_ERR_NONFINITE;
-      s.active = 0;
-    } else if (tot[0] <= s.tol2) {
-      s.active = 0;
-    } else if (s.it >= s.maxit) {
-      s.status = TCAD_ERR_NOCONV;
-      s.active = 0;
-    } else {
-      s.beta = s.rho / s.rho_prev;
-    }
-  }
+  if (Reduce<1>::run(pk, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0)
+    fin_cg_x(ks[fb.inst], tot[0]);
 }
 
 __global__ void __launch_bounds__(NT)
@@ -1201,15 +1210,9 @@ k_eqrb_init(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JB
     v[1] += bv * bv;
   }
   double tot[2];
-  if (Reduce<2>::run(pkb, blockIdx.x, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0) {
-    KState& s = ks[fb.inst];
-    s.bb = tot[0]; s.rho = tot[0]; s.rr = tot[0];
-    const double rt = rtol_inst ? rtol_inst[fb.inst] : rtol;
-    s.tol2 = rt * rt * tot[0];
-    s.it = 0; s.maxit = maxit; s.status = TCAD_OK; s.restart = 0; s.early = 0;
-    if (!isfinite(tot[0]) || !isfinite(tot[1])) s.status = TCAD_ERR_NONFINITE;
-    s.active = (s.status == TCAD_OK && tot[0] > 0.0 && (!active || active[fb.inst])) ? 1 : 0;
-  }
+  if (Reduce<2>::run(pkb, blockIdx.x, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0)
+    fin_cg_init(ks[fb.inst], tot[0], tot[1], rtol_inst ? rtol_inst[fb.inst] : rtol, maxit,
+                !active || active[fb.inst]);
 }
 
 // q = S p (Tr from the red pass of p); alpha = rho / (p, q)
@@ -1234,15 +1237,8 @@ k_eqrb_q(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JBe,
     v[0] += pv * qv;
   }
   double tot[1];
-  if (Reduce<1>::run(pkb, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0) {
-    KState& s = ks[fb.inst];
-    if (!(tot[0] > 0.0) || !isfinite(tot[0])) {
-      s.status = TCAD_ERR_BREAKDOWN;
-      s.active = 0;
-    } else {
-      s.alpha = s.rho / tot[0];
-    }
-  }
+  if (Reduce<1>::run(pkb, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0)
+    fin_cg_q(ks[fb.inst], tot[0]);
 }
 
 // x += alpha p, r -= alpha q, z = Sinv r; (r, z), convergence as k_cg_x
@@ -1264,24 +1260,8 @@ k_eqrb_x(const tcad_pack_t pkb, const double* __restrict__ Sinv, double* __restr
     v[0] += r * z;
   }
   double tot[1];
-  if (Reduce<1>::run(pkb, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0) {
-    KState& s = ks[fb.inst];
-    s.it += 1;
-    s.rho_prev = s.rho;
-    s.rho = tot[0];
-    s.rr = tot[0];
-    if (!isfinite(tot[0])) {
-      s.status = TCAD_ERR_NONFINITE;
-      s.active = 0;
-    } else if (tot[0] <= s.tol2) {
-      s.active = 0;
-    } else if (s.it >= s.maxit) {
-      s.status = TCAD_ERR_NOCONV;
-      s.active = 0;
-    } else {
-      s.beta = s.rho / s.rho_prev;
-    }
-  }
+  if (Reduce<1>::run(pkb, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0)
+    fin_cg_x(ks[fb.inst], tot[0]);
 }
 
 // full update: d_r = Tr (= A_rr^-1 (F_r - A_rb d_b) from the red pass), d_b = x
@@ -1298,6 +1278,10 @@ k_eqrb_merge(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ T
     if (qb.real) d[qb.node] = xb[slot];
   }
 }
+
+}  // namespace tcad
+#include "eq_resident.cuh"
+namespace tcad {
 
 // equilibrium update: clip to +-max_dpsi, psi += d, err = max |d|
 __global__ void __launch_bounds__(NT)
@@ -1544,14 +1528,14 @@ struct WorkRb {
 // Slot-pack flat blocks hold pk->flat_nodes slots (measured, 200-iteration
 // solves on the two-lane 983k-node tri-gate: 419 us per iteration at 512
 // slots and 5 CTAs per SM, 450 at 256 slots, 511 at 256 slots and 4 CTAs,
-// 774 at 128).  A single instance that the resident solve takes (at most
-// kRbResidentCtas blocks of kRbResidentMaxSlots) is split over all SMs
-// instead: whole warps of slots, at most one block per SM.
+// 774 at 128).  A single instance that a resident solve takes (at most
+// kRbResidentCtas blocks of `most` slots) is split over all SMs instead:
+// whole warps of slots, at most one block per SM.
 constexpr int64_t kRbResidentCtas = 148;
-static int64_t rb_flat(const tcad_pack_t* pk, int64_t slots) {
+static int64_t rb_flat(const tcad_pack_t* pk, int64_t slots, int64_t most) {
   if (pk->n_inst != 1) return pk->flat_nodes;
   const int64_t fn = ((slots + kRbResidentCtas - 1) / kRbResidentCtas + 31) / 32 * 32;
-  return fn <= kRbResidentMaxSlots ? fn : pk->flat_nodes;
+  return fn <= most ? fn : pk->flat_nodes;
 }
 // slots / rb_flat + n_inst <= n_nodes / flat_nodes + n_inst, or the resident
 // solve's blocks
@@ -1595,6 +1579,7 @@ struct WorkEq {
   int64_t* flat_off;
   int32_t* flat_inst;
   int32_t* blk;
+  double *partial, *sync;   // as WorkRb's
   size_t bytes;
 };
 
@@ -1615,12 +1600,15 @@ static WorkEq carve_eq(const tcad_pack_t* pk, void* base) {
   w.flat_off = c.take<int64_t>((size_t)pk->n_inst + 1);
   w.flat_inst = c.take<int32_t>(rb_flat_cap(pk));
   w.blk = c.take<int32_t>(rb_flat_cap(pk));
+  w.partial = c.take<double>(8 * rb_flat_cap(pk));
+  w.sync = c.take<double>(sync_doubles());
   w.bytes = c.used;
   return w;
 }
 
 // The slot pack of a pack (host tables; see redblack.cuh): per instance
 // (ceil(Nx/2), Ny Nz, 1) slots of each colour, flat blocks of rb_flat slots
+// (`most`: the resident solve's bound)
 struct RbLayout {
   tcad_pack_t pkb;
   RbMap mp;
@@ -1629,7 +1617,7 @@ struct RbLayout {
 
 template <class W>   // WorkRb or WorkEq: the slot pack's table arrays
 static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream_t s,
-                     bool resident) {
+                     int64_t most) {
   const int ni = pk->n_inst;
   std::vector<int32_t> shp(3 * (size_t)ni), sb(3 * (size_t)ni), fi;
   TCAD_CUDA_CHECK(cudaMemcpyAsync(shp.data(), pk->shape, sizeof(int32_t) * shp.size(),
@@ -1637,21 +1625,19 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
   std::vector<int64_t> noff(ni + 1), foff(ni + 1);
   noff[0] = 0; foff[0] = 0;
-  int64_t fn = pk->flat_nodes;
-  if (resident && ni == 1)
-    fn = rb_flat(pk, (int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2]);
+  int64_t fn = pk->flat_nodes, nflat = 0;
+  if (ni == 1) fn = rb_flat(pk, (int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2], most);
   for (int i = 0; i < ni; ++i) {
     const int64_t hx = (shp[3 * i] + 1) / 2, rows = (int64_t)shp[3 * i + 1] * shp[3 * i + 2];
     sb[3 * i] = (int32_t)hx; sb[3 * i + 1] = (int32_t)rows; sb[3 * i + 2] = 1;
     noff[i + 1] = noff[i] + hx * rows;
     const int64_t nf = (hx * rows + fn - 1) / fn;
     foff[i + 1] = foff[i] + nf;
+    nflat += (hx * rows + pk->flat_nodes - 1) / pk->flat_nodes;
     for (int64_t b = 0; b < nf; ++b) fi.push_back(i);
   }
-  // (without the resident blocks the Krylov partials, 8 n_flat doubles, hold
-  // 4 per slot block, as n_flat >= max(n_inst, n_nodes / flat_nodes))
-  if (noff[ni] > pk->n_nodes || (size_t)foff[ni] > rb_flat_cap(pk) ||
-      (!resident && 4 * foff[ni] > 8 * pk->n_flat))
+  // (n_flat >= max(n_inst, n_nodes / flat_nodes) in a consistent pack)
+  if (noff[ni] > pk->n_nodes || (size_t)foff[ni] > rb_flat_cap(pk) || nflat > 2 * pk->n_flat)
     return TCAD_ERR_ARG;
   TCAD_CUDA_CHECK(cudaMemcpyAsync(wr.shape, sb.data(), sizeof(int32_t) * sb.size(),
                                   cudaMemcpyHostToDevice, s));
@@ -2364,6 +2350,53 @@ static int launch_cg(const tcad_pack_t* pk, const double* J, const double* b, do
   return TCAD_OK;
 }
 
+// k_eqrb_resident over the slot pack's blocks: TCAD_OK with hks[0] filled, or 1
+// when the launch was refused or a wait gave up
+template <int DIM, int K>
+static int launch_eq_resident_t(const RbLayout& L, const WorkEq& we, const double* J,
+                                const double* b, double* d, double rtol, int maxiter,
+                                const Work& w, const uint8_t* active,
+                                std::vector<KState>& hks, cudaStream_t s,
+                                const double* rtol_inst) {
+  const auto kern = k_eqrb_resident<DIM, K>;
+  const size_t smem = (size_t)L.pkb.flat_nodes * (1 + 2 * DIM) * 16;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  CoopLaunch c;
+  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, smem, w.bar, s)) return rc;
+  if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, J, b, d, w.cg.z, w.cg.p, we.xb, we.tR, w.ks,
+                         we.sync, w.bar, rtol, maxiter, active, rtol_inst) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  note_launch();
+  return coop_result(w, hks, s);
+}
+
+static int launch_eq_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& we,
+                              const double* J, const double* b, double* d, double rtol,
+                              int maxiter, const Work& w, const uint8_t* active,
+                              std::vector<KState>& hks, cudaStream_t s,
+                              const double* rtol_inst) {
+  const int fn = L.pkb.flat_nodes;
+  if (fn > kEqResidentMaxSlots) return 1;
+  auto go = [&](auto fnc) {
+    return fnc(L, we, J, b, d, rtol, maxiter, w, active, hks, s, rtol_inst);
+  };
+  if (pk->dim == 2)
+    return fn <= NT       ? go(launch_eq_resident_t<2, 1>)
+           : fn <= 2 * NT ? go(launch_eq_resident_t<2, 2>)
+           : fn <= 4 * NT ? go(launch_eq_resident_t<2, 4>)
+                          : go(launch_eq_resident_t<2, 8>);
+  return fn <= NT       ? go(launch_eq_resident_t<3, 1>)
+         : fn <= 2 * NT ? go(launch_eq_resident_t<3, 2>)
+         : fn <= 4 * NT ? go(launch_eq_resident_t<3, 4>)
+                        : go(launch_eq_resident_t<3, 8>);
+}
+
 // Equilibrium PCG on the red-black Schur complement (k_eqrb_*): the same
 // per-instance loop, masks and compaction as launch_cg, on the black slots;
 // d is the full update.  L: the slot pack (rb_layout over we's tables).
@@ -2377,6 +2410,10 @@ static int launch_cg_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& 
   const int ni = pk->n_inst;
   const bool d2 = pk->dim == 2;
   CgVec cg = w.cg;   // black slot vectors
+  if (g_fused_mode.load() && ni == 1 && (int64_t)nbb <= kRbResidentCtas &&
+      launch_eq_resident(pk, L, we, J, b, d, rtol, maxiter, w, active, hks, s, rtol_inst) ==
+          TCAD_OK)
+    return TCAD_OK;
   TCAD_CUDA_CHECK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned) * ni, s));
   TCAD_CUDA_CHECK(cudaMemsetAsync(we.xb, 0, sizeof(double) * (size_t)pkb.n_nodes, s));
   if (d2) {
@@ -2384,14 +2421,14 @@ static int launch_cg_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& 
     k_eqrb_diag<2><<<nbb, NT, 0, s>>>(pkb, L.mp, we.JRe, we.JBe, we.Sinv);
     k_eqrb_red<2><<<nbb, NT, 0, s>>>(pkb, L.mp, we.JRe, we.xb, we.bR, we.tR, nullptr, nullptr);
     k_eqrb_init<2><<<nbb, NT, 0, s>>>(pkb, L.mp, we.JBe, we.bB, we.tR, we.Sinv, we.xb, cg,
-                                      w.ks, w.partial, w.ticket, rtol, maxiter, active,
+                                      w.ks, we.partial, w.ticket, rtol, maxiter, active,
                                       rtol_inst);
   } else {
     k_eqrb_pack<3><<<nbb, NT, 0, s>>>(pkb, L.mp, J, b, we.JRe, we.JBe, we.bR, we.bB);
     k_eqrb_diag<3><<<nbb, NT, 0, s>>>(pkb, L.mp, we.JRe, we.JBe, we.Sinv);
     k_eqrb_red<3><<<nbb, NT, 0, s>>>(pkb, L.mp, we.JRe, we.xb, we.bR, we.tR, nullptr, nullptr);
     k_eqrb_init<3><<<nbb, NT, 0, s>>>(pkb, L.mp, we.JBe, we.bB, we.tR, we.Sinv, we.xb, cg,
-                                      w.ks, w.partial, w.ticket, rtol, maxiter, active,
+                                      w.ks, we.partial, w.ticket, rtol, maxiter, active,
                                       rtol_inst);
   }
   for (int l = 0; l < 4; ++l) note_launch();
@@ -2407,14 +2444,14 @@ static int launch_cg_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& 
     for (int q = 0; q < check; ++q) {
       if (d2) {
         k_eqrb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, we.JRe, cg.p, nullptr, we.tR, w.ks, dlist);
-        k_eqrb_q<2><<<ng, NT, 0, s>>>(pkb, L.mp, we.JBe, we.tR, cg, w.ks, w.partial, w.ticket,
+        k_eqrb_q<2><<<ng, NT, 0, s>>>(pkb, L.mp, we.JBe, we.tR, cg, w.ks, we.partial, w.ticket,
                                       dlist);
       } else {
         k_eqrb_red<3><<<ng, NT, 0, s>>>(pkb, L.mp, we.JRe, cg.p, nullptr, we.tR, w.ks, dlist);
-        k_eqrb_q<3><<<ng, NT, 0, s>>>(pkb, L.mp, we.JBe, we.tR, cg, w.ks, w.partial, w.ticket,
+        k_eqrb_q<3><<<ng, NT, 0, s>>>(pkb, L.mp, we.JBe, we.tR, cg, w.ks, we.partial, w.ticket,
                                       dlist);
       }
-      k_eqrb_x<<<ng, NT, 0, s>>>(pkb, we.Sinv, we.xb, cg, w.ks, w.partial, w.ticket, dlist);
+      k_eqrb_x<<<ng, NT, 0, s>>>(pkb, we.Sinv, we.xb, cg, w.ks, we.partial, w.ticket, dlist);
       k_cg_p<<<ng, NT, 0, s>>>(pkb, cg, w.ks, dlist);
       for (int l = 0; l < 4; ++l) note_launch();
     }
@@ -2598,7 +2635,7 @@ extern "C" int tcad_block_krylov(const tcad_pack_t* pk, const double* J, const d
     if (work_bytes < tcad_block_workspace_bytes(pk, 2, 0)) return TCAD_ERR_ARG;
     const WorkRb wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
     RbLayout rbl;
-    if ((rc = rb_layout(pk, wrb, rbl, s, true)) != TCAD_OK) return rc;
+    if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots)) != TCAD_OK) return rc;
     const unsigned nbb = (unsigned)rbl.pkb.n_flat;
     if (pk->dim == 2)
       k_rb_pack<2><<<nbb, NT, 0, s>>>(rbl.pkb, rbl.mp, J, wrb.JR, wrb.JB);
@@ -2694,7 +2731,7 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
   RbLayout rbl;
   if (use_rb) {
     wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
-    if (int rc = rb_layout(pk, wrb, rbl, s, true)) return rc;
+    if (int rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots)) return rc;
   }
   std::vector<int32_t> mix_it(ni), mix_st(ni), mix_grew(ni, 0), mix_steps(ni, 0);
   std::vector<double> mix_rr(ni), mix_prev(ni, -1.0);
@@ -3029,7 +3066,7 @@ extern "C" int tcad_equilibrium_solve(const tcad_pack_t* pk, double* psi, double
   RbLayout rbl;
   if (use_rb) {
     we = carve_eq(pk, reinterpret_cast<char*>(work) + off_eq(pk));
-    if (int rc = rb_layout(pk, we, rbl, s, false)) return rc;
+    if (int rc = rb_layout(pk, we, rbl, s, kEqResidentMaxSlots)) return rc;
   }
   for (int it = 0; it < opts->max_iter; ++it) {
     TCAD_CUDA_CHECK(cudaMemcpyAsync(dact, hact.data(), ni, cudaMemcpyHostToDevice, s));

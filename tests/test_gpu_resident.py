@@ -37,3 +37,45 @@ def test_resident_schur_solve_bit_identical_to_per_step(kind, shape):
         assert (ita, sta, rra) == (itb, stb, rrb)
         assert np.array_equal(xa.cpu().numpy(), xb.cpu().numpy())
         assert nb == 2 and na > 2           # colour repack + the single launch
+
+
+@pytest.mark.parametrize("kind,shape", SIZES + [("diode", (301, 511)), ("trigate", (96, 57, 40)),
+                                                ("trigate", (131, 80, 50))])
+def test_resident_equilibrium_bit_identical_to_per_step(kind, shape):
+    """One to eight slots per thread; the whole equilibrium Newton."""
+    res = []
+    for fused in (0, 1):
+        dev = _device(kind, shape)
+        lib = dev.pack.lib
+        prev = lib.tcad_set_krylov_fused(fused)
+        try:
+            n0 = lib.tcad_launch_count()
+            dev.solve_equilibrium()
+            eq = dev.last_equilibrium
+            assert eq["converged"]
+            res.append((dev.psi, dev.n, dev.p, eq["iters"], eq["krylov_iters"],
+                        lib.tcad_launch_count() - n0))
+        finally:
+            lib.tcad_set_krylov_fused(prev)
+    for a, b in zip(res[0][:5], res[1][:5]):
+        assert np.array_equal(a, b)
+    assert res[1][5] <= 3 * res[1][3] + 2 < res[0][5]   # assembly, solve, update per step
+
+
+def test_resident_equilibrium_give_up_falls_back():
+    dev = _device("diode", (21, 10))
+    lib = dev.pack.lib
+    dev.solve_equilibrium()
+    want, g0 = dev.psi, lib.tcad_krylov_fused_gave_up()
+    prev = lib.tcad_set_krylov_fused_test(1)
+    try:
+        import tcad_b200 as tb
+        import warnings
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore")     # one Newton step: not converged
+            dev.solve_equilibrium(tb.NewtonOptions(max_iter=1))
+        assert lib.tcad_krylov_fused_gave_up() == g0 + 1
+    finally:
+        lib.tcad_set_krylov_fused_test(prev)
+    dev.solve_equilibrium()
+    assert np.array_equal(dev.psi, want)
