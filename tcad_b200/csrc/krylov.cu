@@ -667,6 +667,7 @@ k_true_resid(const tcad_pack_t pk, const TJ* __restrict__ J, const T* __restrict
 
 }  // namespace tcad
 #include "redblack.cuh"
+#include "rb_stream.cuh"
 #include "grid_sync.cuh"
 #include "rb_resident.cuh"
 namespace tcad {
@@ -1613,6 +1614,7 @@ struct RbLayout {
   tcad_pack_t pkb;
   RbMap mp;
   std::vector<int64_t> hfoff;
+  bool tiles;   // every flat block starts on a warp tile
 };
 
 template <class W>   // WorkRb or WorkEq: the slot pack's table arrays
@@ -1626,11 +1628,16 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   std::vector<int64_t> noff(ni + 1), foff(ni + 1);
   noff[0] = 0; foff[0] = 0;
   int64_t fn = pk->flat_nodes, nflat = 0;
+  bool room = true;
   if (ni == 1) fn = rb_flat(pk, (int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2], most);
   for (int i = 0; i < ni; ++i) {
     const int64_t hx = (shp[3 * i] + 1) / 2, rows = (int64_t)shp[3 * i + 1] * shp[3 * i + 2];
     sb[3 * i] = (int32_t)hx; sb[3 * i + 1] = (int32_t)rows; sb[3 * i + 2] = 1;
     noff[i + 1] = noff[i] + hx * rows;
+    // whole warp tiles per instance (rb_stream.cuh), where the slot arrays
+    // (n_nodes) have the room
+    room = room && (noff[i + 1] + 31) / 32 * 32 <= pk->n_nodes;
+    if (room) noff[i + 1] = (noff[i + 1] + 31) / 32 * 32;
     const int64_t nf = (hx * rows + fn - 1) / fn;
     foff[i + 1] = foff[i] + nf;
     nflat += (hx * rows + pk->flat_nodes - 1) / pk->flat_nodes;
@@ -1660,6 +1667,8 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   L.mp.node_off = pk->node_off;
   L.mp.n_full = pk->n_nodes;
   L.hfoff = foff;
+  L.tiles = fn % 32 == 0;
+  for (int i = 0; i < ni; ++i) L.tiles = L.tiles && noff[i] % 32 == 0;
   return TCAD_OK;
 }
 
@@ -2096,6 +2105,49 @@ static int launch_bicgstab_rb_fused(const tcad_pack_t* pk, const RbLayout& L,
   return TCAD_OK;
 }
 
+static int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  return std::max(sms, 1);
+}
+
+template <int DIM>
+static bool rb_stream_smem_ok() {
+  bool ok = true;
+  auto set = [&](auto kern) {
+    ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)rb_stream_smem<DIM>()) == cudaSuccess;
+  };
+  set(k_rb_stream<DIM, kRbRed>);
+  set(k_rb_stream<DIM, kRbV>);
+  set(k_rb_stream<DIM, kRbT>);
+  set(k_rb_stream<DIM, kRbTrue>);
+  if (!ok) (void)cudaGetLastError();
+  return ok;
+}
+static bool rb_stream_ready(bool d2) {
+  return d2 ? rb_stream_smem_ok<2>() : rb_stream_smem_ok<3>();
+}
+
+// one streamed pass over ng blocks (dlist: their numbers, null: all); on: the
+// states that say which instances take part (null: all)
+template <int PASS>
+static void rb_stream(bool d2, int sms, const tcad_pack_t& pkb, const RbMap& mp,
+                      const WorkRb& wr, const double* X, double* out, const BiVec& bi,
+                      const Work& w, const KState* on, int rearm, unsigned ng,
+                      const int32_t* dlist, cudaStream_t s) {
+  const double* Jc = PASS == kRbRed ? wr.JR : wr.JB;
+  const unsigned grid = std::min(ng, (unsigned)sms);
+  if (d2)
+    k_rb_stream<2, PASS><<<grid, NT, rb_stream_smem<2>(), s>>>(
+        pkb, mp, Jc, X, out, bi, wr.rhs, wr.xb, on, w.ks, wr.partial, w.ticket, rearm, ng, dlist);
+  else
+    k_rb_stream<3, PASS><<<grid, NT, rb_stream_smem<3>(), s>>>(
+        pkb, mp, Jc, X, out, bi, wr.rhs, wr.xb, on, w.ks, wr.partial, w.ticket, rearm, ng, dlist);
+}
+
 // BiCGStab on the red-black Schur complement of A^ (redblack.cuh): the same
 // per-instance stopping test ||b - A^ x|| <= rtol ||b|| as launch_bicgstab_t,
 // the same vector kernels on the black slot pack, and the full solution x
@@ -2138,6 +2190,11 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
   note_launch();
   TCAD_LAUNCH_CHECK();
   hks.resize(ni);
+  // J streamed through shared memory where the pack is larger than one wave
+  // of blocks and every block starts on a warp tile
+  const int sms = sm_count();
+  const bool stream = L.tiles && pkb.flat_nodes == kRbStreamSlots && (int)nbb > sms &&
+                      rb_stream_ready(d2);
   int check = 4, done_iters = 0, rechecks = 0;
   ActiveGrid grid;
   if (int rc = grid.init(&pkb, s, &L.hfoff)) return rc;
@@ -2146,7 +2203,10 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
     const int32_t* dlist = grid.dlist;
     for (int q = 0; q < check; ++q) {
       k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist);
-      if (d2) {
+      if (stream) {
+        rb_stream<kRbRed>(d2, sms, pkb, L.mp, wr, bi.p, wr.tR, bi, w, w.ks, 0, ng, dlist, s);
+        rb_stream<kRbV>(d2, sms, pkb, L.mp, wr, wr.tR, nullptr, bi, w, w.ks, 0, ng, dlist, s);
+      } else if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.p, wr.tR, w.ks, dlist);
         k_rb_v<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
@@ -2156,7 +2216,10 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
                                     dlist);
       }
       k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist);
-      if (d2) {
+      if (stream) {
+        rb_stream<kRbRed>(d2, sms, pkb, L.mp, wr, bi.s, wr.tR, bi, w, w.ks, 0, ng, dlist, s);
+        rb_stream<kRbT>(d2, sms, pkb, L.mp, wr, wr.tR, nullptr, bi, w, w.ks, 0, ng, dlist, s);
+      } else if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.s, wr.tR, w.ks, dlist);
         k_rb_t<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
@@ -2174,13 +2237,20 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
                                     cudaMemcpyDeviceToHost, s));
     TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
     bool any = false;
-    for (int i = 0; i < ni; ++i) any = any || hks[i].active;
+    for (int i = 0; i < ni; ++i) {
+      if (hks[i].status == TCAD_ERR_CUDA) return TCAD_ERR_CUDA;
+      any = any || hks[i].active;
+    }
     if (any)
       if (int rc = grid.update(hks, wr.blk, s)) return rc;
     if (!any) {
       // true Schur residual (= the full residual); re-arm drifted instances
       const int rearm = rechecks < 8 ? 1 : 0;
-      if (d2) {
+      if (stream) {
+        rb_stream<kRbRed>(d2, sms, pkb, L.mp, wr, wr.xb, wr.tR, bi, w, nullptr, 0, nbb, nullptr, s);
+        rb_stream<kRbTrue>(d2, sms, pkb, L.mp, wr, wr.tR, bi.r, bi, w, nullptr, rearm, nbb,
+                           nullptr, s);
+      } else if (d2) {
         k_rb_red<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JR, wr.xb, wr.tR, nullptr, nullptr);
         k_rb_true<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, wr.rhs, wr.xb, bi.r, w.ks,
                                         wr.partial, w.ticket, rearm);

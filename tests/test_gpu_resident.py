@@ -79,3 +79,71 @@ def test_resident_equilibrium_give_up_falls_back():
         lib.tcad_set_krylov_fused_test(prev)
     dev.solve_equilibrium()
     assert np.array_equal(dev.psi, want)
+
+
+def _batch_system(devs):
+    """The block-scaled Newton systems of several devices in one pack, each
+    at its bulk-guess state."""
+    import torch
+    from tcad_b200 import _lib
+    from tcad_b200.pack import Pack
+    pk = Pack([d.setup for d in devs])
+    g = np.concatenate([d.setup.bulk_guess().ravel() for d in devs])
+    ns = np.concatenate([d.setup.nie_s.ravel() for d in devs])
+    for t, a in ((pk.psi, g), (pk.n, ns * np.exp(g)), (pk.p, ns * np.exp(-g))):
+        t.copy_(torch.from_numpy(a))
+    pk.set_bias()
+    pk.assemble(_lib.MODE_ELIMINATE)
+    st = torch.zeros(len(devs), dtype=torch.int32, device=pk.device)
+    _lib.check(pk.lib.tcad_block_jacobi_setup_rel(pk.pref, _lib.ptr(pk.J), _lib.ptr(pk.F),
+                                                  _lib.ptr(st), _lib.ptr(pk.n), _lib.ptr(pk.p),
+                                                  1e-10, pk.sp()), "bj")
+    assert not st.any()
+    return pk
+
+
+def _batch_solve(pk, rtol, maxit, fused):
+    import ctypes
+    import torch
+    from tcad_b200 import _lib
+    ni = len(pk.setups)
+    x = torch.full_like(pk.du, float("nan"))
+    it, st, rr = (ctypes.c_int32 * ni)(), (ctypes.c_int32 * ni)(), (ctypes.c_double * ni)()
+    prev = pk.lib.tcad_set_krylov_fused(fused)
+    try:
+        _lib.check(pk.lib.tcad_block_krylov(pk.pref, _lib.ptr(pk.J), _lib.ptr(pk.F),
+                                            _lib.ptr(x), 2, rtol, maxit, 0, _lib.ptr(pk.work),
+                                            pk.work.numel(), it, st, rr, pk.sp()), "krylov")
+    finally:
+        pk.lib.tcad_set_krylov_fused(prev)
+    torch.cuda.synchronize()
+    return x, list(it), list(st), list(rr)
+
+
+STREAMED = [[("trigate", (131, 80, 51))], [("mosfet", (801, 400))],
+            [("trigate", (57, 45, 39)), ("trigate", (9, 7, 5)), ("trigate", (56, 48, 46))],
+            [("diode", (401, 351)), ("diode", (21, 10)), ("diode", (300, 203))]]
+
+
+@pytest.mark.parametrize("devs", STREAMED, ids=lambda d: "+".join(str(q[1]) for q in d))
+def test_streamed_schur_solve_meets_the_full_systems_test(devs):
+    """Packs of more blocks than SMs (J streamed through shared memory): one
+    instance and ragged ones, odd rows, partial tiles and blocks."""
+    import torch
+    from tcad_b200 import _lib
+    pk = _batch_system([_device(*d) for d in devs])
+    rtol = 1e-9
+    x, it, st, rr = _batch_solve(pk, rtol, 20000, 1)
+    assert bool(x.isfinite().all())
+    y = torch.empty_like(x)
+    _lib.check(pk.lib.tcad_block_spmv(pk.pref, _lib.ptr(pk.J), _lib.ptr(x), _lib.ptr(y),
+                                      pk.sp()), "spmv")
+    r, b = (pk.F - y).view(3, -1), pk.F.view(3, -1)
+    for i, s in enumerate(pk.setups):
+        a = slice(int(pk.node_off[i]), int(pk.node_off[i]) + s.N)
+        rel = float(torch.linalg.norm(r[:, a]) / torch.linalg.norm(b[:, a]))
+        assert abs(rel - rr[i]) <= 1e-3 * rtol + 0.01 * rr[i], (rel, rr[i])
+        if st[i] == _lib.TCAD_OK:          # block Jacobi stalls on some MOSFETs
+            assert rel <= 1.01 * rtol
+    x, it, st, rr = _batch_solve(pk, 1e-30, 17, 1)
+    assert it == [17] * len(devs) and st == [_lib.TCAD_ERR_NOCONV] * len(devs)
