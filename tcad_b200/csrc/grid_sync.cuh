@@ -49,16 +49,48 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
+// The barrier alone, for CTAs of any size.  bar[0]: arrivals; [2]: a CTA gave
+// up; [3]: the give-up test hook, an arrival to wait for that never comes.
+struct GridBarrier {
+  unsigned* bar;
+  unsigned round;
+
+  // thread 0's part, between two CTA barriers
+  __device__ __forceinline__ int arrive_and_wait() {
+    const unsigned target = round * gridDim.x + ld_acquire(&bar[3]);
+    if (atom_add_acq_rel(&bar[0], 1u) + 1u == target) return 1;
+    unsigned long long t0 = 0;
+    for (unsigned it = 1; (int)(ld_acquire(&bar[0]) - target) < 0; ++it) {
+      if ((it & 255u) != 0u) continue;
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (ld_acquire(&bar[2]) != 0u) return 0;
+      if (now - t0 > kBarrierNs || it > (1u << 30)) {
+        atomicExch(&bar[2], 1u);
+        return 0;
+      }
+    }
+    return 1;
+  }
+
+  // ok: a shared word.  Orders all global writes before it, of any thread of
+  // the grid, before all reads after it.
+  __device__ __forceinline__ bool wait(int* ok) {
+    ++round;
+    __syncthreads();
+    if (threadIdx.x == 0) *ok = arrive_and_wait();
+    __syncthreads();
+    return *ok != 0;
+  }
+};
+
 struct GridSync {
   double* partial;   // sync_doubles()
-  unsigned* bar;     // [0]: arrivals; [2]: a CTA gave up; [3]: the give-up test
-                     // hook, an arrival to wait for that never comes
-  unsigned round;
+  GridBarrier gb;
 
   __device__ __forceinline__ void init(double* part, unsigned* b) {
     partial = part;
-    bar = b;
-    round = 0;
+    gb = GridBarrier{b, 0u};
   }
 
   // tot = the sums over the grid of every thread's v, valid in every thread;
@@ -85,8 +117,8 @@ struct GridSync {
         if (lane == 0) dst[q][warp] = r[q];
       }
     };
-    ++round;
-    double* const buf = partial + (round & 1u) * (size_t)(kSyncSums * kSyncMaxCtas);
+    ++gb.round;
+    double* const buf = partial + (gb.round & 1u) * (size_t)(kSyncSums * kSyncMaxCtas);
     double r[NS];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) r[q] = v[q];
@@ -95,23 +127,7 @@ struct GridSync {
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int q = 0; q < NQ; ++q) buf[q * kSyncMaxCtas + blockIdx.x] = tree(sa[q]);
-      int good = 1;
-      const unsigned target = round * G + ld_acquire(&bar[3]);
-      if (atom_add_acq_rel(&bar[0], 1u) + 1u != target) {
-        unsigned long long t0 = 0;
-        for (unsigned it = 1; (int)(ld_acquire(&bar[0]) - target) < 0; ++it) {
-          if ((it & 255u) != 0u) continue;
-          const unsigned long long now = globaltimer_ns();
-          if (t0 == 0) t0 = now;
-          if (ld_acquire(&bar[2]) != 0u) { good = 0; break; }
-          if (now - t0 > kBarrierNs || it > (1u << 30)) {
-            atomicExch(&bar[2], 1u);
-            good = 0;
-            break;
-          }
-        }
-      }
-      ok = good;
+      ok = gb.arrive_and_wait();
     }
     __syncthreads();
     if (!ok) return false;

@@ -667,9 +667,9 @@ k_true_resid(const tcad_pack_t pk, const TJ* __restrict__ J, const T* __restrict
 
 }  // namespace tcad
 #include "redblack.cuh"
-#include "rb_stream.cuh"
 #include "grid_sync.cuh"
 #include "rb_resident.cuh"
+#include "rb_stream.cuh"
 namespace tcad {
 
 // ---- the whole solve in one cooperative launch (single-instance packs whose
@@ -795,115 +795,6 @@ k_bicgstab_fused(const tcad_pack_t pk, const double* __restrict__ J,
     }
     if (!S.active) break;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) ks[inst] = S;
-}
-
-// ---- the red-black Schur solve in one cooperative launch (single-instance
-// packs whose slot blocks all fit on the GPU at once: one CTA per slot
-// block).  The search direction and s are formed on the fly by the red
-// passes (RbFormP / RbFormS) and stored by the black passes, so an iteration
-// takes five grid barriers: red(p); p + v (alpha); red(s); s + t (early,
-// omega); x (rho, beta, convergence).  Bodies, scalar updates and reduction
-// order are the per-step kernels' own, so the result is bit-identical to
-// launch_bicgstab_rb's one launch per step.  Every wait is bounded as in
-// k_bicgstab_fused; a CTA that gives up returns and the host solves again
-// one launch per step.
-template <int DIM>
-__global__ void __launch_bounds__(NT, 2)
-k_bicgstab_rb_fused(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR,
-                    const double* __restrict__ JB, const double* __restrict__ b,
-                    double* __restrict__ x, double* __restrict__ bR, double* __restrict__ bB,
-                    double* __restrict__ Tr, double* __restrict__ xb,
-                    double* __restrict__ rhs, BiVec w, KState* ks, double* partial,
-                    unsigned* bar, double rtol, int maxit,
-                    const int32_t* __restrict__ pre_status,
-                    const double* __restrict__ rtol_inst, int max_rechecks) {
-  __shared__ KState S;
-  const unsigned G = gridDim.x;
-  const FlatBlock fb = flat_block(pkb, blockIdx.x);
-  const int inst = fb.inst;
-  const int64_t NS = pkb.n_nodes;
-  double* const half[2] = {partial, partial + 4 * (int64_t)pkb.n_flat};
-  int ph = 0;
-  unsigned round = 0;
-  double tot[3];
-  double bb = 0.0;
-  {
-    double v[1] = {rb_split_body<DIM>(pkb, mp, fb, b, bR, bB)};
-    Reduce<1>::store(blockIdx.x, v, half[ph]);
-    if (!grid_barrier(bar, G, round)) return;
-    Reduce<1>::total(pkb, inst, half[ph], tot);
-    ph ^= 1;
-    bb = tot[0];
-  }
-  {
-    double v[1] = {rb_init_body<DIM>(pkb, mp, fb, JB, bR, bB, rhs, xb, w)};
-    Reduce<1>::store(blockIdx.x, v, half[ph]);
-    if (!grid_barrier(bar, G, round)) return;
-    Reduce<1>::total(pkb, inst, half[ph], tot);
-    ph ^= 1;
-    if (threadIdx.x == 0)
-      rb_fin_init(S, tot[0], bb, rtol_inst ? rtol_inst[inst] : rtol, maxit,
-                  pre_status ? pre_status[inst] : TCAD_OK);
-    __syncthreads();
-  }
-  for (int rechecks = 0;; ++rechecks) {
-    while (S.active) {
-      rb_red_body<DIM>(pkb, mp, fb, JR,
-                       RbMakeP{w.r, w.p, w.v, NS, S.beta, S.omega, S.restart}, Tr);
-      if (!grid_barrier(bar, G, round)) return;
-      {
-        double v[1] = {rb_v_body<DIM, true>(pkb, mp, fb, JB, Tr, w, S.beta, S.omega,
-                                            S.restart)};
-        Reduce<1>::store(blockIdx.x, v, half[ph]);
-        if (!grid_barrier(bar, G, round)) return;
-        Reduce<1>::total(pkb, inst, half[ph], tot);
-        ph ^= 1;
-        if (threadIdx.x == 0) fin_v(S, tot[0]);
-        __syncthreads();
-      }
-      if (!S.active) break;
-      rb_red_body<DIM>(pkb, mp, fb, JR, RbMakeS{w.r, w.v, NS, S.alpha}, Tr);
-      if (!grid_barrier(bar, G, round)) return;
-      {
-        double v[3];
-        rb_t_body<DIM, true>(pkb, mp, fb, JB, Tr, w, S.alpha, v);
-        Reduce<3>::store(blockIdx.x, v, half[ph]);
-        if (!grid_barrier(bar, G, round)) return;
-        Reduce<3>::total(pkb, inst, half[ph], tot);
-        ph ^= 1;
-        if (threadIdx.x == 0) {
-          fin_s(S, tot[0]);
-          fin_t(S, tot[1], tot[2]);
-        }
-        __syncthreads();
-      }
-      {
-        double v[3];
-        bi_x_body<double>(pkb, fb, xb, w, S.alpha, S.omega, v);
-        Reduce<3>::store(blockIdx.x, v, half[ph]);
-        if (!grid_barrier(bar, G, round)) return;
-        Reduce<3>::total(pkb, inst, half[ph], tot);
-        ph ^= 1;
-        if (threadIdx.x == 0) fin_x(S, tot[0], tot[1], tot[2]);
-        __syncthreads();
-      }
-    }
-    rb_red_body<DIM>(pkb, mp, fb, JR, RbMakeVal{xb, NS}, Tr);
-    if (!grid_barrier(bar, G, round)) return;
-    {
-      double v[1] = {rb_true_body<DIM>(pkb, mp, fb, JB, Tr, rhs, xb, w.r)};
-      Reduce<1>::store(blockIdx.x, v, half[ph]);
-      if (!grid_barrier(bar, G, round)) return;
-      Reduce<1>::total(pkb, inst, half[ph], tot);
-      ph ^= 1;
-      if (threadIdx.x == 0) fin_true(S, tot[0], rechecks < max_rechecks ? 1 : 0);
-      __syncthreads();
-    }
-    if (!S.active) break;
-  }
-  rb_merge_body<DIM>(pkb, mp, fb, bR, Tr, xb, x,
-                     pre_status && pre_status[inst] != TCAD_OK);
   if (blockIdx.x == 0 && threadIdx.x == 0) ks[inst] = S;
 }
 
@@ -1526,24 +1417,27 @@ struct WorkRb {
   size_t bytes;
 };
 
-// Slot-pack flat blocks hold pk->flat_nodes slots (measured, 200-iteration
+// Slot-pack flat blocks hold kRbStreamSlots = 512 slots (measured, 200-iteration
 // solves on the two-lane 983k-node tri-gate: 419 us per iteration at 512
 // slots and 5 CTAs per SM, 450 at 256 slots, 511 at 256 slots and 4 CTAs,
 // 774 at 128).  A single instance that a resident solve takes (at most
 // kRbResidentCtas blocks of `most` slots) is split over all SMs instead:
 // whole warps of slots, at most one block per SM.
 constexpr int64_t kRbResidentCtas = 148;
-static int64_t rb_flat(const tcad_pack_t* pk, int64_t slots, int64_t most) {
-  if (pk->n_inst != 1) return pk->flat_nodes;
-  const int64_t fn = ((slots + kRbResidentCtas - 1) / kRbResidentCtas + 31) / 32 * 32;
-  return fn <= most ? fn : pk->flat_nodes;
+static int64_t rb_flat(int64_t slots, int64_t most) {
+  const int64_t sms = kRbResidentCtas;
+  const auto even = [&](int64_t blocks) { return ((slots + blocks - 1) / blocks + 31) / 32 * 32; };
+  if (even(sms) <= most) return even(sms);
+  // a larger single instance: as many blocks for every SM, of at most
+  // kRbStreamSlots slots
+  return even(sms * ((slots + sms * kRbStreamSlots - 1) / (sms * kRbStreamSlots)));
 }
-// slots / rb_flat + n_inst <= n_nodes / flat_nodes + n_inst, or the resident
-// solve's blocks
+// n_nodes bounds the slots
 static size_t rb_flat_cap(const tcad_pack_t* pk) {
-  return (size_t)(pk->n_nodes / pk->flat_nodes) + (size_t)pk->n_inst + 1 +
+  return (size_t)(pk->n_nodes / kRbStreamSlots) + (size_t)pk->n_inst + 1 +
          (size_t)(pk->n_inst == 1 ? kRbResidentCtas : 0);
 }
+// (single instance: at most 148 ceil(slots / (148 x 512)) < slots / 512 + 148 blocks)
 
 static WorkRb carve_rb(const tcad_pack_t* pk, void* base) {
   Carve c{reinterpret_cast<char*>(base), 0, 0};
@@ -1627,9 +1521,9 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
   std::vector<int64_t> noff(ni + 1), foff(ni + 1);
   noff[0] = 0; foff[0] = 0;
-  int64_t fn = pk->flat_nodes, nflat = 0;
+  int64_t fn = kRbStreamSlots, nflat = 0;
   bool room = true;
-  if (ni == 1) fn = rb_flat(pk, (int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2], most);
+  if (ni == 1) fn = rb_flat((int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2], most);
   for (int i = 0; i < ni; ++i) {
     const int64_t hx = (shp[3 * i] + 1) / 2, rows = (int64_t)shp[3 * i + 1] * shp[3 * i + 2];
     sb[3 * i] = (int32_t)hx; sb[3 * i + 1] = (int32_t)rows; sb[3 * i + 2] = 1;
@@ -1947,28 +1841,14 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
   return TCAD_OK;
 }
 
-template <int DIM>
-static bool rb_fused_fits(unsigned nb) {
-  int dev = 0, coop = 0, sms = 0, per = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
-    return false;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return false;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bicgstab_rb_fused<DIM>, NT, 0) !=
-      cudaSuccess)
-    return false;
-  return nb >= 1 && (long long)nb <= (long long)per * sms;
-}
-
 // Launch configuration of a cooperative single-launch solve, its barrier
 // flags cleared (and the give-up test hook set)
 struct CoopLaunch {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
 };
-static int coop_launch(CoopLaunch& c, unsigned blocks, size_t smem, unsigned* flags,
-                       cudaStream_t s) {
+static int coop_launch(CoopLaunch& c, unsigned blocks, unsigned threads, size_t smem,
+                       unsigned* flags, cudaStream_t s) {
   TCAD_CUDA_CHECK(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned), s));
   if (g_fused_test_hold.load()) {
     static const unsigned kPhantom = 1u;
@@ -1976,7 +1856,7 @@ static int coop_launch(CoopLaunch& c, unsigned blocks, size_t smem, unsigned* fl
                                     cudaMemcpyHostToDevice, s));
   }
   c.cfg.gridDim = dim3(blocks);
-  c.cfg.blockDim = dim3(NT);
+  c.cfg.blockDim = dim3(threads);
   c.cfg.dynamicSmemBytes = smem;
   c.cfg.stream = s;
   c.at[0].id = cudaLaunchAttributeCooperative;
@@ -1988,10 +1868,11 @@ static int coop_launch(CoopLaunch& c, unsigned blocks, size_t smem, unsigned* fl
 
 // Waits for a single-launch solve and reads its result: 1 when a grid
 // barrier gave up (the caller then solves with one launch per step)
-static int coop_result(const Work& w, std::vector<KState>& hks, cudaStream_t s) {
-  hks.resize(1);
+static int coop_result(const Work& w, int ni, std::vector<KState>& hks, cudaStream_t s) {
+  hks.resize(ni);
   unsigned hbar[4] = {0u, 0u, 0u, 0u};
-  TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState), cudaMemcpyDeviceToHost, s));
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState) * ni, cudaMemcpyDeviceToHost,
+                                  s));
   TCAD_CUDA_CHECK(cudaMemcpyAsync(hbar, w.bar, sizeof(hbar), cudaMemcpyDeviceToHost, s));
   TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
   if (hbar[2] != 0u) {
@@ -2017,7 +1898,7 @@ static int launch_rb_resident_t(const tcad_pack_t* pk, const RbLayout& L, const 
     return 1;
   }
   CoopLaunch c;
-  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, smem, w.bar, s)) return rc;
+  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, s)) return rc;
   const BiVec& bi = w.bi;
   const int rechecks = 8;
   // (a cooperative launch that does not fit is refused, not run)
@@ -2028,7 +1909,7 @@ static int launch_rb_resident_t(const tcad_pack_t* pk, const RbLayout& L, const 
     return 1;
   }
   note_launch();
-  return coop_result(w, hks, s);
+  return coop_result(w, 1, hks, s);
 }
 
 static int launch_bicgstab_rb_resident(const tcad_pack_t* pk, const RbLayout& L,
@@ -2052,59 +1933,6 @@ static int launch_bicgstab_rb_resident(const tcad_pack_t* pk, const RbLayout& L,
                   : go(launch_rb_resident_t<3, 2, false>);
 }
 
-// The whole red-black solve of a single-instance pack in one launch (same
-// arithmetic as launch_bicgstab_rb's per-step loop).  Returns TCAD_OK with
-// hks[0] filled, or 1 when the launch was refused or a grid barrier gave up
-// (the caller then solves one launch per step).
-static int launch_bicgstab_rb_fused(const tcad_pack_t* pk, const RbLayout& L,
-                                    const WorkRb& wr, const double* b, double* x,
-                                    double rtol, int maxiter, const BiVec& bi, const Work& w,
-                                    const int32_t* pre_status, std::vector<KState>& hks,
-                                    cudaStream_t s, const double* rtol_inst) {
-  TCAD_CUDA_CHECK(cudaMemsetAsync(w.bar, 0, 4 * sizeof(unsigned), s));
-  if (g_fused_test_hold.load()) {
-    static const unsigned kPhantom = 1u;
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(w.bar + 3, &kPhantom, sizeof(unsigned),
-                                    cudaMemcpyHostToDevice, s));
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)L.pkb.n_flat);
-  cfg.blockDim = dim3(NT);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  const int rechecks = 8;
-  cudaError_t e =
-      pk->dim == 2
-          ? cudaLaunchKernelEx(&cfg, k_bicgstab_rb_fused<2>, L.pkb, L.mp, (const double*)wr.JR,
-                               (const double*)wr.JB, b, x, wr.bR, wr.bB, wr.tR, wr.xb, wr.rhs,
-                               bi, w.ks, wr.partial, w.bar, rtol, maxiter, pre_status,
-                               rtol_inst, rechecks)
-          : cudaLaunchKernelEx(&cfg, k_bicgstab_rb_fused<3>, L.pkb, L.mp, (const double*)wr.JR,
-                               (const double*)wr.JB, b, x, wr.bR, wr.bB, wr.tR, wr.xb, wr.rhs,
-                               bi, w.ks, wr.partial, w.bar, rtol, maxiter, pre_status,
-                               rtol_inst, rechecks);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return 1;
-  }
-  note_launch();
-  hks.resize(1);
-  unsigned hbar[4] = {0u, 0u, 0u, 0u};
-  TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState), cudaMemcpyDeviceToHost, s));
-  TCAD_CUDA_CHECK(cudaMemcpyAsync(hbar, w.bar, sizeof(hbar), cudaMemcpyDeviceToHost, s));
-  TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
-  if (hbar[2] != 0u) {
-    g_fused_gave_up.fetch_add(1);
-    return 1;
-  }
-  return TCAD_OK;
-}
-
 static int sm_count() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -2120,9 +1948,13 @@ static bool rb_stream_smem_ok() {
     ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)rb_stream_smem<DIM>()) == cudaSuccess;
   };
+  set(k_rb_stream<DIM, kRbRedP>);
+  set(k_rb_stream<DIM, kRbRedS>);
   set(k_rb_stream<DIM, kRbRed>);
   set(k_rb_stream<DIM, kRbV>);
   set(k_rb_stream<DIM, kRbT>);
+  set(k_rb_stream<DIM, kRbVs>);
+  set(k_rb_stream<DIM, kRbTs>);
   set(k_rb_stream<DIM, kRbTrue>);
   if (!ok) (void)cudaGetLastError();
   return ok;
@@ -2131,22 +1963,66 @@ static bool rb_stream_ready(bool d2) {
   return d2 ? rb_stream_smem_ok<2>() : rb_stream_smem_ok<3>();
 }
 
-// one streamed pass over ng blocks (dlist: their numbers, null: all); on: the
-// states that say which instances take part (null: all)
-template <int PASS>
-static void rb_stream(bool d2, int sms, const tcad_pack_t& pkb, const RbMap& mp,
-                      const WorkRb& wr, const double* X, double* out, const BiVec& bi,
-                      const Work& w, const KState* on, int rearm, unsigned ng,
-                      const int32_t* dlist, cudaStream_t s) {
-  const double* Jc = PASS == kRbRed ? wr.JR : wr.JB;
-  const unsigned grid = std::min(ng, (unsigned)sms);
-  if (d2)
-    k_rb_stream<2, PASS><<<grid, NT, rb_stream_smem<2>(), s>>>(
-        pkb, mp, Jc, X, out, bi, wr.rhs, wr.xb, on, w.ks, wr.partial, w.ticket, rearm, ng, dlist);
-  else
-    k_rb_stream<3, PASS><<<grid, NT, rb_stream_smem<3>(), s>>>(
-        pkb, mp, Jc, X, out, bi, wr.rhs, wr.xb, on, w.ks, wr.partial, w.ticket, rearm, ng, dlist);
-}
+// The streamed steps of one solve (rb_stream.cuh) over ng blocks (dlist: their
+// numbers, null: all)
+template <int DIM>
+struct RbStreamLauncher {
+  const tcad_pack_t& pkb;
+  const RbMap& mp;
+  const WorkRb& wr;
+  const BiVec& bi;
+  const Work& w;
+  int sms;
+  cudaStream_t s;
+
+  template <class... P, class... A>
+  int launch(void (*kern)(P...), unsigned ng, size_t smem, A... args) const {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::min(ng, (unsigned)sms));
+    cfg.blockDim = dim3(NTS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    TCAD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+    note_launch();
+    return TCAD_OK;
+  }
+  template <int PASS>
+  int pass(const double* X, bool all, int rearm, unsigned ng, const int32_t* dlist) const {
+    return launch(k_rb_stream<DIM, PASS>, ng, rb_stream_smem<DIM>(), pkb, mp, wr.JR, wr.JB, X,
+                  wr.tR, bi, wr.rhs, w.ks, all, wr.partial, w.ticket, rearm, ng, dlist);
+  }
+  int iteration(bool formed, unsigned ng, const int32_t* dlist) const {
+    int rc = TCAD_OK;
+    auto then = [&](int r) { if (rc == TCAD_OK) rc = r; };
+    if (formed) {
+      then(pass<kRbRedP>(nullptr, false, 0, ng, dlist));
+      then(pass<kRbV>(nullptr, false, 0, ng, dlist));
+      then(pass<kRbRedS>(nullptr, false, 0, ng, dlist));
+      then(pass<kRbT>(nullptr, false, 0, ng, dlist));
+      then(launch(k_rb_stream_x<DIM>, ng, 0, pkb, mp, wr.xb, bi, w.ks, wr.partial, w.ticket, ng,
+                  dlist));
+      return rc;
+    }
+    k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist);
+    then(pass<kRbRed>(bi.p, false, 0, ng, dlist));
+    then(pass<kRbVs>(nullptr, false, 0, ng, dlist));
+    k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist);
+    then(pass<kRbRed>(bi.s, false, 0, ng, dlist));
+    then(pass<kRbTs>(nullptr, false, 0, ng, dlist));
+    k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, wr.partial, w.ticket, dlist);
+    note_launch(3);
+    return rc;
+  }
+  int true_residual(int rearm, unsigned nb) const {
+    const int rc = pass<kRbRed>(wr.xb, true, 0, nb, nullptr);
+    return rc == TCAD_OK ? pass<kRbTrue>(wr.xb, true, rearm, nb, nullptr) : rc;
+  }
+};
 
 // BiCGStab on the red-black Schur complement of A^ (redblack.cuh): the same
 // per-instance stopping test ||b - A^ x|| <= rtol ||b|| as launch_bicgstab_t,
@@ -2165,20 +2041,24 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
   BiVec bi = w.bi;   // black vectors (stride: the slot count)
   bi.ph = bi.p;
   bi.sh = bi.s;
-  if (g_fused_mode.load() && ni == 1) {
-    const int rc = (int64_t)nbb <= kRbResidentCtas
-                       ? launch_bicgstab_rb_resident(pk, L, wr, b, x, rtol, maxiter, w,
-                                                     pre_status, hks, s, rtol_inst)
-                   : (d2 ? rb_fused_fits<2>(nbb) : rb_fused_fits<3>(nbb))
-                       ? launch_bicgstab_rb_fused(pk, L, wr, b, x, rtol, maxiter, bi, w,
-                                                  pre_status, hks, s, rtol_inst)
-                       : 1;
-    if (rc == TCAD_OK) return TCAD_OK;
-  }
+  if (g_fused_mode.load() && ni == 1 && (int64_t)nbb <= kRbResidentCtas &&
+      launch_bicgstab_rb_resident(pk, L, wr, b, x, rtol, maxiter, w, pre_status, hks, s,
+                                  rtol_inst) == TCAD_OK)
+    return TCAD_OK;
+  // J streamed through shared memory where the pack is larger than one wave
+  // of blocks and every block starts on a warp tile
+  const int sms = sm_count();
+  const bool stream = L.tiles && pkb.flat_nodes <= kRbStreamSlots && (int)nbb > sms &&
+                      rb_stream_ready(d2);
+  const bool formed = pkb.n_nodes <= kRbFormSlots;
+  const RbStreamLauncher<2> st2{pkb, L.mp, wr, bi, w, sms, s};
+  const RbStreamLauncher<3> st3{pkb, L.mp, wr, bi, w, sms, s};
+  // colours of b, right-hand side and state of every instance
   TCAD_CUDA_CHECK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned) * ni, s));
-  if (d2) k_rb_split<2><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, wr.partial, w.ticket);
-  else    k_rb_split<3><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, wr.partial, w.ticket);
-  note_launch();
+  if (d2)
+    k_rb_split<2><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, wr.partial, w.ticket);
+  else
+    k_rb_split<3><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, wr.partial, w.ticket);
   if (d2)
     k_rb_init<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.bR, wr.bB, wr.rhs, wr.xb, bi, wr.bbf,
                                     w.ks, wr.partial, w.ticket, rtol, maxiter, pre_status,
@@ -2187,14 +2067,9 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
     k_rb_init<3><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.bR, wr.bB, wr.rhs, wr.xb, bi, wr.bbf,
                                     w.ks, wr.partial, w.ticket, rtol, maxiter, pre_status,
                                     rtol_inst);
-  note_launch();
+  note_launch(2);
   TCAD_LAUNCH_CHECK();
   hks.resize(ni);
-  // J streamed through shared memory where the pack is larger than one wave
-  // of blocks and every block starts on a warp tile
-  const int sms = sm_count();
-  const bool stream = L.tiles && pkb.flat_nodes == kRbStreamSlots && (int)nbb > sms &&
-                      rb_stream_ready(d2);
   int check = 4, done_iters = 0, rechecks = 0;
   ActiveGrid grid;
   if (int rc = grid.init(&pkb, s, &L.hfoff)) return rc;
@@ -2202,11 +2077,13 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
     const unsigned ng = grid.ng;
     const int32_t* dlist = grid.dlist;
     for (int q = 0; q < check; ++q) {
-      k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist);
       if (stream) {
-        rb_stream<kRbRed>(d2, sms, pkb, L.mp, wr, bi.p, wr.tR, bi, w, w.ks, 0, ng, dlist, s);
-        rb_stream<kRbV>(d2, sms, pkb, L.mp, wr, wr.tR, nullptr, bi, w, w.ks, 0, ng, dlist, s);
-      } else if (d2) {
+        if (int rc = d2 ? st2.iteration(formed, ng, dlist) : st3.iteration(formed, ng, dlist))
+          return rc;
+        continue;
+      }
+      k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist);
+      if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.p, wr.tR, w.ks, dlist);
         k_rb_v<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
@@ -2216,10 +2093,7 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
                                     dlist);
       }
       k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist);
-      if (stream) {
-        rb_stream<kRbRed>(d2, sms, pkb, L.mp, wr, bi.s, wr.tR, bi, w, w.ks, 0, ng, dlist, s);
-        rb_stream<kRbT>(d2, sms, pkb, L.mp, wr, wr.tR, nullptr, bi, w, w.ks, 0, ng, dlist, s);
-      } else if (d2) {
+      if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.s, wr.tR, w.ks, dlist);
         k_rb_t<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
@@ -2229,7 +2103,7 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
                                     dlist);
       }
       k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, wr.partial, w.ticket, dlist);
-      for (int l = 0; l < 7; ++l) note_launch();
+      note_launch(7);
     }
     TCAD_LAUNCH_CHECK();
     done_iters += check;
@@ -2247,20 +2121,18 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
       // true Schur residual (= the full residual); re-arm drifted instances
       const int rearm = rechecks < 8 ? 1 : 0;
       if (stream) {
-        rb_stream<kRbRed>(d2, sms, pkb, L.mp, wr, wr.xb, wr.tR, bi, w, nullptr, 0, nbb, nullptr, s);
-        rb_stream<kRbTrue>(d2, sms, pkb, L.mp, wr, wr.tR, bi.r, bi, w, nullptr, rearm, nbb,
-                           nullptr, s);
+        if (int rc = d2 ? st2.true_residual(rearm, nbb) : st3.true_residual(rearm, nbb)) return rc;
       } else if (d2) {
         k_rb_red<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JR, wr.xb, wr.tR, nullptr, nullptr);
         k_rb_true<2><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, wr.rhs, wr.xb, bi.r, w.ks,
                                         wr.partial, w.ticket, rearm);
+        note_launch(2);
       } else {
         k_rb_red<3><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JR, wr.xb, wr.tR, nullptr, nullptr);
         k_rb_true<3><<<nbb, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, wr.rhs, wr.xb, bi.r, w.ks,
                                         wr.partial, w.ticket, rearm);
+        note_launch(2);
       }
-      note_launch();
-      note_launch();
       TCAD_LAUNCH_CHECK();
       TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState) * ni,
                                       cudaMemcpyDeviceToHost, s));
@@ -2436,14 +2308,14 @@ static int launch_eq_resident_t(const RbLayout& L, const WorkEq& we, const doubl
     return 1;
   }
   CoopLaunch c;
-  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, smem, w.bar, s)) return rc;
+  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, s)) return rc;
   if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, J, b, d, w.cg.z, w.cg.p, we.xb, we.tR, w.ks,
                          we.sync, w.bar, rtol, maxiter, active, rtol_inst) != cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
   note_launch();
-  return coop_result(w, hks, s);
+  return coop_result(w, 1, hks, s);
 }
 
 static int launch_eq_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& we,
@@ -2791,9 +2663,8 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
     wilu_use.Mf = nullptr;  // node-order sweeps
     wilu_use.Mb = nullptr;
   }
-  // red-black Schur solves: the slot pack's tables, once per call (a
-  // single-instance pack small enough is solved in one cooperative launch,
-  // k_bicgstab_rb_fused, by launch_bicgstab_rb itself)
+  // red-black Schur solves: the slot pack's tables, once per call (which
+  // single-launch solve takes a pack is launch_bicgstab_rb's own choice)
   // (a workspace sized without the red-black extension -- method 0 -- solves
   // the whole system)
   const bool use_rb = opts->red_black != 0 && work_bytes >= tcad_block_workspace_bytes(pk, 2, 0);

@@ -11,7 +11,7 @@
 // 40 x 24 x 16 tri-gate 38 -> 14 us).
 // Five steps an iteration, each ended by GridSync: red(p), p + v (alpha),
 // red(s), s + t (early, omega), x (rho, beta, convergence); p and s are
-// formed on the fly at the neighbours (RbFormP / RbFormS).  Bodies, scalar
+// formed on the fly at the neighbours (RbFormPCg / RbFormSCg).  Bodies, scalar
 // updates and the order of the sums are those of the per-step kernels, so the
 // result is bit-identical to launch_bicgstab_rb's loop.
 #pragma once

@@ -1,33 +1,50 @@
-// The red and black passes of the red-black BiCGStab as persistent kernels
-// that stream the colour rows of J through shared memory.
+// The red-black BiCGStab of a pack larger than one wave of blocks: J streamed
+// through shared memory.
 //
-// These passes are one read of a colour's J (312 bytes a slot in 3D, 232 in
-// 2D) against 70 to 120 bytes of vectors that mostly stay in L2, so they should
-// run at the copy rate.  With J loaded where it is used (k_rb_red, k_rb_v,
-// k_rb_t) a thread's 39 row entries compete with its gathers for registers:
-// at 48 registers and 5 CTAs per SM the 983k-node tri-gate's passes read J at
-// 2.6 to 3.6 TB/s.  Here one CTA per SM walks the flat blocks, each warp owns
-// two of a block's sixteen warp tiles, and lane 0 copies the warp's tiles of the
-// NEXT block (contiguous runs of 10 KB) with cp.async.bulk as soon as the
-// present ones are consumed: 80 to 160 KB in flight per SM without a register,
-// while the gathers have 255 registers a thread to be in flight together.
-// J is read with an evict-first policy, so that it does not push the vectors
-// out of L2.  983k-node tri-gate, one instance: red 42.7 -> 28.5 us (153 MB of J:
-// 3.6 -> 5.4 TB/s), v 58.0 -> 36.1, t 53.4 -> 33.3; an iteration 240 -> 166 us.
+// A pass (red: t = E x, black: x - F t) is one read of a colour's J (312 bytes a
+// slot in 3D, 232 in 2D) against 70 to 120 bytes of vectors that mostly stay in
+// L2, so it should run at the copy rate.  With J loaded where it is used
+// (k_rb_red, k_rb_v, k_rb_t) a thread's 39 row entries compete with its gathers
+// for registers: at 48 registers and 5 CTAs per SM the 983k-node tri-gate's
+// passes read J at 2.6 to 3.6 TB/s.  Here one CTA of 16 warps per SM walks the
+// flat blocks, each warp owns one warp tile of a block (a contiguous run of
+// 10 KB), and lane 0 copies the warp's tile of the NEXT block with
+// cp.async.bulk as soon as the present one is consumed: up to 160 KB in flight
+// per SM without a register, next to the gathers.  J is read with an
+// evict-first policy, so that it does not push the vectors out of L2.  (8 warps
+// of two buffers each wait for their gathers, 6.6 of 11 stall cycles per issue,
+// and take 28.5 / 36 / 33 us a pass.)
 //
-// Expressions, the slots of a thread and the order of every sum are those of
-// the per-step kernels: bit-identical to them.  A CTA adds its count of blocks
-// to the instance's ticket once (not once per block).
+// Successive launches overlap (programmatic dependent launch): J does not depend
+// on the vectors, so a CTA of the next kernel starts as soon as its SM is free,
+// copies its first tiles, and only then waits for the present kernel to end.
+//
+// Two sequences run an iteration:
+//   formed (vectors that fit in L2 together): red(p), v, red(s), t, x -- p and s
+//     are formed where they are gathered, and s is never stored;
+//   stored: k_bi_p, red, v, k_bi_s, red, t, k_bi_x.
+// Tried and slower: the formed sequence in one cooperative launch (195 us per
+// iteration of the 983k-node tri-gate against 160: a static split leaves every
+// grid barrier 4 to 8 us of waiting for the slowest SM).
 #pragma once
 
 namespace tcad {
 
-constexpr int kRbStreamSlots = 2 * NT;   // the flat block these kernels take
-constexpr int kRbRed = 0, kRbV = 1, kRbT = 2, kRbTrue = 3;
+constexpr int kRbStreamSlots = 512;       // most slots of a flat block
+constexpr int NTS = 512;                  // threads: one slot each
+// passes: red(p) and red(s) formed, red(X); v and t formed, and stored; the true
+// residual
+enum RbPass { kRbRedP, kRbRedS, kRbRed, kRbV, kRbT, kRbVs, kRbTs, kRbTrue };
+constexpr bool rb_is_red(int pass) { return pass <= kRbRed; }
+constexpr int rb_sums(int pass) { return pass == kRbT ? 3 : pass == kRbTs ? 2 : 1; }
+// the formed sequence up to this many slots: its x, r, rh, p, v, t and red result
+// (168 bytes a slot) then stay in L2 (126 MB).  Per iteration, formed / stored:
+// 491k slots 160 / 180 us, 983k slots 335 / 322 us.
+constexpr int64_t kRbFormSlots = 600000;
 
 template <int DIM>
 constexpr size_t rb_stream_smem() {
-  return (size_t)2 * (NT / 32) * Stencil<DIM>::NE * 32 * sizeof(double);
+  return (size_t)(NTS / 32) * Stencil<DIM>::NE * 32 * sizeof(double);
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -51,9 +68,16 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned n
       : "memory");
 }
 
-__device__ __forceinline__ uint64_t evict_first_policy() {
+// J of more than this many bytes is read evict-first; less stays in L2 (126 MB)
+// from one pass to the next along with the vectors
+constexpr int64_t kRbKeepBytes = (int64_t)80 << 20;
+
+__device__ __forceinline__ uint64_t stream_policy(bool keep) {
   uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  if (keep)
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  else
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 
@@ -94,197 +118,402 @@ __device__ __forceinline__ void rb_couple_r(const double* Jt, const double (&xv)
   y2 = d[6] * t0 + d[7] * t1 + d[8] * t2;
 }
 
-// PASS kRbRed:  out = E X (X black, all instances when ks is null)
-//      kRbV:    w.v = w.p - F X (X = E p); (rh, v)
-//      kRbT:    w.t = w.s - F X (X = E s); (t, s), (t, t)
-//      kRbTrue: out = rhs - (xb - F X) (X = E xb); (r, r), every instance
-// `fail`: the states of all instances (status TCAD_ERR_CUDA when a copy did
-// not arrive within its limit)
-template <int DIM, int PASS>
-__global__ void __launch_bounds__(NT, 1)
-k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ Jc,
-            const double* __restrict__ X, double* __restrict__ out, BiVec w,
-            const double* __restrict__ rhs, const double* __restrict__ xb, const KState* ks,
-            KState* fail, double* partial, unsigned* ticket, int rearm, int64_t nblk,
-            const int32_t* __restrict__ blk) {
-  constexpr int NE = Stencil<DIM>::NE, NW = NT / 32, ND = 2 * DIM;
-  constexpr int NS = PASS == kRbT ? 2 : 1;
-  constexpr unsigned kBytes = NE * 32 * sizeof(double);
-  extern __shared__ __align__(128) double s_tiles[];   // [NW][2][NE * 32]
-  __shared__ uint64_t s_bar[NW][2];
-  __shared__ double s_sum[2][NS][NW];
-  __shared__ int s_last;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double* const tile = s_tiles + (size_t)warp * 2 * NE * 32;
-  const int64_t VS = pkb.n_nodes;
-  const uint64_t policy = evict_first_policy();
-  if (lane == 0) {
-    mbar_init(&s_bar[warp][0]);
-    mbar_init(&s_bar[warp][1]);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+// a flat block of the slot pack
+struct RbBlk {
+  int64_t id, begin;
+  int len, inst;   // len 0: nothing to do
+};
+
+__device__ __forceinline__ RbBlk rb_blk(const tcad_pack_t& pkb, int64_t id) {
+  const FlatBlock fb = flat_block(pkb, id);
+  return RbBlk{id, fb.begin, (int)(fb.end - fb.begin), fb.inst};
+}
+
+// shared memory of a streaming CTA (next to the dynamic tiles)
+struct RbStreamShared {
+  uint64_t bar[NTS / 32];
+  double sum[2][3][NTS / 32];
+};
+
+template <int DIM>
+struct RbStreamer {
+  static constexpr int NE = Stencil<DIM>::NE, NW = NTS / 32, ND = 2 * DIM;
+  const tcad_pack_t& pkb;
+  const RbMap& mp;
+  const double *JR, *JB;
+  RbStreamShared& sh;
+  double* tile;      // the warp's buffer
+  uint64_t policy;
+  int lane, warp, par;
+  int64_t pend;      // block whose tile the buffer holds or waits for (-1: none)
+  int pcol;          // and its colour
+  unsigned phase, tries;
+  bool lost;         // a copy did not arrive within its limit
+
+  __device__ __forceinline__ RbStreamer(const tcad_pack_t& pkb_, const RbMap& mp_,
+                                        const double* JR_, const double* JB_,
+                                        RbStreamShared& sh_, double* tiles)
+      : pkb(pkb_), mp(mp_), JR(JR_), JB(JB_), sh(sh_) {
+    lane = threadIdx.x & 31;
+    warp = threadIdx.x >> 5;
+    tile = tiles + (size_t)warp * NE * 32;
+    policy = stream_policy(pkb.n_nodes * (2 * NE * 8) <= kRbKeepBytes);
+    par = 0;
+    pend = -1;
+    pcol = 0;
+    phase = 0u;
+    tries = 1u << 20;
+    lost = false;
+    if (lane == 0) {
+      mbar_init(&sh.bar[warp]);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
   }
-  __syncwarp();
 
-  struct Blk {
-    FlatBlock fb;
-    int64_t id;
-    bool on;
-  };
-  auto fetch = [&](int64_t i) {
-    Blk q;
-    q.on = false;
-    if (i < nblk) {
-      q.id = blk ? (int64_t)blk[i] : i;
-      q.fb = flat_block(pkb, q.id);
-      q.on = !ks || ks[q.fb.inst].active;
+  // start copying the warp's tile of block q, colour col (every lane has
+  // read the buffer)
+  __device__ __forceinline__ void issue(const RbBlk& q, int col) {
+    pend = -1;
+    if (warp * 32 >= q.len) return;
+    pend = q.id;
+    pcol = col;
+    if (lane == 0)
+      bulk_load(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32),
+                NE * 32 * sizeof(double), &sh.bar[warp], policy);
+  }
+  __device__ __forceinline__ void arrive() {
+    if (!mbar_wait(&sh.bar[warp], phase, tries)) {
+      lost = true;
+      tries = 64u;
     }
-    return q;
-  };
-  auto has = [&](const Blk& q, int h) {
-    return q.on && q.fb.begin + (warp + h * NW) * 32 < q.fb.end;
-  };
-  auto issue = [&](const Blk& q, int h) {
-    if (lane == 0 && has(q, h))
-      bulk_load(tile + h * NE * 32, Jc + ((q.fb.begin >> 5) + warp + h * NW) * (NE * 32), kBytes,
-                &s_bar[warp][h], policy);
-  };
-  // once the CTA has stored all its partials of an instance: its ticket, and
-  // the totals by the last CTA
-  auto flush = [&](int inst, unsigned count) {
-    if (threadIdx.x == 0) {
-      __threadfence();
-      const unsigned nb = (unsigned)(pkb.flat_off[inst + 1] - pkb.flat_off[inst]);
-      s_last = atomicAdd(&ticket[inst], count) + count == nb;
+    phase ^= 1u;
+    pend = -1;
+  }
+
+  // block sums of v (all threads) into out[0..NS): warp sums, then the 16 of
+  // them pairwise
+  template <int NS>
+  __device__ __forceinline__ void block_sums(double (&v)[NS], double* out) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+      if (lane == 0) sh.sum[par][q][warp] = v[q];
     }
     __syncthreads();
-    if (s_last) {
-      __threadfence();
-      double tot[NS];
-      Reduce<NS>::total(pkb, inst, partial, tot);
-      if (threadIdx.x == 0) {
-        ticket[inst] = 0u;
-        if (PASS == kRbV) fin_v(fail[inst], tot[0]);
-        if (PASS == kRbT) fin_t(fail[inst], tot[0], tot[NS - 1]);
-        if (PASS == kRbTrue) fin_true(fail[inst], tot[0], rearm);
-      }
+    if (threadIdx.x < NS) {
+      const double* const e = sh.sum[par][threadIdx.x];
+      double s[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s[i] = e[i] + e[i + 8];
+      out[threadIdx.x] = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
     }
-    __syncthreads();
-  };
+    par ^= 1;   // (the next sums go to the other buffer, across a barrier)
+  }
 
-  unsigned phase[2] = {0u, 0u}, tries = 1u << 20, count = 0u;
-  int cinst = -1, par = 0;
-  Blk cur = fetch(blockIdx.x);
-  issue(cur, 0);
-  issue(cur, 1);
-  for (int64_t i = blockIdx.x; i < nblk; i += gridDim.x) {
-    const Blk nxt = fetch(i + gridDim.x);
+  // one block of a pass; nxt, ncol: what the warp's buffer is for after it;
+  // S: the instance's state.  Between x and v, w.p holds p - omega v: a
+  // neighbour's p is then formed from two values, r + beta w.p, the bits of
+  // r + beta (p - omega v); s is formed from r and v and never stored.
+  //   kRbRedP, kRbRedS, kRbRed:  Tr = E p, E s, E X
+  //   kRbV:    w.p = p, w.v = p - F Tr; (rh, v)   (restart: rh = r)
+  //   kRbT:    w.t = s - F Tr; (s, s), (t, s), (t, t)
+  //   kRbVs, kRbTs: the same with p and s as stored, without (s, s)
+  //   kRbTrue: w.r = rhs - (X - F Tr); (r, r)
+  template <int PASS>
+  __device__ __forceinline__ void block(const RbBlk& q, const RbBlk& nxt, int ncol,
+                                        const KState& S, const double* X, double* Tr,
+                                        const BiVec& w, const double* rhs, double* partial) {
+    constexpr int NS = rb_sums(PASS), col = rb_is_red(PASS) ? 0 : 1;
+    const int64_t VS = pkb.n_nodes;
+    const RbGeo g = rb_geo(pkb, mp, q.inst);
+    const double alpha = S.alpha, beta = S.beta;
+    const int restart = S.restart;
+    const bool here = warp * 32 < q.len;
+    if (pend >= 0 && (!here || pend != q.id || pcol != col)) arrive();
+    if (here && pend < 0) issue(q, col);
     double v[NS];
 #pragma unroll
-    for (int q = 0; q < NS; ++q) v[q] = 0.0;
-    if (cur.on) {
-      const RbGeo g = rb_geo(pkb, mp, cur.fb.inst);
+    for (int k = 0; k < NS; ++k) v[k] = 0.0;
+    const int64_t slot = q.begin + threadIdx.x;
+    const bool mine = (int)threadIdx.x < q.len;
+    bool real = false;
+    double xv[ND][3], own[3][3];
+    if (mine) {
+      const RbNode nd = rb_node(g, slot, col);
+      real = nd.real;
+      if (real) {
+        int m[6];
+        rb_nbrs<DIM>(g, nd, (int)(slot - g.soff), m);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (!has(cur, h)) {
-          issue(nxt, h);
-          continue;
-        }
-        const int64_t slot = cur.fb.begin + (warp + h * NW) * 32 + lane;
-        const bool mine = slot < cur.fb.end;
-        bool real = false;
-        double xv[ND][3], own[2][3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) { own[0][c] = 0.0; own[1][c] = 0.0; }
-        if (mine) {
-          const RbNode q = rb_node(g, slot, PASS == kRbRed ? 0 : 1);
-          real = q.real;
-          if (real) {
-            int m[6];
-            rb_nbrs<DIM>(g, q, (int)(slot - g.soff), m);
-            const double* __restrict__ xi = X + g.soff;
-#pragma unroll
-            for (int d = 0; d < ND; ++d)
-#pragma unroll
-              for (int c = 0; c < 3; ++c) xv[d][c] = xi[c * VS + m[d]];
-          }
-          if (PASS != kRbRed) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const int64_t a = c * VS + slot;
-              own[0][c] = PASS == kRbV ? w.p[a] : PASS == kRbT ? w.s[a] : xb[a];
-              if (PASS == kRbV) own[1][c] = w.rh[a];
-              if (PASS == kRbTrue) own[1][c] = rhs[a];
-            }
-          }
-        }
-        if (!mbar_wait(&s_bar[warp][h], phase[h], tries)) {
-          if (lane == 0) {
-            fail[cur.fb.inst].status = TCAD_ERR_CUDA;
-            fail[cur.fb.inst].active = 0;
-          }
-          tries = 64u;
-        }
-        phase[h] ^= 1u;
-        double u[3] = {0.0, 0.0, 0.0};
-        if (real) rb_couple_r<DIM>(tile + h * NE * 32 + lane, xv, u[0], u[1], u[2]);
-        __syncwarp();
-        issue(nxt, h);
-        if (mine) {
+        for (int d = 0; d < ND; ++d)
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            const int64_t a = c * VS + slot;
-            if (PASS == kRbRed) {
-              out[a] = u[c];
-            } else if (PASS == kRbV) {
-              const double y = real ? own[0][c] - u[c] : 0.0;
-              w.v[a] = y;
-              v[0] += own[1][c] * y;
-            } else if (PASS == kRbT) {
-              const double y = real ? own[0][c] - u[c] : 0.0;
-              w.t[a] = y;
-              v[0] += y * own[0][c];
-              v[NS - 1] += y * y;
+            const int64_t a = c * VS + g.soff + m[d];
+            if (PASS == kRbRedP) {
+              const double rv = w.r[a], pv = w.p[a];
+              xv[d][c] = restart ? rv : rv + beta * pv;
+            } else if (PASS == kRbRedS) {
+              xv[d][c] = w.r[a] - alpha * w.v[a];
             } else {
-              const double y = real ? own[0][c] - u[c] : 0.0;
-              const double r = own[1][c] - y;
-              out[a] = r;
-              v[0] += r * r;
+              xv[d][c] = PASS == kRbRed ? X[a] : Tr[a];
             }
           }
+      }
+      if (!rb_is_red(PASS)) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int64_t a = c * VS + slot;
+          own[0][c] = PASS == kRbTrue ? X[a] : PASS == kRbVs ? w.p[a] : PASS == kRbTs ? w.s[a]
+                                                                                     : w.r[a];
+          if (PASS == kRbV) own[1][c] = w.p[a];
+          if (PASS == kRbT) own[1][c] = w.v[a];
+          if (PASS == kRbTrue) own[1][c] = rhs[a];
+          if (PASS == kRbV || PASS == kRbVs) own[2][c] = w.rh[a];
         }
       }
-      if (PASS != kRbRed) {
-        if (cinst >= 0 && cinst != cur.fb.inst) {
-          flush(cinst, count);
-          count = 0u;
+    }
+    if (here) arrive();
+    double u[3] = {0.0, 0.0, 0.0};
+    if (real) rb_couple_r<DIM>(tile + lane, xv, u[0], u[1], u[2]);
+    __syncwarp();
+    issue(nxt, ncol);
+    if (mine) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int64_t a = c * VS + slot;
+        if (rb_is_red(PASS)) {
+          Tr[a] = u[c];
+        } else if (PASS == kRbV) {
+          const double rv = own[0][c], pn = restart ? rv : rv + beta * own[1][c];
+          const double hv = restart ? rv : own[2][c];
+          const double y = real ? pn - u[c] : 0.0;
+          if (restart) w.rh[a] = rv;
+          w.p[a] = pn;
+          w.v[a] = y;
+          v[0] += hv * y;
+        } else if (PASS == kRbT) {
+          const double sv = own[0][c] - alpha * own[1][c];
+          const double y = real ? sv - u[c] : 0.0;
+          w.t[a] = y;
+          v[0] += sv * sv;
+          v[NS - 2] += y * sv;
+          v[NS - 1] += y * y;
+        } else if (PASS == kRbVs) {
+          const double y = real ? own[0][c] - u[c] : 0.0;
+          w.v[a] = y;
+          v[0] += own[2][c] * y;
+        } else if (PASS == kRbTs) {
+          const double y = real ? own[0][c] - u[c] : 0.0;
+          w.t[a] = y;
+          v[0] += y * own[0][c];
+          v[NS - 1] += y * y;
+        } else {
+          const double y = real ? own[0][c] - u[c] : 0.0;
+          const double r = own[1][c] - y;
+          w.r[a] = r;
+          v[0] += r * r;
         }
-        cinst = cur.fb.inst;
-        ++count;
-#pragma unroll
-        for (int q = 0; q < NS; ++q) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-          if (lane == 0) s_sum[par][q][warp] = v[q];
-        }
-        __syncthreads();
-        if (warp == 0) {
-#pragma unroll
-          for (int q = 0; q < NS; ++q) {
-            double r = lane < NW ? s_sum[par][q][lane] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-            if (lane == 0) partial[cur.id * 4 + q] = r;
-          }
-        }
-        par ^= 1;
       }
+    }
+    if (!rb_is_red(PASS)) block_sums<NS>(v, partial + q.id * 4);
+  }
+
+  // the vectors of the x step, loaded one block ahead
+  struct XVec {
+    double e[6][3];   // x, p, r, v, t, rh
+  };
+  __device__ __forceinline__ void x_load(const RbBlk& q, const double* X, const BiVec& w,
+                                         XVec& o) {
+    if ((int)threadIdx.x >= q.len) return;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int64_t a = c * pkb.n_nodes + q.begin + threadIdx.x;
+      o.e[0][c] = X[a]; o.e[1][c] = w.p[a]; o.e[2][c] = w.r[a];
+      o.e[3][c] = w.v[a]; o.e[4][c] = w.t[a]; o.e[5][c] = w.rh[a];
+    }
+  }
+  // x += alpha p + omega s, r = s - omega t, w.p = p - omega v; (rh, r), (r, r),
+  // (rh, rh)
+  __device__ __forceinline__ void x_block(const RbBlk& q, const XVec& o, const KState& S,
+                                          double* X, const BiVec& w, double* partial) {
+    const double alpha = S.alpha, omega = S.omega;
+    double v[3] = {0.0, 0.0, 0.0};
+    if ((int)threadIdx.x < q.len)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int64_t a = c * pkb.n_nodes + q.begin + threadIdx.x;
+        const double sv = o.e[2][c] - alpha * o.e[3][c], hv = o.e[5][c];
+        X[a] = o.e[0][c] + alpha * o.e[1][c] + omega * sv;
+        const double r = sv - omega * o.e[4][c];
+        w.r[a] = r;
+        w.p[a] = o.e[1][c] - omega * o.e[3][c];
+        v[0] += hv * r;
+        v[1] += r * r;
+        v[2] += hv * hv;
+      }
+    block_sums<3>(v, partial + q.id * 4);
+  }
+};
+
+// sums over instance inst's blocks of partial[b * 4 + q], valid in thread 0
+template <int NS>
+__device__ __forceinline__ void rb_totals(const tcad_pack_t& pkb, int inst, const double* partial,
+                                          double (&sum)[NS][NTS / 32], double* tot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t b1 = pkb.flat_off[inst + 1];
+  double v[NS];
+#pragma unroll
+  for (int q = 0; q < NS; ++q) v[q] = 0.0;
+  for (int64_t b = pkb.flat_off[inst] + threadIdx.x; b < b1; b += NTS)
+#pragma unroll
+    for (int q = 0; q < NS; ++q) v[q] += __ldcg(&partial[b * 4 + q]);
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+    if (lane == 0) sum[q][warp] = v[q];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      double s[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s[i] = sum[q][i] + sum[q][i + 8];
+      tot[q] = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+    }
+}
+
+// ---- one step per launch over nblk blocks (blk: their numbers, null: all) of the
+// instances still iterating (all: of every instance).  A CTA adds its count of
+// blocks to the instance's ticket once; the last CTA takes the totals into ks
+// (status TCAD_ERR_CUDA when a copy did not arrive within its limit).
+struct RbTicket {
+  unsigned count = 0u;
+  int inst = -1;
+};
+
+template <int NS, class FIN>
+__device__ __forceinline__ void rb_flush(const tcad_pack_t& pkb, RbTicket& tk, double* partial,
+                                         unsigned* ticket, const FIN& fin) {
+  __shared__ double s_tot[NS][NTS / 32];
+  __shared__ int s_last;
+  if (threadIdx.x < 32) {      // the threads that stored the CTA's partials
+    __threadfence();
+    __syncwarp();
+  }
+  if (threadIdx.x == 0) {
+    const unsigned nb = (unsigned)(pkb.flat_off[tk.inst + 1] - pkb.flat_off[tk.inst]);
+    s_last = atomicAdd(&ticket[tk.inst], tk.count) + tk.count == nb;
+  }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    double tot[NS];
+    rb_totals<NS>(pkb, tk.inst, partial, s_tot, tot);
+    if (threadIdx.x == 0) {
+      ticket[tk.inst] = 0u;
+      fin(tk.inst, tot);
+    }
+  }
+  __syncthreads();
+  tk.count = 0u;
+}
+
+// the i-th block; len 0 when its instance takes no part (ks null: all do)
+__device__ __forceinline__ RbBlk rb_fetch(const tcad_pack_t& pkb, const KState* ks, int64_t i,
+                                          int64_t nblk, const int32_t* blk) {
+  RbBlk q{-1, 0, 0, 0};
+  if (i < nblk) {
+    q = rb_blk(pkb, blk ? (int64_t)blk[i] : i);
+    if (ks && !ks[q.inst].active) q.len = 0;
+  }
+  return q;
+}
+
+// programmatic dependent launch: let the next kernel's CTAs start where SMs are
+// free; wait for the kernels before this one (what they wrote is visible then)
+__device__ __forceinline__ void launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_prior() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <int DIM, int PASS>
+__global__ void __launch_bounds__(NTS, 1)
+k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR,
+            const double* __restrict__ JB, const double* X, double* Tr, BiVec w,
+            const double* rhs, KState* ks, bool all, double* partial, unsigned* ticket,
+            int rearm, int64_t nblk, const int32_t* __restrict__ blk) {
+  constexpr int NS = rb_sums(PASS), col = rb_is_red(PASS) ? 0 : 1;
+  extern __shared__ __align__(128) double s_tiles[];
+  __shared__ RbStreamShared sh;
+  RbStreamer<DIM> st(pkb, mp, JR, JB, sh, s_tiles);
+  auto fin = [&](int inst, const double* tot) {
+    if (PASS == kRbV || PASS == kRbVs) fin_v(ks[inst], tot[0]);
+    if (PASS == kRbT) fin_s(ks[inst], tot[0]);
+    if (PASS == kRbT || PASS == kRbTs) fin_t(ks[inst], tot[NS > 1 ? NS - 2 : 0], tot[NS - 1]);
+    if (PASS == kRbTrue) fin_true(ks[inst], tot[0], rearm);
+  };
+  RbTicket tk;
+  // J and the tables are older than the kernel before this one; its states and
+  // vectors are not
+  RbBlk cur = rb_fetch(pkb, nullptr, blockIdx.x, nblk, blk);
+  st.issue(cur, col);
+  launch_dependents();
+  wait_prior();
+  if (!all && !ks[cur.inst].active) cur.len = 0;
+  for (int64_t i = blockIdx.x; i < nblk; i += gridDim.x) {
+    const RbBlk nxt = rb_fetch(pkb, all ? nullptr : ks, i + gridDim.x, nblk, blk);
+    if (cur.len > 0) {
+      if (!rb_is_red(PASS)) {
+        if (tk.inst >= 0 && tk.inst != cur.inst) rb_flush<NS>(pkb, tk, partial, ticket, fin);
+        tk.inst = cur.inst;
+        ++tk.count;
+      }
+      st.template block<PASS>(cur, nxt, col, ks[cur.inst], X, Tr, w, rhs, partial);
     } else {
-      issue(nxt, 0);
-      issue(nxt, 1);
+      if (st.pend >= 0) st.arrive();
+      st.issue(nxt, col);
     }
     cur = nxt;
   }
-  if (PASS != kRbRed && cinst >= 0) flush(cinst, count);
+  if (tk.inst >= 0) rb_flush<NS>(pkb, tk, partial, ticket, fin);
+  if (st.lost && st.lane == 0) {
+    ks[0].status = TCAD_ERR_CUDA;
+    ks[0].active = 0;
+  }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(NTS, 1)
+k_rb_stream_x(const tcad_pack_t pkb, const RbMap mp, double* X, BiVec w, KState* ks,
+              double* partial, unsigned* ticket, int64_t nblk, const int32_t* __restrict__ blk) {
+  __shared__ RbStreamShared sh;
+  RbStreamer<DIM> st(pkb, mp, nullptr, nullptr, sh, nullptr);
+  typename RbStreamer<DIM>::XVec a, b;
+  auto fin = [&](int inst, const double* tot) { fin_x(ks[inst], tot[0], tot[1], tot[2]); };
+  RbTicket tk;
+  launch_dependents();
+  wait_prior();
+  RbBlk cur = rb_fetch(pkb, ks, blockIdx.x, nblk, blk);
+  st.x_load(cur, X, w, a);
+  for (int64_t i = blockIdx.x; i < nblk; i += gridDim.x) {
+    const RbBlk nxt = rb_fetch(pkb, ks, i + gridDim.x, nblk, blk);
+    st.x_load(nxt, X, w, b);
+    if (cur.len > 0) {
+      if (tk.inst >= 0 && tk.inst != cur.inst) rb_flush<3>(pkb, tk, partial, ticket, fin);
+      tk.inst = cur.inst;
+      ++tk.count;
+      st.x_block(cur, a, ks[cur.inst], X, w, partial);
+    }
+    cur = nxt;
+    a = b;
+  }
+  if (tk.inst >= 0) rb_flush<3>(pkb, tk, partial, ticket, fin);
 }
 
 }  // namespace tcad

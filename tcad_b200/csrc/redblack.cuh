@@ -143,32 +143,6 @@ struct RbVal {
   __device__ __forceinline__ double operator()(int m, int c) const { return xi[c * NS + m]; }
 };
 
-// The search direction p = r + beta (p - omega v) (p = r on a restart) and
-// s = r - alpha v formed on the fly at the other colour's slots, from vectors
-// no CTA writes meanwhile -- the expressions of bi_p_body and bi_s_body (the
-// single-launch solve forms them where the per-step solve stores them)
-struct RbFormP {
-  const double* __restrict__ r;
-  const double* __restrict__ p;
-  const double* __restrict__ v;
-  int64_t NS;
-  double beta, omega;
-  int restart;
-  __device__ __forceinline__ double operator()(int m, int c) const {
-    const double rv = r[c * NS + m];
-    return restart ? rv : rv + beta * (p[c * NS + m] - omega * v[c * NS + m]);
-  }
-};
-struct RbFormS {
-  const double* __restrict__ r;
-  const double* __restrict__ v;
-  int64_t NS;
-  double alpha;
-  __device__ __forceinline__ double operator()(int m, int c) const {
-    return r[c * NS + m] - alpha * v[c * NS + m];
-  }
-};
-
 template <int DIM>
 __device__ __forceinline__ void rb_couple(const double* __restrict__ Jc,
                                           const double* __restrict__ xi, int64_t slot,
@@ -177,9 +151,9 @@ __device__ __forceinline__ void rb_couple(const double* __restrict__ Jc,
   rb_couple_f<DIM>(Jc, RbVal{xi, NS}, slot, m, y0, y1, y2);
 }
 
-// ---- per-block bodies, shared by the per-step kernels below and the
-// single-launch solve (k_bicgstab_rb_fused), so both run the same
-// arithmetic in the same order
+// ---- per-block bodies of the per-step kernels; the single-launch solves
+// (rb_resident.cuh, rb_streamed.cuh) and the streamed passes (rb_stream.cuh)
+// run the same arithmetic in the same order
 
 // bR, bB <- the colours of b at the block's slots; returns the thread's
 // share of (b, b)
@@ -251,42 +225,38 @@ __device__ __forceinline__ double rb_init_body(const tcad_pack_t& pkb, const RbM
   return v;
 }
 
-// red pass: Tr = E X at the block's red slots, X a value functor factory
-// (instance base offset -> functor)
-template <int DIM, class MK>
+// red pass: Tr = E x at the block's red slots
+template <int DIM>
 __device__ __forceinline__ void rb_red_body(const tcad_pack_t& pkb, const RbMap& mp,
                                             const FlatBlock& fb,
-                                            const double* __restrict__ JR, const MK& make,
+                                            const double* __restrict__ JR,
+                                            const double* __restrict__ x,
                                             double* __restrict__ Tr) {
   const RbGeo g = rb_geo(pkb, mp, fb.inst);
   const int64_t NS = pkb.n_nodes;
-  const auto X = make(g.soff);
   for (int64_t slot = fb.begin + threadIdx.x; slot < fb.end; slot += NT) {
     const RbNode q = rb_node(g, slot, 0);
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
     if (q.real) {
       int m[6];
       rb_nbrs<DIM>(g, q, (int)(slot - g.soff), m);
-      rb_couple_f<DIM>(JR, X, slot, m, y0, y1, y2);
+      rb_couple<DIM>(JR, x + g.soff, slot, NS, m, y0, y1, y2);
     }
     Tr[slot] = y0; Tr[NS + slot] = y1; Tr[2 * NS + slot] = y2;
   }
 }
 
-// v = S p (Tr = E p); FORM: p formed and stored first (p = r + beta (p -
-// omega v); restart: rh = p = r), else p as stored; returns (rh, v) share
-template <int DIM, bool FORM>
+// v = S p (Tr = E p); returns (rh, v) share
+template <int DIM>
 __device__ __forceinline__ double rb_v_body(const tcad_pack_t& pkb, const RbMap& mp,
                                             const FlatBlock& fb,
                                             const double* __restrict__ JB,
-                                            const double* __restrict__ Tr, const BiVec& w,
-                                            double beta, double omega, int restart) {
+                                            const double* __restrict__ Tr, const BiVec& w) {
   const RbGeo g = rb_geo(pkb, mp, fb.inst);
   const int64_t NS = pkb.n_nodes;
-  double* __restrict__ P = w.p;
-  double* __restrict__ RH = w.rh;
+  const double* __restrict__ P = w.p;
+  const double* __restrict__ RH = w.rh;
   double* __restrict__ Vo = w.v;
-  const double* __restrict__ R = w.r;
   double v = 0.0;
   for (int64_t slot = fb.begin + threadIdx.x; slot < fb.end; slot += NT) {
     double u[3];
@@ -294,17 +264,7 @@ __device__ __forceinline__ double rb_v_body(const tcad_pack_t& pkb, const RbMap&
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int64_t i = c * NS + slot;
-      double pn, h;
-      if (FORM) {
-        const double rv = R[i];
-        pn = restart ? rv : rv + beta * (P[i] - omega * Vo[i]);
-        P[i] = pn;
-        if (restart) RH[i] = rv;
-        h = restart ? rv : RH[i];
-      } else {
-        pn = P[i];
-        h = RH[i];
-      }
+      const double pn = P[i], h = RH[i];
       const double y = real ? pn - u[c] : 0.0;
       Vo[i] = y;
       v += h * y;
@@ -313,39 +273,28 @@ __device__ __forceinline__ double rb_v_body(const tcad_pack_t& pkb, const RbMap&
   return v;
 }
 
-// t = S s (Tr = E s); FORM: s = r - alpha v formed and stored first (its
-// (s, s) share in v[0], accumulated as bi_s_body does), else s as stored;
-// v[1] = (t, s), v[2] = (t, t) shares
-template <int DIM, bool FORM>
+// t = S s (Tr = E s); v[0] = (t, s), v[1] = (t, t) shares
+template <int DIM>
 __device__ __forceinline__ void rb_t_body(const tcad_pack_t& pkb, const RbMap& mp,
                                           const FlatBlock& fb, const double* __restrict__ JB,
                                           const double* __restrict__ Tr, const BiVec& w,
-                                          double alpha, double (&v)[3]) {
+                                          double (&v)[2]) {
   const RbGeo g = rb_geo(pkb, mp, fb.inst);
   const int64_t NS = pkb.n_nodes;
-  double* __restrict__ S = w.s;
+  const double* __restrict__ S = w.s;
   double* __restrict__ To = w.t;
-  const double* __restrict__ R = w.r;
-  const double* __restrict__ V = w.v;
-  v[0] = 0.0; v[1] = 0.0; v[2] = 0.0;
+  v[0] = 0.0; v[1] = 0.0;
   for (int64_t slot = fb.begin + threadIdx.x; slot < fb.end; slot += NT) {
     double u[3];
     const bool real = rb_black_u<DIM>(g, JB, Tr, slot, NS, u);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int64_t i = c * NS + slot;
-      double sv;
-      if (FORM) {
-        sv = R[i] - alpha * V[i];
-        v[0] += sv * sv;
-        S[i] = sv;
-      } else {
-        sv = S[i];
-      }
+      const double sv = S[i];
       const double y = real ? sv - u[c] : 0.0;
       To[i] = y;
-      v[1] += y * sv;
-      v[2] += y * y;
+      v[0] += y * sv;
+      v[1] += y * y;
     }
   }
 }
@@ -399,30 +348,6 @@ __device__ __forceinline__ void rb_merge_body(const tcad_pack_t& pkb, const RbMa
     }
   }
 }
-
-// functor factories for rb_red_body
-struct RbMakeVal {
-  const double* x;
-  int64_t NS;
-  __device__ __forceinline__ RbVal operator()(int64_t soff) const { return RbVal{x + soff, NS}; }
-};
-struct RbMakeP {
-  const double *r, *p, *v;
-  int64_t NS;
-  double beta, omega;
-  int restart;
-  __device__ __forceinline__ RbFormP operator()(int64_t soff) const {
-    return RbFormP{r + soff, p + soff, v + soff, NS, beta, omega, restart};
-  }
-};
-struct RbMakeS {
-  const double *r, *v;
-  int64_t NS;
-  double alpha;
-  __device__ __forceinline__ RbFormS operator()(int64_t soff) const {
-    return RbFormS{r + soff, v + soff, NS, alpha};
-  }
-};
 
 // ---- one launch per step
 
@@ -499,7 +424,7 @@ k_rb_red(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR,
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pkb, fbi);
   if (ks && !ks[fb.inst].active) return;
-  rb_red_body<DIM>(pkb, mp, fb, JR, RbMakeVal{x, pkb.n_nodes}, Tr);
+  rb_red_body<DIM>(pkb, mp, fb, JR, x, Tr);
 }
 
 // v = S p (Tr = E p from the red pass); (rh, v)
@@ -511,7 +436,7 @@ k_rb_v(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JB,
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pkb, fbi);
   if (!ks[fb.inst].active) return;
-  double vv[1] = {rb_v_body<DIM, false>(pkb, mp, fb, JB, Tr, w, 0.0, 0.0, 0)};
+  double vv[1] = {rb_v_body<DIM>(pkb, mp, fb, JB, Tr, w)};
   double tot[1];
   if (Reduce<1>::run(pkb, fbi, fb.inst, vv, partial, ticket, tot) && threadIdx.x == 0)
     fin_v(ks[fb.inst], tot[0]);
@@ -526,9 +451,8 @@ k_rb_t(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JB,
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pkb, fbi);
   if (!ks[fb.inst].active) return;
-  double v3[3];
-  rb_t_body<DIM, false>(pkb, mp, fb, JB, Tr, w, 0.0, v3);
-  double v[2] = {v3[1], v3[2]};
+  double v[2];
+  rb_t_body<DIM>(pkb, mp, fb, JB, Tr, w, v);
   double tot[2];
   if (Reduce<2>::run(pkb, fbi, fb.inst, v, partial, ticket, tot) && threadIdx.x == 0)
     fin_t(ks[fb.inst], tot[0], tot[1]);

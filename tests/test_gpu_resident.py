@@ -120,7 +120,7 @@ def _batch_solve(pk, rtol, maxit, fused):
     return x, list(it), list(st), list(rr)
 
 
-STREAMED = [[("trigate", (131, 80, 51))], [("mosfet", (801, 400))],
+STREAMED = [[("trigate", (131, 80, 51))], [("mosfet", (801, 400))], [("trigate", (161, 97, 79))],
             [("trigate", (57, 45, 39)), ("trigate", (9, 7, 5)), ("trigate", (56, 48, 46))],
             [("diode", (401, 351)), ("diode", (21, 10)), ("diode", (300, 203))]]
 
