@@ -6,7 +6,10 @@
 // (device Jacobians carry ~10 entries per row), so a warp reads four rows'
 // entries with unit stride.  Dot products reduce per block; the last block
 // to finish sums the block partials in block order (deterministic) and
-// updates the solver scalars on the device.
+// updates the solver's state on the device (BiCGStab's scalars; GMRES's column
+// of H, its Givens rotations and residual norm), so an iteration runs without
+// the host, which looks at the state every few iterations.  Once a state is
+// done, the kernels already queued return at once.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -18,6 +21,7 @@ namespace csr {
 
 constexpr int NT = 256;
 constexpr int kRowsPerBlock = NT / 8;
+constexpr int64_t kGridBlocks = 592;   // 4 per SM: most blocks of a reducing kernel
 
 struct Sys {
   int64_t n;
@@ -213,47 +217,406 @@ __global__ void k_axpbypcz(int64_t n, double a, const double* __restrict__ x, do
   y[i] = v;
 }
 
-// GMRES: h[i] = (V_i, w) for i < m (one pass over w)
-__global__ void __launch_bounds__(NT) k_gs_dots(int64_t n, const double* __restrict__ V,
-                                                int m, const double* __restrict__ w,
-                                                double* __restrict__ partial) {
-  __shared__ double sm[32];
-  for (int i = 0; i < m; ++i) {
-    double v = 0.0;
-    const double* Vi = V + (int64_t)i * n;
-    for (int64_t k = (int64_t)blockIdx.x * NT + threadIdx.x; k < n;
-         k += (int64_t)gridDim.x * NT)
-      v += Vi[k] * w[k];
-    const double r = block_sum<NT>(v, sm);
-    if (threadIdx.x == 0) partial[(int64_t)blockIdx.x * m + i] = r;
+// ---- the last block of a grid to finish (ticket), for its totals
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  if (threadIdx.x == 0) *ticket = 0u;
+  return true;
 }
 
-__global__ void k_gs_sum(const double* __restrict__ partial, int nblk, int m,
-                         double* __restrict__ h) {
+// NS block sums into partial[q gridDim.x + block]; in the last block, the
+// totals (valid in thread 0)
+template <int NS, int T = NT>
+__device__ __forceinline__ bool grid_sums(double (&v)[NS], double* partial, unsigned* ticket,
+                                          double* tot) {
   __shared__ double sm[32];
-  for (int i = 0; i < m; ++i) {
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+    const double r = block_sum<T>(v[q], sm);
+    if (threadIdx.x == 0) partial[(size_t)q * gridDim.x + blockIdx.x] = r;
+  }
+  if (!last_block(ticket)) return false;
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
     double s = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += NT) s += partial[(int64_t)b * m + i];
-    const double r = block_sum<NT>(s, sm);
-    if (threadIdx.x == 0) h[i] = r;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += T)
+      s += __ldcg(&partial[(size_t)q * gridDim.x + b]);
+    tot[q] = block_sum<T>(s, sm);
+  }
+  return true;
+}
+
+// z = M^-1 r at one block row (bs = 3, 6), or one row
+__device__ __forceinline__ void prec_row(int bs, const double* __restrict__ inv, int64_t t,
+                                         const double* v, double* z) {
+  if (bs == 3) {
+    const double* m = inv + 9 * t;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) z[q] = m[3 * q] * v[0] + m[3 * q + 1] * v[1] + m[3 * q + 2] * v[2];
+  } else if (bs == 6) {
+    const double* m = inv + 36 * t;
+    for (int q = 0; q < 6; ++q) {
+      double acc = 0.0;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) acc += m[6 * q + c] * v[c];
+      z[q] = acc;
+    }
+  } else {
+    z[0] = bs == 1 ? inv[t] * v[0] : v[0];
   }
 }
 
-// w -= sum_i h[i] V_i
-__global__ void k_gs_sub(int64_t n, const double* __restrict__ V, int m,
-                         const double* __restrict__ h, double* __restrict__ w) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  double s = w[k];
-  for (int i = 0; i < m; ++i) s -= h[i] * V[(int64_t)i * n + k];
-  w[k] = s;
+// ---- GMRES(m), right preconditioned: one iteration in five launches
+//   spmv   w = A z
+//   dots   h1 = V^T w
+//   sub    w -= V h1, h2 = V^T w      (classical Gram-Schmidt, twice)
+//   norm   w -= V h2, ||w||; the last block: column h1 + h2 of H, its Givens
+//          rotations, the residual norm |g[j + 1]|
+//   next   V_{j+1} = w / ||w||, z = M^-1 V_{j+1}
+// A Jacobian of a few thousand nodes gives the V products 50 blocks of 256 rows,
+// so they are bound by the latency of their loads, one basis vector after the
+// other: a block has 32 warps, which take two vectors at a time for V^T w (w in
+// shared memory, one warp reduction per vector and 256 rows), and four groups
+// of 256 threads, which take every fourth vector for w -= V h.  13,824 rows, up
+// to 100 vectors: 180 us per iteration with the host in it, 44 us with 8 warps and
+// one group, 32 us with this.
+struct GState {
+  int j, done;      // columns finished; 1: residual at the tolerance or breakdown
+  double inv;       // 1 / ||w|| (0 when it vanished)
+};
+struct Gmres {
+  int64_t n;
+  int m;
+  double *V, *w, *h1, *h2, *R, *cs, *sn, *g;   // R: column j at R + j (m + 1)
+  double* partial;                              // [m + 1][blocks]
+  unsigned* ticket;
+  GState* st;
+};
+
+constexpr int NTG = 4 * NT;   // threads of the V products' blocks
+
+// partial sums of h = V^T w over the block's rows sw (256 of them from row0)
+__device__ __forceinline__ void gm_dots(const Gmres& G, int nv, int64_t row0, const double* sw,
+                                        bool first) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cnt = (int)min((int64_t)NT, G.n - row0);
+  double wv[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) wv[u] = sw[lane + 32 * u];   // 0 past the end
+  // two vectors at a time: sixteen loads a lane in flight
+  for (int i = 2 * warp; i < nv; i += 2 * (NTG / 32)) {
+    const bool two = i + 1 < nv;
+    const double* __restrict__ Vi = G.V + (int64_t)i * G.n + row0;
+    const double* __restrict__ Vk = two ? Vi + G.n : Vi;
+    double x[8], y[8], v = 0.0, q = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const bool in = lane + 32 * u < cnt;
+      x[u] = in ? Vi[lane + 32 * u] : 0.0;
+      y[u] = in ? Vk[lane + 32 * u] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      v += x[u] * wv[u];
+      q += y[u] * wv[u];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v += __shfl_down_sync(0xffffffffu, v, o);
+      q += __shfl_down_sync(0xffffffffu, q, o);
+    }
+    if (lane == 0) {
+      double* const d = &G.partial[(size_t)i * gridDim.x + blockIdx.x];
+      *d = first ? v : *d + v;
+      if (two) d[gridDim.x] = first ? q : d[gridDim.x] + q;
+    }
+  }
 }
 
-__global__ void k_scale_copy(int64_t n, double a, const double* __restrict__ x,
-                             double* __restrict__ y) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) y[k] = a * x[k];
+// h = the blocks' partial sums (last block)
+__device__ __forceinline__ void gm_totals(const Gmres& G, int nv, double* h) {
+  const int lane = threadIdx.x & 7;   // 8 lanes a vector
+  for (int i0 = 0; i0 < nv; i0 += NTG / 8) {
+    const int i = i0 + (threadIdx.x >> 3);
+    double v = 0.0;
+    if (i < nv) {
+#pragma unroll 8
+      for (unsigned b = lane; b < gridDim.x; b += 8)
+        v += __ldcg(&G.partial[(size_t)i * gridDim.x + b]);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 8);
+    if (i < nv && lane == 0) h[i] = v;
+  }
+}
+
+// w[row] - sum_i h[i] V_i[row] of the block's 256 rows, in the threads below NT
+// (0 past the end); s4: [4][NT]
+__device__ __forceinline__ double gm_minus(const Gmres& G, int nv, const double* __restrict__ h,
+                                           int64_t row0, double (*s4)[NT]) {
+  const int l = threadIdx.x & (NT - 1), grp = threadIdx.x / NT;
+  const int64_t row = row0 + l;
+  double a = 0.0;
+  if (row < G.n) {
+    const double* __restrict__ Vr = G.V + row;
+#pragma unroll 8
+    for (int i = grp; i < nv; i += 4) a += h[i] * Vr[(int64_t)i * G.n];
+  }
+  s4[grp][l] = a;
+  __syncthreads();
+  if (grp != 0 || row >= G.n) return 0.0;
+  return G.w[row] - ((s4[0][l] + s4[1][l]) + (s4[2][l] + s4[3][l]));
+}
+
+template <bool SUB>
+__global__ void __launch_bounds__(NTG) k_gm_dots(Gmres G) {
+  __shared__ double sw[NT], s4[4][NT];
+  if (G.st->done || G.st->j >= G.m) return;
+  const int nv = G.st->j + 1;
+  bool first = true;
+  for (int64_t row0 = (int64_t)blockIdx.x * NT; row0 < G.n; row0 += (int64_t)gridDim.x * NT) {
+    const int64_t row = row0 + threadIdx.x;
+    const bool mine = threadIdx.x < NT && row < G.n;
+    double w = 0.0;
+    if (SUB) w = gm_minus(G, nv, G.h1, row0, s4);
+    else if (mine) w = G.w[row];
+    if (SUB && mine) G.w[row] = w;
+    if (threadIdx.x < NT) sw[threadIdx.x] = w;
+    __syncthreads();
+    gm_dots(G, nv, row0, sw, first);
+    __syncthreads();
+    first = false;
+  }
+  if (last_block(G.ticket)) gm_totals(G, nv, SUB ? G.h2 : G.h1);
+}
+
+__global__ void __launch_bounds__(NTG) k_gm_norm(Gmres G, double tol) {
+  __shared__ double s4[4][NT];
+  if (G.st->done || G.st->j >= G.m) return;
+  const int j = G.st->j;
+  double v[1] = {0.0}, tot[1];
+  for (int64_t row0 = (int64_t)blockIdx.x * NT; row0 < G.n; row0 += (int64_t)gridDim.x * NT) {
+    const double w = gm_minus(G, j + 1, G.h2, row0, s4);
+    if (threadIdx.x < NT && row0 + threadIdx.x < G.n) G.w[row0 + threadIdx.x] = w;
+    v[0] += w * w;
+    __syncthreads();
+  }
+  if (!grid_sums<1, NTG>(v, G.partial, G.ticket, tot)) return;
+  // column j: the rotations so far (through shared memory: the chain in thread
+  // 0 then waits for arithmetic only), then the new one
+  double* const sh = s4[0];
+  double* const sc = s4[1];
+  double* const ss = s4[2];
+  double* const r = G.R + (size_t)j * (G.m + 1);
+  double a = G.h1[0] + G.h2[0];
+  for (int i0 = 0; i0 < j; i0 += NT) {
+    const int i = i0 + threadIdx.x;
+    __syncthreads();
+    if (threadIdx.x < NT && i < j) {
+      sh[threadIdx.x] = G.h1[i + 1] + G.h2[i + 1];
+      sc[threadIdx.x] = G.cs[i];
+      ss[threadIdx.x] = G.sn[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int k = 0; k < min(NT, j - i0); ++k) {
+        r[i0 + k] = sc[k] * a + ss[k] * sh[k];
+        a = -ss[k] * a + sc[k] * sh[k];
+      }
+  }
+  if (threadIdx.x != 0) return;
+  const double hn = sqrt(tot[0]);
+  const double den = hypot(a, hn);
+  const double c = den > 0.0 ? a / den : 1.0, s = den > 0.0 ? hn / den : 0.0;
+  r[j] = den;
+  G.cs[j] = c;
+  G.sn[j] = s;
+  const double gj = G.g[j], gn = -s * gj;
+  G.g[j + 1] = gn;
+  G.g[j] = c * gj;
+  G.st->inv = hn > 0.0 ? 1.0 / hn : 0.0;
+  G.st->done = (fabs(gn) <= tol || !(den > 0.0)) ? 1 : 0;
+  G.st->j = j + 1;
+}
+
+// V_j = w inv (j the new column), z = M^-1 V_j
+__global__ void __launch_bounds__(NT) k_gm_next(Gmres G, int bs, const double* __restrict__ inv,
+                                                double* __restrict__ z) {
+  if (G.st->done || G.st->j >= G.m) return;
+  const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
+  const int b = bs > 1 ? bs : 1;
+  if (t >= G.n / b) return;
+  const double a = G.st->inv;
+  double* const Vj = G.V + (int64_t)G.st->j * G.n;
+  double v[6], q[6];
+  for (int c = 0; c < b; ++c) {
+    v[c] = a * G.w[b * t + c];
+    Vj[b * t + c] = v[c];
+  }
+  prec_row(bs, inv, t, v, q);
+  for (int c = 0; c < b; ++c) z[b * t + c] = q[c];
+}
+
+// start of a cycle: g = (rn, 0, ...), no columns, w = the residual
+__global__ void k_gm_start(Gmres G, double rn) {
+  for (int i = threadIdx.x; i <= G.m; i += blockDim.x) G.g[i] = i == 0 ? rn : 0.0;
+  if (threadIdx.x == 0) *G.st = GState{0, 0, 1.0 / rn};
+}
+
+// ---- BiCGStab, right preconditioned: one iteration in five launches, each
+// ended by its scalars (last block)
+struct BState {
+  double rho, alpha, omega, beta, rn;   // rn: the residual norm (of s on an early exit)
+  int it, done;                         // done: converged, out of iterations or broken down
+};
+struct Bicg {
+  int64_t n;
+  double *r, *rh, *p, *v, *ph, *s, *sh, *t, *x;
+  double* partial;
+  unsigned* ticket;
+  BState* st;
+  double tol;
+  int maxit;
+};
+
+// the test at the top of an iteration on (rh, r): rho, beta for it
+__device__ __forceinline__ void bi_top(BState& st, double rhr, double tol, int maxit) {
+  if (!(st.rn > tol) || st.it >= maxit || rhr == 0.0 || !isfinite(rhr)) st.done = 1;
+  st.beta = (rhr / st.rho) * (st.alpha / st.omega);
+  st.rho = rhr;
+}
+
+// p = r + beta p - beta omega v, ph = M^-1 p
+__global__ void __launch_bounds__(NT) k_cb_p(Bicg B, int bs, const double* __restrict__ inv) {
+  const BState st = *B.st;
+  if (st.done) return;
+  const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
+  const int b = bs > 1 ? bs : 1;
+  if (t >= B.n / b) return;
+  const double bw = -st.beta * st.omega;
+  double v[6], q[6];
+  for (int c = 0; c < b; ++c) {
+    const int64_t i = b * t + c;
+    v[c] = B.r[i] + st.beta * B.p[i] + bw * B.v[i];
+    B.p[i] = v[c];
+  }
+  prec_row(bs, inv, t, v, q);
+  for (int c = 0; c < b; ++c) B.ph[b * t + c] = q[c];
+}
+
+// s = r - alpha v, sh = M^-1 s; (s, s): early exit
+__global__ void __launch_bounds__(NT) k_cb_s(Bicg B, int bs, const double* __restrict__ inv) {
+  const BState st = *B.st;
+  if (st.done) return;
+  const int b = bs > 1 ? bs : 1;
+  double sum[1] = {0.0}, tot[1];
+  for (int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x; t < B.n / b;
+       t += (int64_t)gridDim.x * NT) {
+    double v[6], q[6];
+    for (int c = 0; c < b; ++c) {
+      const int64_t i = b * t + c;
+      v[c] = B.r[i] - st.alpha * B.v[i];
+      B.s[i] = v[c];
+      sum[0] += v[c] * v[c];
+    }
+    prec_row(bs, inv, t, v, q);
+    for (int c = 0; c < b; ++c) B.sh[b * t + c] = q[c];
+  }
+  if (grid_sums<1>(sum, B.partial, B.ticket, tot) && threadIdx.x == 0) {
+    ++B.st->it;
+    if (sqrt(tot[0]) <= B.tol) {
+      B.st->rn = sqrt(tot[0]);
+      B.st->done = 2;               // x += alpha ph is left to do
+    }
+  }
+}
+
+// one row of A x by its 8 lanes (valid in lane 0)
+__device__ __forceinline__ double row_dot(const Sys& A, int64_t row, const double* __restrict__ x,
+                                          int lane) {
+  double s = 0.0;
+  if (row < A.n) {
+    const int a = A.ptr[row], b = A.ptr[row + 1];
+    for (int q = a + lane; q < b; q += 8) s += A.val[q] * x[A.idx[q]];
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, 8);
+  return s;
+}
+
+// v = A ph, (rh, v) -> alpha;  T: t = A sh, (t, t), (s, t) -> omega
+template <bool T>
+__global__ void __launch_bounds__(NT) k_cb_spmv(Sys A, Bicg B) {
+  if (B.st->done) return;
+  const int lane = threadIdx.x & 7;
+  double sum[2] = {0.0, 0.0}, tot[2];
+  for (int64_t r0 = (int64_t)blockIdx.x * kRowsPerBlock; r0 < A.n;
+       r0 += (int64_t)gridDim.x * kRowsPerBlock) {
+    const int64_t row = r0 + (threadIdx.x >> 3);
+    const double y = row_dot(A, row, T ? B.sh : B.ph, lane);
+    if (row < A.n && lane == 0) {
+      if (T) {
+        B.t[row] = y;
+        sum[0] += y * y;
+        sum[1] += B.s[row] * y;
+      } else {
+        B.v[row] = y;
+        sum[0] += B.rh[row] * y;
+      }
+    }
+  }
+  if (!grid_sums<2>(sum, B.partial, B.ticket, tot) || threadIdx.x != 0) return;
+  if (T) {
+    // (h[0] = (t, t), h[1] = (s, t) in the reference's naming of the step)
+    B.st->omega = tot[0] > 0.0 ? tot[1] / tot[0] : 0.0;
+  } else if (tot[0] == 0.0 || !isfinite(tot[0])) {
+    B.st->done = 1;
+  } else {
+    B.st->alpha = B.st->rho / tot[0];
+  }
+}
+
+// x += alpha ph + omega sh, r = s - omega t; (r, r), (rh, r)
+__global__ void __launch_bounds__(NT) k_cb_x(Bicg B) {
+  const BState st = *B.st;
+  if (st.done) return;
+  double sum[2] = {0.0, 0.0}, tot[2];
+  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < B.n;
+       i += (int64_t)gridDim.x * NT) {
+    B.x[i] = st.alpha * B.ph[i] + B.x[i] + st.omega * B.sh[i];
+    const double r = B.s[i] - st.omega * B.t[i];
+    B.r[i] = r;
+    sum[0] += r * r;
+    sum[1] += B.rh[i] * r;
+  }
+  if (!grid_sums<2>(sum, B.partial, B.ticket, tot) || threadIdx.x != 0) return;
+  B.st->rn = sqrt(tot[0]);
+  if (st.omega == 0.0) B.st->done = 1;
+  bi_top(*B.st, tot[1], B.tol, B.maxit);
+}
+
+// rh = r, p = v = 0; (r, r): the first iteration's scalars
+__global__ void __launch_bounds__(NT) k_cb_start(Bicg B) {
+  double sum[1] = {0.0}, tot[1];
+  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < B.n;
+       i += (int64_t)gridDim.x * NT) {
+    const double r = B.r[i];
+    B.rh[i] = r;
+    B.p[i] = 0.0;
+    B.v[i] = 0.0;
+    sum[0] += r * r;
+  }
+  if (!grid_sums<1>(sum, B.partial, B.ticket, tot) || threadIdx.x != 0) return;
+  *B.st = BState{1.0, 1.0, 1.0, 0.0, sqrt(tot[0]), 0, 0};
+  bi_top(*B.st, tot[0], B.tol, B.maxit);
 }
 
 // x += sum_i c[i] Z_i  (Z_i = M^-1 V_i folded later) -- here: y = sum_i c[i] V_i
@@ -329,6 +692,7 @@ extern "C" size_t tcad_csr_workspace_bytes(int64_t n, int method, int restart) {
   v += 4096 * 4 * sizeof(double) + 64 * sizeof(double) + 256;
   v += (size_t)4096 * (m + 1) * sizeof(double);      // Gram-Schmidt partials
   v += (size_t)(m + 1) * sizeof(double) + vec;       // coefficients, true residual
+  v += (size_t)(m + 1) * (m + 6) * sizeof(double);   // GMRES: H, rotations, sums
   return v + (1u << 20);                             // alignment slack
 }
 
@@ -389,144 +753,106 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
   const double tol = std::max(atol, rtol * bnorm);
   int it = 0;
   double rn = 0.0;
+  const unsigned gv = (unsigned)std::min<int64_t>(kGridBlocks, (N + NT - 1) / NT);
   if (method == 0) {
-    double* r = reinterpret_cast<double*>(take(N * 8));
-    double* rh = reinterpret_cast<double*>(take(N * 8));
-    double* p = reinterpret_cast<double*>(take(N * 8));
-    double* v = reinterpret_cast<double*>(take(N * 8));
-    double* ph = reinterpret_cast<double*>(take(N * 8));
-    double* sv = reinterpret_cast<double*>(take(N * 8));
-    double* sh = reinterpret_cast<double*>(take(N * 8));
-    double* t = reinterpret_cast<double*>(take(N * 8));
+    Bicg B;
+    double** const vec[8] = {&B.r, &B.rh, &B.p, &B.v, &B.ph, &B.s, &B.sh, &B.t};
+    for (double** q : vec) *q = reinterpret_cast<double*>(take(N * 8));
+    B.n = N;
+    B.x = x;
+    B.partial = c.partial;
+    B.ticket = c.ticket;
+    B.st = reinterpret_cast<BState*>(c.scal + 8);
+    B.tol = tol;
+    B.maxit = maxiter;
     // r = b - A x
-    spmv(c, x, r);
-    axpy(c, 1.0, b, -1.0, r);
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(rh, r, N * 8, cudaMemcpyDeviceToDevice, s));
-    TCAD_CUDA_CHECK(cudaMemsetAsync(p, 0, N * 8, s));
-    TCAD_CUDA_CHECK(cudaMemsetAsync(v, 0, N * 8, s));
-    Dots dr{{r}, {r}, 1};
-    if ((rc = dots(c, dr, h))) return rc;
-    rn = std::sqrt(h[0]);
-    double rho_prev = 1.0, alpha = 1.0, omega = 1.0;
-    while (rn > tol && it < maxiter) {
-      Dots d1{{rh}, {r}, 1};
-      if ((rc = dots(c, d1, h))) return rc;
-      const double rho = h[0];
-      if (rho == 0.0 || !std::isfinite(rho)) break;  // breakdown: report as is
-      const double beta = (rho / rho_prev) * (alpha / omega);
-      axpy(c, 1.0, r, beta, p, -beta * omega, v);   // p = r + beta p - beta omega v
-      prec(c, p, ph);
-      spmv(c, ph, v);
-      Dots d2{{rh}, {v}, 1};
-      if ((rc = dots(c, d2, h))) return rc;
-      if (h[0] == 0.0 || !std::isfinite(h[0])) break;
-      alpha = rho / h[0];
-      TCAD_CUDA_CHECK(cudaMemcpyAsync(sv, r, N * 8, cudaMemcpyDeviceToDevice, s));
-      axpy(c, -alpha, v, 1.0, sv);                   // s = r - alpha v
-      Dots d3{{sv}, {sv}, 1};
-      if ((rc = dots(c, d3, h))) return rc;
-      ++it;
-      if (std::sqrt(h[0]) <= tol) {
-        axpy(c, alpha, ph, 1.0, x);
-        rn = std::sqrt(h[0]);
-        break;
+    spmv(c, x, B.r);
+    axpy(c, 1.0, b, -1.0, B.r);
+    k_cb_start<<<gv, NT, 0, s>>>(B);
+    note_launch();
+    const unsigned gb = g1(c.bs > 1 ? N / c.bs : N);
+    const unsigned gr = (unsigned)std::min<int64_t>(kGridBlocks,
+                                                    (N + kRowsPerBlock - 1) / kRowsPerBlock);
+    BState st;
+    for (int check = 4;; check = std::min(2 * check, 32)) {
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(&st, B.st, sizeof(st), cudaMemcpyDeviceToHost, s));
+      TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+      if (st.done) break;
+      for (int q = 0; q < check; ++q) {
+        k_cb_p<<<gb, NT, 0, s>>>(B, c.bs, c.inv);
+        k_cb_spmv<false><<<gr, NT, 0, s>>>(c.A, B);
+        k_cb_s<<<(unsigned)std::min<int64_t>(kGridBlocks, gb), NT, 0, s>>>(B, c.bs, c.inv);
+        k_cb_spmv<true><<<gr, NT, 0, s>>>(c.A, B);
+        k_cb_x<<<gv, NT, 0, s>>>(B);
+        note_launch(5);
       }
-      prec(c, sv, sh);
-      spmv(c, sh, t);
-      Dots d4{{t, t}, {sv, t}, 2};
-      if ((rc = dots(c, d4, h))) return rc;
-      omega = h[1] > 0.0 ? h[0] / h[1] : 0.0;
-      axpy(c, alpha, ph, 1.0, x, omega, sh);         // x += alpha ph + omega sh
-      TCAD_CUDA_CHECK(cudaMemcpyAsync(r, sv, N * 8, cudaMemcpyDeviceToDevice, s));
-      axpy(c, -omega, t, 1.0, r);                    // r = s - omega t
-      Dots d5{{r}, {r}, 1};
-      if ((rc = dots(c, d5, h))) return rc;
-      rn = std::sqrt(h[0]);
-      rho_prev = rho;
-      if (omega == 0.0) break;
+      TCAD_LAUNCH_CHECK();
     }
+    if (st.done == 2) axpy(c, st.alpha, B.ph, 1.0, x);
+    rn = st.rn;
+    it = st.it;
   } else {
-    double* V = reinterpret_cast<double*>(take((size_t)(m + 1) * N * 8));
-    double* w = reinterpret_cast<double*>(take(N * 8));
+    Gmres G;
+    G.n = N;
+    G.m = m;
+    G.V = reinterpret_cast<double*>(take((size_t)(m + 1) * N * 8));
+    G.w = reinterpret_cast<double*>(take(N * 8));
     double* z = reinterpret_cast<double*>(take(N * 8));
     double* y = reinterpret_cast<double*>(take(N * 8));
-    double* gp = reinterpret_cast<double*>(take((size_t)4096 * (m + 1) * 8));
-    double* hd = c.scal;  // up to m+1 <= 64 scalars
-    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hv(m + 1);
-    double* hdev = nullptr;
-    double* hbuf = nullptr;
-    hdev = reinterpret_cast<double*>(take((size_t)(m + 1) * 8));
-    (void)hd;
-    hbuf = hv.data();
-    const unsigned gb = (unsigned)std::min<int64_t>(4096, (N + NT - 1) / NT);
+    G.partial = reinterpret_cast<double*>(take((size_t)kGridBlocks * (m + 1) * 8));
+    G.R = reinterpret_cast<double*>(take((size_t)m * (m + 1) * 8));
+    double** const vec[5] = {&G.h1, &G.h2, &G.cs, &G.sn, &G.g};
+    for (double** q : vec) *q = reinterpret_cast<double*>(take((size_t)(m + 1) * 8));
+    G.ticket = c.ticket;
+    G.st = reinterpret_cast<GState*>(c.scal + 8);
+    std::vector<double> R((size_t)m * (m + 1)), g(m + 1), yv(m);
+    const unsigned gb = g1(c.bs > 1 ? N / c.bs : N);
     // maxiter counts restart cycles, as scipy's gmres does
     for (int cycle = 0;; ++cycle) {
       // r = b - A x -> V_0
-      spmv(c, x, w);
-      axpy(c, 1.0, b, -1.0, w);
-      Dots dr{{w}, {w}, 1};
+      spmv(c, x, G.w);
+      axpy(c, 1.0, b, -1.0, G.w);
+      Dots dr{{G.w}, {G.w}, 1};
       if ((rc = dots(c, dr, h))) return rc;
       rn = std::sqrt(h[0]);
       if (rn <= tol || cycle >= maxiter || !std::isfinite(rn)) break;
-      k_scale_copy<<<g1(N), NT, 0, s>>>(N, 1.0 / rn, w, V);
-      note_launch();
-      std::fill(g.begin(), g.end(), 0.0);
-      g[0] = rn;
-      int j = 0;
-      for (; j < m; ++j) {
-        prec(c, V + (size_t)j * N, z);
-        spmv(c, z, w);
-        // classical Gram-Schmidt, twice
-        std::vector<double> hj(j + 2, 0.0);
-        for (int pass = 0; pass < 2; ++pass) {
-          k_gs_dots<<<gb, NT, 0, s>>>(N, V, j + 1, w, gp);
-          note_launch();
-          k_gs_sum<<<1, NT, 0, s>>>(gp, (int)gb, j + 1, hdev);
-          note_launch();
-          k_gs_sub<<<g1(N), NT, 0, s>>>(N, V, j + 1, hdev, w);
-          note_launch();
-          TCAD_CUDA_CHECK(cudaMemcpyAsync(hbuf, hdev, sizeof(double) * (j + 1),
-                                          cudaMemcpyDeviceToHost, s));
-          TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
-          for (int i = 0; i <= j; ++i) hj[i] += hbuf[i];
+      k_gm_start<<<1, NT, 0, s>>>(G, rn);
+      k_gm_next<<<gb, NT, 0, s>>>(G, c.bs, c.inv, z);
+      note_launch(2);
+      GState st{0, 0, 0.0};
+      int queued = 0;
+      for (int check = 4; !st.done && st.j < m; check = std::min(2 * check, 32)) {
+        const int todo = std::min(check, m - queued);
+        for (int q = 0; q < todo; ++q) {
+          spmv(c, z, G.w);
+          k_gm_dots<false><<<gv, NTG, 0, s>>>(G);
+          k_gm_dots<true><<<gv, NTG, 0, s>>>(G);
+          k_gm_norm<<<gv, NTG, 0, s>>>(G, tol);
+          k_gm_next<<<gb, NT, 0, s>>>(G, c.bs, c.inv, z);
+          note_launch(4);
         }
-        Dots dw{{w}, {w}, 1};
-        if ((rc = dots(c, dw, h))) return rc;
-        hj[j + 1] = std::sqrt(h[0]);
-        if (hj[j + 1] > 0.0) {
-          k_scale_copy<<<g1(N), NT, 0, s>>>(N, 1.0 / hj[j + 1], w, V + (size_t)(j + 1) * N);
-          note_launch();
-        }
-        // Givens rotations on column j
-        for (int i = 0; i < j; ++i) {
-          const double a = cs[i] * hj[i] + sn[i] * hj[i + 1];
-          hj[i + 1] = -sn[i] * hj[i] + cs[i] * hj[i + 1];
-          hj[i] = a;
-        }
-        const double den = std::hypot(hj[j], hj[j + 1]);
-        cs[j] = den > 0.0 ? hj[j] / den : 1.0;
-        sn[j] = den > 0.0 ? hj[j + 1] / den : 0.0;
-        hj[j] = den;
-        hj[j + 1] = 0.0;
-        g[j + 1] = -sn[j] * g[j];
-        g[j] = cs[j] * g[j];
-        for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = hj[i];
-        ++it;
-        if (std::fabs(g[j + 1]) <= tol || !(den > 0.0)) {
-          ++j;
-          break;
-        }
+        queued += todo;
+        TCAD_LAUNCH_CHECK();
+        TCAD_CUDA_CHECK(cudaMemcpyAsync(&st, G.st, sizeof(st), cudaMemcpyDeviceToHost, s));
+        TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
       }
+      const int j = st.j;
+      it += j;
       // solve the j x j triangle, x += M^-1 (V y)
-      std::vector<double> yv(j, 0.0);
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(R.data(), G.R, sizeof(double) * (size_t)j * (m + 1),
+                                      cudaMemcpyDeviceToHost, s));
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(g.data(), G.g, sizeof(double) * (m + 1),
+                                      cudaMemcpyDeviceToHost, s));
+      TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
       for (int i = j - 1; i >= 0; --i) {
         double sacc = g[i];
-        for (int k = i + 1; k < j; ++k) sacc -= H[(size_t)i * m + k] * yv[k];
-        yv[i] = H[(size_t)i * m + i] != 0.0 ? sacc / H[(size_t)i * m + i] : 0.0;
+        for (int k = i + 1; k < j; ++k) sacc -= R[(size_t)k * (m + 1) + i] * yv[k];
+        const double d = R[(size_t)i * (m + 1) + i];
+        yv[i] = d != 0.0 ? sacc / d : 0.0;
       }
-      TCAD_CUDA_CHECK(cudaMemcpyAsync(hdev, yv.data(), sizeof(double) * j,
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(G.h1, yv.data(), sizeof(double) * j,
                                       cudaMemcpyHostToDevice, s));
-      k_lincomb<<<g1(N), NT, 0, s>>>(N, V, j, hdev, y);
+      k_lincomb<<<g1(N), NT, 0, s>>>(N, G.V, j, G.h1, y);
       note_launch();
       prec(c, y, z);
       axpy(c, 1.0, z, 1.0, x);
