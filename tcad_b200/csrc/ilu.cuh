@@ -21,6 +21,8 @@
 // writes of a level are visible to the block after the barrier).
 #pragma once
 
+#include "async_copy.cuh"
+
 namespace tcad {
 
 constexpr int kIluThreads = 256;
@@ -53,6 +55,30 @@ __device__ __forceinline__ void mul33(const double* A, const double* B, double* 
       C[3 * r + c] = A[3 * r + 0] * B[0 + c] + A[3 * r + 1] * B[3 + c] + A[3 * r + 2] * B[6 + c];
 }
 
+// inv = D^-1; the identity and false when D is singular
+__device__ __forceinline__ bool inverse33(const double* D, double* inv) {
+  const double c00 = D[4] * D[8] - D[5] * D[7];
+  const double c01 = D[5] * D[6] - D[3] * D[8];
+  const double c02 = D[3] * D[7] - D[4] * D[6];
+  const double det = D[0] * c00 + D[1] * c01 + D[2] * c02;
+  if (!(isfinite(det) && fabs(det) >= 1e-300)) {
+#pragma unroll
+    for (int e = 0; e < 9; ++e) inv[e] = (e % 4 == 0) ? 1.0 : 0.0;
+    return false;
+  }
+  const double id = 1.0 / det;
+  inv[0] = c00 * id;
+  inv[1] = (D[2] * D[7] - D[1] * D[8]) * id;
+  inv[2] = (D[1] * D[5] - D[2] * D[4]) * id;
+  inv[3] = c01 * id;
+  inv[4] = (D[0] * D[8] - D[2] * D[6]) * id;
+  inv[5] = (D[2] * D[3] - D[0] * D[5]) * id;
+  inv[6] = c02 * id;
+  inv[7] = (D[1] * D[6] - D[0] * D[7]) * id;
+  inv[8] = (D[0] * D[4] - D[1] * D[3]) * id;
+  return true;
+}
+
 __device__ __forceinline__ void load9(const double* __restrict__ X, int64_t NN, int64_t k,
                                       int e0, double* out) {
 #pragma unroll
@@ -82,13 +108,24 @@ __device__ __forceinline__ void add_nb_vec(const double* b, double v0, double v1
 // node (c, w) -- row c of the shorter side, position w along it -- of the
 // plane whose first node is `base` sits in slot 2*base + (c + w)*Lc + c.
 // A plane with Lc <= Lw rows has (Lc + Lw - 1) Lc <= 2 Lc Lw slots, so the
-// slots of all planes fit in 2 * n_nodes.  Per slot (FP32, a preconditioner
-// needs no more): forward Q, Q G B_walk, Q G B_cross (27 values),
-// backward Q G B_walk', Q G B_cross' (18) -- G folded in, so
+// slots of all planes fit in 2 * n_nodes.  Each sweep has an array of records, one
+// per slot: two 3 x 3 products (FP32, a preconditioner needs no more) --
+// Q G B_walk, Q G B_cross forward, Q G B_walk', Q G B_cross' backward -- and a
+// vector (FP64), so that
 //   forward  a = Q r - (Q G B_walk) a_prev - (Q G B_cross) a_cross
-//   backward x = a - (Q G B_walk') x_next - (Q G B_cross') x_cross'.
-// The right-hand side is permuted into slot order and the result back by
-// two node-parallel kernels.
+//   backward x = a - (Q G B_walk') x_next - (Q G B_cross') x_cross'
+// and all that a level reads is one contiguous run, copied in bulk.  Q r is formed
+// node-parallel while r is permuted into the forward records; the forward sweep
+// leaves a in the backward records and the backward one x in their place.
+constexpr int kIluRec = 28;   // floats of a record (7 x 16 bytes: an odd stride, no
+                              // bank conflicts): 18, 2 of pad, 3 doubles, 1 of pad
+constexpr int kIluVec = 20;   // where the vector starts
+__device__ __forceinline__ double2* ilu_vec(float* M, int64_t slot) {
+  return reinterpret_cast<double2*>(M + slot * kIluRec + kIluVec);
+}
+constexpr int kIluStages = 16;
+constexpr int kIluSweepThreads = 4 * 128 + 32;   // 4 groups of 128 rows, or 2 of 256
+
 struct IluGeo {
   bool byj;      // rows are j (ny <= nx), walk along i
   int Lc, Lw;    // rows, positions per row
@@ -110,48 +147,12 @@ __device__ __forceinline__ int64_t ilu_slot(const IluGeo& q, int i, int j) {
   return q.soff + (int64_t)(c + w) * q.Lc + c;
 }
 
-// store the forward / backward sweep data of node k (FP32, slot order)
-__device__ __forceinline__ void ilu_store_slot(const double* __restrict__ J, int64_t NN,
-                                               int64_t k, const IluGeo& q, int i, int j,
-                                               int nx, int ny, const double* Qk,
-                                               float* __restrict__ Mf, float* __restrict__ Mb,
-                                               int64_t NS) {
-  double G[9], QG[9], b[5], T1[9];
-  load9(J, NN, k, 0, G);
-  mul33(Qk, G, QG);
-  const int64_t sl = ilu_slot(q, i, j);
-  const int c = q.byj ? j : i, w = q.byj ? i : j;
-  // direction indices: W 0, E 1, S 2, N 3
-  const int dwp = q.byj ? 0 : 2, dcp = q.byj ? 2 : 0;
-  const int dwn = q.byj ? 1 : 3, dcn = q.byj ? 3 : 1;
-#pragma unroll
-  for (int e = 0; e < 9; ++e) Mf[(int64_t)e * NS + sl] = (float)Qk[e];
-  const bool has[4] = {w > 0, c > 0, w < q.Lw - 1, c < q.Lc - 1};
-  const int dir[4] = {dwp, dcp, dwn, dcn};
-#pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    if (has[m]) {
-      load_nb(J, NN, k, dir[m], b);
-      mul_dense_nb(QG, b, T1);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 9; ++e) T1[e] = 0.0;
-    }
-    float* dst = m < 2 ? Mf + (int64_t)(9 + 9 * m) * NS : Mb + (int64_t)(9 * (m - 2)) * NS;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) dst[(int64_t)e * NS + sl] = (float)T1[e];
-  }
-  (void)nx; (void)ny;
-}
-
-// r (node order) -> rs (slot order) for the instances preconditioned here;
-// the others' ph = p is written by k_ilu_unperm.
 // Factor: Q_k for every node of each instance whose pre_status is TCAD_OK;
 // status[inst] = TCAD_ERR_SINGULAR when a D~ block is singular.
 __global__ void __launch_bounds__(kIluThreads)
 k_ilu2d_factor(const tcad_pack_t pk, const double* __restrict__ J, double* __restrict__ Q,
                const int32_t* __restrict__ pre_status, int32_t* __restrict__ status,
-               int nzmax, float* __restrict__ Mf, float* __restrict__ Mb) {
+               int nzmax) {
   const int inst = blockIdx.x / nzmax, z = blockIdx.x % nzmax;
   if (pre_status && pre_status[inst] != TCAD_OK) return;
   const Inst g = load_inst(pk, inst);
@@ -196,30 +197,10 @@ k_ilu2d_factor(const tcad_pack_t pk, const double* __restrict__ J, double* __res
       mul33(G, S, D);
 #pragma unroll
       for (int e = 0; e < 9; ++e) D[e] = (e % 4 == 0 ? 1.0 : 0.0) - D[e];
-      const double c00 = D[4] * D[8] - D[5] * D[7];
-      const double c01 = D[5] * D[6] - D[3] * D[8];
-      const double c02 = D[3] * D[7] - D[4] * D[6];
-      const double det = D[0] * c00 + D[1] * c01 + D[2] * c02;
       double inv[9];
-      if (isfinite(det) && fabs(det) >= 1e-300) {
-        const double id = 1.0 / det;
-        inv[0] = c00 * id;
-        inv[1] = (D[2] * D[7] - D[1] * D[8]) * id;
-        inv[2] = (D[1] * D[5] - D[2] * D[4]) * id;
-        inv[3] = c01 * id;
-        inv[4] = (D[0] * D[8] - D[2] * D[6]) * id;
-        inv[5] = (D[2] * D[3] - D[0] * D[5]) * id;
-        inv[6] = c02 * id;
-        inv[7] = (D[1] * D[6] - D[0] * D[7]) * id;
-        inv[8] = (D[0] * D[4] - D[1] * D[3]) * id;
-      } else {
-        if (status) atomicExch(&status[inst], TCAD_ERR_SINGULAR);
-#pragma unroll
-        for (int e = 0; e < 9; ++e) inv[e] = (e % 4 == 0) ? 1.0 : 0.0;
-      }
+      if (!inverse33(D, inv) && status) atomicExch(&status[inst], TCAD_ERR_SINGULAR);
 #pragma unroll
       for (int e = 0; e < 9; ++e) Q[(int64_t)e * NN + k] = inv[e];
-      if (Mf) ilu_store_slot(J, NN, k, ilu_geo(g, base), i, j, nx, ny, inv, Mf, Mb, 2 * NN);
     }
     __syncthreads();
   }
@@ -444,11 +425,107 @@ namespace tcad {
 
 constexpr int NT_ILU_FLAT = 256;  // flat (node-parallel) permutation kernels
 
+// Factor of the 2D instances with slot data: thread c owns row c and walks
+// along it, level by level as the sweeps do.  Its own previous Q G B_walk' is in
+// registers and the row below's Q G B_cross' in shared memory -- the terms of
+// the recursion and, rounded to FP32, the backward records -- and the next
+// position's blocks of J are loaded while this one is worked on.  (Recomputing
+// the neighbours' products from J and Q in global memory at every level took
+// 609 us on a batch of up to 120 x 60 devices, this takes 174.)
+__global__ void __launch_bounds__(kIluThreads)
+k_ilu_factor_rows(const tcad_pack_t pk, const double* __restrict__ J, double* __restrict__ Q,
+                  const int32_t* __restrict__ pre_status, float* __restrict__ Mf,
+                  float* __restrict__ Mb) {
+  const int inst = blockIdx.x;
+  if (pre_status[inst] != TCAD_OK) return;
+  const Inst g = load_inst(pk, inst);
+  const IluGeo q = ilu_geo(g, g.off);
+  const int Lc = q.Lc, Lw = q.Lw, nd = Lc + Lw - 1, c = threadIdx.x;
+  const int64_t NN = pk.n_nodes;
+  // neighbour directions (W 0, E 1, S 2, N 3): along the row and across rows
+  const int dwp = q.byj ? 0 : 2, dcp = q.byj ? 2 : 0, dwn = q.byj ? 1 : 3, dcn = q.byj ? 3 : 1;
+  __shared__ double tn[2][9][kIluThreads];
+  struct Nd {
+    double G[9], b[4][5];
+  };
+  auto node = [&](int w) { return g.off + (q.byj ? (int64_t)c * g.nx + w : (int64_t)w * g.nx + c); };
+  auto valid = [&](int d) { return c < Lc && d - c >= 0 && d - c < Lw; };
+  auto load = [&](int d, Nd& o) {
+    if (!valid(d)) return;
+    const int w = d - c;
+    const int64_t k = node(w);
+    load9(J, NN, k, 0, o.G);
+    const int dir[4] = {dwp, dcp, dwn, dcn};
+    const bool has[4] = {w > 0, c > 0, w < Lw - 1, c < Lc - 1};
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if (has[m]) load_nb(J, NN, k, dir[m], o.b[m]);
+      else
+#pragma unroll
+        for (int e = 0; e < 5; ++e) o.b[m][e] = 0.0;
+    }
+  };
+  double tw[9];   // Q G B_walk' of the previous position
+#pragma unroll
+  for (int e = 0; e < 9; ++e) tw[e] = 0.0;
+  Nd cur;
+  load(0, cur);
+  for (int d = 0; d < nd; ++d) {
+    Nd nxt;
+    load(d + 1, nxt);
+    if (valid(d)) {
+      const int w = d - c;
+      double S[9], T[9], D[9], Qk[9], QG[9];
+      mul_nb_dense(cur.b[0], tw, S);
+      if (c > 0) {
+        double tc[9];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) tc[e] = tn[(d & 1) ^ 1][e][c - 1];
+        mul_nb_dense(cur.b[1], tc, T);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) S[e] += T[e];
+      }
+      mul33(cur.G, S, D);
+#pragma unroll
+      for (int e = 0; e < 9; ++e) D[e] = (e % 4 == 0 ? 1.0 : 0.0) - D[e];
+      inverse33(D, Qk);
+      const int64_t k = node(w);
+#pragma unroll
+      for (int e = 0; e < 9; ++e) Q[(int64_t)e * NN + k] = Qk[e];
+      mul33(Qk, cur.G, QG);
+      float rec[2][kIluVec];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        mul_dense_nb(QG, cur.b[m], T);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+          rec[m >> 1][9 * (m & 1) + e] = (float)T[e];
+          if (m == 2) tw[e] = T[e];
+          if (m == 3) tn[d & 1][e][c] = T[e];
+        }
+      }
+      const int64_t sl = q.soff + (int64_t)d * Lc + c;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        rec[h][18] = rec[h][19] = 0.0f;
+        float4* const dst = reinterpret_cast<float4*>((h ? Mb : Mf) + sl * kIluRec);
+#pragma unroll
+        for (int e = 0; e < kIluVec / 4; ++e)
+          dst[e] = make_float4(rec[h][4 * e], rec[h][4 * e + 1], rec[h][4 * e + 2],
+                               rec[h][4 * e + 3]);
+      }
+    }
+    __syncthreads();
+    cur = nxt;
+  }
+}
+
+// the forward records' vectors = Q r for the instances preconditioned here
 template <class T>
 __global__ void __launch_bounds__(NT_ILU_FLAT)
-k_ilu_perm(const tcad_pack_t pk, const T* __restrict__ r, double* __restrict__ rs,
-           const KState* ks, const uint8_t* __restrict__ mask, const int32_t* __restrict__ blk,
-           int64_t NS) {
+k_ilu_perm(const tcad_pack_t pk, const double* __restrict__ Q, const T* __restrict__ r,
+           float* __restrict__ Mf, const KState* ks, const uint8_t* __restrict__ mask,
+           const int32_t* __restrict__ blk) {
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (ks && !ks[fb.inst].active) return;
@@ -457,21 +534,25 @@ k_ilu_perm(const tcad_pack_t pk, const T* __restrict__ r, double* __restrict__ r
   const IluGeo q = ilu_geo(g, g.off);
   const int64_t NN = pk.n_nodes;
   for (int64_t k = fb.begin + threadIdx.x; k < fb.end; k += NT_ILU_FLAT) {
-    const int64_t loc = k - g.off;
-    const int i = (int)(loc % g.nx), j = (int)(loc / g.nx);
-    const int64_t sl = ilu_slot(q, i, j);
-    rs[sl] = (double)r[k];
-    rs[NS + sl] = (double)r[NN + k];
-    rs[2 * NS + sl] = (double)r[2 * NN + k];
+    const unsigned loc = (unsigned)(k - g.off);
+    const int j = (int)(loc / (unsigned)g.nx), i = (int)(loc - (unsigned)j * (unsigned)g.nx);
+    double Qk[9];
+    load9(Q, NN, k, 0, Qk);
+    const double r0 = (double)r[k], r1 = (double)r[NN + k], r2 = (double)r[2 * NN + k];
+    double2* const dst = ilu_vec(Mf, ilu_slot(q, i, j));
+    dst[0] = make_double2(Qk[0] * r0 + Qk[1] * r1 + Qk[2] * r2,
+                          Qk[3] * r0 + Qk[4] * r1 + Qk[5] * r2);
+    dst[1] = make_double2(Qk[6] * r0 + Qk[7] * r1 + Qk[8] * r2, 0.0);
   }
 }
 
-// out (node order) = xs (slot order); instances not preconditioned: out = r
+// out (node order) = the backward records' vectors; instances not preconditioned:
+// out = r
 template <class T>
 __global__ void __launch_bounds__(NT_ILU_FLAT)
-k_ilu_unperm(const tcad_pack_t pk, const double* __restrict__ xs, const T* __restrict__ r,
+k_ilu_unperm(const tcad_pack_t pk, float* __restrict__ Mb, const T* __restrict__ r,
              T* __restrict__ out, const KState* ks, const uint8_t* __restrict__ mask,
-             const int32_t* __restrict__ blk, int64_t NS) {
+             const int32_t* __restrict__ blk) {
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (ks && !ks[fb.inst].active) return;
@@ -485,140 +566,140 @@ k_ilu_unperm(const tcad_pack_t pk, const double* __restrict__ xs, const T* __res
   const Inst g = load_inst(pk, fb.inst);
   const IluGeo q = ilu_geo(g, g.off);
   for (int64_t k = fb.begin + threadIdx.x; k < fb.end; k += NT_ILU_FLAT) {
-    const int64_t loc = k - g.off;
-    const int i = (int)(loc % g.nx), j = (int)(loc / g.nx);
-    const int64_t sl = ilu_slot(q, i, j);
-    out[k] = (T)xs[sl]; out[NN + k] = (T)xs[NS + sl]; out[2 * NN + k] = (T)xs[2 * NS + sl];
+    const unsigned loc = (unsigned)(k - g.off);
+    const int j = (int)(loc / (unsigned)g.nx), i = (int)(loc - (unsigned)j * (unsigned)g.nx);
+    const double2* const src = ilu_vec(Mb, ilu_slot(q, i, j));
+    const double2 a = src[0], b = src[1];
+    out[k] = (T)a.x; out[NN + k] = (T)a.y; out[2 * NN + k] = (T)b.x;
   }
 }
 
-// The sweeps, one CTA per 2D instance (Lc <= kIluThreads): thread c owns
-// row c.  Level d's data of thread c is slot soff + d Lc + c, so a level's
-// loads are coalesced across the block; they are issued two levels ahead
-// into one of three register sets chosen by d mod 3 (uniform in the block).
-// xs holds a after the forward sweep and x after the backward one.
-__global__ void __launch_bounds__(kIluThreads)
-k_ilu_sweep(const tcad_pack_t pk, const float* __restrict__ Mf, const float* __restrict__ Mb,
-            const double* __restrict__ rs, double* __restrict__ xs, const KState* ks,
-            const uint8_t* __restrict__ mask, int64_t NS) {
+// The sweeps, one CTA per 2D instance (Lc <= rows <= kIluThreads).
+//
+// A sweep is a chain of nx + ny - 1 levels, so what counts is a level's
+// dependent part: the values of the level before from shared memory, five
+// dependent multiply-adds and the store of the result.  Everything else is kept
+// off it:
+// - GROUPS groups of `rows` threads take the levels in turn (thread c of a group:
+//   row c).  Only the group whose turn it is waits for the one before (a named
+//   barrier that the latter arrives at without waiting); the others meanwhile
+//   wait for their next level's records, read them and convert them (18 FP32 to
+//   FP64 conversions a thread: 200 cycles of that pipe, more than the level).
+// - One more warp fills a ring of up to kIluStages levels in shared memory with
+//   bulk copies, one contiguous run a level.
+// Devices of up to 120 x 60, both sweeps: 175 us with one group of 256 threads that loaded
+// two levels ahead into registers from 30 arrays; 54 us now.
+// `ring`: bytes of dynamic shared memory, at least GROUPS levels of the longest Lc.
+template <int GROUPS>
+__global__ void __launch_bounds__(kIluSweepThreads)
+k_ilu_sweep(const tcad_pack_t pk, float* Mf, float* Mb, KState* ks,
+            const uint8_t* __restrict__ mask, int rows, int ring) {
+  extern __shared__ __align__(128) unsigned char s_ring[];
+  __shared__ uint64_t s_full[kIluStages], s_empty[kIluStages];
+  __shared__ double fr[2][3][kIluThreads];
   const int inst = blockIdx.x;
-  if (ks && !ks[inst].active) return;
+  if (!ks[inst].active) return;
   if (mask && !mask[inst]) return;
   const Inst g = load_inst(pk, inst);
   const IluGeo q = ilu_geo(g, g.off);
   const int Lc = q.Lc, Lw = q.Lw, nd = Lc + Lw - 1;
-  const int c = threadIdx.x;
-  const bool lane = c < Lc;
-  __shared__ double fr[2][kIluThreads][3];
-  struct Fd {
-    float q[9], mw[9], mc[9];
-    double r[3];
-  };
-  struct Bd {
-    float mw[9], mc[9];
-    double a[3];
-  };
-  auto valid = [&](int d) { const int w = d - c; return lane && d >= 0 && d < nd && w >= 0 && w < Lw; };
-  auto fload = [&](int d, Fd& o) {
-    if (!valid(d)) return;
-    const int64_t sl = q.soff + (int64_t)d * Lc + c;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      o.q[e] = Mf[(int64_t)e * NS + sl];
-      o.mw[e] = Mf[(int64_t)(9 + e) * NS + sl];
-      o.mc[e] = Mf[(int64_t)(18 + e) * NS + sl];
+  const int level = Lc * kIluRec * (int)sizeof(float);
+  const int D = min(kIluStages, ring / level);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < D; ++i) {
+      mbar_init(&s_full[i]);
+      mbar_init(&s_empty[i], rows / 32);   // one arrival per warp of a group
     }
-    o.r[0] = rs[sl]; o.r[1] = rs[NS + sl]; o.r[2] = rs[2 * NS + sl];
-  };
-  auto bload = [&](int d, Bd& o) {
-    if (!valid(d)) return;
-    const int64_t sl = q.soff + (int64_t)d * Lc + c;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      o.mw[e] = Mb[(int64_t)e * NS + sl];
-      o.mc[e] = Mb[(int64_t)(9 + e) * NS + sl];
-    }
-    o.a[0] = xs[sl]; o.a[1] = xs[NS + sl]; o.a[2] = xs[2 * NS + sl];
-  };
-  double p0 = 0.0, p1 = 0.0, p2 = 0.0;  // own previous result (same row)
-  int cur = 0;
-  auto fstep = [&](int d, const Fd& X) {
-    if (valid(d)) {
-      const int w = d - c;
-      const double* fc = fr[cur ^ 1][c > 0 ? c - 1 : 0];
-      const double c0 = c > 0 ? fc[0] : 0.0, c1 = c > 0 ? fc[1] : 0.0, c2 = c > 0 ? fc[2] : 0.0;
-      const double w0 = w > 0 ? p0 : 0.0, w1 = w > 0 ? p1 : 0.0, w2 = w > 0 ? p2 : 0.0;
-      double a[3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-        a[r] = ((double)X.q[3 * r] * X.r[0] + (double)X.q[3 * r + 1] * X.r[1] +
-                (double)X.q[3 * r + 2] * X.r[2]) -
-               ((double)X.mw[3 * r] * w0 + (double)X.mw[3 * r + 1] * w1 +
-                (double)X.mw[3 * r + 2] * w2) -
-               ((double)X.mc[3 * r] * c0 + (double)X.mc[3 * r + 1] * c1 +
-                (double)X.mc[3 * r + 2] * c2);
-      p0 = a[0]; p1 = a[1]; p2 = a[2];
-      double* f = fr[cur][c];
-      f[0] = a[0]; f[1] = a[1]; f[2] = a[2];
-      const int64_t sl = q.soff + (int64_t)d * Lc + c;
-      xs[sl] = a[0]; xs[NS + sl] = a[1]; xs[2 * NS + sl] = a[2];
-    }
-    __syncthreads();
-    cur ^= 1;
-  };
-  auto bstep = [&](int d, const Bd& X) {
-    if (valid(d)) {
-      const int w = d - c;
-      const double* fc = fr[cur ^ 1][c < Lc - 1 ? c + 1 : c];
-      const bool hc = c < Lc - 1, hw = w < Lw - 1;
-      const double c0 = hc ? fc[0] : 0.0, c1 = hc ? fc[1] : 0.0, c2 = hc ? fc[2] : 0.0;
-      const double w0 = hw ? p0 : 0.0, w1 = hw ? p1 : 0.0, w2 = hw ? p2 : 0.0;
-      double x[3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-        x[r] = X.a[r] -
-               ((double)X.mw[3 * r] * w0 + (double)X.mw[3 * r + 1] * w1 +
-                (double)X.mw[3 * r + 2] * w2) -
-               ((double)X.mc[3 * r] * c0 + (double)X.mc[3 * r + 1] * c1 +
-                (double)X.mc[3 * r + 2] * c2);
-      p0 = x[0]; p1 = x[1]; p2 = x[2];
-      double* f = fr[cur][c];
-      f[0] = x[0]; f[1] = x[1]; f[2] = x[2];
-      const int64_t sl = q.soff + (int64_t)d * Lc + c;
-      xs[sl] = x[0]; xs[NS + sl] = x[1]; xs[2 * NS + sl] = x[2];
-    }
-    __syncthreads();
-    cur ^= 1;
-  };
-  {  // forward, levels 0 .. nd-1, data two levels ahead
-    Fd S0, S1, S2;
-    fload(0, S0);
-    fload(1, S1);
-    for (int d = 0; d < nd; d += 3) {
-      fload(d + 2, S2);
-      fstep(d, S0);
-      if (d + 1 >= nd) break;
-      fload(d + 3, S0);
-      fstep(d + 1, S1);
-      if (d + 2 >= nd) break;
-      fload(d + 4, S1);
-      fstep(d + 2, S2);
-    }
+    fence_async();
   }
-  {  // backward, levels nd-1 .. 0
-    Bd S0, S1, S2;
-    bload(nd - 1, S0);
-    bload(nd - 2, S1);
-    for (int d = nd - 1; d >= 0; d -= 3) {
-      bload(d - 2, S2);
-      bstep(d, S0);
-      if (d - 1 < 0) break;
-      bload(d - 3, S0);
-      bstep(d - 1, S1);
-      if (d - 2 < 0) break;
-      bload(d - 4, S1);
-      bstep(d - 2, S2);
+  for (int i = threadIdx.x; i < 2 * 3 * kIluThreads; i += blockDim.x) (&fr[0][0][0])[i] = 0.0;
+  __syncthreads();
+  bool lost = false;
+  unsigned tries = kMbarTries;
+  auto wait = [&](uint64_t* b, unsigned parity) {
+    if (!mbar_wait(b, parity, tries)) {
+      lost = true;
+      tries = kMbarFewTries;
     }
+  };
+  const int grp = threadIdx.x / rows;             // GROUPS: the copying warp
+  const int c = threadIdx.x - grp * rows, lane = threadIdx.x & 31;
+  auto sweep = [&](bool fwd, int base) {          // base: levels of the ring used so far
+    auto at = [&](int s) { return fwd ? s : nd - 1 - s; };
+    if (grp == GROUPS) {
+      if (lane != 0) return;
+      const float* const M = fwd ? Mf : Mb;
+      int st = base % D;
+      unsigned par = (base / D) & 1;
+      for (int s = 0; s < nd; ++s) {
+        wait(&s_empty[st], par ^ 1u);             // the first round finds them empty
+        mbar_expect(&s_full[st], level);
+        bulk_copy(s_ring + st * level, M + (q.soff + (int64_t)at(s) * Lc) * kIluRec, level,
+                  &s_full[st]);
+        if (++st == D) { st = 0; par ^= 1u; }
+      }
+      return;
+    }
+    const int cn = fwd ? max(c - 1, 0) : min(c + 1, Lc - 1);   // (its record is 0 at the edge)
+    int st = (base + grp) % D;
+    unsigned par = ((base + grp) / D) & 1;
+    for (int s = grp; s < nd; s += GROUPS) {
+      const int w = at(s) - c;
+      const bool mine = c < Lc && w >= 0 && w < Lw;
+      wait(&s_full[st], par);
+      double mw[9], mc[9], a[3];
+      if (mine) {
+        const float4* const m4 =
+            reinterpret_cast<const float4*>(s_ring + st * level + c * 4 * kIluRec);
+        float f[kIluVec];
+#pragma unroll
+        for (int e = 0; e < kIluVec / 4; ++e) {
+          const float4 v = m4[e];
+          f[4 * e] = v.x; f[4 * e + 1] = v.y; f[4 * e + 2] = v.z; f[4 * e + 3] = v.w;
+        }
+#pragma unroll
+        for (int e = 0; e < 9; ++e) { mw[e] = (double)f[e]; mc[e] = (double)f[9 + e]; }
+        const double2* const r2 = reinterpret_cast<const double2*>(m4 + kIluVec / 4);
+        const double2 u = r2[0], v = r2[1];
+        a[0] = u.x; a[1] = u.y; a[2] = v.x;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_empty[st]);
+      st += GROUPS;
+      if (st >= D) { st -= D; par ^= 1u; }
+      // level s - 1 is in fr (its group arrived; the first level has none)
+      if (s > 0)
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + s % GROUPS), "r"(2 * rows) : "memory");
+      if (mine) {
+        const double(*const f)[kIluThreads] = fr[(s & 1) ^ 1];
+        const double p0 = f[0][c], p1 = f[1][c], p2 = f[2][c];
+        const double x0 = f[0][cn], x1 = f[1][cn], x2 = f[2][cn];
+        const bool first = fwd ? w == 0 : w == Lw - 1;   // no position before this one
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          const double ow = mw[3 * e] * p0 + mw[3 * e + 1] * p1 + mw[3 * e + 2] * p2;
+          const double ox = mc[3 * e] * x0 + mc[3 * e + 1] * x1 + mc[3 * e + 2] * x2;
+          a[e] = (a[e] - (first ? 0.0 : ow)) - ox;
+          fr[s & 1][e][c] = a[e];
+        }
+      }
+      if (s + 1 < nd)
+        asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s + 1) % GROUPS), "r"(2 * rows) : "memory");
+      if (mine) {
+        double2* const dst = ilu_vec(Mb, q.soff + (int64_t)at(s) * Lc + c);
+        dst[0] = make_double2(a[0], a[1]);
+        dst[1] = make_double2(a[2], 0.0);
+      }
+    }
+  };
+  sweep(true, 0);
+  __threadfence();
+  fence_async();   // the forward results, before the bulk copies that read them
+  __syncthreads();
+  sweep(false, nd);
+  if (lost) {
+    ks[inst].status = TCAD_ERR_CUDA;
+    ks[inst].active = 0;
   }
 }
 

@@ -1374,16 +1374,15 @@ struct WorkIlu {
   double* sh;
   uint8_t* mask;    // instances preconditioned with ILU(0)
   int32_t* pre;     // factor pre-status (-1: skip)
-  float* Mf;        // 2D: forward sweep data in anti-diagonal slot order [27][2n]
-  float* Mb;        //     backward sweep data [18][2n]
-  double* rs;       //     right-hand side in slot order [3][2n]
-  double* xs;       //     sweep result in slot order [3][2n]
+  float* Mf;        // 2D: forward sweep records in anti-diagonal slot order [2n][kIluRec]
+  float* Mb;        //     backward sweep records
+  int rows;         //     longest shorter side of the pack (Mf non-null)
   size_t bytes;
 };
 
 static WorkIlu carve_ilu(const tcad_pack_t* pk, void* base) {
   Carve c{reinterpret_cast<char*>(base), 0, 0};
-  WorkIlu w{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
+  WorkIlu w{};
   const size_t v3 = 3 * (size_t)pk->n_nodes;
   w.Q = c.take<double>(9 * (size_t)pk->n_nodes);
   w.ph = c.take<double>(v3);
@@ -1392,10 +1391,8 @@ static WorkIlu carve_ilu(const tcad_pack_t* pk, void* base) {
   w.pre = c.take<int32_t>(pk->n_inst);
   if (pk->dim == 2) {
     const size_t ns = 2 * (size_t)pk->n_nodes;
-    w.Mf = c.take<float>(27 * ns);
-    w.Mb = c.take<float>(18 * ns);
-    w.rs = c.take<double>(3 * ns);
-    w.xs = c.take<double>(3 * ns);
+    w.Mf = c.take<float>(kIluRec * ns);
+    w.Mb = c.take<float>(kIluRec * ns);
   }
   w.bytes = c.used;
   return w;
@@ -1598,6 +1595,11 @@ static Work carve(const tcad_pack_t* pk, void* base, size_t cap) {
   return w;
 }
 
+// Threads per group and ring of the slot-order sweeps for shorter sides of up to
+// `rows`: a dozen levels ahead, as far as shared memory goes (6 for 256 rows)
+static int ilu_rows(int rows) { return (rows + 31) / 32 * 32; }
+static int ilu_ring(int rows) { return std::min(12 * rows * kIluRec * 4, 200 << 10); }
+
 // out = M^-1 r: the coalesced slot-order sweeps when the factor wrote them
 // (2D, every shorter side <= kIluThreads), else the node-order sweeps
 template <class T>
@@ -1607,11 +1609,15 @@ static void ilu_apply_t(const tcad_pack_t* pk, const double* J, const double* Q,
                         cudaStream_t s) {
   const int ni = pk->n_inst;
   if (ilc && ilc->Mf) {
-    const int64_t NS = 2 * pk->n_nodes;
-    k_ilu_perm<T><<<ng, NT_ILU_FLAT, 0, s>>>(*pk, r, ilc->rs, w.ks, mask, dlist, NS);
-    k_ilu_sweep<<<(unsigned)ni, kIluThreads, 0, s>>>(*pk, ilc->Mf, ilc->Mb, ilc->rs, ilc->xs,
-                                                     w.ks, mask, NS);
-    k_ilu_unperm<T><<<ng, NT_ILU_FLAT, 0, s>>>(*pk, ilc->xs, r, out, w.ks, mask, dlist, NS);
+    k_ilu_perm<T><<<ng, NT_ILU_FLAT, 0, s>>>(*pk, Q, r, ilc->Mf, w.ks, mask, dlist);
+    const int rows = ilu_rows(ilc->rows), ring = ilu_ring(ilc->rows);
+    if (rows <= 128)
+      k_ilu_sweep<4><<<(unsigned)ni, 4 * rows + 32, ring, s>>>(*pk, ilc->Mf, ilc->Mb, w.ks, mask,
+                                                               rows, ring);
+    else
+      k_ilu_sweep<2><<<(unsigned)ni, 2 * rows + 32, ring, s>>>(*pk, ilc->Mf, ilc->Mb, w.ks, mask,
+                                                               rows, ring);
+    k_ilu_unperm<T><<<ng, NT_ILU_FLAT, 0, s>>>(*pk, ilc->Mb, r, out, w.ks, mask, dlist);
     note_launch(3);
     return;
   }
@@ -1815,7 +1821,10 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
                                     cudaMemcpyDeviceToHost, s));
     TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
     bool any = false;
-    for (int i = 0; i < ni; ++i) any = any || hks[i].active;
+    for (int i = 0; i < ni; ++i) {
+      if (hks[i].status == TCAD_ERR_CUDA) return TCAD_ERR_CUDA;   // a sweep lost a copy
+      any = any || hks[i].active;
+    }
     if (any)
       if (int rc = grid.update(hks, w.blk, s)) return rc;
     if (!any) {
@@ -2529,7 +2538,7 @@ extern "C" int tcad_block_ilu_setup(const tcad_pack_t* pk, const double* J, doub
   const int nzm = pack_nzmax(pk, (cudaStream_t)stream);
   if (nzm < 1) return TCAD_ERR_CUDA;
   k_ilu2d_factor<<<(unsigned)(pk->n_inst * nzm), kIluThreads, 0, (cudaStream_t)stream>>>(
-      *pk, J, Q, nullptr, status, nzm, nullptr, nullptr);
+      *pk, J, Q, nullptr, status, nzm);
   note_launch();
   TCAD_LAUNCH_CHECK();
   return TCAD_OK;
@@ -2656,10 +2665,17 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
   const WorkIlu wilu = use_ilu ? carve_ilu(pk, reinterpret_cast<char*>(work) +
                                                    ((w.bytes + 255) & ~(size_t)255) +
                                                    ((w32.bytes + 255) & ~(size_t)255))
-                               : WorkIlu{nullptr, nullptr, nullptr, nullptr, nullptr,
-                                         nullptr, nullptr, nullptr, nullptr, 0};
+                               : WorkIlu{};
   WorkIlu wilu_use = wilu;
-  if (use_ilu && (pk->dim != 2 || pack_max_short_side(pk, s) > kIluThreads)) {
+  if (use_ilu && pk->dim == 2) wilu_use.rows = pack_max_short_side(pk, s);
+  const auto sweeps_ready = [] {
+    return cudaFuncSetAttribute(k_ilu_sweep<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                ilu_ring(kIluThreads)) == cudaSuccess &&
+           cudaFuncSetAttribute(k_ilu_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                ilu_ring(kIluThreads)) == cudaSuccess;
+  };
+  if (use_ilu && (pk->dim != 2 || wilu_use.rows > kIluThreads || !sweeps_ready())) {
+    (void)cudaGetLastError();
     wilu_use.Mf = nullptr;  // node-order sweeps
     wilu_use.Mb = nullptr;
   }
@@ -2863,8 +2879,12 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
         TCAD_CUDA_CHECK(cudaMemcpyAsync(wilu.pre, pre.data(), sizeof(int32_t) * ni,
                                         cudaMemcpyHostToDevice, s));
         TCAD_CUDA_CHECK(cudaMemcpyAsync(wilu.mask, msk.data(), ni, cudaMemcpyHostToDevice, s));
-        k_ilu2d_factor<<<(unsigned)(ni * nzmax), kIluThreads, 0, s>>>(
-            *pk, J, wilu.Q, wilu.pre, nullptr, nzmax, wilu_use.Mf, wilu_use.Mb);
+        if (wilu_use.Mf)
+          k_ilu_factor_rows<<<(unsigned)ni, ilu_rows(wilu_use.rows), 0, s>>>(
+              *pk, J, wilu.Q, wilu.pre, wilu_use.Mf, wilu_use.Mb);
+        else
+          k_ilu2d_factor<<<(unsigned)(ni * nzmax), kIluThreads, 0, s>>>(*pk, J, wilu.Q, wilu.pre,
+                                                                       nullptr, nzmax);
         note_launch();
         TCAD_LAUNCH_CHECK();
       }

@@ -47,27 +47,6 @@ constexpr size_t rb_stream_smem() {
   return (size_t)(NTS / 32) * Stencil<DIM>::NE * 32 * sizeof(double);
 }
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* b) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
-}
-
-// bulk copy of n bytes (a multiple of 16) global -> shared, completing on b
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned n, uint64_t* b,
-                                          uint64_t policy) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)),
-               "r"(n)
-               : "memory");
-  asm volatile(
-      "cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes.L2::cache_hint "
-      "[%0], [%1], %2, [%3], %4;" ::"r"(smem_addr(dst)),
-      "l"(src), "r"(n), "r"(smem_addr(b)), "l"(policy)
-      : "memory");
-}
-
 // J of more than this many bytes is read evict-first; less stays in L2 (126 MB)
 // from one pass to the next along with the vectors
 constexpr int64_t kRbKeepBytes = (int64_t)80 << 20;
@@ -79,23 +58,6 @@ __device__ __forceinline__ uint64_t stream_policy(bool keep) {
   else
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
-}
-
-// wait for the phase, at most `tries` polls (each suspends for a while)
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity, unsigned tries) {
-  const unsigned a = smem_addr(b);
-  for (unsigned i = 0; i < tries; ++i) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
 }
 
 // rb_couple_f on gathered values xv[d][c]; Jt: the slot's column of its tile
@@ -162,11 +124,11 @@ struct RbStreamer {
     pend = -1;
     pcol = 0;
     phase = 0u;
-    tries = 1u << 20;
+    tries = kMbarTries;
     lost = false;
     if (lane == 0) {
       mbar_init(&sh.bar[warp]);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      fence_async();
     }
     __syncwarp();
   }
@@ -178,14 +140,17 @@ struct RbStreamer {
     if (warp * 32 >= q.len) return;
     pend = q.id;
     pcol = col;
-    if (lane == 0)
-      bulk_load(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32),
-                NE * 32 * sizeof(double), &sh.bar[warp], policy);
+    if (lane == 0) {
+      constexpr unsigned n = NE * 32 * sizeof(double);
+      mbar_expect(&sh.bar[warp], n);
+      bulk_copy(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32), n, &sh.bar[warp],
+                policy);
+    }
   }
   __device__ __forceinline__ void arrive() {
     if (!mbar_wait(&sh.bar[warp], phase, tries)) {
       lost = true;
-      tries = 64u;
+      tries = kMbarFewTries;
     }
     phase ^= 1u;
     pend = -1;
