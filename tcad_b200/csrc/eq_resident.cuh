@@ -22,8 +22,7 @@ __global__ void __launch_bounds__(NT, 1)
 k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ J,
                 const double* __restrict__ F, double* __restrict__ d, double* zg, double* pg,
                 double* xg, double* Tr, KState* ks, double* part, unsigned* bar, double rtol,
-                int maxit, const uint8_t* __restrict__ active,
-                const double* __restrict__ rtol_inst) {
+                int maxit, const double* __restrict__ rtol_inst) {
   constexpr int NE = 1 + 2 * DIM, ND = 2 * DIM;
   extern __shared__ __align__(16) double s_rows[];   // [2][NE][flat_nodes]
   GridSync gs;
@@ -126,8 +125,7 @@ k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict_
     sum[1] += bv * bv;
   }
   if (!gs.sum<2>(sum, tot)) return;
-  fin_cg_init(S, tot[0], tot[1], rtol_inst ? rtol_inst[inst] : rtol, maxit,
-              !active || active[inst]);
+  fin_cg_init(S, tot[0], tot[1], rtol_inst ? rtol_inst[inst] : rtol, maxit, true);
   S.beta = 0.0;   // the first direction is z: p = z + 0 * 0
   while (S.active) {
     const double beta = S.beta;

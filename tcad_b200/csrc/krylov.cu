@@ -798,6 +798,11 @@ k_bicgstab_fused(const tcad_pack_t pk, const double* __restrict__ J,
   if (blockIdx.x == 0 && threadIdx.x == 0) ks[inst] = S;
 }
 
+// a Krylov solve that another preconditioner may still finish
+__host__ __device__ __forceinline__ bool solve_failed(int32_t status) {
+  return status == TCAD_ERR_NOCONV || status == TCAD_ERR_BREAKDOWN;
+}
+
 // --------------------------------------------------------------------------
 // Newton update (device2d.py:2079-2100): per-instance max update into err
 __global__ void __launch_bounds__(NT)
@@ -805,9 +810,15 @@ k_newton_update(const tcad_pack_t pk, double* __restrict__ psi, double* __restri
                 double* __restrict__ pp, const double* __restrict__ du, double max_dpsi,
                 double floor_, const uint8_t* __restrict__ active,
                 unsigned long long* __restrict__ err, int relative, int dry, double sfloor,
-                const double* __restrict__ sfloor_inst = nullptr) {
+                const double* __restrict__ sfloor_inst = nullptr,
+                const unsigned* __restrict__ bar = nullptr,
+                const KState* __restrict__ keep_failed = nullptr) {
   const FlatBlock fb = flat_block(pk, blockIdx.x);
   if (active && !active[fb.inst]) return;
+  // queued behind a single-launch solve whose result the host has not seen:
+  // no step when a wait of it gave up, or when a failed solve is to be retried
+  if (bar && bar[2] != 0u) return;
+  if (keep_failed && solve_failed(keep_failed[fb.inst].status)) return;
   if (sfloor_inst) sfloor = sfloor_inst[fb.inst];  // the floor the step was scaled with
   __shared__ double sm[32];
   const int64_t NN = pk.n_nodes;
@@ -1179,9 +1190,10 @@ namespace tcad {
 __global__ void __launch_bounds__(NT)
 k_eq_update(const tcad_pack_t pk, double* __restrict__ psi, const double* __restrict__ d,
             double max_dpsi, const uint8_t* __restrict__ active,
-            unsigned long long* __restrict__ err) {
+            unsigned long long* __restrict__ err, const unsigned* __restrict__ bar = nullptr) {
   const FlatBlock fb = flat_block(pk, blockIdx.x);
   if (active && !active[fb.inst]) return;
+  if (bar && bar[2] != 0u) return;   // the queued solve before it gave up
   __shared__ double sm[32];
   double e = 0.0;
   for (int64_t k = fb.begin + threadIdx.x; k < fb.end; k += NT) {
@@ -1581,7 +1593,7 @@ static Work carve(const tcad_pack_t* pk, void* base, size_t cap) {
   w.cg.p = w.bi.r + 2 * pk->n_nodes;
   w.cg.q = w.bi.rh;
   w.partial = c.take<double>(8 * (size_t)pk->n_flat);
-  w.bar = c.take<unsigned>(4);
+  w.bar = c.take<unsigned>(4);   // bar .. sfl: one run (StepControl)
   w.ks = c.take<KState>(pk->n_inst);
   w.ticket = c.take<unsigned>(pk->n_inst);
   w.status = c.take<int32_t>(pk->n_inst);
@@ -1850,19 +1862,60 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
   return TCAD_OK;
 }
 
-// Launch configuration of a cooperative single-launch solve, its barrier
-// flags cleared (and the give-up test hook set)
+// The host's image of the run bar .. sfl of a single-instance workspace: what a
+// Newton step sets before its kernels (one copy up) and reads after them (one
+// copy down), so that the step has one synchronisation
+struct StepControl {
+  std::vector<unsigned char> img;
+  unsigned char* dev;
+  explicit StepControl(const Work& w)
+      : img(reinterpret_cast<unsigned char*>(w.sfl + 1) -
+            reinterpret_cast<unsigned char*>(w.bar)),
+        dev(reinterpret_cast<unsigned char*>(w.bar)) {}
+  template <class T>
+  T& at(const T* field) {
+    return *reinterpret_cast<T*>(img.data() + (reinterpret_cast<const unsigned char*>(field) - dev));
+  }
+  int up(cudaStream_t s) {
+    TCAD_CUDA_CHECK(cudaMemcpyAsync(dev, img.data(), img.size(), cudaMemcpyHostToDevice, s));
+    return TCAD_OK;
+  }
+  int down(cudaStream_t s) {
+    TCAD_CUDA_CHECK(cudaMemcpyAsync(img.data(), dev, img.size(), cudaMemcpyDeviceToHost, s));
+    TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+    return TCAD_OK;
+  }
+  // barrier flags and status cleared, the give-up test hook set
+  void clear(const Work& w) {
+    std::fill(img.begin(), img.end(), (unsigned char)0);
+    at(w.bar + 3) = g_fused_test_hold.load() ? 1u : 0u;
+  }
+};
+
+// JR, JB <- the colour rows of the prepared J
+static void rb_pack(const tcad_pack_t* pk, const RbLayout& L, const WorkRb& wr, const double* J,
+                    cudaStream_t s) {
+  const unsigned nbb = (unsigned)L.pkb.n_flat;
+  if (pk->dim == 2) k_rb_pack<2><<<nbb, NT, 0, s>>>(L.pkb, L.mp, J, wr.JR, wr.JB);
+  else              k_rb_pack<3><<<nbb, NT, 0, s>>>(L.pkb, L.mp, J, wr.JR, wr.JB);
+  note_launch();
+}
+
+// Launch configuration of a cooperative single-launch solve; clear: its barrier
+// flags cleared (and the give-up test hook set) first
 struct CoopLaunch {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
 };
 static int coop_launch(CoopLaunch& c, unsigned blocks, unsigned threads, size_t smem,
-                       unsigned* flags, cudaStream_t s) {
-  TCAD_CUDA_CHECK(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned), s));
-  if (g_fused_test_hold.load()) {
-    static const unsigned kPhantom = 1u;
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(flags + 3, &kPhantom, sizeof(unsigned),
-                                    cudaMemcpyHostToDevice, s));
+                       unsigned* flags, bool clear, cudaStream_t s) {
+  if (clear) {
+    TCAD_CUDA_CHECK(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned), s));
+    if (g_fused_test_hold.load()) {
+      static const unsigned kPhantom = 1u;
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(flags + 3, &kPhantom, sizeof(unsigned),
+                                      cudaMemcpyHostToDevice, s));
+    }
   }
   c.cfg.gridDim = dim3(blocks);
   c.cfg.blockDim = dim3(threads);
@@ -1891,14 +1944,14 @@ static int coop_result(const Work& w, int ni, std::vector<KState>& hks, cudaStre
   return TCAD_OK;
 }
 
-// k_bicgstab_rb_resident over the slot pack's blocks.  Returns TCAD_OK with
-// hks[0] filled, or 1 when the launch was refused or a wait gave up.
+// k_bicgstab_rb_resident over the slot pack's blocks, queued: 1 when the launch
+// was refused.  Jn: J in node order (a solve with its rows in shared memory
+// takes them from there), null: the packed colour rows.  clear: see coop_launch.
 template <int DIM, int K, bool JS>
-static int launch_rb_resident_t(const tcad_pack_t* pk, const RbLayout& L, const WorkRb& wr,
-                                const double* b, double* x, double rtol, int maxiter,
-                                const Work& w, const int32_t* pre_status,
-                                std::vector<KState>& hks, cudaStream_t s,
-                                const double* rtol_inst) {
+static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double* Jn,
+                               const double* b, double* x, double rtol, int maxiter,
+                               const Work& w, const int32_t* pre_status, bool clear,
+                               cudaStream_t s, const double* rtol_inst) {
   const auto kern = k_bicgstab_rb_resident<DIM, K, JS>;
   const size_t smem = JS ? (size_t)L.pkb.flat_nodes * Stencil<DIM>::NE * 16 : 0;
   if (JS && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1907,39 +1960,45 @@ static int launch_rb_resident_t(const tcad_pack_t* pk, const RbLayout& L, const 
     return 1;
   }
   CoopLaunch c;
-  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, s)) return rc;
+  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, clear, s)) return rc;
   const BiVec& bi = w.bi;
   const int rechecks = 8;
   // (a cooperative launch that does not fit is refused, not run)
-  if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, (const double*)wr.JR, (const double*)wr.JB,
-                         b, x, wr.bR, wr.tR, wr.xb, wr.rhs, bi.r, bi.p, bi.v, w.ks, wr.sync,
+  if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, Jn, (const double*)wr.JR,
+                         (const double*)wr.JB, b, x, wr.bR, wr.tR, wr.xb, wr.rhs, bi.r, bi.p, bi.v, w.ks, wr.sync,
                          w.bar, rtol, maxiter, pre_status, rtol_inst, rechecks) != cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
   note_launch();
-  return coop_result(w, 1, hks, s);
+  return TCAD_OK;
 }
 
-static int launch_bicgstab_rb_resident(const tcad_pack_t* pk, const RbLayout& L,
-                                       const WorkRb& wr, const double* b, double* x,
-                                       double rtol, int maxiter, const Work& w,
-                                       const int32_t* pre_status, std::vector<KState>& hks,
-                                       cudaStream_t s, const double* rtol_inst) {
+// whether a resident solve takes the pack, and whether it holds J's rows
+static bool rb_resident(const tcad_pack_t* pk, const RbLayout& L) {
+  return pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
+         L.pkb.flat_nodes <= kRbResidentMaxSlots && g_fused_mode.load();
+}
+static bool rb_resident_js(const tcad_pack_t* pk, const RbLayout& L) {
+  return L.pkb.flat_nodes <= rb_resident_js_slots(pk->dim == 2 ? TCAD_NE2 : TCAD_NE3);
+}
+
+static int queue_rb_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkRb& wr,
+                             const double* Jn, const double* b, double* x, double rtol,
+                             int maxiter, const Work& w, const int32_t* pre_status, bool clear,
+                             cudaStream_t s, const double* rtol_inst) {
   const int fn = L.pkb.flat_nodes;
-  if (fn > kRbResidentMaxSlots || fn % 32) return 1;
-  const bool d2 = pk->dim == 2;
-  const bool js = fn <= rb_resident_js_slots(d2 ? TCAD_NE2 : TCAD_NE3);
+  const bool js = rb_resident_js(pk, L);
   auto go = [&](auto fnc) {
-    return fnc(pk, L, wr, b, x, rtol, maxiter, w, pre_status, hks, s, rtol_inst);
+    return fnc(L, wr, Jn, b, x, rtol, maxiter, w, pre_status, clear, s, rtol_inst);
   };
-  if (d2)
-    return fn <= NT ? go(launch_rb_resident_t<2, 1, true>)
-           : js     ? go(launch_rb_resident_t<2, 2, true>)
-                    : go(launch_rb_resident_t<2, 2, false>);
-  return fn <= NT ? go(launch_rb_resident_t<3, 1, true>)
-         : js     ? go(launch_rb_resident_t<3, 2, true>)
-                  : go(launch_rb_resident_t<3, 2, false>);
+  if (pk->dim == 2)
+    return fn <= NT ? go(queue_rb_resident_t<2, 1, true>)
+           : js     ? go(queue_rb_resident_t<2, 2, true>)
+                    : go(queue_rb_resident_t<2, 2, false>);
+  return fn <= NT ? go(queue_rb_resident_t<3, 1, true>)
+         : js     ? go(queue_rb_resident_t<3, 2, true>)
+                  : go(queue_rb_resident_t<3, 2, false>);
 }
 
 static int sm_count() {
@@ -2037,12 +2096,12 @@ struct RbStreamLauncher {
 // per-instance stopping test ||b - A^ x|| <= rtol ||b|| as launch_bicgstab_t,
 // the same vector kernels on the black slot pack, and the full solution x
 // (node layout) at the end.  JR / JB must hold the colour rows of the current
-// J (k_rb_pack after the block-Jacobi set-up).
+// J (k_rb_pack after the block-Jacobi set-up).  per_step: no single launch.
 static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkRb& wr,
                               const double* b, double* x, double rtol, int maxiter,
                               const Work& w, const int32_t* pre_status,
                               std::vector<KState>& hks, cudaStream_t s,
-                              const double* rtol_inst) {
+                              const double* rtol_inst, bool per_step = false) {
   const tcad_pack_t& pkb = L.pkb;
   const unsigned nbb = (unsigned)pkb.n_flat;
   const int ni = pk->n_inst;
@@ -2050,9 +2109,10 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
   BiVec bi = w.bi;   // black vectors (stride: the slot count)
   bi.ph = bi.p;
   bi.sh = bi.s;
-  if (g_fused_mode.load() && ni == 1 && (int64_t)nbb <= kRbResidentCtas &&
-      launch_bicgstab_rb_resident(pk, L, wr, b, x, rtol, maxiter, w, pre_status, hks, s,
-                                  rtol_inst) == TCAD_OK)
+  if (rb_resident(pk, L) && !per_step &&
+      queue_rb_resident(pk, L, wr, nullptr, b, x, rtol, maxiter, w, pre_status, true, s,
+                        rtol_inst) == TCAD_OK &&
+      coop_result(w, 1, hks, s) == TCAD_OK)
     return TCAD_OK;
   // J streamed through shared memory where the pack is larger than one wave
   // of blocks and every block starts on a warp tile
@@ -2301,14 +2361,12 @@ static int launch_cg(const tcad_pack_t* pk, const double* J, const double* b, do
   return TCAD_OK;
 }
 
-// k_eqrb_resident over the slot pack's blocks: TCAD_OK with hks[0] filled, or 1
-// when the launch was refused or a wait gave up
+// k_eqrb_resident over the slot pack's blocks, queued with its barrier flags
+// cleared by the caller: 1 when the launch was refused
 template <int DIM, int K>
-static int launch_eq_resident_t(const RbLayout& L, const WorkEq& we, const double* J,
-                                const double* b, double* d, double rtol, int maxiter,
-                                const Work& w, const uint8_t* active,
-                                std::vector<KState>& hks, cudaStream_t s,
-                                const double* rtol_inst) {
+static int queue_eq_resident_t(const RbLayout& L, const WorkEq& we, const double* J,
+                               const double* b, double* d, double rtol, int maxiter,
+                               const Work& w, cudaStream_t s, const double* rtol_inst) {
   const auto kern = k_eqrb_resident<DIM, K>;
   const size_t smem = (size_t)L.pkb.flat_nodes * (1 + 2 * DIM) * 16;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -2317,35 +2375,36 @@ static int launch_eq_resident_t(const RbLayout& L, const WorkEq& we, const doubl
     return 1;
   }
   CoopLaunch c;
-  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, s)) return rc;
+  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, false, s)) return rc;
   if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, J, b, d, w.cg.z, w.cg.p, we.xb, we.tR, w.ks,
-                         we.sync, w.bar, rtol, maxiter, active, rtol_inst) != cudaSuccess) {
+                         we.sync, w.bar, rtol, maxiter, rtol_inst) != cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
   note_launch();
-  return coop_result(w, 1, hks, s);
+  return TCAD_OK;
 }
 
-static int launch_eq_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& we,
-                              const double* J, const double* b, double* d, double rtol,
-                              int maxiter, const Work& w, const uint8_t* active,
-                              std::vector<KState>& hks, cudaStream_t s,
-                              const double* rtol_inst) {
+static bool eq_resident(const tcad_pack_t* pk, const RbLayout& L) {
+  return pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
+         L.pkb.flat_nodes <= kEqResidentMaxSlots && g_fused_mode.load();
+}
+
+static int queue_eq_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& we,
+                             const double* J, const double* b, double* d, double rtol,
+                             int maxiter, const Work& w, cudaStream_t s,
+                             const double* rtol_inst) {
   const int fn = L.pkb.flat_nodes;
-  if (fn > kEqResidentMaxSlots) return 1;
-  auto go = [&](auto fnc) {
-    return fnc(L, we, J, b, d, rtol, maxiter, w, active, hks, s, rtol_inst);
-  };
+  auto go = [&](auto fnc) { return fnc(L, we, J, b, d, rtol, maxiter, w, s, rtol_inst); };
   if (pk->dim == 2)
-    return fn <= NT       ? go(launch_eq_resident_t<2, 1>)
-           : fn <= 2 * NT ? go(launch_eq_resident_t<2, 2>)
-           : fn <= 4 * NT ? go(launch_eq_resident_t<2, 4>)
-                          : go(launch_eq_resident_t<2, 8>);
-  return fn <= NT       ? go(launch_eq_resident_t<3, 1>)
-         : fn <= 2 * NT ? go(launch_eq_resident_t<3, 2>)
-         : fn <= 4 * NT ? go(launch_eq_resident_t<3, 4>)
-                        : go(launch_eq_resident_t<3, 8>);
+    return fn <= NT       ? go(queue_eq_resident_t<2, 1>)
+           : fn <= 2 * NT ? go(queue_eq_resident_t<2, 2>)
+           : fn <= 4 * NT ? go(queue_eq_resident_t<2, 4>)
+                          : go(queue_eq_resident_t<2, 8>);
+  return fn <= NT       ? go(queue_eq_resident_t<3, 1>)
+         : fn <= 2 * NT ? go(queue_eq_resident_t<3, 2>)
+         : fn <= 4 * NT ? go(queue_eq_resident_t<3, 4>)
+                        : go(queue_eq_resident_t<3, 8>);
 }
 
 // Equilibrium PCG on the red-black Schur complement (k_eqrb_*): the same
@@ -2361,10 +2420,6 @@ static int launch_cg_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& 
   const int ni = pk->n_inst;
   const bool d2 = pk->dim == 2;
   CgVec cg = w.cg;   // black slot vectors
-  if (g_fused_mode.load() && ni == 1 && (int64_t)nbb <= kRbResidentCtas &&
-      launch_eq_resident(pk, L, we, J, b, d, rtol, maxiter, w, active, hks, s, rtol_inst) ==
-          TCAD_OK)
-    return TCAD_OK;
   TCAD_CUDA_CHECK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned) * ni, s));
   TCAD_CUDA_CHECK(cudaMemsetAsync(we.xb, 0, sizeof(double) * (size_t)pkb.n_nodes, s));
   if (d2) {
@@ -2587,12 +2642,7 @@ extern "C" int tcad_block_krylov(const tcad_pack_t* pk, const double* J, const d
     const WorkRb wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
     RbLayout rbl;
     if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots)) != TCAD_OK) return rc;
-    const unsigned nbb = (unsigned)rbl.pkb.n_flat;
-    if (pk->dim == 2)
-      k_rb_pack<2><<<nbb, NT, 0, s>>>(rbl.pkb, rbl.mp, J, wrb.JR, wrb.JB);
-    else
-      k_rb_pack<3><<<nbb, NT, 0, s>>>(rbl.pkb, rbl.mp, J, wrb.JR, wrb.JB);
-    note_launch();
+    rb_pack(pk, rbl, wrb, J, s);
     TCAD_LAUNCH_CHECK();
     rc = launch_bicgstab_rb(pk, rbl, wrb, b, x, rtol, maxiter, w, nullptr, hks, s, nullptr);
   } else {
@@ -2719,7 +2769,14 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
     for (int64_t t = 0; t < pk->n_tiles; ++t) htile_inst[t] = htile[4 * t];
     listed.assign(ni, 2);  // forces a first decision
   }
+  // One instance whose FP64 solves are resident: a step's kernels -- assembly,
+  // set-up, solve, update -- are queued behind one copy up and followed by one
+  // copy down, one synchronisation a step (the update looks on the device
+  // whether the solve it follows may be applied)
+  StepControl ctl(w);
+  const bool lean_call = ni == 1 && opts->precision == 64 && use_rb && rb_resident(pk, rbl);
   for (int it = 0; it < opts->max_iter; ++it) {
+    const bool lean = lean_call && !ilu_on[0] && hact[0];
     if (ni > 1 && listed != hact) {
       listed = hact;
       int64_t act_blocks = 0;
@@ -2745,6 +2802,17 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
         tl = nullptr; fl = nullptr; ntl = 0; nfl = 0;
       }
     }
+    // density floor of each instance's relative unknowns: the polishing
+    // steps use their own (far below the densities), the others sfloor
+    for (int i = 0; i < ni; ++i)
+      hsfl[i] = (polish_left[i] > 0 && opts->polish_scale_floor > 0.0)
+                    ? opts->polish_scale_floor : sfloor;
+    if (lean) {
+      ctl.clear(w);
+      ctl.at(w.eta) = heta[0];
+      ctl.at(w.sfl) = hsfl[0];
+      if (int rc = ctl.up(s)) return rc;
+    }
     int rc = sg_assemble_tiles(pk, psi, n, p, F, J, TCAD_MODE_ELIMINATE, tl, ntl, s);
     if (rc != TCAD_OK) return rc;
     if (opts->dt > 0.0) {  // one step of the theta scheme: storage term
@@ -2752,14 +2820,11 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
                          opts->dt, opts->theta, F, J, fl, nfl, s);
       if (rc != TCAD_OK) return rc;
     }
-    TCAD_CUDA_CHECK(cudaMemsetAsync(w.status, 0, sizeof(int32_t) * ni, s));
-    // density floor of each instance's relative unknowns: the polishing
-    // steps use their own (far below the densities), the others sfloor
-    for (int i = 0; i < ni; ++i)
-      hsfl[i] = (polish_left[i] > 0 && opts->polish_scale_floor > 0.0)
-                    ? opts->polish_scale_floor : sfloor;
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(w.sfl, hsfl.data(), sizeof(double) * ni,
-                                    cudaMemcpyHostToDevice, s));
+    if (!lean) {
+      TCAD_CUDA_CHECK(cudaMemsetAsync(w.status, 0, sizeof(int32_t) * ni, s));
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(w.sfl, hsfl.data(), sizeof(double) * ni,
+                                      cudaMemcpyHostToDevice, s));
+    }
     if (!fl || nfl > 0) {
       const bool rel = opts->density_scaling != 0;
       const double* sn_ = rel ? n : nullptr;
@@ -2772,16 +2837,40 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
     }
     note_launch();
     TCAD_LAUNCH_CHECK();
-    // inactive instances: pre-mark so their Krylov stays idle
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(hstat.data(), w.status, sizeof(int32_t) * ni,
-                                    cudaMemcpyDeviceToHost, s));
-    TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
-    for (int i = 0; i < ni; ++i)
-      if (!hact[i] && hstat[i] == TCAD_OK) hstat[i] = -1;  // idle marker
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(w.status, hstat.data(), sizeof(int32_t) * ni,
-                                    cudaMemcpyHostToDevice, s));
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(w.eta, heta.data(), sizeof(double) * ni,
-                                    cudaMemcpyHostToDevice, s));
+    bool stepped = false;   // the lean step solved and (unless it is retried) updated
+    if (lean) {
+      const bool retry_ok = opts->precond == 2 && use_ilu;
+      const bool js = rb_resident_js(pk, rbl);
+      if (!js) rb_pack(pk, rbl, wrb, J, s);
+      if (queue_rb_resident(pk, rbl, wrb, js ? J : nullptr, F, du, opts->rtol,
+                            opts->krylov_maxiter, w, w.status, false, s, w.eta) == TCAD_OK) {
+        k_newton_update<<<nb, NT, 0, s>>>(*pk, psi, n, p, du, opts->max_dpsi, opts->dens_floor,
+                                          nullptr, w.err, opts->density_scaling, 0, sfloor,
+                                          w.sfl, w.bar, retry_ok ? w.ks : nullptr);
+        note_launch();
+        TCAD_LAUNCH_CHECK();
+        stepped = true;
+      }
+      if (int rd = ctl.down(s)) return rd;
+      hstat[0] = ctl.at(w.status);
+      if (stepped && ctl.at(w.bar + 2) != 0u) {
+        g_fused_gave_up.fetch_add(1);
+        stepped = false;
+      }
+      hks[0] = ctl.at(w.ks);
+      herr[0] = ctl.at(w.err);
+    } else {
+      // inactive instances: pre-mark so their Krylov stays idle
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(hstat.data(), w.status, sizeof(int32_t) * ni,
+                                      cudaMemcpyDeviceToHost, s));
+      TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+      for (int i = 0; i < ni; ++i)
+        if (!hact[i] && hstat[i] == TCAD_OK) hstat[i] = -1;  // idle marker
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(w.status, hstat.data(), sizeof(int32_t) * ni,
+                                      cudaMemcpyHostToDevice, s));
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(w.eta, heta.data(), sizeof(double) * ni,
+                                      cudaMemcpyHostToDevice, s));
+    }
     // instances whose step is solved in FP64 this iteration, and those whose
     // (FP32-solved) step is applied before the FP64 solve starts
     std::vector<uint8_t> grp64(ni, 0), grp32(ni, 0);
@@ -2792,7 +2881,7 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
     }
     bool any32 = false, any64 = false;
     for (int i = 0; i < ni; ++i) { any32 = any32 || grp32[i]; }
-    TCAD_CUDA_CHECK(cudaMemsetAsync(w.err, 0, sizeof(unsigned long long) * ni, s));
+    if (!stepped) TCAD_CUDA_CHECK(cudaMemsetAsync(w.err, 0, sizeof(unsigned long long) * ni, s));
     if (any32) {
       // FP32 inner Krylov inside FP64 iterative refinement
       std::vector<int32_t> st32(ni);
@@ -2861,14 +2950,16 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
     // failed is solved again with ILU(0) before its update is applied
     std::vector<uint8_t> solve_set(grp64), done_set(ni, 0);
     for (int pass = 0; pass < 2 && any64; ++pass) {
+      const bool done_here = stepped && pass == 0;   // by the lean step
       std::vector<int32_t> st64(ni);
       bool any_ilu = false;
       for (int i = 0; i < ni; ++i) {
         st64[i] = solve_set[i] ? hstat[i] : -1;
         any_ilu = any_ilu || (solve_set[i] && ilu_on[i]);
       }
-      TCAD_CUDA_CHECK(cudaMemcpyAsync(w.status, st64.data(), sizeof(int32_t) * ni,
-                                      cudaMemcpyHostToDevice, s));
+      if (!done_here)
+        TCAD_CUDA_CHECK(cudaMemcpyAsync(w.status, st64.data(), sizeof(int32_t) * ni,
+                                        cudaMemcpyHostToDevice, s));
       if (any_ilu) {  // factor the ILU instances of this solve
         std::vector<int32_t> pre(ni);
         std::vector<uint8_t> msk(ni);
@@ -2894,7 +2985,9 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
       // keep the FP64 operator
       bool any_polish = false;
       for (int i = 0; i < ni; ++i) any_polish = any_polish || (solve_set[i] && polish_left[i] > 0);
-      if (opts->precision == TCAD_PRECISION_J32 && !any_ilu && !any_polish) {
+      if (done_here) {
+        rc = TCAD_OK;
+      } else if (opts->precision == TCAD_PRECISION_J32 && !any_ilu && !any_polish) {
         const int ne = pk->dim == 2 ? TCAD_NE2 : TCAD_NE3;
         k_to_f32<<<fl ? (unsigned)nfl : nb, NT, 0, s>>>(*pk, ne, J, w32.J32, fl);
         note_launch();
@@ -2903,15 +2996,11 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
                                               opts->krylov_maxiter, w.bi, w, w.status, hks, s,
                                               w.eta);
       } else if (use_rb && !any_ilu) {
-        const unsigned nbb = (unsigned)rbl.pkb.n_flat;
-        if (pk->dim == 2)
-          k_rb_pack<2><<<nbb, NT, 0, s>>>(rbl.pkb, rbl.mp, J, wrb.JR, wrb.JB);
-        else
-          k_rb_pack<3><<<nbb, NT, 0, s>>>(rbl.pkb, rbl.mp, J, wrb.JR, wrb.JB);
-        note_launch();
+        rb_pack(pk, rbl, wrb, J, s);
         TCAD_LAUNCH_CHECK();
+        // (a lean step that comes here was refused or gave up)
         rc = launch_bicgstab_rb(pk, rbl, wrb, F, du, opts->rtol, opts->krylov_maxiter, w,
-                                w.status, hks, s, w.eta);
+                                w.status, hks, s, w.eta, lean);
       } else {
         rc = launch_bicgstab(pk, J, F, du, opts->rtol, opts->krylov_maxiter, w, w.status, hks,
                              s, w.eta, any_ilu ? &wilu_use : nullptr, nzmax);
@@ -2925,9 +3014,7 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
         result[i].krylov_iters += hks[i].it;
         result[i].status = hks[i].status;
         result[i].relres = hks[i].bb > 0.0 ? std::sqrt(hks[i].rr / hks[i].bb) : 0.0;
-        const bool failed = hks[i].status == TCAD_ERR_NOCONV ||
-                            hks[i].status == TCAD_ERR_BREAKDOWN;
-        if (pass == 0 && failed && opts->precond == 2 && use_ilu && !ilu_on[i]) {
+        if (pass == 0 && solve_failed(hks[i].status) && opts->precond == 2 && use_ilu && !ilu_on[i]) {
           ilu_on[i] = 1;  // from now on this instance is ILU-preconditioned
           retry[i] = 1;
           any_retry = true;
@@ -2940,6 +3027,12 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
       }
       // apply this pass's accepted steps (the retried ones are solved again;
       // their du is overwritten by the next pass)
+      if (done_here) {
+        if (!any_retry) break;
+        stepped = false;   // the retry's update is still to come
+        solve_set = retry;
+        continue;
+      }
       TCAD_CUDA_CHECK(cudaMemcpyAsync(active, apply.data(), ni, cudaMemcpyHostToDevice, s));
       k_newton_update<<<nb, NT, 0, s>>>(*pk, psi, n, p, du, opts->max_dpsi, opts->dens_floor,
                                         active, w.err, opts->density_scaling, 0, sfloor,
@@ -2949,9 +3042,11 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
       if (!any_retry) break;
       solve_set = retry;
     }
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(herr.data(), w.err, sizeof(unsigned long long) * ni,
-                                    cudaMemcpyDeviceToHost, s));
-    TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+    if (!stepped) {
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(herr.data(), w.err, sizeof(unsigned long long) * ni,
+                                      cudaMemcpyDeviceToHost, s));
+      TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+    }
     bool any = false;
     for (int i = 0; i < ni; ++i) {
       if (!hact[i]) continue;
@@ -3029,24 +3124,48 @@ extern "C" int tcad_equilibrium_solve(const tcad_pack_t* pk, double* psi, double
     we = carve_eq(pk, reinterpret_cast<char*>(work) + off_eq(pk));
     if (int rc = rb_layout(pk, we, rbl, s, kEqResidentMaxSlots)) return rc;
   }
+  StepControl ctl(w);
   for (int it = 0; it < opts->max_iter; ++it) {
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(dact, hact.data(), ni, cudaMemcpyHostToDevice, s));
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(w.eta, heta.data(), sizeof(double) * ni,
-                                    cudaMemcpyHostToDevice, s));
-    int rc = tcad_poisson_assemble(pk, psi, F, J, TCAD_MODE_ELIMINATE, stream);
-    if (rc != TCAD_OK) return rc;
-    rc = use_rb ? launch_cg_rb(pk, rbl, we, J, F, d, opts->rtol, opts->krylov_maxiter, w, dact,
-                               hks, s, w.eta)
-                : launch_cg(pk, J, F, d, opts->rtol, opts->krylov_maxiter, w, dact, hks, s,
-                            w.eta);
-    if (rc != TCAD_OK) return rc;
-    TCAD_CUDA_CHECK(cudaMemsetAsync(w.err, 0, sizeof(unsigned long long) * ni, s));
-    k_eq_update<<<nb, NT, 0, s>>>(*pk, psi, d, opts->max_dpsi, dact, w.err);
-    note_launch();
-    TCAD_LAUNCH_CHECK();
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(herr.data(), w.err, sizeof(unsigned long long) * ni,
-                                    cudaMemcpyDeviceToHost, s));
-    TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+    // the resident solve of one instance: one copy up, the kernels, one copy down
+    // (as the coupled Newton's lean step)
+    bool stepped = false;
+    if (use_rb && eq_resident(pk, rbl)) {
+      ctl.clear(w);
+      ctl.at(w.eta) = heta[0];
+      if (int rc = ctl.up(s)) return rc;
+      int rc = tcad_poisson_assemble(pk, psi, F, J, TCAD_MODE_ELIMINATE, stream);
+      if (rc != TCAD_OK) return rc;
+      if (queue_eq_resident(pk, rbl, we, J, F, d, opts->rtol, opts->krylov_maxiter, w, s,
+                            w.eta) == TCAD_OK) {
+        k_eq_update<<<nb, NT, 0, s>>>(*pk, psi, d, opts->max_dpsi, nullptr, w.err, w.bar);
+        note_launch();
+        TCAD_LAUNCH_CHECK();
+        if ((rc = ctl.down(s))) return rc;
+        stepped = ctl.at(w.bar + 2) == 0u;
+        if (!stepped) g_fused_gave_up.fetch_add(1);
+        hks.assign(1, ctl.at(w.ks));
+        herr[0] = ctl.at(w.err);
+      }
+    }
+    if (!stepped) {
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(dact, hact.data(), ni, cudaMemcpyHostToDevice, s));
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(w.eta, heta.data(), sizeof(double) * ni,
+                                      cudaMemcpyHostToDevice, s));
+      int rc = tcad_poisson_assemble(pk, psi, F, J, TCAD_MODE_ELIMINATE, stream);
+      if (rc != TCAD_OK) return rc;
+      rc = use_rb ? launch_cg_rb(pk, rbl, we, J, F, d, opts->rtol, opts->krylov_maxiter, w, dact,
+                                 hks, s, w.eta)
+                  : launch_cg(pk, J, F, d, opts->rtol, opts->krylov_maxiter, w, dact, hks, s,
+                              w.eta);
+      if (rc != TCAD_OK) return rc;
+      TCAD_CUDA_CHECK(cudaMemsetAsync(w.err, 0, sizeof(unsigned long long) * ni, s));
+      k_eq_update<<<nb, NT, 0, s>>>(*pk, psi, d, opts->max_dpsi, dact, w.err);
+      note_launch();
+      TCAD_LAUNCH_CHECK();
+      TCAD_CUDA_CHECK(cudaMemcpyAsync(herr.data(), w.err, sizeof(unsigned long long) * ni,
+                                      cudaMemcpyDeviceToHost, s));
+      TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+    }
     bool any = false;
     for (int i = 0; i < ni; ++i) {
       if (!hact[i]) continue;

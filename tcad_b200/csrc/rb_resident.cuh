@@ -53,8 +53,8 @@ struct RbFormSCg {
 
 template <int DIM, int K, bool JS>
 __global__ void __launch_bounds__(NT, 1)
-k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR,
-                       const double* __restrict__ JB, const double* __restrict__ b,
+k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ Jn,
+                       const double* __restrict__ JR, const double* __restrict__ JB, const double* __restrict__ b,
                        double* __restrict__ x, double* bRg, double* Tr, double* xbg,
                        double* rhsg, double* rg, double* pg, double* vg, KState* ks,
                        double* part, unsigned* bar, double rtol, int maxit,
@@ -69,7 +69,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
   const RbGeo g = rb_geo(pkb, mp, inst);
   const int64_t NS = pkb.n_nodes, NN = mp.n_full;
   const int nloc = (int)(fb.end - fb.begin);
-  const double *jr, *jb;   // J rows of the CTA's slots, warp tiles from slot jbase
+  const double *jr, *jb;   // J rows of the CTA's slots in warp tiles
   if constexpr (JS) {
     // flat_nodes is a multiple of 32, so the CTA's rows are whole warp tiles,
     // one contiguous run per colour
@@ -77,10 +77,22 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
     const double2* const gr = reinterpret_cast<const double2*>(JR + rb_jidx<NE>(0, fb.begin));
     const double2* const gb = reinterpret_cast<const double2*>(JB + rb_jidx<NE>(0, fb.begin));
     double2* const s2 = reinterpret_cast<double2*>(s_rows);
+    if (Jn) {   // from J in node order (zeros at pads, as k_rb_pack)
+      for (int l = threadIdx.x; l < nloc; l += NT)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const RbNode q = rb_node(g, fb.begin + l, c);
+          double* const dst = s_rows + 2 * c * n2 + rb_jidx<NE>(0, l);
+#pragma unroll 13
+          for (int e = 0; e < NE; ++e)
+            dst[32 * e] = q.real ? Jn[(int64_t)e * NN + q.node] : 0.0;
+        }
+    } else {
 #pragma unroll 8
-    for (int i = threadIdx.x; i < n2; i += NT) s2[i] = gr[i];
+      for (int i = threadIdx.x; i < n2; i += NT) s2[i] = gr[i];
 #pragma unroll 8
-    for (int i = threadIdx.x; i < n2; i += NT) s2[n2 + i] = gb[i];
+      for (int i = threadIdx.x; i < n2; i += NT) s2[n2 + i] = gb[i];
+    }
     jr = s_rows;
     jb = s_rows + 2 * n2;
   } else {
