@@ -9,29 +9,37 @@
 // (600k nodes) stay resident and an iteration is bound by the latency of its
 // three steps -- red(p), q (alpha), x (beta) -- instead of four launches and
 // two last-block reductions.  240 x 120 MOSFET: 24 -> 6.5 us per iteration.
+// Instances of at most kClusterMaxCtas x kEqResidentMaxSlots slots have a cluster
+// each instead (SYNC = ClusterSync): barriers inside a cluster cost a fifth, and a
+// batch's instances run side by side, each to its own convergence.
 // Expressions and the order of the sums are the per-step kernels', so the
-// update is bit-identical to launch_cg_rb's loop.
+// update is bit-identical to launch_cg_rb's loop over the same blocks.
 #pragma once
 
 namespace tcad {
 
 constexpr int kEqResidentMaxSlots = 8 * NT;
 
-template <int DIM, int K>
+template <int DIM, int K, class SYNC>
 __global__ void __launch_bounds__(NT, 1)
 k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ J,
                 const double* __restrict__ F, double* __restrict__ d, double* zg, double* pg,
                 double* xg, double* Tr, KState* ks, double* part, unsigned* bar, double rtol,
-                int maxit, const double* __restrict__ rtol_inst) {
+                int maxit, const uint8_t* __restrict__ active,
+                const double* __restrict__ rtol_inst, int rows) {
   constexpr int NE = 1 + 2 * DIM, ND = 2 * DIM;
-  extern __shared__ __align__(16) double s_rows[];   // [2][NE][flat_nodes]
-  GridSync gs;
+  extern __shared__ __align__(16) double s_rows[];   // [2][NE][rows]
+  SYNC gs;
   gs.init(part, bar);
-  const FlatBlock fb = flat_block(pkb, blockIdx.x);
+  const RbShare fb = rb_share(pkb, gs);
   const int inst = fb.inst;
+  if (active && !active[inst]) {
+    if (fb.lead && threadIdx.x == 0) ks[inst].active = 0;
+    return;
+  }
   const RbGeo g = rb_geo(pkb, mp, inst);
   const int64_t NN = mp.n_full;
-  const int nloc = (int)(fb.end - fb.begin), fn = pkb.flat_nodes;
+  const int nloc = fb.len, fn = rows;
   double* const sR = s_rows;
   double* const sB = s_rows + (int64_t)NE * fn;
   const int64_t q0 = fb.begin + threadIdx.x;   // slot k of the thread: q0 + k NT
@@ -110,7 +118,7 @@ k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict_
 #pragma unroll
   for (int k = 0; k < K; ++k)
     if (own[k]) Tr[q0 + k * NT] = red(k, [](int) { return 0.0; }, r[k]);
-  if (!gs.sum<0>(nullptr, nullptr)) return;
+  if (!gs.template sum<0>(nullptr, nullptr)) return;
   sum[0] = 0.0; sum[1] = 0.0;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
@@ -124,7 +132,7 @@ k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict_
     sum[0] += bv * z[k];
     sum[1] += bv * bv;
   }
-  if (!gs.sum<2>(sum, tot)) return;
+  if (!gs.template sum<2>(sum, tot)) return;
   fin_cg_init(S, tot[0], tot[1], rtol_inst ? rtol_inst[inst] : rtol, maxit, true);
   S.beta = 0.0;   // the first direction is z: p = z + 0 * 0
   while (S.active) {
@@ -136,7 +144,7 @@ k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict_
       if (own[k])
         Tr[q0 + k * NT] =
             red(k, [&](int m) { return __ldcg(zi + m) + beta * __ldcg(pi + m); }, 0.0);
-    if (!gs.sum<0>(nullptr, nullptr)) return;
+    if (!gs.template sum<0>(nullptr, nullptr)) return;
     sum[0] = 0.0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -147,7 +155,7 @@ k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict_
       q[k] = realb[k] ? -sB[threadIdx.x + k * NT] * pv + black(k) : 0.0;
       sum[0] += pv * q[k];
     }
-    if (!gs.sum<1>(sum, tot)) return;
+    if (!gs.template sum<1>(sum, tot)) return;
     fin_cg_q(S, tot[0]);
     if (!S.active) break;
     sum[0] = 0.0;
@@ -161,14 +169,14 @@ k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict_
       zg[q0 + k * NT] = z[k];
       sum[0] += rn * z[k];
     }
-    if (!gs.sum<1>(sum, tot)) return;
+    if (!gs.template sum<1>(sum, tot)) return;
     fin_cg_x(S, tot[0]);
   }
   // d_r = A_rr^-1 (F_r - A_rb d_b), d_b = x
 #pragma unroll
   for (int k = 0; k < K; ++k)
     if (own[k]) xg[q0 + k * NT] = x[k];
-  if (!gs.sum<0>(nullptr, nullptr)) return;
+  if (!gs.template sum<0>(nullptr, nullptr)) return;
   const double* const xi = xg + g.soff;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
@@ -177,7 +185,7 @@ k_eqrb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict_
     if (realr[k]) d[nr.node] = red(k, [&](int m) { return __ldcg(xi + m); }, F[nr.node]);
     if (realb[k]) d[nk.node] = x[k];
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) ks[inst] = S;
+  if (fb.lead && threadIdx.x == 0) ks[inst] = S;
 }
 
 }  // namespace tcad

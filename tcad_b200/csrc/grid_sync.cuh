@@ -144,4 +144,90 @@ struct GridSync {
   }
 };
 
+// The same for one thread-block cluster (hardware barrier, no bound needed: the
+// CTAs of a cluster are always resident together, and a barrier of it cannot be
+// waited for by fewer).  A CTA stores its sums into every peer's shared memory
+// before it arrives, so the totals are at hand after the wait.  Per step on 8 / 16
+// CTAs: 0.21 us without sums, 0.65 / 0.78 with one, 0.76 / 1.09 with three.
+constexpr int kClusterMaxCtas = 16;
+
+struct ClusterSync {
+  unsigned rank, ctas;
+  int par;
+
+  __device__ __forceinline__ void init(double*, unsigned*) {
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+    par = 0;
+  }
+
+  template <int NQ>
+  __device__ __forceinline__ bool sum(const double* v, double* tot) {
+    static_assert(NQ <= kSyncSums, "sums per step");
+    constexpr int NT = kFlatThreads, NW = NT / 32, NS = NQ > 0 ? NQ : 1;
+    __shared__ double sa[NS][NW], slot[2][NS][kClusterMaxCtas];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if constexpr (NQ > 0) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        double r = v[q];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+        if (lane == 0) sa[q][warp] = r;
+      }
+      __syncthreads();
+      if (threadIdx.x < ctas) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          const double* const w = sa[q];   // (the last tree of block_sum)
+          const double r = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+          unsigned peer;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                       : "=r"(peer)
+                       : "r"((unsigned)__cvta_generic_to_shared(&slot[par][q][rank])),
+                         "r"(threadIdx.x));
+          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer), "d"(r) : "memory");
+        }
+      }
+      __syncwarp();
+    }
+    asm volatile(
+        "barrier.cluster.arrive.release.aligned;\n\t"
+        "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if constexpr (NQ > 0) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        double r = 0.0 + (lane < (int)ctas ? slot[par][q][lane] : 0.0);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+        tot[q] = __shfl_sync(0xffffffffu, r, 0);
+      }
+      par ^= 1;
+    }
+    return true;
+  }
+};
+
+// A resident CTA's share of the slot pack: a flat block of the grid, or of a
+// cluster that has an instance to itself
+struct RbShare {
+  int inst, len;
+  int64_t begin;
+  bool lead;   // writes the instance's state
+};
+template <class SYNC>
+__device__ __forceinline__ RbShare rb_share(const tcad_pack_t& pkb, const SYNC&) {
+  const FlatBlock fb = flat_block(pkb, blockIdx.x);
+  return RbShare{fb.inst, (int)(fb.end - fb.begin), fb.begin, blockIdx.x == 0};
+}
+__device__ __forceinline__ RbShare rb_share(const tcad_pack_t& pkb, const ClusterSync& cs) {
+  const int inst = (int)(blockIdx.x / cs.ctas);
+  const int64_t slots = (int64_t)pkb.shape[3 * inst] * pkb.shape[3 * inst + 1];
+  const int64_t chunk = ((slots + cs.ctas - 1) / cs.ctas + 31) / 32 * 32;
+  const int64_t at = cs.rank * chunk;
+  const int64_t len = slots - at < chunk ? slots - at : chunk;
+  return RbShare{inst, (int)(len > 0 ? len : 0), pkb.node_off[inst] + (len > 0 ? at : 0),
+                 cs.rank == 0};
+}
+
 }  // namespace tcad

@@ -1433,13 +1433,28 @@ struct WorkRb {
 // kRbResidentCtas blocks of `most` slots) is split over all SMs instead:
 // whole warps of slots, at most one block per SM.
 constexpr int64_t kRbResidentCtas = 148;
-static int64_t rb_flat(int64_t slots, int64_t most) {
+static int64_t rb_cluster_slots(const tcad_pack_t* pk) {
+  return std::min(kRbResidentMaxSlots,
+                  rb_resident_js_slots(pk->dim == 2 ? TCAD_NE2 : TCAD_NE3));
+}
+// CTAs of the cluster that takes an instance of `slots` slots, `most` a CTA (0:
+// none does): 8 while that is at most two slots a thread
+static int cluster_ctas(int64_t slots, int64_t most) {
+  if (slots <= 8 * std::min<int64_t>(most, 2 * NT)) return 8;
+  return slots <= 16 * most ? 16 : 0;
+}
+static int64_t even_share(int64_t slots, int64_t blocks) {
+  return ((slots + blocks - 1) / blocks + 31) / 32 * 32;
+}
+// slots per flat block of a single instance; `most`, `most_cluster`: what one CTA
+// of the grid's and the cluster's resident solve takes
+static int64_t rb_flat(int64_t slots, int64_t most, int64_t most_cluster) {
   const int64_t sms = kRbResidentCtas;
-  const auto even = [&](int64_t blocks) { return ((slots + blocks - 1) / blocks + 31) / 32 * 32; };
-  if (even(sms) <= most) return even(sms);
+  if (const int c = cluster_ctas(slots, most_cluster)) return even_share(slots, c);
+  if (even_share(slots, sms) <= most) return even_share(slots, sms);
   // a larger single instance: as many blocks for every SM, of at most
   // kRbStreamSlots slots
-  return even(sms * ((slots + sms * kRbStreamSlots - 1) / (sms * kRbStreamSlots)));
+  return even_share(slots, sms * ((slots + sms * kRbStreamSlots - 1) / (sms * kRbStreamSlots)));
 }
 // n_nodes bounds the slots
 static size_t rb_flat_cap(const tcad_pack_t* pk) {
@@ -1512,17 +1527,19 @@ static WorkEq carve_eq(const tcad_pack_t* pk, void* base) {
 
 // The slot pack of a pack (host tables; see redblack.cuh): per instance
 // (ceil(Nx/2), Ny Nz, 1) slots of each colour, flat blocks of rb_flat slots
-// (`most`: the resident solve's bound)
+// (`most`, `most_cluster`: the resident solves' bounds per CTA)
 struct RbLayout {
   tcad_pack_t pkb;
   RbMap mp;
   std::vector<int64_t> hfoff;
   bool tiles;   // every flat block starts on a warp tile
+  int cluster;  // CTAs of the clusters that take every instance (0: some is too large)
+  int share;    // most slots of one of their CTAs
 };
 
 template <class W>   // WorkRb or WorkEq: the slot pack's table arrays
 static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream_t s,
-                     int64_t most) {
+                     int64_t most, int64_t most_cluster) {
   const int ni = pk->n_inst;
   std::vector<int32_t> shp(3 * (size_t)ni), sb(3 * (size_t)ni), fi;
   TCAD_CUDA_CHECK(cudaMemcpyAsync(shp.data(), pk->shape, sizeof(int32_t) * shp.size(),
@@ -1532,7 +1549,7 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   noff[0] = 0; foff[0] = 0;
   int64_t fn = kRbStreamSlots, nflat = 0;
   bool room = true;
-  if (ni == 1) fn = rb_flat((int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2], most);
+  if (ni == 1) fn = rb_flat((int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2], most, most_cluster);
   for (int i = 0; i < ni; ++i) {
     const int64_t hx = (shp[3 * i] + 1) / 2, rows = (int64_t)shp[3 * i + 1] * shp[3 * i + 2];
     sb[3 * i] = (int32_t)hx; sb[3 * i + 1] = (int32_t)rows; sb[3 * i + 2] = 1;
@@ -1570,6 +1587,10 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   L.mp.node_off = pk->node_off;
   L.mp.n_full = pk->n_nodes;
   L.hfoff = foff;
+  int64_t largest = 0;
+  for (int i = 0; i < ni; ++i) largest = std::max<int64_t>(largest, (int64_t)sb[3 * i] * sb[3 * i + 1]);
+  L.cluster = cluster_ctas(largest, most_cluster);
+  L.share = L.cluster ? (int)even_share(largest, L.cluster) : 0;
   L.tiles = fn % 32 == 0;
   for (int i = 0; i < ni; ++i) L.tiles = L.tiles && noff[i] % 32 == 0;
   return TCAD_OK;
@@ -1928,6 +1949,31 @@ static int coop_launch(CoopLaunch& c, unsigned blocks, unsigned threads, size_t 
   return TCAD_OK;
 }
 
+// Launch configuration of a cluster per instance; 1 when such clusters do not
+// fit on the GPU
+template <class... P>
+static int cluster_launch(CoopLaunch& c, void (*kern)(P...), int ni, int ctas, size_t smem,
+                          cudaStream_t s) {
+  c.cfg.gridDim = dim3((unsigned)(ni * ctas));
+  c.cfg.blockDim = dim3(NT);
+  c.cfg.dynamicSmemBytes = smem;
+  c.cfg.stream = s;
+  c.at[0].id = cudaLaunchAttributeClusterDimension;
+  c.at[0].val.clusterDim.x = (unsigned)ctas;
+  c.at[0].val.clusterDim.y = 1;
+  c.at[0].val.clusterDim.z = 1;
+  c.cfg.attrs = c.at;
+  c.cfg.numAttrs = 1;
+  int fit = 0;
+  if ((ctas > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                        1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&fit, kern, &c.cfg) != cudaSuccess || fit < 1) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  return TCAD_OK;
+}
+
 // Waits for a single-launch solve and reads its result: 1 when a grid
 // barrier gave up (the caller then solves with one launch per step)
 static int coop_result(const Work& w, int ni, std::vector<KState>& hks, cudaStream_t s) {
@@ -1947,26 +1993,32 @@ static int coop_result(const Work& w, int ni, std::vector<KState>& hks, cudaStre
 // k_bicgstab_rb_resident over the slot pack's blocks, queued: 1 when the launch
 // was refused.  Jn: J in node order (a solve with its rows in shared memory
 // takes them from there), null: the packed colour rows.  clear: see coop_launch.
-template <int DIM, int K, bool JS>
+template <int DIM, int K, bool JS, class SYNC>
 static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double* Jn,
                                const double* b, double* x, double rtol, int maxiter,
                                const Work& w, const int32_t* pre_status, bool clear,
                                cudaStream_t s, const double* rtol_inst) {
-  const auto kern = k_bicgstab_rb_resident<DIM, K, JS>;
-  const size_t smem = JS ? (size_t)L.pkb.flat_nodes * Stencil<DIM>::NE * 16 : 0;
+  constexpr bool kCluster = std::is_same<SYNC, ClusterSync>::value;
+  const auto kern = k_bicgstab_rb_resident<DIM, K, JS, SYNC>;
+  const int share = kCluster ? L.share : L.pkb.flat_nodes;
+  const size_t smem = JS ? (size_t)share * Stencil<DIM>::NE * 16 : 0;
   if (JS && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem) != cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
   CoopLaunch c;
-  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, clear, s)) return rc;
+  if (kCluster && clear) TCAD_CUDA_CHECK(cudaMemsetAsync(w.bar, 0, 4 * sizeof(unsigned), s));
+  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, smem, s)
+                        : coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, clear, s))
+    return rc;
   const BiVec& bi = w.bi;
   const int rechecks = 8;
   // (a cooperative launch that does not fit is refused, not run)
   if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, Jn, (const double*)wr.JR,
-                         (const double*)wr.JB, b, x, wr.bR, wr.tR, wr.xb, wr.rhs, bi.r, bi.p, bi.v, w.ks, wr.sync,
-                         w.bar, rtol, maxiter, pre_status, rtol_inst, rechecks) != cudaSuccess) {
+                         (const double*)wr.JB, b, x, wr.bR, wr.tR, wr.xb, wr.rhs, bi.r, bi.p,
+                         bi.v, w.ks, wr.sync, w.bar, rtol, maxiter, pre_status, rtol_inst,
+                         rechecks) != cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
@@ -1976,29 +2028,40 @@ static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double
 
 // whether a resident solve takes the pack, and whether it holds J's rows
 static bool rb_resident(const tcad_pack_t* pk, const RbLayout& L) {
-  return pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
-         L.pkb.flat_nodes <= kRbResidentMaxSlots && g_fused_mode.load();
+  return g_fused_mode.load() &&
+         (L.cluster || (pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
+                        L.pkb.flat_nodes <= kRbResidentMaxSlots));
 }
 static bool rb_resident_js(const tcad_pack_t* pk, const RbLayout& L) {
-  return L.pkb.flat_nodes <= rb_resident_js_slots(pk->dim == 2 ? TCAD_NE2 : TCAD_NE3);
+  return L.cluster ||
+         L.pkb.flat_nodes <= rb_resident_js_slots(pk->dim == 2 ? TCAD_NE2 : TCAD_NE3);
 }
 
 static int queue_rb_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkRb& wr,
                              const double* Jn, const double* b, double* x, double rtol,
                              int maxiter, const Work& w, const int32_t* pre_status, bool clear,
                              cudaStream_t s, const double* rtol_inst) {
-  const int fn = L.pkb.flat_nodes;
-  const bool js = rb_resident_js(pk, L);
+  const bool js = rb_resident_js(pk, L), d2 = pk->dim == 2;
   auto go = [&](auto fnc) {
     return fnc(L, wr, Jn, b, x, rtol, maxiter, w, pre_status, clear, s, rtol_inst);
   };
-  if (pk->dim == 2)
-    return fn <= NT ? go(queue_rb_resident_t<2, 1, true>)
-           : js     ? go(queue_rb_resident_t<2, 2, true>)
-                    : go(queue_rb_resident_t<2, 2, false>);
-  return fn <= NT ? go(queue_rb_resident_t<3, 1, true>)
-         : js     ? go(queue_rb_resident_t<3, 2, true>)
-                  : go(queue_rb_resident_t<3, 2, false>);
+  // (the test hook holds up a grid barrier; clusters have none)
+  if (L.cluster && !g_fused_test_hold.load()) {
+    if (d2)
+      return L.share <= NT ? go(queue_rb_resident_t<2, 1, true, ClusterSync>)
+                           : go(queue_rb_resident_t<2, 2, true, ClusterSync>);
+    return L.share <= NT ? go(queue_rb_resident_t<3, 1, true, ClusterSync>)
+                         : go(queue_rb_resident_t<3, 2, true, ClusterSync>);
+  }
+  if (pk->n_inst != 1) return 1;
+  const int fn = L.pkb.flat_nodes;
+  if (d2)
+    return fn <= NT ? go(queue_rb_resident_t<2, 1, true, GridSync>)
+           : js     ? go(queue_rb_resident_t<2, 2, true, GridSync>)
+                    : go(queue_rb_resident_t<2, 2, false, GridSync>);
+  return fn <= NT ? go(queue_rb_resident_t<3, 1, true, GridSync>)
+         : js     ? go(queue_rb_resident_t<3, 2, true, GridSync>)
+                  : go(queue_rb_resident_t<3, 2, false, GridSync>);
 }
 
 static int sm_count() {
@@ -2112,7 +2175,7 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
   if (rb_resident(pk, L) && !per_step &&
       queue_rb_resident(pk, L, wr, nullptr, b, x, rtol, maxiter, w, pre_status, true, s,
                         rtol_inst) == TCAD_OK &&
-      coop_result(w, 1, hks, s) == TCAD_OK)
+      coop_result(w, ni, hks, s) == TCAD_OK)
     return TCAD_OK;
   // J streamed through shared memory where the pack is larger than one wave
   // of blocks and every block starts on a warp tile
@@ -2361,23 +2424,29 @@ static int launch_cg(const tcad_pack_t* pk, const double* J, const double* b, do
   return TCAD_OK;
 }
 
-// k_eqrb_resident over the slot pack's blocks, queued with its barrier flags
-// cleared by the caller: 1 when the launch was refused
-template <int DIM, int K>
+// k_eqrb_resident over the slot pack's blocks or a cluster per instance, queued;
+// its barrier flags are cleared by the caller: 1 when the launch was refused
+template <int DIM, int K, class SYNC>
 static int queue_eq_resident_t(const RbLayout& L, const WorkEq& we, const double* J,
                                const double* b, double* d, double rtol, int maxiter,
-                               const Work& w, cudaStream_t s, const double* rtol_inst) {
-  const auto kern = k_eqrb_resident<DIM, K>;
-  const size_t smem = (size_t)L.pkb.flat_nodes * (1 + 2 * DIM) * 16;
+                               const Work& w, const uint8_t* active, cudaStream_t s,
+                               const double* rtol_inst) {
+  constexpr bool kCluster = std::is_same<SYNC, ClusterSync>::value;
+  const auto kern = k_eqrb_resident<DIM, K, SYNC>;
+  const int share = kCluster ? L.share : L.pkb.flat_nodes;
+  const size_t smem = (size_t)share * (1 + 2 * DIM) * 16;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
   CoopLaunch c;
-  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, false, s)) return rc;
+  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, smem, s)
+                        : coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, false, s))
+    return rc;
   if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, J, b, d, w.cg.z, w.cg.p, we.xb, we.tR, w.ks,
-                         we.sync, w.bar, rtol, maxiter, rtol_inst) != cudaSuccess) {
+                         we.sync, w.bar, rtol, maxiter, active, rtol_inst, share) !=
+      cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
@@ -2386,25 +2455,31 @@ static int queue_eq_resident_t(const RbLayout& L, const WorkEq& we, const double
 }
 
 static bool eq_resident(const tcad_pack_t* pk, const RbLayout& L) {
-  return pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
-         L.pkb.flat_nodes <= kEqResidentMaxSlots && g_fused_mode.load();
+  return g_fused_mode.load() &&
+         (L.cluster || (pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
+                        L.pkb.flat_nodes <= kEqResidentMaxSlots));
 }
 
 static int queue_eq_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& we,
                              const double* J, const double* b, double* d, double rtol,
-                             int maxiter, const Work& w, cudaStream_t s,
+                             int maxiter, const Work& w, const uint8_t* active, cudaStream_t s,
                              const double* rtol_inst) {
-  const int fn = L.pkb.flat_nodes;
-  auto go = [&](auto fnc) { return fnc(L, we, J, b, d, rtol, maxiter, w, s, rtol_inst); };
-  if (pk->dim == 2)
-    return fn <= NT       ? go(queue_eq_resident_t<2, 1>)
-           : fn <= 2 * NT ? go(queue_eq_resident_t<2, 2>)
-           : fn <= 4 * NT ? go(queue_eq_resident_t<2, 4>)
-                          : go(queue_eq_resident_t<2, 8>);
-  return fn <= NT       ? go(queue_eq_resident_t<3, 1>)
-         : fn <= 2 * NT ? go(queue_eq_resident_t<3, 2>)
-         : fn <= 4 * NT ? go(queue_eq_resident_t<3, 4>)
-                        : go(queue_eq_resident_t<3, 8>);
+  auto go = [&](auto fnc) { return fnc(L, we, J, b, d, rtol, maxiter, w, active, s, rtol_inst); };
+  auto pick = [&](auto sync, int fn) {
+    using S = decltype(sync);
+    if (pk->dim == 2)
+      return fn <= NT       ? go(queue_eq_resident_t<2, 1, S>)
+             : fn <= 2 * NT ? go(queue_eq_resident_t<2, 2, S>)
+             : fn <= 4 * NT ? go(queue_eq_resident_t<2, 4, S>)
+                            : go(queue_eq_resident_t<2, 8, S>);
+    return fn <= NT       ? go(queue_eq_resident_t<3, 1, S>)
+           : fn <= 2 * NT ? go(queue_eq_resident_t<3, 2, S>)
+           : fn <= 4 * NT ? go(queue_eq_resident_t<3, 4, S>)
+                          : go(queue_eq_resident_t<3, 8, S>);
+  };
+  // (the test hook holds up a grid barrier; clusters have none)
+  if (L.cluster && !g_fused_test_hold.load()) return pick(ClusterSync{}, L.share);
+  return pk->n_inst == 1 ? pick(GridSync{}, L.pkb.flat_nodes) : 1;
 }
 
 // Equilibrium PCG on the red-black Schur complement (k_eqrb_*): the same
@@ -2420,6 +2495,14 @@ static int launch_cg_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& 
   const int ni = pk->n_inst;
   const bool d2 = pk->dim == 2;
   CgVec cg = w.cg;   // black slot vectors
+  if (ni > 1 && eq_resident(pk, L) &&
+      queue_eq_resident(pk, L, we, J, b, d, rtol, maxiter, w, active, s, rtol_inst) == TCAD_OK) {
+    hks.resize(ni);
+    TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState) * ni,
+                                    cudaMemcpyDeviceToHost, s));
+    TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+    return TCAD_OK;
+  }
   TCAD_CUDA_CHECK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned) * ni, s));
   TCAD_CUDA_CHECK(cudaMemsetAsync(we.xb, 0, sizeof(double) * (size_t)pkb.n_nodes, s));
   if (d2) {
@@ -2641,7 +2724,7 @@ extern "C" int tcad_block_krylov(const tcad_pack_t* pk, const double* J, const d
     if (work_bytes < tcad_block_workspace_bytes(pk, 2, 0)) return TCAD_ERR_ARG;
     const WorkRb wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
     RbLayout rbl;
-    if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots)) != TCAD_OK) return rc;
+    if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk))) != TCAD_OK) return rc;
     rb_pack(pk, rbl, wrb, J, s);
     TCAD_LAUNCH_CHECK();
     rc = launch_bicgstab_rb(pk, rbl, wrb, b, x, rtol, maxiter, w, nullptr, hks, s, nullptr);
@@ -2738,7 +2821,7 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
   RbLayout rbl;
   if (use_rb) {
     wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
-    if (int rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots)) return rc;
+    if (int rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk))) return rc;
   }
   std::vector<int32_t> mix_it(ni), mix_st(ni), mix_grew(ni, 0), mix_steps(ni, 0);
   std::vector<double> mix_rr(ni), mix_prev(ni, -1.0);
@@ -3122,21 +3205,21 @@ extern "C" int tcad_equilibrium_solve(const tcad_pack_t* pk, double* psi, double
   RbLayout rbl;
   if (use_rb) {
     we = carve_eq(pk, reinterpret_cast<char*>(work) + off_eq(pk));
-    if (int rc = rb_layout(pk, we, rbl, s, kEqResidentMaxSlots)) return rc;
+    if (int rc = rb_layout(pk, we, rbl, s, kEqResidentMaxSlots, kEqResidentMaxSlots)) return rc;
   }
   StepControl ctl(w);
   for (int it = 0; it < opts->max_iter; ++it) {
     // the resident solve of one instance: one copy up, the kernels, one copy down
     // (as the coupled Newton's lean step)
     bool stepped = false;
-    if (use_rb && eq_resident(pk, rbl)) {
+    if (ni == 1 && use_rb && eq_resident(pk, rbl)) {
       ctl.clear(w);
       ctl.at(w.eta) = heta[0];
       if (int rc = ctl.up(s)) return rc;
       int rc = tcad_poisson_assemble(pk, psi, F, J, TCAD_MODE_ELIMINATE, stream);
       if (rc != TCAD_OK) return rc;
-      if (queue_eq_resident(pk, rbl, we, J, F, d, opts->rtol, opts->krylov_maxiter, w, s,
-                            w.eta) == TCAD_OK) {
+      if (queue_eq_resident(pk, rbl, we, J, F, d, opts->rtol, opts->krylov_maxiter, w, nullptr,
+                            s, w.eta) == TCAD_OK) {
         k_eq_update<<<nb, NT, 0, s>>>(*pk, psi, d, opts->max_dpsi, nullptr, w.err, w.bar);
         note_launch();
         TCAD_LAUNCH_CHECK();

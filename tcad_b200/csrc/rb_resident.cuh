@@ -13,7 +13,10 @@
 // red(s), s + t (early, omega), x (rho, beta, convergence); p and s are
 // formed on the fly at the neighbours (RbFormPCg / RbFormSCg).  Bodies, scalar
 // updates and the order of the sums are those of the per-step kernels, so the
-// result is bit-identical to launch_bicgstab_rb's loop.
+// result is bit-identical to launch_bicgstab_rb's loop over the same blocks.
+//
+// Instances whose rows fit in the shared memory of one cluster have a cluster
+// each (SYNC = ClusterSync, eq_resident.cuh).
 #pragma once
 
 namespace tcad {
@@ -51,7 +54,7 @@ struct RbFormSCg {
   }
 };
 
-template <int DIM, int K, bool JS>
+template <int DIM, int K, bool JS, class SYNC>
 __global__ void __launch_bounds__(NT, 1)
 k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ Jn,
                        const double* __restrict__ JR, const double* __restrict__ JB, const double* __restrict__ b,
@@ -62,16 +65,16 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
                        const double* __restrict__ rtol_inst, int max_rechecks) {
   constexpr int NE = Stencil<DIM>::NE;
   extern __shared__ __align__(16) double s_rows[];
-  GridSync gs;
+  SYNC gs;
   gs.init(part, bar);
-  const FlatBlock fb = flat_block(pkb, blockIdx.x);
+  const RbShare fb = rb_share(pkb, gs);
   const int inst = fb.inst;
   const RbGeo g = rb_geo(pkb, mp, inst);
   const int64_t NS = pkb.n_nodes, NN = mp.n_full;
-  const int nloc = (int)(fb.end - fb.begin);
+  const int nloc = fb.len;
   const double *jr, *jb;   // J rows of the CTA's slots in warp tiles
   if constexpr (JS) {
-    // flat_nodes is a multiple of 32, so the CTA's rows are whole warp tiles,
+    // a share is a multiple of 32 slots, so the CTA's rows are whole warp tiles,
     // one contiguous run per colour
     const int n2 = (nloc + 31) / 32 * NE * 16;
     const double2* const gr = reinterpret_cast<const double2*>(JR + rb_jidx<NE>(0, fb.begin));
@@ -160,7 +163,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
       }
     }
   }
-  if (!gs.sum<1>(sum, tot)) return;
+  if (!gs.template sum<1>(sum, tot)) return;
   const double bb = tot[0];
   // rhs = bB - F bR; x = 0, r = rh = rhs, p = v = 0
   sum[0] = 0.0;
@@ -180,14 +183,14 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
       }
     }
   }
-  if (!gs.sum<1>(sum, tot)) return;
+  if (!gs.template sum<1>(sum, tot)) return;
   rb_fin_init(S, tot[0], bb, rtol_inst ? rtol_inst[inst] : rtol, maxit,
               pre_status ? pre_status[inst] : TCAD_OK);
 
   for (int rechecks = 0;; ++rechecks) {
     while (S.active) {
       red(RbFormPCg{rg + g.soff, pg + g.soff, vg + g.soff, NS, S.beta, S.omega, S.restart});
-      if (!gs.sum<0>(nullptr, nullptr)) return;
+      if (!gs.template sum<0>(nullptr, nullptr)) return;
       sum[0] = 0.0;
 #pragma unroll
       for (int k = 0; k < K; ++k) {
@@ -207,11 +210,11 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
           sum[0] += rh[k][c] * y;
         }
       }
-      if (!gs.sum<1>(sum, tot)) return;
+      if (!gs.template sum<1>(sum, tot)) return;
       fin_v(S, tot[0]);
       if (!S.active) break;
       red(RbFormSCg{rg + g.soff, vg + g.soff, NS, S.alpha});
-      if (!gs.sum<0>(nullptr, nullptr)) return;
+      if (!gs.template sum<0>(nullptr, nullptr)) return;
       sum[0] = 0.0; sum[1] = 0.0; sum[2] = 0.0;
 #pragma unroll
       for (int k = 0; k < K; ++k) {
@@ -229,7 +232,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
           sum[2] += y * y;
         }
       }
-      if (!gs.sum<3>(sum, tot)) return;
+      if (!gs.template sum<3>(sum, tot)) return;
       fin_s(S, tot[0]);
       fin_t(S, tot[1], tot[2]);
       sum[0] = 0.0; sum[1] = 0.0; sum[2] = 0.0;
@@ -247,7 +250,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
           sum[2] += rh[k][c] * rh[k][c];
         }
       }
-      if (!gs.sum<3>(sum, tot)) return;
+      if (!gs.template sum<3>(sum, tot)) return;
       fin_x(S, tot[0], tot[1], tot[2]);
     }
     // true Schur residual r = rhs - S x
@@ -256,9 +259,9 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
       if (own[k])
 #pragma unroll
         for (int c = 0; c < 3; ++c) xbg[c * NS + q0 + k * NT] = xb[k][c];
-    if (!gs.sum<0>(nullptr, nullptr)) return;
+    if (!gs.template sum<0>(nullptr, nullptr)) return;
     red(RbValCg{xbg + g.soff, NS});
-    if (!gs.sum<0>(nullptr, nullptr)) return;
+    if (!gs.template sum<0>(nullptr, nullptr)) return;
     sum[0] = 0.0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -274,7 +277,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
         sum[0] += a * a;
       }
     }
-    if (!gs.sum<1>(sum, tot)) return;
+    if (!gs.template sum<1>(sum, tot)) return;
     fin_true(S, tot[0], rechecks < max_rechecks ? 1 : 0);
     if (!S.active) break;
   }
@@ -290,7 +293,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
       if (realb[k]) x[c * NN + nk.node] = idle ? 0.0 : xb[k][c];
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) ks[inst] = S;
+  if (fb.lead && threadIdx.x == 0) ks[inst] = S;
 }
 
 }  // namespace tcad

@@ -1,7 +1,8 @@
 """The resident single-launch solves (one CTA per SM, rows in shared memory,
 vectors in registers) against the launch-per-step loops at the sizes where
-their layout changes: one and two slots per thread, rows in shared memory and
-not, a last block of a few slots, odd rows (pad slots), the smallest meshes.
+their layout changes: a cluster of 8 or 16 CTAs and the whole grid, one and two
+slots per thread, rows in shared memory and not, a last block of a few slots, odd
+rows (pad slots), the smallest meshes.
 Same bodies, scalar updates and order of sums: bit-identical."""
 import numpy as np
 import pytest
@@ -10,7 +11,8 @@ from test_gpu_redblack import _scaled_system, _solve_counted
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [("diode", (2, 2)), ("diode", (21, 10)), ("mosfet", (301, 260)), ("mosfet", (385, 385)),
+SIZES = [("diode", (2, 2)), ("diode", (21, 10)), ("diode", (126, 122)), ("diode", (129, 119)),
+         ("trigate", (31, 22, 16)), ("trigate", (32, 22, 16)), ("mosfet", (301, 260)), ("mosfet", (385, 385)),
          ("trigate", (9, 7, 5)), ("trigate", (57, 45, 39)), ("trigate", (56, 48, 46))]
 
 
@@ -39,7 +41,8 @@ def test_resident_schur_solve_bit_identical_to_per_step(kind, shape):
         assert nb == 2 and na > 2           # colour repack + the single launch
 
 
-@pytest.mark.parametrize("kind,shape", SIZES + [("diode", (301, 511)), ("trigate", (96, 57, 40)),
+@pytest.mark.parametrize("kind,shape", SIZES + [("diode", (257, 254)), ("diode", (261, 252)),
+                                                ("diode", (301, 511)), ("trigate", (96, 57, 40)),
                                                 ("trigate", (131, 80, 50))])
 def test_resident_equilibrium_bit_identical_to_per_step(kind, shape):
     """One to eight slots per thread; the whole equilibrium Newton."""
@@ -147,3 +150,27 @@ def test_streamed_schur_solve_meets_the_full_systems_test(devs):
             assert rel <= 1.01 * rtol
     x, it, st, rr = _batch_solve(pk, 1e-30, 17, 1)
     assert it == [17] * len(devs) and st == [_lib.TCAD_ERR_NOCONV] * len(devs)
+
+
+@pytest.mark.parametrize("devs", [[("diode", (21, 10)), ("mosfet", (64, 41)), ("diode", (2, 2))],
+                                  [("trigate", (9, 7, 5)), ("trigate", (24, 16, 13))],
+                                  [("trigate", (9, 7, 5)), ("trigate", (40, 24, 22))]],
+                         ids=lambda d: "+".join(str(q[1]) for q in d))
+def test_cluster_batches_equal_alone(devs):
+    """A cluster per instance (or, where one is too large for it, the per-step
+    kernels): equilibrium and the coupled solve of every instance as alone."""
+    import tcad_b200 as tb
+    from tcad_b200.batch import DeviceBatch
+    opts = tb.NewtonOptions(precond="block_jacobi")
+    b = DeviceBatch([_device(*d) for d in devs])
+    b.solve_equilibrium(opts)
+    eq = [b.state(i)[0] for i in range(len(devs))]
+    name = {"diode": "anode", "mosfet": "drain", "trigate": "drain"}
+    res = b.solve_bias([{name[d[0]]: 0.05} for d in devs], opts)
+    assert all(r["converged"] for r in res)
+    for i, d in enumerate(devs):
+        dev = _device(*d)
+        dev.solve_equilibrium(opts)
+        assert np.abs(dev.psi - eq[i]).max() * dev.VT < 1e-10, d
+        dev.solve_bias({name[d[0]]: 0.05}, opts)
+        assert np.abs(dev.psi - b.state(i)[0]).max() * dev.VT < 1e-9, d
