@@ -55,6 +55,13 @@ __device__ __forceinline__ void cp_async_wait_one() {
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
 }
 
+// What bounds it is instructions and their latency, not bytes (456 MB take 70 us on
+// the 983k-node tri-gate; 2,800 instructions per 32 nodes, FP64 pipe 21 %): the edges'
+// exponentials and divisions, so every quotient with a divisor used more than once --
+// the spacings (once per tile), the recombination's denominators -- is a product with
+// its reciprocal and a correction, and a tile's halo edges are one call of the edge
+// function.  tri-gate 160x96x64: 252 us with a division each, 183 now; MOSFET 256x128
+// (128 tiles): 14.3, 10.3.
 // CTAs per SM the coupled assembly is compiled for (register budget):
 // 4 in 2D (64 registers, no spills), 3 in 3D (80 registers; the z-march
 // carries two edges and two node states in registers, and at 64 registers
@@ -73,6 +80,9 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
   __shared__ uint8_t s_flag[TY + 2][TX + 2];
   __shared__ Edge s_ex[TY][TX + 1];  // x-edge slot a: nodes (i0-1+a, i0+a)
   __shared__ Edge s_ey[TY + 1][TX];  // y-edge slot b: nodes (j0-1+b, j0+b)
+  // the tile's spacings with their reciprocals, by edge slot; z: slot q & 1 for the
+  // edge below plane q
+  __shared__ Divisor s_hx[TX + 1], s_hy[TY + 1], s_hz[2];
 
   const int64_t t = tiles ? (int64_t)tiles[blockIdx.x] : (int64_t)blockIdx.x;
   const int inst = pk.tile[4 * t + 0], i0 = pk.tile[4 * t + 1];
@@ -88,6 +98,16 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
   const double* par = pk.par + TCAD_NPAR * inst;
   const int kend = DIM == 3 ? min(k0 + pk.tile_z, g.nz) : 1;
 
+  if (tid <= TX) {
+    const int q = i0 - 1 + tid;
+    s_hx[tid] = Divisor::of(q >= 0 && q + 1 < g.nx ? pk.h[0][ax0 + q] : 1.0);
+  } else if (tid >= 64 && tid <= 64 + TY) {
+    const int q = j0 - 1 + tid - 64;
+    s_hy[tid - 64] = Divisor::of(q >= 0 && q + 1 < g.ny ? pk.h[1][ay0 + q] : 1.0);
+  } else if (DIM == 3 && tid == 128) {
+    s_hz[k0 & 1] = Divisor::of(k0 > 0 ? pk.h[2][az0 + k0 - 1] : 1.0);
+  }
+
   // z-march registers (3D): own node values of the current / next plane
   NodeVals cur{0.0, 0.0, 0.0}, nxt{0.0, 0.0, 0.0};
   Edge eD, eU;
@@ -101,7 +121,7 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
     const int64_t q = g.off + (int64_t)k0 * sxy + (int64_t)j * g.nx + i;
     const int64_t ql = q - sxy;
     sg_edge(psi[ql], cur.psi, nn[ql], cur.n, pp[ql], cur.p, pk.an[2][ql], pk.ap[2][ql],
-            pk.dl[2][ql], pk.h[2][az0 + k0 - 1], eD);
+            pk.dl[2][ql], Divisor::of(pk.h[2][az0 + k0 - 1]), eD);
   }
 
   // this thread's share of plane kz's staging copies into buffer st: its own
@@ -158,6 +178,8 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
       else cp_async_commit();
     }
     // ---- stage the plane (tile + 1-node halo, no corners) in shared memory
+    if (DIM == 3 && tid == 128)
+      s_hz[(kz + 1) & 1] = Divisor::of(kz + 1 < g.nz ? pk.h[2][az0 + kz] : 1.0);
     s_psi[ty + 1][tx + 1] = cur.psi;
     s_n[ty + 1][tx + 1] = cur.n;
     s_p[ty + 1][tx + 1] = cur.p;
@@ -189,49 +211,37 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
     if constexpr (STAGED) cp_async_wait_one();   // this plane's copies (own thread)
     __syncthreads();
 
-    // ---- evaluate every edge touching the tile once
-    auto xedge = [&](int row, int a) {
-      const int ilo = i0 - 1 + a, jj = j0 + row;
+    // ---- evaluate every edge touching the tile once: edge(xed, r, c) is the x- or
+    // y-edge (xed) whose low node is row r, column c of the padded tile
+    auto edge = [&](bool xed, int r, int c) {
+      const int li = i0 - 1 + c, lj = j0 - 1 + r;
+      const bool on = xed ? li >= 0 && li + 1 < g.nx && lj < g.ny
+                          : lj >= 0 && lj + 1 < g.ny && li < g.nx;
       Edge e;
-      if (ilo >= 0 && ilo + 1 < g.nx && jj < g.ny) {
-        const int64_t q = plane + (int64_t)jj * g.nx + ilo;
+      if (on) {
+        const int64_t q = plane + (int64_t)lj * g.nx + li;
+        const int r1 = xed ? r : r + 1, c1 = xed ? c + 1 : c;
         double an, ap, dl;
         if constexpr (STAGED) {
-          an = stg->ax[0][row][a]; ap = stg->ax[1][row][a]; dl = stg->ax[2][row][a];
+          const double* const s = xed ? &stg->ax[0][r - 1][c] : &stg->ay[0][r][c - 1];
+          const int d = xed ? TY * (TX + 1) : (TY + 1) * TX;
+          an = s[0]; ap = s[d]; dl = s[2 * d];
         } else {
-          an = pk.an[0][q]; ap = pk.ap[0][q]; dl = pk.dl[0][q];
+          an = (xed ? pk.an[0] : pk.an[1])[q];
+          ap = (xed ? pk.ap[0] : pk.ap[1])[q];
+          dl = (xed ? pk.dl[0] : pk.dl[1])[q];
         }
-        sg_edge(s_psi[row + 1][a], s_psi[row + 1][a + 1], s_n[row + 1][a],
-                s_n[row + 1][a + 1], s_p[row + 1][a], s_p[row + 1][a + 1], an, ap, dl,
-                pk.h[0][ax0 + ilo], e);
+        sg_edge(s_psi[r][c], s_psi[r1][c1], s_n[r][c], s_n[r1][c1], s_p[r][c], s_p[r1][c1],
+                an, ap, dl, xed ? s_hx[c] : s_hy[r], e);
       } else {
         zero_edge(e);
       }
-      s_ex[row][a] = e;
+      *(xed ? &s_ex[r - 1][c] : &s_ey[r][c - 1]) = e;
     };
-    auto yedge = [&](int col, int b) {
-      const int jlo = j0 - 1 + b, ii = i0 + col;
-      Edge e;
-      if (jlo >= 0 && jlo + 1 < g.ny && ii < g.nx) {
-        const int64_t q = plane + (int64_t)jlo * g.nx + ii;
-        double an, ap, dl;
-        if constexpr (STAGED) {
-          an = stg->ay[0][b][col]; ap = stg->ay[1][b][col]; dl = stg->ay[2][b][col];
-        } else {
-          an = pk.an[1][q]; ap = pk.ap[1][q]; dl = pk.dl[1][q];
-        }
-        sg_edge(s_psi[b][col + 1], s_psi[b + 1][col + 1], s_n[b][col + 1],
-                s_n[b + 1][col + 1], s_p[b][col + 1], s_p[b + 1][col + 1], an, ap, dl,
-                pk.h[1][ay0 + jlo], e);
-      } else {
-        zero_edge(e);
-      }
-      s_ey[b][col] = e;
-    };
-    xedge(ty, tx + 1);  // own E edge
-    yedge(tx, ty + 1);  // own N edge
-    if (tid < TY) xedge(tid, 0);                        // tile's west halo edges
-    else if (tid < TY + TX) yedge(tid - TY, 0);         // tile's south halo edges
+    edge(true, ty + 1, tx + 1);   // own E edge
+    edge(false, ty + 1, tx + 1);  // own N edge
+    // the tile's west halo edges (threads 0..7) and south halo edges (8..39)
+    if (tid < TY + TX) edge(tid < TY, tid < TY ? tid + 1 : 0, tid < TY ? 0 : tid - TY + 1);
     if (DIM == 3) {
       if (own && kz + 1 < g.nz) {
         const int64_t q = plane + (int64_t)j * g.nx + i;
@@ -242,7 +252,7 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
           an = pk.an[2][q]; ap = pk.ap[2][q]; dl = pk.dl[2][q];
         }
         sg_edge(cur.psi, nxt.psi, cur.n, nxt.n, cur.p, nxt.p, an, ap, dl,
-                pk.h[2][az0 + kz], eU);
+                s_hz[(kz + 1) & 1], eU);
       } else {
         zero_edge(eU);
       }
@@ -276,9 +286,6 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
         const Edge& E = s_ex[ty][tx + 1];
         const Edge& S = s_ey[ty][tx];
         const Edge& N = s_ey[ty + 1][tx];
-        const double hW = vW ? pk.h[0][ax0 + i - 1] : 1.0, hE = vE ? pk.h[0][ax0 + i] : 1.0;
-        const double hS = vS ? pk.h[1][ay0 + j - 1] : 1.0, hN = vN ? pk.h[1][ay0 + j] : 1.0;
-        const double hD = vD ? pk.h[2][az0 + kz - 1] : 1.0, hU = vU ? pk.h[2][az0 + kz] : 1.0;
         // divergences: div[lo] += f; div[hi] -= f  (device2d.py:1512-1525)
         double f0, f1, f2;
         {
@@ -312,27 +319,27 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
         // diagonal block, summed in the reference's stamp order per axis
         // (low-role edge first, then high-role edge)
         double d00 = 0.0, d10 = 0.0, d11 = 0.0, d20 = 0.0, d22 = 0.0;
-        auto lo_role = [&](const Edge& e, double face, double h) {  // node = low end
-          d00 = d00 + (-(face / h));
+        auto lo_role = [&](const Edge& e, double face, const Divisor& h) {  // node = low end
+          d00 = d00 + (-h.divide(face));
           d10 = d10 + (-(face * e.npsi));
           d11 = d11 + face * e.nlo;
           d20 = d20 + (-(face * e.ppsi));
           d22 = d22 + face * e.plo;
         };
-        auto hi_role = [&](const Edge& e, double face, double h) {  // node = high end
-          d00 = d00 + (-(face / h));
+        auto hi_role = [&](const Edge& e, double face, const Divisor& h) {  // node = high end
+          d00 = d00 + (-h.divide(face));
           d10 = d10 + (-(face * e.npsi));
           d11 = d11 + (-face) * e.nhi;
           d20 = d20 + (-(face * e.ppsi));
           d22 = d22 + (-face) * e.phi;
         };
-        if (vE) lo_role(E, fx, hE);
-        if (vW) hi_role(W, fx, hW);
-        if (vN) lo_role(N, fy, hN);
-        if (vS) hi_role(S, fy, hS);
+        if (vE) lo_role(E, fx, s_hx[tx + 1]);
+        if (vW) hi_role(W, fx, s_hx[tx]);
+        if (vN) lo_role(N, fy, s_hy[ty + 1]);
+        if (vS) hi_role(S, fy, s_hy[ty]);
         if (DIM == 3) {
-          if (vU) lo_role(eU, fz, hU);
-          if (vD) hi_role(eD, fz, hD);
+          if (vU) lo_role(eU, fz, s_hz[(kz + 1) & 1]);
+          if (vD) hi_role(eD, fz, s_hz[kz & 1]);
         }
         d11 = d11 + (-dRsn) * dV;
         d22 = d22 + dRsp * dV;
@@ -347,11 +354,11 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
         // off-diagonal blocks, W,E,S,N,D,U; in ELIMINATE mode a contact
         // neighbour's known update is folded into F and its block emptied
         const bool elim = mode == TCAD_MODE_ELIMINATE;
-        auto emit = [&](int d, bool valid, bool lo_end, const Edge& e, double face, double h,
-                        uint8_t nflag, int64_t m) {
+        auto emit = [&](int d, bool valid, bool lo_end, const Edge& e, double face,
+                        const Divisor& h, uint8_t nflag, int64_t m) {
           double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, a4 = 0.0;
           if (valid) {
-            a0 = face / h;
+            a0 = h.divide(face);
             a1 = face * e.npsi;
             a3 = face * e.ppsi;
             if (lo_end) { a2 = face * e.nhi; a4 = face * e.phi; }          // nbr = high end
@@ -369,13 +376,13 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
           st(nb(d, 0), a0); st(nb(d, 1), a1); st(nb(d, 2), a2); st(nb(d, 3), a3);
           st(nb(d, 4), a4);
         };
-        emit(0, vW, false, W, fx, hW, s_flag[ty + 1][tx], k - 1);
-        emit(1, vE, true, E, fx, hE, s_flag[ty + 1][tx + 2], k + 1);
-        emit(2, vS, false, S, fy, hS, s_flag[ty][tx + 1], k - g.nx);
-        emit(3, vN, true, N, fy, hN, s_flag[ty + 2][tx + 1], k + g.nx);
+        emit(0, vW, false, W, fx, s_hx[tx], s_flag[ty + 1][tx], k - 1);
+        emit(1, vE, true, E, fx, s_hx[tx + 1], s_flag[ty + 1][tx + 2], k + 1);
+        emit(2, vS, false, S, fy, s_hy[ty], s_flag[ty][tx + 1], k - g.nx);
+        emit(3, vN, true, N, fy, s_hy[ty + 1], s_flag[ty + 2][tx + 1], k + g.nx);
         if (DIM == 3) {
-          emit(4, vD, false, eD, fz, hD, vD ? pk.bcflag[k - sxy] : 0, k - sxy);
-          emit(5, vU, true, eU, fz, hU, vU ? pk.bcflag[k + sxy] : 0, k + sxy);
+          emit(4, vD, false, eD, fz, s_hz[kz & 1], vD ? pk.bcflag[k - sxy] : 0, k - sxy);
+          emit(5, vU, true, eU, fz, s_hz[(kz + 1) & 1], vU ? pk.bcflag[k + sxy] : 0, k + sxy);
         }
         F[k] = F0;
         F[NN + k] = F1;
@@ -431,14 +438,14 @@ __global__ void k_contact_current(const tcad_pack_t pk, const double* __restrict
       const int64_t m = k + stride[a];
       Edge e;
       sg_edge(psi[k], psi[m], nn[k], nn[m], pp[k], pp[m], pk.an[a][k], pk.ap[a][k],
-              pk.dl[a][k], pk.h[a][aoff[a] + coord[a]], e);
+              pk.dl[a][k], Divisor::of(pk.h[a][aoff[a] + coord[a]]), e);
       dn = dn + e.Jn; dp = dp + e.Jp;
     }
     if (coord[a] >= 1) {             // edge from the low neighbour (node = high end)
       const int64_t m = k - stride[a];
       Edge e;
       sg_edge(psi[m], psi[k], nn[m], nn[k], pp[m], pp[k], pk.an[a][m], pk.ap[a][m],
-              pk.dl[a][m], pk.h[a][aoff[a] + coord[a] - 1], e);
+              pk.dl[a][m], Divisor::of(pk.h[a][aoff[a] + coord[a] - 1]), e);
       dn = dn - e.Jn; dp = dp - e.Jp;
     }
     tn = a == 0 ? face[a] * dn : tn + face[a] * dn;
@@ -481,7 +488,7 @@ __global__ void k_edge_currents(const tcad_pack_t pk, int axis,
       const int64_t m = k + stride;
       Edge e;
       sg_edge(psi[k], psi[m], nn[k], nn[m], pp[k], pp[m], pk.an[axis][k], pk.ap[axis][k],
-              pk.dl[axis][k], pk.h[axis][aoff + c], e);
+              pk.dl[axis][k], Divisor::of(pk.h[axis][aoff + c]), e);
       a = e.Jn; b = e.Jp;
     }
     Jn[k] = a;

@@ -12,10 +12,42 @@ __device__ __forceinline__ double clip700(double x) {
   return x < -700.0 ? -700.0 : (x > 700.0 ? 700.0 : x);
 }
 
-// B(x) and B'(x) of the series branch |x| < 1e-4 (kernels.py:92-96,105-109).
-__device__ __forceinline__ void bern_series(double x, double& B, double& dB) {
-  B = (1.0 - x / 2.0) + (x * x) / 12.0;
-  dB = (-0.5 + x / 6.0) - (x * x * x) / 180.0;
+// a / b from r = 1/b, bit for bit (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990: with r the rounded
+// reciprocal, one residual correction of a r gives the rounded quotient, barring
+// underflow and overflow).
+__device__ __forceinline__ double div_in_range(double a, double b, double r) {
+  const double q = a * r;
+  return fma(fma(-q, b, a), r, q);
+}
+// ... of any a: where a or the quotient is zero, infinite, NaN or of a magnitude near
+// the end of the range it is a r.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+  const double q = a * r;
+  const double c = fma(fma(-q, b, a), r, q);
+  return fabs(a) > 1e-270 && fabs(q) > 1e-270 && fabs(q) < 1e270 ? c : q;
+}
+
+// A divisor of several quotients and its reciprocal.
+struct Divisor {
+  double b, r;
+  static __device__ __forceinline__ Divisor of(double b) { return Divisor{b, 1.0 / b}; }
+  __device__ __forceinline__ double divide(double a) const { return div_by(a, b, r); }
+};
+
+// B(x), B'(x) and those of -x of the series band |x| < 1e-4 (kernels.py:92-96,
+// 105-109), B = (1 - x/2) + x^2/12 and B' = (-1/2 + x/6) - x^3/180; the terms of
+// -x are those of x or their negatives.  (A quotient that underflows is far below
+// the last bit of the sum it is added to.)
+__device__ __forceinline__ void bern_series(double x, double& Bp, double& Bm, double& dBp,
+                                            double& dBm) {
+  const double x2 = div_in_range(x * x, 12.0, 1.0 / 12.0);
+  const double x1 = div_in_range(x, 6.0, 1.0 / 6.0);
+  const double x3 = div_in_range(x * x * x, 180.0, 1.0 / 180.0);
+  Bp = (1.0 - x / 2.0) + x2;
+  Bm = (1.0 + x / 2.0) + x2;
+  dBp = (-0.5 + x1) - x3;
+  dBm = (-0.5 - x1) + x3;
 }
 
 // B(x), B(-x), B'(x), B'(-x).  Three argument bands:
@@ -38,25 +70,32 @@ __device__ __forceinline__ void bern_series(double x, double& B, double& dB) {
 //                       values agree with the reference's formulas to a few
 //                       ulp (derivatives within 1e-13 relative; measured
 //                       over 4e5 arguments against kernels.py).
+//
+// The lanes of a warp are seldom in one band and an edge is mostly its
+// exponentials and divisions, so the last two bands share one expm1 and its
+// reciprocal, and quotients with a divisor whose reciprocal is at hand (or a
+// constant) are a product and its correction: a mixed warp runs 2 expm1 and 3
+// divisions (3 and 12 band by band).
 __device__ __forceinline__ void bern4(double x, double& Bp, double& Bm, double& dBp,
                                       double& dBm) {
   x = clip700(x);
   const double a = fabs(x);
   if (a < 1e-4) {
-    bern_series(x, Bp, dBp);
-    bern_series(-x, Bm, dBm);
+    bern_series(x, Bp, Bm, dBp, dBm);
     return;
   }
-  if (a < 1e-2) {
-    const double ep = expm1(x), em = expm1(-x);
-    Bp = x / ep;
-    Bm = (-x) / em;
-    dBp = Bp * (1.0 / x - 1.0 / (-em));
-    dBm = Bm * (1.0 / (-x) - 1.0 / (-ep));
-    return;
-  }
-  const double e = expm1(a);
+  const bool mid = a < 1e-2;
+  const double e = expm1(mid ? x : a);
   const double r = 1.0 / e;
+  if (mid) {
+    const double em = expm1(-x);
+    const double rm = 1.0 / em, rx = 1.0 / x;
+    Bp = div_in_range(x, e, r);
+    Bm = div_in_range(-x, em, rm);
+    dBp = Bp * (rx + rm);    // B (1/x - 1/(1 - e^-x)), 1 - e^-x = -em
+    dBm = Bm * (r - rx);
+    return;
+  }
   const double r1 = 1.0 + r;
   const double S = a * r;
   const double L = S + a;
@@ -90,9 +129,9 @@ __device__ __forceinline__ void zero_edge(Edge& e) {
 // pytcad/device2d.py:1451-1479.
 __device__ __forceinline__ void sg_edge(double psi_lo, double psi_hi, double n_lo,
                                         double n_hi, double p_lo, double p_hi, double an,
-                                        double ap, double dl, double h, Edge& e) {
+                                        double ap, double dl, Divisor h, Edge& e) {
   const double dpsi = psi_hi - psi_lo;
-  e.f = dpsi / h;
+  e.f = h.divide(dpsi);
   double Bp, Bm, dBp, dBm, Bph, Bmh, dBph, dBmh;
   bern4(dpsi + dl, Bp, Bm, dBp, dBm);
   if (dl == 0.0) {
@@ -129,8 +168,9 @@ __device__ __forceinline__ void recomb(double n, double p, double nie, double ta
   const double den = taup * (nph + nie) + taun * (pph + nie);
   double R = excess / den;
   const double den2 = den * den;
-  double dRdn = (pph * den - excess * taup) / den2;
-  double dRdp = (nph * den - excess * taun) / den2;
+  const Divisor by2 = Divisor::of(den2);
+  double dRdn = by2.divide(pph * den - excess * taup);
+  double dRdp = by2.divide(nph * den - excess * taun);
   if (par[TCAD_P_AUGER] != 0.0) {
     const double Cn = par[TCAD_P_CN], Cp = par[TCAD_P_CP];
     const double cc = Cn * nph + Cp * pph;
@@ -138,9 +178,10 @@ __device__ __forceinline__ void recomb(double n, double p, double nie, double ta
     dRdn = dRdn + Cn * excess + cc * pph;
     dRdp = dRdp + Cp * excess + cc * nph;
   }
-  Rs = R / R0;
-  dRsn = dRdn * Ns / R0;
-  dRsp = dRdp * Ns / R0;
+  const Divisor by0 = Divisor::of(R0);
+  Rs = by0.divide(R);
+  dRsn = by0.divide(dRdn * Ns);
+  dRsp = by0.divide(dRdp * Ns);
 }
 
 }  // namespace tcad
