@@ -399,15 +399,43 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
 
 // ---------------------------------------------------------------------------
 // raw continuity residual F_n + F_p at listed nodes (terminal currents)
+//
+// A contact has tens to hundreds of nodes, so its current is latency: the chain of one
+// node and the launches.  An edge goes to a lane of its own (2D: 4 lanes a node, 3D: 8
+// of which 6 have one) and not to a thread's loop, and a list that a thread-block
+// cluster takes (up to 8 CTAs: 512 nodes in 2D, 256 in 3D) is summed by the same
+// launch; a longer one by k_sum_list, in the same order.  Two contacts of a 201x101
+// diode read one after the other: 66 us with a thread per node and two launches each,
+// 56 now, the rest the two copies back and their synchronisations.
+constexpr int kCurThreads = 256;
+constexpr int kCurCluster = 8;
 template <int DIM>
-__global__ void k_contact_current(const tcad_pack_t pk, const double* __restrict__ psi,
-                                  const double* __restrict__ nn,
-                                  const double* __restrict__ pp,
-                                  const int64_t* __restrict__ nodes, int64_t count,
-                                  double* __restrict__ out) {
-  // out[t] = raw F_n, out[count + t] = raw F_p of node nodes[t]
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
+constexpr int kCurLanes = DIM == 2 ? 4 : 8;
+
+// fixed-order sum of vals[0..count) + vals[count..2 count) by one block
+__device__ __forceinline__ void sum_list(const double* vals, int64_t count, double* out) {
+  __shared__ double sm[32];
+  double s = 0.0;
+  for (int64_t q = threadIdx.x; q < count; q += kCurThreads) s += vals[q] + vals[count + q];
+  const double r = block_sum<kCurThreads>(s, sm);
+  if (threadIdx.x == 0) out[0] = r;
+}
+__global__ void k_sum_list(const double* vals, int64_t count, double* out) {
+  sum_list(vals, count, out);
+}
+
+// out[t] = raw F_n, out[count + t] = raw F_p of node nodes[t] (count > 0); SUM (the
+// grid is one cluster): out_sum[0] = their sum
+template <int DIM, bool SUM>
+__global__ void __launch_bounds__(kCurThreads)
+k_contact_current(const tcad_pack_t pk, const double* __restrict__ psi,
+                  const double* __restrict__ nn, const double* __restrict__ pp,
+                  const int64_t* __restrict__ nodes, int64_t count, double* out,
+                  double* out_sum) {
+  constexpr int LANES = kCurLanes<DIM>;
+  const int64_t slot = ((int64_t)blockIdx.x * kCurThreads + threadIdx.x) / LANES;
+  const int64_t t = slot < count ? slot : count - 1;
+  const int edge = threadIdx.x % LANES, a = edge >> 1;   // axis; even: to the high neighbour
   const int64_t k = nodes[t];
   // locate the instance by a binary search on node_off
   int lo = 0, hi = pk.n_inst;
@@ -416,55 +444,86 @@ __global__ void k_contact_current(const tcad_pack_t pk, const double* __restrict
     if (pk.node_off[mid] <= k) lo = mid; else hi = mid;
   }
   const Inst g = load_inst(pk, lo);
-  const int64_t loc = k - g.off;
-  const int64_t sxy = (int64_t)g.nx * g.ny;
-  const int i = (int)(loc % g.nx), j = (int)((loc / g.nx) % g.ny);
-  const int kz = DIM == 3 ? (int)(loc / sxy) : 0;
-  const int64_t ax0 = pk.axis_off[3 * lo], ay0 = pk.axis_off[3 * lo + 1];
-  const int64_t az0 = pk.axis_off[3 * lo + 2];
-  const double* par = pk.par + TCAD_NPAR * lo;
-  const double dvx = pk.dv[0][ax0 + i], dvy = pk.dv[1][ay0 + j];
-  const double dvz = DIM == 3 ? pk.dv[2][az0 + kz] : 1.0;
+  const int loc = (int)(k - g.off);   // (an instance has fewer than 2^31 nodes)
+  const int sxy = g.nx * g.ny;
+  const int kz = DIM == 3 ? loc / sxy : 0;
+  const int j = (loc - kz * sxy) / g.nx, i = loc - kz * sxy - j * g.nx;
+  const int64_t* const aoff = pk.axis_off + 3 * lo;
+  const double dvx = pk.dv[0][aoff[0] + i], dvy = pk.dv[1][aoff[1] + j];
+  const double dvz = DIM == 3 ? pk.dv[2][aoff[2] + kz] : 1.0;
   const double face[3] = {DIM == 2 ? dvy : dvy * dvz, DIM == 2 ? dvx : dvx * dvz, dvx * dvy};
   const double dV = DIM == 2 ? dvy * dvx : (dvz * dvy) * dvx;
-  const int coord[3] = {i, j, kz};
-  const int extent[3] = {g.nx, g.ny, g.nz};
-  const int64_t stride[3] = {1, g.nx, sxy};
-  const int64_t aoff[3] = {ax0, ay0, az0};
-  double tn = 0.0, tp = 0.0;
-  for (int a = 0; a < DIM; ++a) {
-    double dn = 0.0, dp = 0.0;
-    if (coord[a] + 1 < extent[a]) {  // edge to the high neighbour (node = low end)
-      const int64_t m = k + stride[a];
+  double Jn = 0.0, Jp = 0.0;
+  if (a < DIM) {
+    const int c = a == 0 ? i : (a == 1 ? j : kz);
+    const int extent = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
+    const int64_t stride = a == 0 ? 1 : (a == 1 ? g.nx : sxy);
+    const bool up = (edge & 1) == 0;
+    if (up ? c + 1 < extent : c >= 1) {
+      const int64_t l = up ? k : k - stride, m = l + stride;   // its low and high node
       Edge e;
-      sg_edge(psi[k], psi[m], nn[k], nn[m], pp[k], pp[m], pk.an[a][k], pk.ap[a][k],
-              pk.dl[a][k], Divisor::of(pk.h[a][aoff[a] + coord[a]]), e);
-      dn = dn + e.Jn; dp = dp + e.Jp;
+      sg_edge(psi[l], psi[m], nn[l], nn[m], pp[l], pp[m], pk.an[a][l], pk.ap[a][l],
+              pk.dl[a][l], Divisor::of(pk.h[a][aoff[a] + c - (up ? 0 : 1)]), e);
+      Jn = e.Jn; Jp = e.Jp;
     }
-    if (coord[a] >= 1) {             // edge from the low neighbour (node = high end)
-      const int64_t m = k - stride[a];
-      Edge e;
-      sg_edge(psi[m], psi[k], nn[m], nn[k], pp[m], pp[k], pk.an[a][m], pk.ap[a][m],
-              pk.dl[a][m], Divisor::of(pk.h[a][aoff[a] + coord[a] - 1]), e);
-      dn = dn - e.Jn; dp = dp - e.Jp;
-    }
-    tn = a == 0 ? face[a] * dn : tn + face[a] * dn;
-    tp = a == 0 ? face[a] * dp : tp + face[a] * dp;
   }
   double Rs, dRsn, dRsp;
-  recomb(nn[k], pp[k], pk.nie[k], pk.tau_n[k], pk.tau_p[k], par, Rs, dRsn, dRsp);
-  out[t] = tn - Rs * dV;
-  out[count + t] = tp + Rs * dV;
+  recomb(nn[k], pp[k], pk.nie[k], pk.tau_n[k], pk.tau_p[k], pk.par + TCAD_NPAR * lo, Rs, dRsn,
+         dRsp);
+  // the node's sums, axis by axis (an edge that is not there adds a zero)
+  double tn = 0.0, tp = 0.0;
+#pragma unroll
+  for (int q = 0; q < DIM; ++q) {
+    const double dn = (0.0 + __shfl_sync(0xffffffffu, Jn, 2 * q, LANES)) -
+                      __shfl_sync(0xffffffffu, Jn, 2 * q + 1, LANES);
+    const double dp = (0.0 + __shfl_sync(0xffffffffu, Jp, 2 * q, LANES)) -
+                      __shfl_sync(0xffffffffu, Jp, 2 * q + 1, LANES);
+    tn = q == 0 ? face[q] * dn : tn + face[q] * dn;
+    tp = q == 0 ? face[q] * dp : tp + face[q] * dp;
+  }
+  if (edge == 0 && slot < count) {
+    out[t] = tn - Rs * dV;
+    out[count + t] = tp + Rs * dV;
+  }
+  if constexpr (SUM) {
+    asm volatile(
+        "barrier.cluster.arrive.release.aligned;\n\t"
+        "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (blockIdx.x == 0) sum_list(out, count, out_sum);
+  }
 }
 
-// fixed-order sum of vals[0..count) by one block
-__global__ void k_sum_list(const double* __restrict__ vals, int64_t count,
-                           double* __restrict__ out) {
-  __shared__ double sm[32];
-  double s = 0.0;
-  for (int64_t q = threadIdx.x; q < count; q += blockDim.x) s += vals[q] + vals[count + q];
-  const double r = block_sum<256>(s, sm);
-  if (threadIdx.x == 0) out[0] = r;
+template <int DIM>
+static int contact_current(const tcad_pack_t& pk, const double* psi, const double* n,
+                           const double* p, const int64_t* nodes, int64_t count,
+                           double* partial, double* out_sum, cudaStream_t s) {
+  const int64_t blocks = (count * kCurLanes<DIM> + kCurThreads - 1) / kCurThreads;
+  if (blocks >= 1 && blocks <= kCurCluster) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kCurThreads);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    TCAD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_contact_current<DIM, true>, pk, psi, n, p, nodes,
+                                       count, partial, out_sum));
+    note_launch();
+    return TCAD_OK;
+  }
+  if (count > 0) {
+    k_contact_current<DIM, false><<<(unsigned)blocks, kCurThreads, 0, s>>>(
+        pk, psi, n, p, nodes, count, partial, nullptr);
+    note_launch();
+    TCAD_LAUNCH_CHECK();
+  }
+  k_sum_list<<<1, kCurThreads, 0, s>>>(partial, count, out_sum);
+  note_launch();
+  TCAD_LAUNCH_CHECK();
+  return TCAD_OK;
 }
 
 template <int DIM>
@@ -727,20 +786,8 @@ extern "C" int tcad_contact_current(const tcad_pack_t* pk, const double* psi,
                                     const int64_t* nodes, int64_t count, double* partial,
                                     int64_t partial_len, double* out_sum, void* stream) {
   if (!pack_ok(pk) || count < 0 || partial_len < 2 * count) return TCAD_ERR_ARG;
-  cudaStream_t s = (cudaStream_t)stream;
-  if (count > 0) {
-    const unsigned nb_ = (unsigned)((count + 255) / 256);
-    if (pk->dim == 2)
-      k_contact_current<2><<<nb_, 256, 0, s>>>(*pk, psi, n, p, nodes, count, partial);
-    else
-      k_contact_current<3><<<nb_, 256, 0, s>>>(*pk, psi, n, p, nodes, count, partial);
-    note_launch();
-    TCAD_LAUNCH_CHECK();
-  }
-  k_sum_list<<<1, 256, 0, s>>>(partial, count, out_sum);
-  note_launch();
-  TCAD_LAUNCH_CHECK();
-  return TCAD_OK;
+  return (pk->dim == 2 ? contact_current<2> : contact_current<3>)(
+      *pk, psi, n, p, nodes, count, partial, out_sum, (cudaStream_t)stream);
 }
 
 extern "C" int tcad_edge_currents(const tcad_pack_t* pk, int axis, const double* psi,
