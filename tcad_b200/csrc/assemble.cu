@@ -61,18 +61,27 @@ __device__ __forceinline__ void cp_async_wait_one() {
 // the spacings (once per tile), the recombination's denominators -- is a product with
 // its reciprocal and a correction, and a tile's halo edges are one call of the edge
 // function.  tri-gate 160x96x64: 252 us with a division each, 183 now; MOSFET 256x128
-// (128 tiles): 14.3, 10.3.
+// (128 tiles): 14.3, 10.3 (9.9 with WIDE below, where the call takes longer than the
+// kernel).
 // CTAs per SM the coupled assembly is compiled for (register budget):
 // 4 in 2D (64 registers, no spills), 3 in 3D (80 registers; the z-march
 // carries two edges and two node states in registers, and at 64 registers
 // the spills cost more than the fourth CTA gains)
-template <int DIM, bool STAGED>
-__global__ void __launch_bounds__(kTileThreads, DIM == 2 ? 4 : (STAGED ? 2 : 3))
+// WIDE (2D, up to a tile per SM): a thread for every edge of the tile instead of its E,
+// N and halo edge one after the other; with one CTA an SM its latency is all there is
+// (128 tiles: 8.8 us, WIDE 6.6; 144: 8.8, 6.7), with more the narrow CTAs run together
+// (150 tiles: 8.7, WIDE 10.2; 512: 14.5, 22.2).
+constexpr unsigned kWideTiles = 148;
+constexpr int kWideThreads = (2 * TX * TY + TX + TY + 31) / 32 * 32;
+template <int DIM, bool STAGED, bool WIDE = false>
+__global__ void __launch_bounds__(WIDE ? kWideThreads : kTileThreads,
+                                  WIDE ? 1 : DIM == 2 ? 4 : (STAGED ? 2 : 3))
 k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
               const double* __restrict__ nn, const double* __restrict__ pp,
               double* __restrict__ F, double* __restrict__ J, int mode,
               const int32_t* __restrict__ tiles) {
   static_assert(DIM == 3 || !STAGED, "plane staging is the 3D z-march's");
+  static_assert(DIM == 2 || !WIDE, "the z-march keeps a thread per node");
   constexpr int NE = DIM == 2 ? TCAD_NE2 : TCAD_NE3;
   extern __shared__ __align__(16) unsigned char s_dyn[];
   PlaneStage* const stage = reinterpret_cast<PlaneStage*>(s_dyn);
@@ -90,7 +99,7 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
   const Inst g = load_inst(pk, inst);
   const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
   const int i = i0 + tx, j = j0 + ty;
-  const bool own = (i < g.nx) && (j < g.ny);
+  const bool own = (!WIDE || ty < TY) && (i < g.nx) && (j < g.ny);
   const int64_t ax0 = pk.axis_off[3 * inst], ay0 = pk.axis_off[3 * inst + 1];
   const int64_t az0 = pk.axis_off[3 * inst + 2];
   const int64_t sxy = (int64_t)g.nx * g.ny;
@@ -180,17 +189,21 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
     // ---- stage the plane (tile + 1-node halo, no corners) in shared memory
     if (DIM == 3 && tid == 128)
       s_hz[(kz + 1) & 1] = Divisor::of(kz + 1 < g.nz ? pk.h[2][az0 + kz] : 1.0);
-    s_psi[ty + 1][tx + 1] = cur.psi;
-    s_n[ty + 1][tx + 1] = cur.n;
-    s_p[ty + 1][tx + 1] = cur.p;
-    s_flag[ty + 1][tx + 1] = own ? pk.bcflag[plane + (int64_t)j * g.nx + i] : 0;
-    if (tid < 2 * TY + 2 * TX) {
+    if (!WIDE || ty < TY) {
+      s_psi[ty + 1][tx + 1] = cur.psi;
+      s_n[ty + 1][tx + 1] = cur.n;
+      s_p[ty + 1][tx + 1] = cur.p;
+      s_flag[ty + 1][tx + 1] = own ? pk.bcflag[plane + (int64_t)j * g.nx + i] : 0;
+    }
+    // (the halo's threads: with WIDE those that have no node)
+    const int hid = WIDE ? tid - kTileThreads : tid;
+    if (hid >= 0 && hid < 2 * TY + 2 * TX) {
       int r, c, hi, hj;
-      if (tid < 2 * TY) {  // x halo: columns 0 and TX+1
-        r = 1 + (tid >> 1);
-        c = (tid & 1) ? TX + 1 : 0;
+      if (hid < 2 * TY) {  // x halo: columns 0 and TX+1
+        r = 1 + (hid >> 1);
+        c = (hid & 1) ? TX + 1 : 0;
       } else {             // y halo: rows 0 and TY+1
-        const int u = tid - 2 * TY;
+        const int u = hid - 2 * TY;
         c = 1 + (u >> 1);
         r = (u & 1) ? TY + 1 : 0;
       }
@@ -238,10 +251,19 @@ k_sg_assemble(const tcad_pack_t pk, const double* __restrict__ psi,
       }
       *(xed ? &s_ex[r - 1][c] : &s_ey[r][c - 1]) = e;
     };
-    edge(true, ty + 1, tx + 1);   // own E edge
-    edge(false, ty + 1, tx + 1);  // own N edge
-    // the tile's west halo edges (threads 0..7) and south halo edges (8..39)
-    if (tid < TY + TX) edge(tid < TY, tid < TY ? tid + 1 : 0, tid < TY ? 0 : tid - TY + 1);
+    // the tile's halo edge number w: west (0..7), then south (8..39)
+    auto halo_row = [&](int w) { return w < TY ? w + 1 : 0; };
+    auto halo_col = [&](int w) { return w < TY ? 0 : w - TY + 1; };
+    if constexpr (WIDE) {   // warps 0..7 the E edges, 8..15 the N edges, then the halo
+      const int part = tid / kTileThreads, w = tid - 2 * kTileThreads;
+      const int r = part < 2 ? ty - part * TY + 1 : halo_row(w);
+      const int c = part < 2 ? tx + 1 : halo_col(w);
+      if (w < TX + TY) edge(part == 0 || (part == 2 && w < TY), r, c);
+    } else {
+      edge(true, ty + 1, tx + 1);   // own E edge
+      edge(false, ty + 1, tx + 1);  // own N edge
+      if (tid < TY + TX) edge(tid < TY, halo_row(tid), halo_col(tid));
+    }
     if (DIM == 3) {
       if (own && kz + 1 < g.nz) {
         const int64_t q = plane + (int64_t)j * g.nx + i;
@@ -753,7 +775,9 @@ int sg_assemble_tiles(const tcad_pack_t* pk, const double* psi, const double* n,
   if (!pack_ok(pk) || pk->n_tiles <= 0) return TCAD_ERR_ARG;
   const unsigned nt = (unsigned)(tiles ? n_list : pk->n_tiles);
   if (nt == 0) return TCAD_OK;
-  if (pk->dim == 2) {
+  if (pk->dim == 2 && nt <= kWideTiles) {
+    k_sg_assemble<2, false, true><<<nt, kWideThreads, 0, s>>>(*pk, psi, n, p, F, J, mode, tiles);
+  } else if (pk->dim == 2) {
     k_sg_assemble<2, false><<<nt, kTileThreads, 0, s>>>(*pk, psi, n, p, F, J, mode, tiles);
   } else if (pk->asm_stage) {
     TCAD_CUDA_CHECK(cudaFuncSetAttribute(k_sg_assemble<3, true>,
