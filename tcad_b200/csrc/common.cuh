@@ -19,6 +19,42 @@ namespace tcad {
 // Count of kernels this library launched (defined in capi.cu).
 void note_launch(uint64_t n = 1);
 
+// ---- programmatic dependent launch
+// A kernel of a chain lets the next one's CTAs start where SMs are free, then waits
+// for the kernels before it (what they wrote is visible then).  Every kernel that
+// launch_chained() starts waits, so a kernel that passed its wait follows all that
+// came before.  What a chained kernel reads before its wait, or through a pointer
+// that lets the compiler move the load there (__restrict__), must be older than the
+// kernel before it.  (Iterations of five to eleven launches of 2 to 10 us each, small
+// systems: GMRES of 13.8k unknowns 37 -> 31 us an iteration; BiCGStab with ILU(0) of 16
+// MOSFETs 207 -> 193.)
+__device__ __forceinline__ void launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_prior() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void chain_in() {
+  launch_dependents();
+  wait_prior();
+}
+// (an error is also the stream's last error, as for <<< >>>)
+template <class... P, class... A>
+inline cudaError_t launch_chained(cudaStream_t s, unsigned grid, unsigned block, size_t smem,
+                                  void (*kern)(P...), A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 constexpr int kFlatThreads = 256;
 constexpr int kTileThreads = TCAD_TILE_X * TCAD_TILE_Y;           // 256
 

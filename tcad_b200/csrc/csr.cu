@@ -30,8 +30,8 @@ struct Sys {
   const double* val;
 };
 
-__global__ void __launch_bounds__(NT) k_spmv(Sys A, const double* __restrict__ x,
-                                             double* __restrict__ y) {
+__global__ void __launch_bounds__(NT) k_spmv(Sys A, const double* x, double* y) {
+  chain_in();
   const int64_t row = (int64_t)blockIdx.x * kRowsPerBlock + (threadIdx.x >> 3);
   const int lane = threadIdx.x & 7;
   double s = 0.0;
@@ -378,6 +378,7 @@ __device__ __forceinline__ double gm_minus(const Gmres& G, int nv, const double*
 
 template <bool SUB>
 __global__ void __launch_bounds__(NTG) k_gm_dots(Gmres G) {
+  chain_in();
   __shared__ double sw[NT], s4[4][NT];
   if (G.st->done || G.st->j >= G.m) return;
   const int nv = G.st->j + 1;
@@ -399,6 +400,7 @@ __global__ void __launch_bounds__(NTG) k_gm_dots(Gmres G) {
 }
 
 __global__ void __launch_bounds__(NTG) k_gm_norm(Gmres G, double tol) {
+  chain_in();
   __shared__ double s4[4][NT];
   if (G.st->done || G.st->j >= G.m) return;
   const int j = G.st->j;
@@ -449,7 +451,8 @@ __global__ void __launch_bounds__(NTG) k_gm_norm(Gmres G, double tol) {
 
 // V_j = w inv (j the new column), z = M^-1 V_j
 __global__ void __launch_bounds__(NT) k_gm_next(Gmres G, int bs, const double* __restrict__ inv,
-                                                double* __restrict__ z) {
+                                                double* z) {
+  chain_in();
   if (G.st->done || G.st->j >= G.m) return;
   const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
   const int b = bs > 1 ? bs : 1;
@@ -496,6 +499,7 @@ __device__ __forceinline__ void bi_top(BState& st, double rhr, double tol, int m
 
 // p = r + beta p - beta omega v, ph = M^-1 p
 __global__ void __launch_bounds__(NT) k_cb_p(Bicg B, int bs, const double* __restrict__ inv) {
+  chain_in();
   const BState st = *B.st;
   if (st.done) return;
   const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
@@ -514,6 +518,7 @@ __global__ void __launch_bounds__(NT) k_cb_p(Bicg B, int bs, const double* __res
 
 // s = r - alpha v, sh = M^-1 s; (s, s): early exit
 __global__ void __launch_bounds__(NT) k_cb_s(Bicg B, int bs, const double* __restrict__ inv) {
+  chain_in();
   const BState st = *B.st;
   if (st.done) return;
   const int b = bs > 1 ? bs : 1;
@@ -555,6 +560,7 @@ __device__ __forceinline__ double row_dot(const Sys& A, int64_t row, const doubl
 // v = A ph, (rh, v) -> alpha;  T: t = A sh, (t, t), (s, t) -> omega
 template <bool T>
 __global__ void __launch_bounds__(NT) k_cb_spmv(Sys A, Bicg B) {
+  chain_in();
   if (B.st->done) return;
   const int lane = threadIdx.x & 7;
   double sum[2] = {0.0, 0.0}, tot[2];
@@ -586,6 +592,7 @@ __global__ void __launch_bounds__(NT) k_cb_spmv(Sys A, Bicg B) {
 
 // x += alpha ph + omega sh, r = s - omega t; (r, r), (rh, r)
 __global__ void __launch_bounds__(NT) k_cb_x(Bicg B) {
+  chain_in();
   const BState st = *B.st;
   if (st.done) return;
   double sum[2] = {0.0, 0.0}, tot[2];
@@ -651,7 +658,8 @@ struct Ctx {
 inline unsigned g1(int64_t n) { return (unsigned)((n + NT - 1) / NT); }
 
 int spmv(const Ctx& c, const double* x, double* y) {
-  k_spmv<<<(unsigned)((c.A.n + kRowsPerBlock - 1) / kRowsPerBlock), NT, 0, c.s>>>(c.A, x, y);
+  launch_chained(c.s, (unsigned)((c.A.n + kRowsPerBlock - 1) / kRowsPerBlock), NT, 0, k_spmv, c.A, x,
+                 y);
   note_launch();
   return TCAD_OK;
 }
@@ -779,11 +787,12 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
       TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
       if (st.done) break;
       for (int q = 0; q < check; ++q) {
-        k_cb_p<<<gb, NT, 0, s>>>(B, c.bs, c.inv);
-        k_cb_spmv<false><<<gr, NT, 0, s>>>(c.A, B);
-        k_cb_s<<<(unsigned)std::min<int64_t>(kGridBlocks, gb), NT, 0, s>>>(B, c.bs, c.inv);
-        k_cb_spmv<true><<<gr, NT, 0, s>>>(c.A, B);
-        k_cb_x<<<gv, NT, 0, s>>>(B);
+        launch_chained(s, gb, NT, 0, k_cb_p, B, c.bs, c.inv);
+        launch_chained(s, gr, NT, 0, k_cb_spmv<false>, c.A, B);
+        launch_chained(s, (unsigned)std::min<int64_t>(kGridBlocks, gb), NT, 0, k_cb_s, B, c.bs,
+                       c.inv);
+        launch_chained(s, gr, NT, 0, k_cb_spmv<true>, c.A, B);
+        launch_chained(s, gv, NT, 0, k_cb_x, B);
         note_launch(5);
       }
       TCAD_LAUNCH_CHECK();
@@ -825,10 +834,10 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
         const int todo = std::min(check, m - queued);
         for (int q = 0; q < todo; ++q) {
           spmv(c, z, G.w);
-          k_gm_dots<false><<<gv, NTG, 0, s>>>(G);
-          k_gm_dots<true><<<gv, NTG, 0, s>>>(G);
-          k_gm_norm<<<gv, NTG, 0, s>>>(G, tol);
-          k_gm_next<<<gb, NT, 0, s>>>(G, c.bs, c.inv, z);
+          launch_chained(s, gv, NTG, 0, k_gm_dots<false>, G);
+          launch_chained(s, gv, NTG, 0, k_gm_dots<true>, G);
+          launch_chained(s, gv, NTG, 0, k_gm_norm, G, tol);
+          launch_chained(s, gb, NT, 0, k_gm_next, G, c.bs, c.inv, z);
           note_launch(4);
         }
         queued += todo;

@@ -523,9 +523,10 @@ k_ilu_factor_rows(const tcad_pack_t pk, const double* __restrict__ J, double* __
 // the forward records' vectors = Q r for the instances preconditioned here
 template <class T>
 __global__ void __launch_bounds__(NT_ILU_FLAT)
-k_ilu_perm(const tcad_pack_t pk, const double* __restrict__ Q, const T* __restrict__ r,
+k_ilu_perm(const tcad_pack_t pk, const double* __restrict__ Q, const T* r,
            float* __restrict__ Mf, const KState* ks, const uint8_t* __restrict__ mask,
            const int32_t* __restrict__ blk) {
+  chain_in();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (ks && !ks[fb.inst].active) return;
@@ -550,9 +551,10 @@ k_ilu_perm(const tcad_pack_t pk, const double* __restrict__ Q, const T* __restri
 // out = r
 template <class T>
 __global__ void __launch_bounds__(NT_ILU_FLAT)
-k_ilu_unperm(const tcad_pack_t pk, float* __restrict__ Mb, const T* __restrict__ r,
-             T* __restrict__ out, const KState* ks, const uint8_t* __restrict__ mask,
+k_ilu_unperm(const tcad_pack_t pk, float* Mb, const T* r,
+             T* out, const KState* ks, const uint8_t* __restrict__ mask,
              const int32_t* __restrict__ blk) {
+  chain_in();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (ks && !ks[fb.inst].active) return;
@@ -594,6 +596,7 @@ template <int GROUPS>
 __global__ void __launch_bounds__(kIluSweepThreads)
 k_ilu_sweep(const tcad_pack_t pk, float* Mf, float* Mb, KState* ks,
             const uint8_t* __restrict__ mask, int rows, int ring) {
+  chain_in();
   extern __shared__ __align__(128) unsigned char s_ring[];
   __shared__ uint64_t s_full[kIluStages], s_empty[kIluStages];
   __shared__ double fr[2][3][kIluThreads];

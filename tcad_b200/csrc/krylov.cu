@@ -588,6 +588,7 @@ k_bi_init(const tcad_pack_t pk, const T* __restrict__ b, T* __restrict__ x, BiVe
 template <class T>
 __global__ void __launch_bounds__(NT, 4)
 k_bi_p(const tcad_pack_t pk, BiVecT<T> w, const KState* ks, const int32_t* __restrict__ blk) {
+  chain_in();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   const KState s = ks[fb.inst];
@@ -599,6 +600,7 @@ template <int DIM, class T, class TJ = T>
 __global__ void __launch_bounds__(NT)
 k_bi_v(const tcad_pack_t pk, const TJ* __restrict__ J, BiVecT<T> w, KState* ks,
        double* partial, unsigned* ticket, const int32_t* __restrict__ blk) {
+  chain_in();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (!ks[fb.inst].active) return;
@@ -612,6 +614,7 @@ template <class T>
 __global__ void __launch_bounds__(NT, 4)
 k_bi_s(const tcad_pack_t pk, BiVecT<T> w, KState* ks, double* partial, unsigned* ticket,
        const int32_t* __restrict__ blk) {
+  chain_in();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   const KState s0 = ks[fb.inst];
@@ -626,6 +629,7 @@ template <int DIM, class T, class TJ = T>
 __global__ void __launch_bounds__(NT)
 k_bi_t(const tcad_pack_t pk, const TJ* __restrict__ J, BiVecT<T> w, KState* ks,
        double* partial, unsigned* ticket, const int32_t* __restrict__ blk) {
+  chain_in();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (!ks[fb.inst].active) return;
@@ -638,8 +642,9 @@ k_bi_t(const tcad_pack_t pk, const TJ* __restrict__ J, BiVecT<T> w, KState* ks,
 
 template <class T>
 __global__ void __launch_bounds__(NT, 3)
-k_bi_x(const tcad_pack_t pk, T* __restrict__ x, BiVecT<T> w, KState* ks, double* partial,
+k_bi_x(const tcad_pack_t pk, T* x, BiVecT<T> w, KState* ks, double* partial,
        unsigned* ticket, const int32_t* __restrict__ blk) {
+  chain_in();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   const KState s0 = ks[fb.inst];
@@ -1642,15 +1647,15 @@ static void ilu_apply_t(const tcad_pack_t* pk, const double* J, const double* Q,
                         cudaStream_t s) {
   const int ni = pk->n_inst;
   if (ilc && ilc->Mf) {
-    k_ilu_perm<T><<<ng, NT_ILU_FLAT, 0, s>>>(*pk, Q, r, ilc->Mf, w.ks, mask, dlist);
+    launch_chained(s, ng, NT_ILU_FLAT, 0, k_ilu_perm<T>, *pk, Q, r, ilc->Mf, w.ks, mask, dlist);
     const int rows = ilu_rows(ilc->rows), ring = ilu_ring(ilc->rows);
     if (rows <= 128)
-      k_ilu_sweep<4><<<(unsigned)ni, 4 * rows + 32, ring, s>>>(*pk, ilc->Mf, ilc->Mb, w.ks, mask,
-                                                               rows, ring);
+      launch_chained(s, (unsigned)ni, 4 * rows + 32, ring, k_ilu_sweep<4>, *pk, ilc->Mf, ilc->Mb,
+                     w.ks, mask, rows, ring);
     else
-      k_ilu_sweep<2><<<(unsigned)ni, 2 * rows + 32, ring, s>>>(*pk, ilc->Mf, ilc->Mb, w.ks, mask,
-                                                               rows, ring);
-    k_ilu_unperm<T><<<ng, NT_ILU_FLAT, 0, s>>>(*pk, ilc->Mb, r, out, w.ks, mask, dlist);
+      launch_chained(s, (unsigned)ni, 2 * rows + 32, ring, k_ilu_sweep<2>, *pk, ilc->Mf, ilc->Mb,
+                     w.ks, mask, rows, ring);
+    launch_chained(s, ng, NT_ILU_FLAT, 0, k_ilu_unperm<T>, *pk, ilc->Mb, r, out, w.ks, mask, dlist);
     note_launch(3);
     return;
   }
@@ -1818,15 +1823,15 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
     const unsigned ng = grid.ng;
     const int32_t* dlist = grid.dlist;
     for (int q = 0; q < check; ++q) {
-      k_bi_p<<<ng, NT, 0, s>>>(*pk, bi, w.ks, dlist);
+      launch_chained(s, ng, NT, 0, k_bi_p<T>, *pk, bi, w.ks, dlist);
       note_launch();
       if (Qilu) {  // ph = M^-1 p
         ilu_apply_t<T>(pk, Jilu, Qilu, bi.p, bi.ph, w, ilu_mask, nzmax, ilc, ng, dlist, s);
       }
       if (pk->dim == 2)
-        k_bi_v<2><<<ng, NT, 0, s>>>(*pk, J, bi, w.ks, w.partial, w.ticket, dlist);
+        launch_chained(s, ng, NT, 0, k_bi_v<2, T, TJ>, *pk, J, bi, w.ks, w.partial, w.ticket, dlist);
       else
-        k_bi_v<3><<<ng, NT, 0, s>>>(*pk, J, bi, w.ks, w.partial, w.ticket, dlist);
+        launch_chained(s, ng, NT, 0, k_bi_v<3, T, TJ>, *pk, J, bi, w.ks, w.partial, w.ticket, dlist);
       note_launch();
       // (The s and t steps stay two launches here: k_bi_st, which forms the
       // neighbours' s from their r and v, measured 120 us against 20 + 80 us
@@ -1834,18 +1839,18 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
       // neighbour value instead of one; the single-launch solve of small
       // packs, which is latency-bound, keeps the fused form.)
       {
-        k_bi_s<<<ng, NT, 0, s>>>(*pk, bi, w.ks, w.partial, w.ticket, dlist);
+        launch_chained(s, ng, NT, 0, k_bi_s<T>, *pk, bi, w.ks, w.partial, w.ticket, dlist);
         note_launch();
         if (Qilu) {  // sh = M^-1 s
           ilu_apply_t<T>(pk, Jilu, Qilu, bi.s, bi.sh, w, ilu_mask, nzmax, ilc, ng, dlist, s);
         }
         if (pk->dim == 2)
-          k_bi_t<2><<<ng, NT, 0, s>>>(*pk, J, bi, w.ks, w.partial, w.ticket, dlist);
+          launch_chained(s, ng, NT, 0, k_bi_t<2, T, TJ>, *pk, J, bi, w.ks, w.partial, w.ticket, dlist);
         else
-          k_bi_t<3><<<ng, NT, 0, s>>>(*pk, J, bi, w.ks, w.partial, w.ticket, dlist);
+          launch_chained(s, ng, NT, 0, k_bi_t<3, T, TJ>, *pk, J, bi, w.ks, w.partial, w.ticket, dlist);
         note_launch();
       }
-      k_bi_x<<<ng, NT, 0, s>>>(*pk, x, bi, w.ks, w.partial, w.ticket, dlist);
+      launch_chained(s, ng, NT, 0, k_bi_x<T>, *pk, x, bi, w.ks, w.partial, w.ticket, dlist);
       note_launch();
     }
     TCAD_LAUNCH_CHECK();
@@ -2108,17 +2113,7 @@ struct RbStreamLauncher {
 
   template <class... P, class... A>
   int launch(void (*kern)(P...), unsigned ng, size_t smem, A... args) const {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(std::min(ng, (unsigned)sms));
-    cfg.blockDim = dim3(NTS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    TCAD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+    TCAD_CUDA_CHECK(launch_chained(s, std::min(ng, (unsigned)sms), NTS, smem, kern, args...));
     note_launch();
     return TCAD_OK;
   }

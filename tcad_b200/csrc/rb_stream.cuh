@@ -398,15 +398,6 @@ __device__ __forceinline__ RbBlk rb_fetch(const tcad_pack_t& pkb, const KState* 
   return q;
 }
 
-// programmatic dependent launch: let the next kernel's CTAs start where SMs are
-// free; wait for the kernels before this one (what they wrote is visible then)
-__device__ __forceinline__ void launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void wait_prior() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 template <int DIM, int PASS>
 __global__ void __launch_bounds__(NTS, 1)
 k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR,
