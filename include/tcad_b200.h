@@ -213,12 +213,14 @@ size_t tcad_block_workspace_bytes(const tcad_pack_t* pk, int method, int restart
 
 /* Launch shape of the node-block-Jacobi BiCGStab (an implementation switch;
  * the reference has no counterpart: pytcad/linsolve.py:725-985 is one
- * scipy call).  on = 1 (the default): a single-instance pack whose flat
- * blocks all fit on the GPU at once is solved in ONE cooperative launch --
- * one CTA per flat block, bounded grid barriers between the steps, the same
- * arithmetic in the same order as the launch-per-step kernels, so the
- * result is bit-identical; on = 0: one launch per step always.  Process-
- * wide; returns the previous setting. */
+ * scipy call).  on = 1 (the default): small solves take ONE launch with
+ * everything resident -- a single-instance pack whose blocks all fit on the
+ * GPU at once (cooperative, bounded grid barriers between the steps) and, on
+ * the red-black system, every pack whose instances each fit a thread-block
+ * cluster; tcad_csr_krylov's GMRES runs a restart cycle of up to 37,296 rows
+ * so -- the same arithmetic in the same order as the launch-per-step
+ * kernels, so the result is bit-identical (GMRES: to rounding); on = 0: one launch per step
+ * always.  Process-wide; returns the previous setting. */
 int tcad_set_krylov_fused(int on);
 
 /* Test hook of the fused solve's failure path (no counterpart in the
@@ -387,9 +389,8 @@ typedef struct tcad_newton_opts {
    * no coupling inside a colour of (i + j + k) & 1, so the red unknowns are
    * eliminated exactly: half the unknowns, the same matrix bytes per
    * product, about half the iterations); the stopping test stays the full
-   * system's ||b - A x|| <= eta ||b||.  A single-instance pack whose slot
-   * blocks fit on the GPU at once is solved in one cooperative launch (the
-   * same arithmetic).  ILU(0) solves, FP32 operators and a workspace sized
+   * system's ||b - A x|| <= eta ||b||.  Small packs are solved in one launch
+   * (tcad_set_krylov_fused; the same arithmetic).  ILU(0) solves, FP32 operators and a workspace sized
    * without the red-black extension (tcad_block_workspace_bytes method 0)
    * keep the full system.  tcad_equilibrium_solve: its PCG runs on the
    * red-black Schur complement of the scalar Poisson system (every

@@ -55,6 +55,12 @@ inline cudaError_t launch_chained(cudaStream_t s, unsigned grid, unsigned block,
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// tcad_set_krylov_fused, tcad_set_krylov_fused_test; count a launch that gave up
+// (defined in krylov.cu)
+bool krylov_fused();
+bool krylov_fused_hold();
+void krylov_note_gave_up();
+
 constexpr int kFlatThreads = 256;
 constexpr int kTileThreads = TCAD_TILE_X * TCAD_TILE_Y;           // 256
 

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "grid_sync.cuh"
 
 namespace tcad {
 namespace csr {
@@ -303,19 +304,18 @@ struct Gmres {
 
 constexpr int NTG = 4 * NT;   // threads of the V products' blocks
 
-// partial sums of h = V^T w over the block's rows sw (256 of them from row0)
-__device__ __forceinline__ void gm_dots(const Gmres& G, int nv, int64_t row0, const double* sw,
-                                        bool first) {
+// partial sums of h = V^T w over the block's cnt <= 256 rows sw from row0 (0 past cnt)
+__device__ __forceinline__ void gm_dots(const Gmres& G, int nv, int64_t row0, int cnt,
+                                        const double* sw, bool first, double* partial) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int cnt = (int)min((int64_t)NT, G.n - row0);
   double wv[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) wv[u] = sw[lane + 32 * u];   // 0 past the end
   // two vectors at a time: sixteen loads a lane in flight
   for (int i = 2 * warp; i < nv; i += 2 * (NTG / 32)) {
     const bool two = i + 1 < nv;
-    const double* __restrict__ Vi = G.V + (int64_t)i * G.n + row0;
-    const double* __restrict__ Vk = two ? Vi + G.n : Vi;
+    const double* const Vi = G.V + (int64_t)i * G.n + row0;
+    const double* const Vk = two ? Vi + G.n : Vi;
     double x[8], y[8], v = 0.0, q = 0.0;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -334,15 +334,15 @@ __device__ __forceinline__ void gm_dots(const Gmres& G, int nv, int64_t row0, co
       q += __shfl_down_sync(0xffffffffu, q, o);
     }
     if (lane == 0) {
-      double* const d = &G.partial[(size_t)i * gridDim.x + blockIdx.x];
+      double* const d = &partial[(size_t)i * gridDim.x + blockIdx.x];
       *d = first ? v : *d + v;
       if (two) d[gridDim.x] = first ? q : d[gridDim.x] + q;
     }
   }
 }
 
-// h = the blocks' partial sums (last block)
-__device__ __forceinline__ void gm_totals(const Gmres& G, int nv, double* h) {
+// h = the blocks' partial sums
+__device__ __forceinline__ void gm_totals(int nv, const double* partial, double* h) {
   const int lane = threadIdx.x & 7;   // 8 lanes a vector
   for (int i0 = 0; i0 < nv; i0 += NTG / 8) {
     const int i = i0 + (threadIdx.x >> 3);
@@ -350,7 +350,7 @@ __device__ __forceinline__ void gm_totals(const Gmres& G, int nv, double* h) {
     if (i < nv) {
 #pragma unroll 8
       for (unsigned b = lane; b < gridDim.x; b += 8)
-        v += __ldcg(&G.partial[(size_t)i * gridDim.x + b]);
+        v += __ldcg(&partial[(size_t)i * gridDim.x + b]);
     }
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 8);
@@ -358,22 +358,21 @@ __device__ __forceinline__ void gm_totals(const Gmres& G, int nv, double* h) {
   }
 }
 
-// w[row] - sum_i h[i] V_i[row] of the block's 256 rows, in the threads below NT
-// (0 past the end); s4: [4][NT]
-__device__ __forceinline__ double gm_minus(const Gmres& G, int nv, const double* __restrict__ h,
-                                           int64_t row0, double (*s4)[NT]) {
+// w[l] - sum_i h[i] V_i[row0 + l] of the block's cnt <= 256 rows, in the threads l < NT
+// (0 past cnt); s4: [4][NT]
+__device__ __forceinline__ double gm_minus(const Gmres& G, int nv, const double* h, int64_t row0,
+                                           int cnt, const double* w, double (*s4)[NT]) {
   const int l = threadIdx.x & (NT - 1), grp = threadIdx.x / NT;
-  const int64_t row = row0 + l;
   double a = 0.0;
-  if (row < G.n) {
-    const double* __restrict__ Vr = G.V + row;
+  if (l < cnt) {
+    const double* const Vr = G.V + row0 + l;
 #pragma unroll 8
     for (int i = grp; i < nv; i += 4) a += h[i] * Vr[(int64_t)i * G.n];
   }
   s4[grp][l] = a;
   __syncthreads();
-  if (grp != 0 || row >= G.n) return 0.0;
-  return G.w[row] - ((s4[0][l] + s4[1][l]) + (s4[2][l] + s4[3][l]));
+  if (grp != 0 || l >= cnt) return 0.0;
+  return w[l] - ((s4[0][l] + s4[1][l]) + (s4[2][l] + s4[3][l]));
 }
 
 template <bool SUB>
@@ -385,18 +384,19 @@ __global__ void __launch_bounds__(NTG) k_gm_dots(Gmres G) {
   bool first = true;
   for (int64_t row0 = (int64_t)blockIdx.x * NT; row0 < G.n; row0 += (int64_t)gridDim.x * NT) {
     const int64_t row = row0 + threadIdx.x;
-    const bool mine = threadIdx.x < NT && row < G.n;
+    const int cnt = (int)min((int64_t)NT, G.n - row0);
+    const bool mine = (int)threadIdx.x < cnt;
     double w = 0.0;
-    if (SUB) w = gm_minus(G, nv, G.h1, row0, s4);
+    if (SUB) w = gm_minus(G, nv, G.h1, row0, cnt, G.w + row0, s4);
     else if (mine) w = G.w[row];
     if (SUB && mine) G.w[row] = w;
     if (threadIdx.x < NT) sw[threadIdx.x] = w;
     __syncthreads();
-    gm_dots(G, nv, row0, sw, first);
+    gm_dots(G, nv, row0, cnt, sw, first, G.partial);
     __syncthreads();
     first = false;
   }
-  if (last_block(G.ticket)) gm_totals(G, nv, SUB ? G.h2 : G.h1);
+  if (last_block(G.ticket)) gm_totals(nv, G.partial, SUB ? G.h2 : G.h1);
 }
 
 __global__ void __launch_bounds__(NTG) k_gm_norm(Gmres G, double tol) {
@@ -406,8 +406,9 @@ __global__ void __launch_bounds__(NTG) k_gm_norm(Gmres G, double tol) {
   const int j = G.st->j;
   double v[1] = {0.0}, tot[1];
   for (int64_t row0 = (int64_t)blockIdx.x * NT; row0 < G.n; row0 += (int64_t)gridDim.x * NT) {
-    const double w = gm_minus(G, j + 1, G.h2, row0, s4);
-    if (threadIdx.x < NT && row0 + threadIdx.x < G.n) G.w[row0 + threadIdx.x] = w;
+    const int cnt = (int)min((int64_t)NT, G.n - row0);
+    const double w = gm_minus(G, j + 1, G.h2, row0, cnt, G.w + row0, s4);
+    if ((int)threadIdx.x < cnt) G.w[row0 + threadIdx.x] = w;
     v[0] += w * w;
     __syncthreads();
   }
@@ -466,6 +467,122 @@ __global__ void __launch_bounds__(NT) k_gm_next(Gmres G, int bs, const double* _
   }
   prec_row(bs, inv, t, v, q);
   for (int c = 0; c < b; ++c) z[b * t + c] = q[c];
+}
+
+// ---- a whole restart cycle in one cooperative launch, for systems of at most
+// kGmCycleCtas x kGmRows rows
+//
+// Five launches of such an iteration are latency (30 us at 13,824 rows, chained; 20
+// here).  Whole solves, five launches an iteration / one a cycle: 288 rows 1.6 / 1.05
+// ms, 13,824 rows 28.4 / 19.8, 36,960 rows 68.5 / 43.2; above 37,296 a CTA would
+// need more rows than its shared memory and registers are laid out for.  Here a CTA keeps kGmRows rows of w in shared memory and an
+// iteration is four grid barriers: h1 = V^T A z; w -= V h1, h2 = V^T w; w -= V h2,
+// ||w||; V_{j+1}, z (whose neighbours' rows the next product reads).  Every CTA adds
+// the partial sums for itself and applies the Givens rotations to its own copy of the
+// column -- the same numbers everywhere -- in one warp while the others form V_{j+1}
+// and z.  kGmRows: whole 3 x 3 and 6 x 6 blocks.  Needs V_0 and z (k_gm_start,
+// k_gm_next); leaves G.w as it was, so that a cycle whose barrier gave up can be run
+// again step by step.
+constexpr int kGmRows = 252;
+constexpr int kGmCycleCtas = 148;
+constexpr int kGmCycleCols = 1000;   // columns of a cycle whose state fits in shared memory
+constexpr size_t gm_cycle_smem(int m) { return 4 * (size_t)(m + 1) * sizeof(double); }
+
+__global__ void __launch_bounds__(NTG, 1)
+k_gm_cycle(Sys A, Gmres G, int bs, const double* __restrict__ inv, double* z, double tol, double g0,
+           unsigned* bar) {
+  extern __shared__ double s_dyn[];   // h1, h2, cs, sn
+  __shared__ double sw[NT], s4[4][NT], sm[32], s_norm, s_g;
+  __shared__ int ok, s_done;
+  double* const h1 = s_dyn;
+  double* const h2 = h1 + (G.m + 1);
+  double* const cs = h2 + (G.m + 1);
+  double* const sn = cs + (G.m + 1);
+  GridBarrier gb{bar, 0u};
+  double* const part[2] = {G.partial, G.partial + (size_t)gridDim.x * (G.m + 1)};
+  double* const pnorm = G.partial + 2 * (size_t)gridDim.x * (G.m + 1);
+  const int64_t row0 = (int64_t)blockIdx.x * kGmRows;
+  const int cnt = (int)min((int64_t)kGmRows, G.n - row0);
+  const int tid = threadIdx.x, b = bs > 1 ? bs : 1;
+  if (tid == 0) {
+    s_g = g0;
+    s_done = 0;
+  }
+  if (tid < NT) sw[tid] = 0.0;
+  __syncthreads();
+  for (int j = 0; j < G.m; ++j) {
+    // w = A z, eight lanes a row
+    for (int r0 = 0; r0 < cnt; r0 += NTG / 8) {
+      const int r = r0 + (tid >> 3);
+      double s = 0.0;
+      if (r < cnt) {
+        const int e = A.ptr[row0 + r + 1];
+        for (int q = A.ptr[row0 + r] + (tid & 7); q < e; q += 8) s += A.val[q] * __ldcg(z + A.idx[q]);
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, 8);
+      if (r < cnt && (tid & 7) == 0) sw[r] = s;
+    }
+    __syncthreads();
+    gm_dots(G, j + 1, row0, cnt, sw, true, part[0]);
+    if (!gb.wait(&ok)) return;
+    gm_totals(j + 1, part[0], h1);
+    __syncthreads();
+    double w = gm_minus(G, j + 1, h1, row0, cnt, sw, s4);
+    __syncthreads();
+    if (tid < NT) sw[tid] = w;
+    __syncthreads();
+    gm_dots(G, j + 1, row0, cnt, sw, true, part[1]);
+    if (!gb.wait(&ok)) return;
+    gm_totals(j + 1, part[1], h2);
+    __syncthreads();
+    w = gm_minus(G, j + 1, h2, row0, cnt, sw, s4);
+    __syncthreads();
+    if (tid < NT) sw[tid] = w;
+    double tot = block_sum<NTG>(w * w, sm);
+    if (tid == 0) pnorm[blockIdx.x] = tot;
+    if (!gb.wait(&ok)) return;
+    tot = block_sum<NTG>(tid < (int)gridDim.x ? __ldcg(pnorm + tid) : 0.0, sm);
+    if (tid == 0) s_norm = sqrt(tot);
+    __syncthreads();
+    const double hn = s_norm, a1 = hn > 0.0 ? 1.0 / hn : 0.0;
+    // V_{j+1}, z; meanwhile the last thread: column j's rotations
+    if (tid < cnt / b) {
+      const int64_t t = row0 / b + tid;
+      double* const Vj = G.V + (int64_t)(j + 1) * G.n;
+      double v[6], q[6];
+      for (int c = 0; c < b; ++c) {
+        v[c] = a1 * sw[b * tid + c];
+        Vj[b * t + c] = v[c];
+      }
+      prec_row(bs, inv, t, v, q);
+      for (int c = 0; c < b; ++c) z[b * t + c] = q[c];
+    } else if (tid == NTG - 1) {
+      const bool out = blockIdx.x == 0;
+      double* const r = G.R + (size_t)j * (G.m + 1);
+      double a = h1[0] + h2[0];
+      for (int k = 0; k < j; ++k) {
+        const double hk = h1[k + 1] + h2[k + 1];
+        if (out) r[k] = cs[k] * a + sn[k] * hk;
+        a = -sn[k] * a + cs[k] * hk;
+      }
+      const double den = hypot(a, hn);
+      const double c = den > 0.0 ? a / den : 1.0, s = den > 0.0 ? hn / den : 0.0;
+      cs[j] = c;
+      sn[j] = s;
+      const double gj = s_g, gn = -s * gj;
+      s_g = gn;
+      s_done = (fabs(gn) <= tol || !(den > 0.0)) ? 1 : 0;
+      if (out) {
+        r[j] = den;
+        G.g[j] = c * gj;
+        G.g[j + 1] = gn;
+        *G.st = GState{j + 1, s_done, a1};
+      }
+    }
+    if (!gb.wait(&ok)) return;
+    if (s_done) return;
+  }
 }
 
 // start of a cycle: g = (rn, 0, ...), no columns, w = the residual
@@ -688,6 +805,41 @@ int axpy(const Ctx& c, double a, const double* x, double b, double* y, double cc
   return TCAD_OK;
 }
 
+// one cycle by k_gm_cycle, its state into st; done = false: it did not run to its end
+int gm_cycle(const Ctx& c, const Gmres& G, double* z, double tol, double rn, GState& st,
+             bool& done) {
+  done = false;
+  unsigned* const bar = c.ticket + 32;
+  unsigned h[4] = {0u, 0u, 0u, krylov_fused_hold() ? 1u : 0u};
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(bar, h, sizeof(h), cudaMemcpyHostToDevice, c.s));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((G.n + kGmRows - 1) / kGmRows));
+  cfg.blockDim = dim3(NTG);
+  cfg.dynamicSmemBytes = gm_cycle_smem(G.m);
+  cfg.stream = c.s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, k_gm_cycle, c.A, G, c.bs, (const double*)c.inv, z, tol, rn, bar) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
+    return TCAD_OK;
+  }
+  note_launch();
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(&st, G.st, sizeof(st), cudaMemcpyDeviceToHost, c.s));
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(h, bar, sizeof(h), cudaMemcpyDeviceToHost, c.s));
+  TCAD_CUDA_CHECK(cudaStreamSynchronize(c.s));
+  if (h[2] != 0u) {
+    krylov_note_gave_up();
+    st = GState{0, 0, 0.0};
+  } else {
+    done = true;
+  }
+  return TCAD_OK;
+}
+
 }  // namespace
 
 extern "C" size_t tcad_csr_workspace_bytes(int64_t n, int method, int restart) {
@@ -829,8 +981,17 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
       k_gm_next<<<gb, NT, 0, s>>>(G, c.bs, c.inv, z);
       note_launch(2);
       GState st{0, 0, 0.0};
+      bool whole = N <= (int64_t)kGmCycleCtas * kGmRows && m <= kGmCycleCols && krylov_fused();
+      if (whole) {
+        if ((rc = gm_cycle(c, G, z, tol, rn, st, whole))) return rc;
+        if (!whole) {   // the launch was refused or gave up: the cycle step by step
+          k_gm_start<<<1, NT, 0, s>>>(G, rn);
+          k_gm_next<<<gb, NT, 0, s>>>(G, c.bs, c.inv, z);
+          note_launch(2);
+        }
+      }
       int queued = 0;
-      for (int check = 4; !st.done && st.j < m; check = std::min(2 * check, 32)) {
+      for (int check = 4; !whole && !st.done && st.j < m; check = std::min(2 * check, 32)) {
         const int todo = std::min(check, m - queued);
         for (int q = 0; q < todo; ++q) {
           spmv(c, z, G.w);

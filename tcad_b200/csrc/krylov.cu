@@ -1668,6 +1668,9 @@ static void ilu_apply_t(const tcad_pack_t* pk, const double* J, const double* Q,
 static std::atomic<int> g_fused_mode{1};   // 0: one launch per step always
 static std::atomic<int> g_fused_test_hold{0};        // give-up test hook (bar[3] = 1)
 static std::atomic<uint64_t> g_fused_gave_up{0};     // fused launches that gave up
+bool krylov_fused() { return g_fused_mode.load() != 0; }
+bool krylov_fused_hold() { return g_fused_test_hold.load() != 0; }
+void krylov_note_gave_up() { g_fused_gave_up.fetch_add(1); }
 
 // k_bicgstab_fused<DIM> needs every flat block resident at once
 template <int DIM>
