@@ -559,7 +559,7 @@ def run_ours(args):
             # committed ncu summary of one iteration on one lane, scaled by the
             # pack's node count
             "roofline": {
-                "kernel": ("k_bi_p + k_rb_red + k_rb_v + k_bi_s + k_rb_red + k_rb_t + k_bi_x "
+                "kernel": ("k_bi_p + k_rb_stream (red, v) + k_bi_s + k_rb_stream (red, t) + k_bi_x "
                            "(one red-black Schur BiCGStab iteration, all lanes)" if rb else
                            "k_bi_p + k_bi_v + k_bi_s + k_bi_t + k_bi_x (one BiCGStab "
                            "iteration, all lanes)"),
