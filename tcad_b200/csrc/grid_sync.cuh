@@ -93,8 +93,8 @@ struct GridSync {
     gb = GridBarrier{b, 0u};
   }
 
-  // tot = the sums over the grid of every thread's v, valid in every thread;
-  // NQ = 0: a barrier alone.  Orders all global writes before it, of any
+  // tot = the sums over the grid of the first kFlatThreads threads' v, valid in
+  // every thread; NQ = 0: a barrier alone.  Orders all global writes before it, of any
   // thread of the grid, before all reads after it.
   template <int NQ>
   __device__ __forceinline__ bool sum(const double* v, double* tot) {
@@ -114,7 +114,7 @@ struct GridSync {
       for (int q = 0; q < NQ; ++q) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r[q] += __shfl_down_sync(0xffffffffu, r[q], o);
-        if (lane == 0) dst[q][warp] = r[q];
+        if (lane == 0 && warp < NW) dst[q][warp] = r[q];
       }
     };
     ++gb.round;
@@ -173,7 +173,7 @@ struct ClusterSync {
         double r = v[q];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-        if (lane == 0) sa[q][warp] = r;
+        if (lane == 0 && warp < NW) sa[q][warp] = r;
       }
       __syncthreads();
       if (threadIdx.x < ctas) {

@@ -1960,10 +1960,10 @@ static int coop_launch(CoopLaunch& c, unsigned blocks, unsigned threads, size_t 
 // Launch configuration of a cluster per instance; 1 when such clusters do not
 // fit on the GPU
 template <class... P>
-static int cluster_launch(CoopLaunch& c, void (*kern)(P...), int ni, int ctas, size_t smem,
-                          cudaStream_t s) {
+static int cluster_launch(CoopLaunch& c, void (*kern)(P...), int ni, int ctas, int threads,
+                          size_t smem, cudaStream_t s) {
   c.cfg.gridDim = dim3((unsigned)(ni * ctas));
-  c.cfg.blockDim = dim3(NT);
+  c.cfg.blockDim = dim3((unsigned)threads);
   c.cfg.dynamicSmemBytes = smem;
   c.cfg.stream = s;
   c.at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2001,14 +2001,15 @@ static int coop_result(const Work& w, int ni, std::vector<KState>& hks, cudaStre
 // k_bicgstab_rb_resident over the slot pack's blocks, queued: 1 when the launch
 // was refused.  Jn: J in node order (a solve with its rows in shared memory
 // takes them from there), null: the packed colour rows.  clear: see coop_launch.
-template <int DIM, int K, bool JS, class SYNC>
+template <int DIM, int K, int T, bool JS, class SYNC>
 static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double* Jn,
                                const double* b, double* x, double rtol, int maxiter,
                                const Work& w, const int32_t* pre_status, bool clear,
                                cudaStream_t s, const double* rtol_inst) {
   constexpr bool kCluster = std::is_same<SYNC, ClusterSync>::value;
-  const auto kern = k_bicgstab_rb_resident<DIM, K, JS, SYNC>;
+  const auto kern = k_bicgstab_rb_resident<DIM, K, T, JS, SYNC>;
   const int share = kCluster ? L.share : L.pkb.flat_nodes;
+  if (share > T * K) return 1;
   const size_t smem = JS ? (size_t)share * Stencil<DIM>::NE * 16 : 0;
   if (JS && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem) != cudaSuccess) {
@@ -2017,8 +2018,8 @@ static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double
   }
   CoopLaunch c;
   if (kCluster && clear) TCAD_CUDA_CHECK(cudaMemsetAsync(w.bar, 0, 4 * sizeof(unsigned), s));
-  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, smem, s)
-                        : coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, clear, s))
+  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, T, smem, s)
+                        : coop_launch(c, (unsigned)L.pkb.n_flat, T, smem, w.bar, clear, s))
     return rc;
   const BiVec& bi = w.bi;
   const int rechecks = 8;
@@ -2053,23 +2054,29 @@ static int queue_rb_resident(const tcad_pack_t* pk, const RbLayout& L, const Wor
   auto go = [&](auto fnc) {
     return fnc(L, wr, Jn, b, x, rtol, maxiter, w, pre_status, clear, s, rtol_inst);
   };
+  // 3D shares above NT slots: a thread for each slot.  Two slots a thread leave no
+  // registers for the gathers (54 loads a slot in red(p)): 64 x 48 x 32 tri-gate 32.5 us
+  // an iteration, with 352 threads 19.1; 31 x 22 x 16 in a cluster 22.0 and 10.2; 56 x
+  // 48 x 46, rows from L2, 39.0 and with 512 threads 28.5.  2D (36 loads): 512 x 256 MOSFET 16.0 with two slots a thread, 17.7
+  // with 448 threads.
+  constexpr int T3 = rb_resident_js_slots(TCAD_NE3);
   // (the test hook holds up a grid barrier; clusters have none)
   if (L.cluster && !g_fused_test_hold.load()) {
     if (d2)
-      return L.share <= NT ? go(queue_rb_resident_t<2, 1, true, ClusterSync>)
-                           : go(queue_rb_resident_t<2, 2, true, ClusterSync>);
-    return L.share <= NT ? go(queue_rb_resident_t<3, 1, true, ClusterSync>)
-                         : go(queue_rb_resident_t<3, 2, true, ClusterSync>);
+      return L.share <= NT ? go(queue_rb_resident_t<2, 1, NT, true, ClusterSync>)
+                           : go(queue_rb_resident_t<2, 2, NT, true, ClusterSync>);
+    return L.share <= NT ? go(queue_rb_resident_t<3, 1, NT, true, ClusterSync>)
+                         : go(queue_rb_resident_t<3, 1, T3, true, ClusterSync>);
   }
   if (pk->n_inst != 1) return 1;
   const int fn = L.pkb.flat_nodes;
   if (d2)
-    return fn <= NT ? go(queue_rb_resident_t<2, 1, true, GridSync>)
-           : js     ? go(queue_rb_resident_t<2, 2, true, GridSync>)
-                    : go(queue_rb_resident_t<2, 2, false, GridSync>);
-  return fn <= NT ? go(queue_rb_resident_t<3, 1, true, GridSync>)
-         : js     ? go(queue_rb_resident_t<3, 2, true, GridSync>)
-                  : go(queue_rb_resident_t<3, 2, false, GridSync>);
+    return fn <= NT ? go(queue_rb_resident_t<2, 1, NT, true, GridSync>)
+           : js     ? go(queue_rb_resident_t<2, 2, NT, true, GridSync>)
+                    : go(queue_rb_resident_t<2, 2, NT, false, GridSync>);
+  return fn <= NT ? go(queue_rb_resident_t<3, 1, NT, true, GridSync>)
+         : js     ? go(queue_rb_resident_t<3, 1, T3, true, GridSync>)
+                  : go(queue_rb_resident_t<3, 1, 2 * NT, false, GridSync>);
 }
 
 static int sm_count() {
@@ -2439,7 +2446,7 @@ static int queue_eq_resident_t(const RbLayout& L, const WorkEq& we, const double
     return 1;
   }
   CoopLaunch c;
-  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, smem, s)
+  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, NT, smem, s)
                         : coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, false, s))
     return rc;
   if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, J, b, d, w.cg.z, w.cg.p, we.xb, we.tR, w.ks,

@@ -1,6 +1,6 @@
 // The red-black Schur BiCGStab of a small single-instance pack in one
-// cooperative launch with everything resident: one CTA per SM (and per flat
-// block of the slot pack, K * 256 slots at most), the CTA's rows of both
+// cooperative launch with everything resident: one CTA of T threads per SM (and
+// per flat block of the slot pack, K T slots at most), the CTA's rows of both
 // colours of J in shared memory when they fit (JS), its slots' vectors in
 // registers.  Global memory holds only what neighbours read: r, p, v and Tr.
 //
@@ -54,8 +54,8 @@ struct RbFormSCg {
   }
 };
 
-template <int DIM, int K, bool JS, class SYNC>
-__global__ void __launch_bounds__(NT, 1)
+template <int DIM, int K, int T, bool JS, class SYNC>
+__global__ void __launch_bounds__(T, 1)
 k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ Jn,
                        const double* __restrict__ JR, const double* __restrict__ JB, const double* __restrict__ b,
                        double* __restrict__ x, double* bRg, double* Tr, double* xbg,
@@ -81,7 +81,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
     const double2* const gb = reinterpret_cast<const double2*>(JB + rb_jidx<NE>(0, fb.begin));
     double2* const s2 = reinterpret_cast<double2*>(s_rows);
     if (Jn) {   // from J in node order (zeros at pads, as k_rb_pack)
-      for (int l = threadIdx.x; l < nloc; l += NT)
+      for (int l = threadIdx.x; l < nloc; l += T)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const RbNode q = rb_node(g, fb.begin + l, c);
@@ -92,9 +92,9 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
         }
     } else {
 #pragma unroll 8
-      for (int i = threadIdx.x; i < n2; i += NT) s2[i] = gr[i];
+      for (int i = threadIdx.x; i < n2; i += T) s2[i] = gr[i];
 #pragma unroll 8
-      for (int i = threadIdx.x; i < n2; i += NT) s2[n2 + i] = gb[i];
+      for (int i = threadIdx.x; i < n2; i += T) s2[n2 + i] = gb[i];
     }
     jr = s_rows;
     jb = s_rows + 2 * n2;
@@ -106,7 +106,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
   bool own[K], realr[K], realb[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const int q = threadIdx.x + k * NT;
+    const int q = threadIdx.x + k * T;
     own[k] = q < nloc;
     const int64_t slot = fb.begin + (own[k] ? q : 0);
     const RbNode nr = rb_node(g, slot, 0), nk = rb_node(g, slot, 1);
@@ -122,8 +122,41 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
   }
   const int64_t q0 = fb.begin + threadIdx.x;     // slot of (k, c): q0 + k NT + c NS
   double r[K][3], rh[K][3], p[K][3], v[K][3], s[K][3], t[K][3], xb[K][3], tr[K][3];
-  double tot[3], sum[3];
+  double tot[3], sum[3] = {0.0, 0.0, 0.0};
   KState S;
+  // The sums in the per-step kernels' order: a thread below NT adds the terms of its
+  // slots q and q + NT, the latter from operands that the thread which has it (T > NT)
+  // hands over (operands, not products: a term is one fused multiply-add).
+  constexpr int HI = T > NT ? T - NT : 1;
+  __shared__ double s_ops[T > NT ? 6 : 1][HI];
+  const bool low = T <= NT || threadIdx.x < NT;
+  const auto add = [&](int i, double u, double w, const auto& term) {
+    if (low) {
+      term(u, w);
+    } else {
+      s_ops[i][threadIdx.x - NT] = u;
+      s_ops[3 + i][threadIdx.x - NT] = w;
+    }
+  };
+  const auto collect = [&](const auto& term) {
+    if constexpr (T > NT) {
+      __syncthreads();
+      if (low && (int)threadIdx.x + NT < nloc)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) term(s_ops[i][threadIdx.x], s_ops[3 + i][threadIdx.x]);
+    }
+  };
+  const auto product = [&](double u, double w) { sum[0] += u * w; };      // (u, w)
+  const auto squares = [&](double u, double w) {                          // (u, u), (w, u), (w, w)
+    sum[0] += u * u;
+    sum[1] += w * u;
+    sum[2] += w * w;
+  };
+  const auto residual = [&](double u, double w) {                         // (u, w), (w, w), (u, u)
+    sum[0] += u * w;
+    sum[1] += w * w;
+    sum[2] += u * u;
+  };
 
   // red pass: tr = E X, stored for the neighbours
   auto red = [&](const auto& X) {
@@ -131,17 +164,17 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
     for (int k = 0; k < K; ++k) {
       tr[k][0] = 0.0; tr[k][1] = 0.0; tr[k][2] = 0.0;
       if (realr[k])
-        rb_couple_f<DIM>(jr, X, threadIdx.x + k * NT, mr[k], tr[k][0], tr[k][1], tr[k][2]);
+        rb_couple_f<DIM>(jr, X, threadIdx.x + k * T, mr[k], tr[k][0], tr[k][1], tr[k][2]);
       if (own[k])
 #pragma unroll
-        for (int c = 0; c < 3; ++c) Tr[c * NS + q0 + k * NT] = tr[k][c];
+        for (int c = 0; c < 3; ++c) Tr[c * NS + q0 + k * T] = tr[k][c];
     }
   };
-  // u = F T at slot k (0 at a pad)
-  auto black = [&](int k, const double* T, double* u) {
+  // u = F y at slot k (0 at a pad)
+  auto black = [&](int k, const double* y, double* u) {
     u[0] = 0.0; u[1] = 0.0; u[2] = 0.0;
     if (realb[k])
-      rb_couple_f<DIM>(jb, RbValCg{T + g.soff, NS}, threadIdx.x + k * NT, mb[k], u[0], u[1],
+      rb_couple_f<DIM>(jb, RbValCg{y + g.soff, NS}, threadIdx.x + k * T, mb[k], u[0], u[1],
                        u[2]);
   };
 
@@ -153,15 +186,22 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
     if (!own[k]) continue;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      const RbNode q = rb_node(g, q0 + k * NT, c);
+      const RbNode q = rb_node(g, q0 + k * T, c);
 #pragma unroll
       for (int e = 0; e < 3; ++e) {
         const double bv = q.real ? b[e * NN + q.node] : 0.0;
         if (c) bB[k][e] = bv;
-        else bRg[e * NS + q0 + k * NT] = bv;
-        sum[0] += bv * bv;
+        else bRg[e * NS + q0 + k * T] = bv;
+        if (low) sum[0] += bv * bv;
+        else s_ops[3 * c + e][threadIdx.x - NT] = bv;
       }
     }
+  }
+  if constexpr (T > NT) {
+    __syncthreads();
+    if (low && (int)threadIdx.x + NT < nloc)
+#pragma unroll
+      for (int i = 0; i < 6; ++i) sum[0] += s_ops[i][threadIdx.x] * s_ops[i][threadIdx.x];
   }
   if (!gs.template sum<1>(sum, tot)) return;
   const double bb = tot[0];
@@ -177,12 +217,13 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
       xb[k][c] = 0.0; r[k][c] = y; rh[k][c] = y; p[k][c] = 0.0; v[k][c] = 0.0;
       s[k][c] = 0.0; t[k][c] = 0.0;
       if (own[k]) {
-        const int64_t q = c * NS + q0 + k * NT;
+        const int64_t q = c * NS + q0 + k * T;
         rhsg[q] = y; rg[q] = y; pg[q] = 0.0; vg[q] = 0.0;
-        sum[0] += y * y;
+        add(c, y, y, product);
       }
     }
   }
+  collect(product);
   if (!gs.template sum<1>(sum, tot)) return;
   rb_fin_init(S, tot[0], bb, rtol_inst ? rtol_inst[inst] : rtol, maxit,
               pre_status ? pre_status[inst] : TCAD_OK);
@@ -205,11 +246,12 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
           const double y = realb[k] ? pn - u[c] : 0.0;
           p[k][c] = pn;
           v[k][c] = y;
-          pg[c * NS + q0 + k * NT] = pn;
-          vg[c * NS + q0 + k * NT] = y;
-          sum[0] += rh[k][c] * y;
+          pg[c * NS + q0 + k * T] = pn;
+          vg[c * NS + q0 + k * T] = y;
+          add(c, rh[k][c], y, product);
         }
       }
+      collect(product);
       if (!gs.template sum<1>(sum, tot)) return;
       fin_v(S, tot[0]);
       if (!S.active) break;
@@ -224,14 +266,13 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           const double sv = r[k][c] - S.alpha * v[k][c];
-          sum[0] += sv * sv;
           const double y = realb[k] ? sv - u[c] : 0.0;
           s[k][c] = sv;
           t[k][c] = y;
-          sum[1] += y * sv;
-          sum[2] += y * y;
+          add(c, sv, y, squares);
         }
       }
+      collect(squares);
       if (!gs.template sum<3>(sum, tot)) return;
       fin_s(S, tot[0]);
       fin_t(S, tot[1], tot[2]);
@@ -244,12 +285,11 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
           xb[k][c] = xb[k][c] + S.alpha * p[k][c] + S.omega * s[k][c];
           const double rn = s[k][c] - S.omega * t[k][c];
           r[k][c] = rn;
-          rg[c * NS + q0 + k * NT] = rn;
-          sum[0] += rh[k][c] * rn;
-          sum[1] += rn * rn;
-          sum[2] += rh[k][c] * rh[k][c];
+          rg[c * NS + q0 + k * T] = rn;
+          add(c, rh[k][c], rn, residual);
         }
       }
+      collect(residual);
       if (!gs.template sum<3>(sum, tot)) return;
       fin_x(S, tot[0], tot[1], tot[2]);
     }
@@ -258,7 +298,7 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
     for (int k = 0; k < K; ++k)
       if (own[k])
 #pragma unroll
-        for (int c = 0; c < 3; ++c) xbg[c * NS + q0 + k * NT] = xb[k][c];
+        for (int c = 0; c < 3; ++c) xbg[c * NS + q0 + k * T] = xb[k][c];
     if (!gs.template sum<0>(nullptr, nullptr)) return;
     red(RbValCg{xbg + g.soff, NS});
     if (!gs.template sum<0>(nullptr, nullptr)) return;
@@ -271,12 +311,13 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const double y = realb[k] ? xb[k][c] - u[c] : 0.0;
-        const double a = rhsg[c * NS + q0 + k * NT] - y;
+        const double a = rhsg[c * NS + q0 + k * T] - y;
         r[k][c] = a;
-        rg[c * NS + q0 + k * NT] = a;
-        sum[0] += a * a;
+        rg[c * NS + q0 + k * T] = a;
+        add(c, a, a, product);
       }
     }
+    collect(product);
     if (!gs.template sum<1>(sum, tot)) return;
     fin_true(S, tot[0], rechecks < max_rechecks ? 1 : 0);
     if (!S.active) break;
@@ -286,10 +327,10 @@ k_bicgstab_rb_resident(const tcad_pack_t pkb, const RbMap mp, const double* __re
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     if (!own[k]) continue;
-    const RbNode nr = rb_node(g, q0 + k * NT, 0), nk = rb_node(g, q0 + k * NT, 1);
+    const RbNode nr = rb_node(g, q0 + k * T, 0), nk = rb_node(g, q0 + k * T, 1);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      if (realr[k]) x[c * NN + nr.node] = idle ? 0.0 : bRg[c * NS + q0 + k * NT] - tr[k][c];
+      if (realr[k]) x[c * NN + nr.node] = idle ? 0.0 : bRg[c * NS + q0 + k * T] - tr[k][c];
       if (realb[k]) x[c * NN + nk.node] = idle ? 0.0 : xb[k][c];
     }
   }
