@@ -2431,13 +2431,13 @@ static int launch_cg(const tcad_pack_t* pk, const double* J, const double* b, do
 
 // k_eqrb_resident over the slot pack's blocks or a cluster per instance, queued;
 // its barrier flags are cleared by the caller: 1 when the launch was refused
-template <int DIM, int K, class SYNC>
+template <int DIM, int K, int T, class SYNC>
 static int queue_eq_resident_t(const RbLayout& L, const WorkEq& we, const double* J,
                                const double* b, double* d, double rtol, int maxiter,
                                const Work& w, const uint8_t* active, cudaStream_t s,
                                const double* rtol_inst) {
   constexpr bool kCluster = std::is_same<SYNC, ClusterSync>::value;
-  const auto kern = k_eqrb_resident<DIM, K, SYNC>;
+  const auto kern = k_eqrb_resident<DIM, K, T, SYNC>;
   const int share = kCluster ? L.share : L.pkb.flat_nodes;
   const size_t smem = (size_t)share * (1 + 2 * DIM) * 16;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -2446,8 +2446,8 @@ static int queue_eq_resident_t(const RbLayout& L, const WorkEq& we, const double
     return 1;
   }
   CoopLaunch c;
-  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, NT, smem, s)
-                        : coop_launch(c, (unsigned)L.pkb.n_flat, NT, smem, w.bar, false, s))
+  if (int rc = kCluster ? cluster_launch(c, kern, L.pkb.n_inst, L.cluster, T, smem, s)
+                        : coop_launch(c, (unsigned)L.pkb.n_flat, T, smem, w.bar, false, s))
     return rc;
   if (cudaLaunchKernelEx(&c.cfg, kern, L.pkb, L.mp, J, b, d, w.cg.z, w.cg.p, we.xb, we.tR, w.ks,
                          we.sync, w.bar, rtol, maxiter, active, rtol_inst, share) !=
@@ -2472,15 +2472,21 @@ static int queue_eq_resident(const tcad_pack_t* pk, const RbLayout& L, const Wor
   auto go = [&](auto fnc) { return fnc(L, we, J, b, d, rtol, maxiter, w, active, s, rtol_inst); };
   auto pick = [&](auto sync, int fn) {
     using S = decltype(sync);
+    // Above NT slots a CTA more threads instead of two or four slots each: 240 x 120
+    // MOSFET (clusters of 900 slots) 11.0 ms at 4 x 256, 10.05 at 2 x 512, 10.9 at 1 x
+    // 1,024; 96 x 56 x 40 tri-gate (grid, 727 slots) 6.91, 6.78, 6.56.  Eight slots a
+    // thread leave no shared memory for the sums' operands.
+    constexpr bool kGrid = std::is_same<S, GridSync>::value;
+    constexpr int K4 = kGrid ? 1 : 2, T4 = 4 * NT / K4;
     if (pk->dim == 2)
-      return fn <= NT       ? go(queue_eq_resident_t<2, 1, S>)
-             : fn <= 2 * NT ? go(queue_eq_resident_t<2, 2, S>)
-             : fn <= 4 * NT ? go(queue_eq_resident_t<2, 4, S>)
-                            : go(queue_eq_resident_t<2, 8, S>);
-    return fn <= NT       ? go(queue_eq_resident_t<3, 1, S>)
-           : fn <= 2 * NT ? go(queue_eq_resident_t<3, 2, S>)
-           : fn <= 4 * NT ? go(queue_eq_resident_t<3, 4, S>)
-                          : go(queue_eq_resident_t<3, 8, S>);
+      return fn <= NT       ? go(queue_eq_resident_t<2, 1, NT, S>)
+             : fn <= 2 * NT ? go(queue_eq_resident_t<2, 1, 2 * NT, S>)
+             : fn <= 4 * NT ? go(queue_eq_resident_t<2, K4, T4, S>)
+                            : go(queue_eq_resident_t<2, 8, NT, S>);
+    return fn <= NT       ? go(queue_eq_resident_t<3, 1, NT, S>)
+           : fn <= 2 * NT ? go(queue_eq_resident_t<3, 1, 2 * NT, S>)
+           : fn <= 4 * NT ? go(queue_eq_resident_t<3, K4, T4, S>)
+                          : go(queue_eq_resident_t<3, 8, NT, S>);
   };
   // (the test hook holds up a grid barrier; clusters have none)
   if (L.cluster && !g_fused_test_hold.load()) return pick(ClusterSync{}, L.share);
