@@ -233,6 +233,14 @@ int tcad_set_krylov_fused(int on);
 int tcad_set_krylov_fused_test(int hold);
 uint64_t tcad_krylov_fused_gave_up(void);
 
+/* Test hook (host arithmetic only; shape: HOST memory, [3 n_inst] Nx, Ny, Nz):
+ * where the red-black solves put the slots of a pack's instances -- start
+ * [n_inst + 1], the last the end -- and the CTAs of the cluster that each
+ * instance has in a coupled solve (0: none).  TCAD_ERR_ARG where the slot
+ * arrays (n_nodes) do not hold them. */
+int tcad_slot_layout_test(const int32_t* shape, int n_inst, int64_t n_nodes, int dim,
+                          int64_t* start, int32_t* cluster);
+
 /* Node-block-Jacobi set-up (pytcad/linsolve.py:363-427): inverts every
  * diagonal 3x3 block of J in place and replaces F by the block-scaled
  * right-hand side b^ = D^-1 (-F).  status[inst] gets TCAD_ERR_SINGULAR for a

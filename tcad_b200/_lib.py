@@ -93,6 +93,8 @@ _SIGS = {
     "tcad_set_krylov_fused": (ctypes.c_int, [ctypes.c_int]),
     "tcad_set_krylov_fused_test": (ctypes.c_int, [ctypes.c_int]),
     "tcad_krylov_fused_gave_up": (ctypes.c_uint64, []),
+    "tcad_slot_layout_test": (ctypes.c_int, [_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int,
+                                             _p, _p]),
     "tcad_state_extrapolate": (ctypes.c_int, [_p, _p, _p, _p, _p, _p, _p, _p, _p]),
     "tcad_block_jacobi_setup": (ctypes.c_int, [_p, _p, _p, _p, _p]),
     "tcad_block_jacobi_setup_rel": (ctypes.c_int, [_p, _p, _p, _p, _p, _p, ctypes.c_double,

@@ -1438,9 +1438,8 @@ struct WorkRb {
 // kRbResidentCtas blocks of `most` slots) is split over all SMs instead:
 // whole warps of slots, at most one block per SM.
 constexpr int64_t kRbResidentCtas = 148;
-static int64_t rb_cluster_slots(const tcad_pack_t* pk) {
-  return std::min(kRbResidentMaxSlots,
-                  rb_resident_js_slots(pk->dim == 2 ? TCAD_NE2 : TCAD_NE3));
+static int64_t rb_cluster_slots(int dim) {
+  return std::min(kRbResidentMaxSlots, rb_resident_js_slots(dim == 2 ? TCAD_NE2 : TCAD_NE3));
 }
 // CTAs of the cluster that takes an instance of `slots` slots, `most` a CTA (0:
 // none does): 8 while that is at most two slots a thread
@@ -1530,6 +1529,35 @@ static WorkEq carve_eq(const tcad_pack_t* pk, void* base) {
   return w;
 }
 
+// Where the slots of a pack's instances lie (host arithmetic on its shapes):
+// ceil(Nx/2) Ny Nz of each colour per instance, in arrays of n_nodes
+struct RbSlots {
+  std::vector<int64_t> start;   // first slot of each instance; [n_inst]: their end
+  int64_t largest = 0;          // slots of the largest instance
+  bool tiles = true;            // every instance starts on a warp tile
+  bool fit = true;              // the arrays hold them
+  RbSlots(const int32_t* shape, int ni, int64_t n_nodes) : start((size_t)ni + 1, 0) {
+    bool room = true;
+    for (int i = 0; i < ni; ++i) {
+      const int64_t slots =
+          (int64_t)((shape[3 * i] + 1) / 2) * shape[3 * i + 1] * shape[3 * i + 2];
+      largest = std::max(largest, slots);
+      tiles = tiles && start[i] % 32 == 0;
+      start[i + 1] = start[i] + slots;
+      // whole warp tiles per instance (rb_stream.cuh), where the slot arrays
+      // (n_nodes) have the room
+      room = room && (start[i + 1] + 31) / 32 * 32 <= n_nodes;
+      if (room) start[i + 1] = (start[i + 1] + 31) / 32 * 32;
+    }
+    fit = start[ni] <= n_nodes;
+  }
+  // CTAs of the cluster that takes any instance in a coupled solve (0: none does):
+  // a cluster copies its rows of J as whole warp tiles, so they have to start on one
+  int coupled_cluster(int dim) const {
+    return tiles ? cluster_ctas(largest, rb_cluster_slots(dim)) : 0;
+  }
+};
+
 // The slot pack of a pack (host tables; see redblack.cuh): per instance
 // (ceil(Nx/2), Ny Nz, 1) slots of each colour, flat blocks of rb_flat slots
 // (`most`, `most_cluster`: the resident solves' bounds per CTA)
@@ -1550,26 +1578,21 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   TCAD_CUDA_CHECK(cudaMemcpyAsync(shp.data(), pk->shape, sizeof(int32_t) * shp.size(),
                                   cudaMemcpyDeviceToHost, s));
   TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
-  std::vector<int64_t> noff(ni + 1), foff(ni + 1);
-  noff[0] = 0; foff[0] = 0;
+  const RbSlots at(shp.data(), ni, pk->n_nodes);
+  const std::vector<int64_t>& noff = at.start;
+  std::vector<int64_t> foff(ni + 1, 0);
   int64_t fn = kRbStreamSlots, nflat = 0;
-  bool room = true;
-  if (ni == 1) fn = rb_flat((int64_t)((shp[0] + 1) / 2) * shp[1] * shp[2], most, most_cluster);
+  if (ni == 1) fn = rb_flat(at.largest, most, most_cluster);
   for (int i = 0; i < ni; ++i) {
     const int64_t hx = (shp[3 * i] + 1) / 2, rows = (int64_t)shp[3 * i + 1] * shp[3 * i + 2];
     sb[3 * i] = (int32_t)hx; sb[3 * i + 1] = (int32_t)rows; sb[3 * i + 2] = 1;
-    noff[i + 1] = noff[i] + hx * rows;
-    // whole warp tiles per instance (rb_stream.cuh), where the slot arrays
-    // (n_nodes) have the room
-    room = room && (noff[i + 1] + 31) / 32 * 32 <= pk->n_nodes;
-    if (room) noff[i + 1] = (noff[i + 1] + 31) / 32 * 32;
     const int64_t nf = (hx * rows + fn - 1) / fn;
     foff[i + 1] = foff[i] + nf;
     nflat += (hx * rows + pk->flat_nodes - 1) / pk->flat_nodes;
     for (int64_t b = 0; b < nf; ++b) fi.push_back(i);
   }
   // (n_flat >= max(n_inst, n_nodes / flat_nodes) in a consistent pack)
-  if (noff[ni] > pk->n_nodes || (size_t)foff[ni] > rb_flat_cap(pk) || nflat > 2 * pk->n_flat)
+  if (!at.fit || (size_t)foff[ni] > rb_flat_cap(pk) || nflat > 2 * pk->n_flat)
     return TCAD_ERR_ARG;
   TCAD_CUDA_CHECK(cudaMemcpyAsync(wr.shape, sb.data(), sizeof(int32_t) * sb.size(),
                                   cudaMemcpyHostToDevice, s));
@@ -1592,12 +1615,9 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   L.mp.node_off = pk->node_off;
   L.mp.n_full = pk->n_nodes;
   L.hfoff = foff;
-  int64_t largest = 0;
-  for (int i = 0; i < ni; ++i) largest = std::max<int64_t>(largest, (int64_t)sb[3 * i] * sb[3 * i + 1]);
-  L.cluster = cluster_ctas(largest, most_cluster);
-  L.share = L.cluster ? (int)even_share(largest, L.cluster) : 0;
-  L.tiles = fn % 32 == 0;
-  for (int i = 0; i < ni; ++i) L.tiles = L.tiles && noff[i] % 32 == 0;
+  L.cluster = cluster_ctas(at.largest, most_cluster);
+  L.share = L.cluster ? (int)even_share(at.largest, L.cluster) : 0;
+  L.tiles = fn % 32 == 0 && at.tiles;
   return TCAD_OK;
 }
 
@@ -2035,9 +2055,10 @@ static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double
   return TCAD_OK;
 }
 
-// whether a resident solve takes the pack, and whether it holds J's rows
+// whether a resident solve takes the pack (its blocks start on warp tiles), and
+// whether it holds J's rows
 static bool rb_resident(const tcad_pack_t* pk, const RbLayout& L) {
-  return g_fused_mode.load() &&
+  return g_fused_mode.load() && L.tiles &&
          (L.cluster || (pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
                         L.pkb.flat_nodes <= kRbResidentMaxSlots));
 }
@@ -2590,6 +2611,15 @@ extern "C" int tcad_set_krylov_fused_test(int hold) {
 
 extern "C" uint64_t tcad_krylov_fused_gave_up(void) { return g_fused_gave_up.load(); }
 
+extern "C" int tcad_slot_layout_test(const int32_t* shape, int n_inst, int64_t n_nodes, int dim,
+                                     int64_t* start, int32_t* cluster) {
+  if (!shape || n_inst < 1 || (dim != 2 && dim != 3) || !start || !cluster) return TCAD_ERR_ARG;
+  const RbSlots at(shape, n_inst, n_nodes);
+  std::copy(at.start.begin(), at.start.end(), start);
+  *cluster = at.coupled_cluster(dim);
+  return at.fit ? TCAD_OK : TCAD_ERR_ARG;
+}
+
 extern "C" int tcad_set_krylov_fused(int on) {
   return g_fused_mode.exchange(on ? 1 : 0);
 }
@@ -2735,7 +2765,7 @@ extern "C" int tcad_block_krylov(const tcad_pack_t* pk, const double* J, const d
     if (work_bytes < tcad_block_workspace_bytes(pk, 2, 0)) return TCAD_ERR_ARG;
     const WorkRb wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
     RbLayout rbl;
-    if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk))) != TCAD_OK) return rc;
+    if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk->dim))) != TCAD_OK) return rc;
     rb_pack(pk, rbl, wrb, J, s);
     TCAD_LAUNCH_CHECK();
     rc = launch_bicgstab_rb(pk, rbl, wrb, b, x, rtol, maxiter, w, nullptr, hks, s, nullptr);
@@ -2832,7 +2862,7 @@ extern "C" int tcad_newton_solve(const tcad_pack_t* pk, double* psi, double* n, 
   RbLayout rbl;
   if (use_rb) {
     wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
-    if (int rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk))) return rc;
+    if (int rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk->dim))) return rc;
   }
   std::vector<int32_t> mix_it(ni), mix_st(ni), mix_grew(ni, 0), mix_steps(ni, 0);
   std::vector<double> mix_rr(ni), mix_prev(ni, -1.0);

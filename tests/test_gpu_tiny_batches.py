@@ -1,0 +1,41 @@
+"""Batches made of tiny meshes, whose slots do not fill warp tiles: every instance's
+equilibrium and coupled solve as alone (psi within 1e-10 / 1e-9 V, the batches'
+tolerances)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _device(*shape):
+    """A p-n diode along x with a contact at both ends."""
+    import tcad_b200 as tb
+    ax = [np.linspace(0.0, 2e-4 if a == 0 else 1e-4, n) for a, n in enumerate(shape)]
+    dop = np.where(np.meshgrid(*ax[::-1], indexing="ij")[-1] < 1e-4, -1e17, 1e18)
+    dev = (tb.Device2D if len(shape) == 2 else tb.Device3D)(
+        (tb.Mesh2D if len(shape) == 2 else tb.Mesh3D)(*ax), dop)
+    rest = [q.ravel() for q in np.meshgrid(*[np.arange(n) for n in shape[1:]], indexing="ij")]
+    for name, i in (("anode", 0), ("cathode", shape[0] - 1)):
+        dev.add_contact(name, np.full(rest[0].size, i), *rest)
+    return dev
+
+
+PACKS = [[(5, 3)] * 2, [(5, 3), (41, 21)]]
+
+
+@pytest.mark.parametrize("shapes", PACKS, ids=lambda q: "+".join(str(s) for s in q))
+def test_tiny_batches_equal_alone(shapes):
+    import tcad_b200 as tb
+    from tcad_b200.batch import DeviceBatch
+    opts = tb.NewtonOptions(precond="block_jacobi")
+    b = DeviceBatch([_device(*s) for s in shapes])
+    b.solve_equilibrium(opts)
+    eq = [b.state(i)[0] for i in range(len(shapes))]
+    res = b.solve_bias([{"anode": 0.05}] * len(shapes), opts)
+    assert all(r["converged"] for r in res)
+    for i, s in enumerate(shapes):
+        dev = _device(*s)
+        dev.solve_equilibrium(opts)
+        assert np.abs(dev.psi - eq[i]).max() * dev.VT < 1e-10, s
+        dev.solve_bias({"anode": 0.05}, opts)
+        assert np.abs(dev.psi - b.state(i)[0]).max() * dev.VT < 1e-9, s
