@@ -1537,18 +1537,26 @@ struct RbSlots {
   bool tiles = true;            // every instance starts on a warp tile
   bool fit = true;              // the arrays hold them
   RbSlots(const int32_t* shape, int ni, int64_t n_nodes) : start((size_t)ni + 1, 0) {
-    bool room = true;
-    for (int i = 0; i < ni; ++i) {
-      const int64_t slots =
-          (int64_t)((shape[3 * i] + 1) / 2) * shape[3 * i + 1] * shape[3 * i + 2];
-      largest = std::max(largest, slots);
-      tiles = tiles && start[i] % 32 == 0;
-      start[i + 1] = start[i] + slots;
-      // whole warp tiles per instance (rb_stream.cuh), where the slot arrays
-      // (n_nodes) have the room
-      room = room && (start[i + 1] + 31) / 32 * 32 <= n_nodes;
-      if (room) start[i + 1] = (start[i + 1] + 31) / 32 * 32;
+    const auto slots = [&](int i) {
+      return (int64_t)((shape[3 * i] + 1) / 2) * shape[3 * i + 1] * shape[3 * i + 2];
+    };
+    const auto place = [&](int64_t unit) {   // starts on multiples of unit
+      for (int i = 0; i < ni; ++i) {
+        start[i] = (start[i] + unit - 1) / unit * unit;
+        start[i + 1] = start[i] + slots(i);
+      }
+    };
+    for (int i = 0; i < ni; ++i) largest = std::max(largest, slots(i));
+    // every instance on a warp tile, or -- where the slot arrays (n_nodes) do not have
+    // the room for that, as in a batch of tiny meshes -- all of them without gaps
+    place(32);
+    if (start[ni] > n_nodes) {
+      start[0] = 0;
+      place(1);
     }
+    for (int i = 0; i < ni; ++i) tiles = tiles && start[i] % 32 == 0;
+    const int64_t end = (start[ni] + 31) / 32 * 32;
+    if (tiles && end <= n_nodes) start[ni] = end;
     fit = start[ni] <= n_nodes;
   }
   // CTAs of the cluster that takes any instance in a coupled solve (0: none does):

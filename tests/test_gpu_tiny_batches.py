@@ -20,10 +20,11 @@ def _device(*shape):
     return dev
 
 
-PACKS = [[(5, 3)] * 2, [(5, 3), (41, 21)]]
+PACKS = [[(5, 3)] * 2, [(5, 3), (41, 21)], [(2, 2)] * 8, [(5, 5)] * 3, [(9, 7)] * 64,
+         [(3, 3, 3)] * 3, [(5, 3), (3, 3), (5, 3)]]
 
 
-@pytest.mark.parametrize("shapes", PACKS, ids=lambda q: "+".join(str(s) for s in q))
+@pytest.mark.parametrize("shapes", PACKS, ids=lambda q: f"{len(q)}x{q[0]}")
 def test_tiny_batches_equal_alone(shapes):
     import tcad_b200 as tb
     from tcad_b200.batch import DeviceBatch

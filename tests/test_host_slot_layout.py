@@ -19,15 +19,31 @@ def _layout(shapes):
     return rc, start, cluster.value, n
 
 
-PACKS = [[(5, 3)] * 2, [(3, 3)] * 2, [(41, 21), (5, 3), (5, 3)], [(5, 3), (41, 21)],
+PACKS = [[(5, 5)] * 3, [(5, 11)] * 4, [(2, 2)] * 8, [(3, 3, 3)] * 3, [(9, 7)] * 64,
+         [(5, 3), (3, 3), (5, 3)], [(5, 3)] * 2, [(3, 3)] * 2, [(41, 21), (5, 3), (5, 3)], [(5, 3), (41, 21)],
          [(64, 41), (21, 10), (2, 2)], [(9, 7, 5), (24, 16, 13)], [(5, 3, 1)] * 2]
 
 
-@pytest.mark.parametrize("shapes", PACKS, ids=lambda q: "+".join(str(s) for s in q))
+@pytest.mark.parametrize("shapes", PACKS, ids=lambda q: f"{len(q)}x{q[0]}")
 def test_clusters_start_on_warp_tiles(shapes):
     rc, start, cluster, _ = _layout(shapes)
     assert rc == 0
     assert cluster == 0 or not (start[:-1] % 32).any()
+
+
+def test_any_pack_fits():
+    """Half the nodes and a slot per odd row: without gaps the slots of any pack are in
+    n_nodes, in order and without overlap."""
+    rng = np.random.default_rng(7)
+    for _ in range(400):
+        dim, ni = int(rng.integers(2, 4)), int(rng.integers(1, 40))
+        top = int(rng.choice([4, 8, 20, 70]))
+        shapes = [tuple(int(v) for v in rng.integers(2, top, dim)) for _ in range(ni)]
+        rc, start, cluster, n = _layout(shapes)
+        slots = [(s[0] + 1) // 2 * int(np.prod(s[1:])) for s in shapes]
+        assert rc == 0 and start[0] == 0 and start[-1] <= n, shapes
+        assert (np.diff(start) >= slots).all(), shapes
+        assert cluster == 0 or not (start[:-1] % 32).any(), shapes
 
 
 def test_single_instances_keep_their_cluster():
