@@ -159,6 +159,15 @@ struct ClusterSync {
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
     par = 0;
+    // a peer's shared memory may be written once the peer runs (a CTA without slots
+    // of its own would get to its first sum before that)
+    barrier();
+  }
+
+  __device__ __forceinline__ void barrier() {
+    asm volatile(
+        "barrier.cluster.arrive.release.aligned;\n\t"
+        "barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 
   template <int NQ>
@@ -191,9 +200,7 @@ struct ClusterSync {
       }
       __syncwarp();
     }
-    asm volatile(
-        "barrier.cluster.arrive.release.aligned;\n\t"
-        "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    barrier();
     if constexpr (NQ > 0) {
 #pragma unroll
       for (int q = 0; q < NQ; ++q) {
