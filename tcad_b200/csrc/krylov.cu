@@ -1441,11 +1441,23 @@ constexpr int64_t kRbResidentCtas = 148;
 static int64_t rb_cluster_slots(int dim) {
   return std::min(kRbResidentMaxSlots, rb_resident_js_slots(dim == 2 ? TCAD_NE2 : TCAD_NE3));
 }
-// CTAs of the cluster that takes an instance of `slots` slots, `most` a CTA (0:
-// none does): 8 while that is at most two slots a thread
-static int cluster_ctas(int64_t slots, int64_t most) {
-  if (slots <= 8 * std::min<int64_t>(most, 2 * NT)) return 8;
-  return slots <= 16 * most ? 16 : 0;
+// CTAs of the cluster that takes each of n instances of at most `slots` slots, `most` a
+// CTA (0: none does).  One instance: 8 while that is at most two slots a thread, else 16.
+// A batch: the fewest that hold the largest instance at four slots a thread, then twice
+// as many while all clusters still run at once, a CTA per SM -- what is left over at a
+// full GPU waits for a cluster to end, and larger clusters spend more of their time in
+// barriers.  Equilibria of n devices, per step / clusters of 8 / this: 20 x 20 diodes,
+// 1,024 of them 2.74 / 5.66 / 1.90 ms; 60 x 40, 256 3.67 / 4.72 / 2.02; MOSFETs of up to
+// 120 x 60, 128 39.8 / 15.2 / 11.1.  Coupled, an iteration: 20 x 20, 1,024 152 / 399 /
+// 53 us; 14 x 10 x 9 tri-gates, 128 59 / 64 / 21.
+static int cluster_ctas(int64_t slots, int64_t most, int n) {
+  const bool two = slots <= 8 * std::min<int64_t>(most, 2 * NT);
+  int c = two ? 8 : 16;
+  if (n > 1) {
+    for (c = 1; c < kClusterMaxCtas && slots > c * std::min<int64_t>(most, 4 * NT);) c *= 2;
+    while (c < (two ? 8 : kClusterMaxCtas) && 2 * c * (int64_t)n <= kRbResidentCtas) c *= 2;
+  }
+  return slots <= c * most ? c : 0;
 }
 static int64_t even_share(int64_t slots, int64_t blocks) {
   return ((slots + blocks - 1) / blocks + 31) / 32 * 32;
@@ -1454,7 +1466,7 @@ static int64_t even_share(int64_t slots, int64_t blocks) {
 // of the grid's and the cluster's resident solve takes
 static int64_t rb_flat(int64_t slots, int64_t most, int64_t most_cluster) {
   const int64_t sms = kRbResidentCtas;
-  if (const int c = cluster_ctas(slots, most_cluster)) return even_share(slots, c);
+  if (const int c = cluster_ctas(slots, most_cluster, 1)) return even_share(slots, c);
   if (even_share(slots, sms) <= most) return even_share(slots, sms);
   // a larger single instance: as many blocks for every SM, of at most
   // kRbStreamSlots slots
@@ -1562,7 +1574,7 @@ struct RbSlots {
   // CTAs of the cluster that takes any instance in a coupled solve (0: none does):
   // a cluster copies its rows of J as whole warp tiles, so they have to start on one
   int coupled_cluster(int dim) const {
-    return tiles ? cluster_ctas(largest, rb_cluster_slots(dim)) : 0;
+    return tiles ? cluster_ctas(largest, rb_cluster_slots(dim), (int)start.size() - 1) : 0;
   }
 };
 
@@ -1623,7 +1635,7 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   L.mp.node_off = pk->node_off;
   L.mp.n_full = pk->n_nodes;
   L.hfoff = foff;
-  L.cluster = cluster_ctas(at.largest, most_cluster);
+  L.cluster = cluster_ctas(at.largest, most_cluster, ni);
   L.share = L.cluster ? (int)even_share(at.largest, L.cluster) : 0;
   L.tiles = fn % 32 == 0 && at.tiles;
   return TCAD_OK;

@@ -42,12 +42,13 @@ def test_tiny_batches_equal_alone(shapes):
         assert np.abs(dev.psi - b.state(i)[0]).max() * dev.VT < 1e-9, s
 
 
-def test_clusters_with_empty_blocks_bit_identical_to_per_step():
-    """64 instances of 32 slots: seven of a cluster's eight CTAs have none and reach the
-    first sum at once, and the clusters do not all fit on the GPU together.  One block
-    of slots, so the sums are the per-step kernels'."""
+@pytest.mark.parametrize("n", [2, 18, 64, 400])
+def test_clusters_with_empty_blocks_bit_identical_to_per_step(n):
+    """Instances of 32 slots: of a cluster's eight CTAs (two of 64, one of 400) only the
+    first has any, the others reach the first sum at once.  One block of slots, so the
+    sums are the per-step kernels'."""
     from test_gpu_resident import _batch_solve, _batch_system
-    pk = _batch_system([_device(8, 8)] * 64)
+    pk = _batch_system([_device(8, 8)] * n)
     want = _batch_solve(pk, 1e-9, 200, 0)
     n0 = pk.lib.tcad_launch_count()
     for _ in range(20):

@@ -51,3 +51,19 @@ def test_single_instances_keep_their_cluster():
                         ((120, 120), 16), ((31, 22, 16), 16), ((201, 101), 0)):
         rc, start, cluster, _ = _layout([shape])
         assert (rc, start[0], cluster) == (0, 0, ctas), shape
+
+
+@pytest.mark.parametrize("shape,n,ctas", [((20, 20), 2, 8), ((20, 20), 18, 8), ((20, 20), 19, 4),
+                                          ((20, 20), 64, 2), ((20, 20), 1024, 1),
+                                          ((60, 40), 16, 8), ((60, 40), 256, 4),
+                                          ((120, 60), 16, 8), ((120, 60), 512, 8),
+                                          ((118, 120), 2, 16), ((118, 120), 64, 16),
+                                          ((14, 10, 9), 256, 2), ((30, 22, 16), 4, 16)])
+def test_cluster_size_looks_at_the_batch(shape, n, ctas):
+    """A batch's clusters all run at once (148 CTAs) unless they are the smallest that
+    hold its largest instance (480 slots a CTA in 2D, 352 in 3D)."""
+    rc, _, cluster, _ = _layout([shape] * n)
+    slots, most = (shape[0] + 1) // 2 * int(np.prod(shape[1:])), 480 if len(shape) == 2 else 352
+    assert (rc, cluster) == (0, ctas)
+    assert slots <= cluster * most
+    assert n * cluster <= 148 or cluster == 1 or slots > cluster // 2 * most
