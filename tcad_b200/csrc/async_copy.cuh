@@ -41,23 +41,30 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned n
       : "memory");
 }
 
-// wait for the phase, at most `tries` polls (each suspends for a while)
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity, unsigned tries) {
-  const unsigned a = smem_addr(b);
-  for (unsigned i = 0; i < tries; ++i) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
+__device__ __forceinline__ bool mbar_try(uint64_t* b, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_addr(b)), "r"(parity)
+      : "memory");
+  return ok != 0;
 }
-constexpr unsigned kMbarTries = 1u << 20;   // of a wait; after one that ran out
-constexpr unsigned kMbarFewTries = 64u;
+// wait for the phase, at most kBarrierNs of device time (a try suspends for a while);
+// lost: no longer than a try.  A thread whose wait ran out does not wait for other
+// copies, starts none, and waits once more for its own in flight before it returns.
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity, bool lost = false) {
+  unsigned long long t0 = 0;
+  for (unsigned i = 1; !mbar_try(b, parity); ++i) {
+    if (lost) return false;
+    if ((i & 15u) != 0u) continue;
+    const unsigned long long now = globaltimer_ns();
+    if (t0 == 0) t0 = now;
+    if (now - t0 > kBarrierNs || i > (1u << 30)) return false;
+  }
+  return true;
+}
 
 }  // namespace tcad

@@ -55,6 +55,15 @@ inline cudaError_t launch_chained(cudaStream_t s, unsigned grid, unsigned block,
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// ---- device time, and the longest wait for anything (a barrier, a copy)
+constexpr unsigned long long kBarrierNs = 1000000000ull;   // 1 s
+
+__device__ __forceinline__ unsigned long long globaltimer_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 // tcad_set_krylov_fused, tcad_set_krylov_fused_test; count a launch that gave up
 // (defined in krylov.cu)
 bool krylov_fused();

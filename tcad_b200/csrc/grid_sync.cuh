@@ -23,18 +23,11 @@
 
 namespace tcad {
 
-constexpr unsigned long long kBarrierNs = 1000000000ull;   // 1 s
 constexpr int kSyncMaxCtas = kFlatThreads;                 // one partial per thread
 constexpr int kSyncSums = 3;                               // sums per step, at most
 
 // doubles of the partials' two buffers
 constexpr size_t sync_doubles() { return 2 * kSyncSums * (size_t)kSyncMaxCtas; }
-
-__device__ __forceinline__ unsigned long long globaltimer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 
 __device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
   unsigned old;

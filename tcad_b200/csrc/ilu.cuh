@@ -588,14 +588,15 @@ k_ilu_unperm(const tcad_pack_t pk, float* Mb, const T* r,
 //   wait for their next level's records, read them and convert them (18 FP32 to
 //   FP64 conversions a thread: 200 cycles of that pipe, more than the level).
 // - One more warp fills a ring of up to kIluStages levels in shared memory with
-//   bulk copies, one contiguous run a level.
+//   bulk copies, one contiguous run a level.  (Its thread takes about as long as a
+//   level: one more wait of it per level cost a third of the sweep.)
 // Devices of up to 120 x 60, both sweeps: 175 us with one group of 256 threads that loaded
 // two levels ahead into registers from 30 arrays; 54 us now.
 // `ring`: bytes of dynamic shared memory, at least GROUPS levels of the longest Lc.
 template <int GROUPS>
 __global__ void __launch_bounds__(kIluSweepThreads)
 k_ilu_sweep(const tcad_pack_t pk, float* Mf, float* Mb, KState* ks,
-            const uint8_t* __restrict__ mask, int rows, int ring) {
+            const uint8_t* __restrict__ mask, int rows, int ring, bool hold) {
   chain_in();
   extern __shared__ __align__(128) unsigned char s_ring[];
   __shared__ uint64_t s_full[kIluStages], s_empty[kIluStages];
@@ -617,13 +618,12 @@ k_ilu_sweep(const tcad_pack_t pk, float* Mf, float* Mb, KState* ks,
   }
   for (int i = threadIdx.x; i < 2 * 3 * kIluThreads; i += blockDim.x) (&fr[0][0][0])[i] = 0.0;
   __syncthreads();
+  // A wait that runs out: the thread does not say that it has read a level from then
+  // on, so the copying thread's own wait runs out and it starts no more copies.
   bool lost = false;
-  unsigned tries = kMbarTries;
+  int issued = 0;                                 // levels whose copy was started
   auto wait = [&](uint64_t* b, unsigned parity) {
-    if (!mbar_wait(b, parity, tries)) {
-      lost = true;
-      tries = kMbarFewTries;
-    }
+    if (!mbar_wait(b, parity, lost)) lost = true;
   };
   const int grp = threadIdx.x / rows;             // GROUPS: the copying warp
   const int c = threadIdx.x - grp * rows, lane = threadIdx.x & 31;
@@ -634,13 +634,23 @@ k_ilu_sweep(const tcad_pack_t pk, float* Mf, float* Mb, KState* ks,
       const float* const M = fwd ? Mf : Mb;
       int st = base % D;
       unsigned par = (base / D) & 1;
-      for (int s = 0; s < nd; ++s) {
-        wait(&s_empty[st], par ^ 1u);             // the first round finds them empty
+      int s = 0;
+      if (hold) {                                 // (test hook: a copy that never comes)
+        mbar_expect(&s_full[st], level);
+        if (++st == D) { st = 0; par ^= 1u; }
+        s = 1;
+      }
+      for (; s < nd; ++s) {
+        if (!mbar_wait(&s_empty[st], par ^ 1u)) {   // the first round finds them empty
+          lost = true;
+          break;
+        }
         mbar_expect(&s_full[st], level);
         bulk_copy(s_ring + st * level, M + (q.soff + (int64_t)at(s) * Lc) * kIluRec, level,
                   &s_full[st]);
         if (++st == D) { st = 0; par ^= 1u; }
       }
+      issued = base + s;
       return;
     }
     const int cn = fwd ? max(c - 1, 0) : min(c + 1, Lc - 1);   // (its record is 0 at the edge)
@@ -667,7 +677,7 @@ k_ilu_sweep(const tcad_pack_t pk, float* Mf, float* Mb, KState* ks,
         a[0] = u.x; a[1] = u.y; a[2] = v.x;
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[st]);
+      if (lane == 0 && !lost) mbar_arrive(&s_empty[st]);
       st += GROUPS;
       if (st >= D) { st -= D; par ^= 1u; }
       // level s - 1 is in fr (its group arrived; the first level has none)
@@ -698,8 +708,12 @@ k_ilu_sweep(const tcad_pack_t pk, float* Mf, float* Mb, KState* ks,
   sweep(true, 0);
   __threadfence();
   fence_async();   // the forward results, before the bulk copies that read them
-  __syncthreads();
-  sweep(false, nd);
+  if (!__syncthreads_or(lost)) sweep(false, nd);
+  if (!__syncthreads_or(lost)) return;
+  // the copies in flight: the last D that were started
+  if (grp == GROUPS && lane == 0)
+    for (int i = max(issued - D, 0); i < issued; ++i)
+      (void)mbar_wait(&s_full[i % D], (i / D) & 1);
   if (lost) {
     ks[inst].status = TCAD_ERR_CUDA;
     ks[inst].active = 0;

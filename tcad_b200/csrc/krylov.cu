@@ -1678,6 +1678,11 @@ static Work carve(const tcad_pack_t* pk, void* base, size_t cap) {
 static int ilu_rows(int rows) { return (rows + 31) / 32 * 32; }
 static int ilu_ring(int rows) { return std::min(12 * rows * kIluRec * 4, 200 << 10); }
 
+// test hook: a grid barrier's arrival (bar[3] = 1), a copy of the ILU sweeps that never come
+enum { kHoldNone, kHoldBarrier, kHoldCopy = 3 };
+static std::atomic<int> g_fused_test_hold{kHoldNone};
+static int test_hold() { return g_fused_test_hold.load(); }
+
 // out = M^-1 r: the coalesced slot-order sweeps when the factor wrote them
 // (2D, every shorter side <= kIluThreads), else the node-order sweeps
 template <class T>
@@ -1689,12 +1694,13 @@ static void ilu_apply_t(const tcad_pack_t* pk, const double* J, const double* Q,
   if (ilc && ilc->Mf) {
     launch_chained(s, ng, NT_ILU_FLAT, 0, k_ilu_perm<T>, *pk, Q, r, ilc->Mf, w.ks, mask, dlist);
     const int rows = ilu_rows(ilc->rows), ring = ilu_ring(ilc->rows);
+    const bool hold = test_hold() == kHoldCopy;
     if (rows <= 128)
       launch_chained(s, (unsigned)ni, 4 * rows + 32, ring, k_ilu_sweep<4>, *pk, ilc->Mf, ilc->Mb,
-                     w.ks, mask, rows, ring);
+                     w.ks, mask, rows, ring, hold);
     else
       launch_chained(s, (unsigned)ni, 2 * rows + 32, ring, k_ilu_sweep<2>, *pk, ilc->Mf, ilc->Mb,
-                     w.ks, mask, rows, ring);
+                     w.ks, mask, rows, ring, hold);
     launch_chained(s, ng, NT_ILU_FLAT, 0, k_ilu_unperm<T>, *pk, ilc->Mb, r, out, w.ks, mask, dlist);
     note_launch(3);
     return;
@@ -1706,10 +1712,9 @@ static void ilu_apply_t(const tcad_pack_t* pk, const double* J, const double* Q,
 
 // ---- fused (one cooperative launch) BiCGStab: when and how
 static std::atomic<int> g_fused_mode{1};   // 0: one launch per step always
-static std::atomic<int> g_fused_test_hold{0};        // give-up test hook (bar[3] = 1)
 static std::atomic<uint64_t> g_fused_gave_up{0};     // fused launches that gave up
 bool krylov_fused() { return g_fused_mode.load() != 0; }
-bool krylov_fused_hold() { return g_fused_test_hold.load() != 0; }
+bool krylov_fused_hold() { return test_hold() == kHoldBarrier; }
 void krylov_note_gave_up() { g_fused_gave_up.fetch_add(1); }
 
 // k_bicgstab_fused<DIM> needs every flat block resident at once
@@ -1795,7 +1800,7 @@ static int launch_bicgstab_fused(const tcad_pack_t* pk, const double* J, const d
                                  std::vector<KState>& hks, cudaStream_t s,
                                  const double* rtol_inst) {
   TCAD_CUDA_CHECK(cudaMemsetAsync(w.bar, 0, 4 * sizeof(unsigned), s));
-  if (g_fused_test_hold.load()) {
+  if (krylov_fused_hold()) {
     static const unsigned kPhantom = 1u;
     TCAD_CUDA_CHECK(cudaMemcpyAsync(w.bar + 3, &kPhantom, sizeof(unsigned),
                                     cudaMemcpyHostToDevice, s));
@@ -1957,7 +1962,7 @@ struct StepControl {
   // barrier flags and status cleared, the give-up test hook set
   void clear(const Work& w) {
     std::fill(img.begin(), img.end(), (unsigned char)0);
-    at(w.bar + 3) = g_fused_test_hold.load() ? 1u : 0u;
+    at(w.bar + 3) = krylov_fused_hold() ? 1u : 0u;
   }
 };
 
@@ -1980,7 +1985,7 @@ static int coop_launch(CoopLaunch& c, unsigned blocks, unsigned threads, size_t 
                        unsigned* flags, bool clear, cudaStream_t s) {
   if (clear) {
     TCAD_CUDA_CHECK(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned), s));
-    if (g_fused_test_hold.load()) {
+    if (krylov_fused_hold()) {
       static const unsigned kPhantom = 1u;
       TCAD_CUDA_CHECK(cudaMemcpyAsync(flags + 3, &kPhantom, sizeof(unsigned),
                                       cudaMemcpyHostToDevice, s));
@@ -2102,7 +2107,7 @@ static int queue_rb_resident(const tcad_pack_t* pk, const RbLayout& L, const Wor
   // with 448 threads.
   constexpr int T3 = rb_resident_js_slots(TCAD_NE3);
   // (the test hook holds up a grid barrier; clusters have none)
-  if (L.cluster && !g_fused_test_hold.load()) {
+  if (L.cluster && !krylov_fused_hold()) {
     if (d2)
       return L.share <= NT ? go(queue_rb_resident_t<2, 1, NT, true, ClusterSync>)
                            : go(queue_rb_resident_t<2, 2, NT, true, ClusterSync>);
@@ -2530,7 +2535,7 @@ static int queue_eq_resident(const tcad_pack_t* pk, const RbLayout& L, const Wor
                           : go(queue_eq_resident_t<3, 8, NT, S>);
   };
   // (the test hook holds up a grid barrier; clusters have none)
-  if (L.cluster && !g_fused_test_hold.load()) return pick(ClusterSync{}, L.share);
+  if (L.cluster && !krylov_fused_hold()) return pick(ClusterSync{}, L.share);
   return pk->n_inst == 1 ? pick(GridSync{}, L.pkb.flat_nodes) : 1;
 }
 
@@ -2626,7 +2631,9 @@ static int launch_cg_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& 
 using namespace tcad;
 
 extern "C" int tcad_set_krylov_fused_test(int hold) {
-  return g_fused_test_hold.exchange(hold ? 1 : 0);
+  return g_fused_test_hold.exchange(hold == kHoldCopy ? kHoldCopy
+                                    : hold            ? kHoldBarrier
+                                                      : kHoldNone);
 }
 
 extern "C" uint64_t tcad_krylov_fused_gave_up(void) { return g_fused_gave_up.load(); }

@@ -109,7 +109,7 @@ struct RbStreamer {
   int lane, warp, par;
   int64_t pend;      // block whose tile the buffer holds or waits for (-1: none)
   int pcol;          // and its colour
-  unsigned phase, tries;
+  unsigned phase;
   bool lost;         // a copy did not arrive within its limit
 
   __device__ __forceinline__ RbStreamer(const tcad_pack_t& pkb_, const RbMap& mp_,
@@ -124,7 +124,6 @@ struct RbStreamer {
     pend = -1;
     pcol = 0;
     phase = 0u;
-    tries = kMbarTries;
     lost = false;
     if (lane == 0) {
       mbar_init(&sh.bar[warp]);
@@ -140,7 +139,7 @@ struct RbStreamer {
     if (warp * 32 >= q.len) return;
     pend = q.id;
     pcol = col;
-    if (lane == 0) {
+    if (lane == 0 && !lost) {
       constexpr unsigned n = NE * 32 * sizeof(double);
       mbar_expect(&sh.bar[warp], n);
       bulk_copy(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32), n, &sh.bar[warp],
@@ -148,12 +147,16 @@ struct RbStreamer {
     }
   }
   __device__ __forceinline__ void arrive() {
-    if (!mbar_wait(&sh.bar[warp], phase, tries)) {
-      lost = true;
-      tries = kMbarFewTries;
+    if (!lost) {
+      lost = !mbar_wait(&sh.bar[warp], phase);
+      if (!lost) phase ^= 1u;
     }
-    phase ^= 1u;
     pend = -1;
+  }
+  // at the kernel's end: whether a copy was lost (lane 0 has then waited for it again)
+  __device__ __forceinline__ bool end() {
+    if (lost && lane == 0) (void)mbar_wait(&sh.bar[warp], phase);
+    return lost;
   }
 
   // block sums of v (all threads) into out[0..NS): warp sums, then the 16 of
@@ -438,7 +441,7 @@ k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR
     cur = nxt;
   }
   if (tk.inst >= 0) rb_flush<NS>(pkb, tk, partial, ticket, fin);
-  if (st.lost && st.lane == 0) {
+  if (st.end() && st.lane == 0) {
     ks[0].status = TCAD_ERR_CUDA;
     ks[0].active = 0;
   }
