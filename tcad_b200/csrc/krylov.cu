@@ -1337,7 +1337,9 @@ struct Work {
   BiVec bi;
   CgVec cg;
   double* partial;  // 2 x 4 x n_flat: block partial sums (the fused solve alternates halves)
-  unsigned* bar;    // fused solve's grid barrier: counter, generation, gave-up flag
+  // flags: arrivals at the fused solves' grid barrier; a streamed pass lost a copy; a
+  // barrier gave up; the test hook's arrival
+  unsigned* bar;
   KState* ks;
   unsigned* ticket;
   int32_t* status;
@@ -1678,8 +1680,9 @@ static Work carve(const tcad_pack_t* pk, void* base, size_t cap) {
 static int ilu_rows(int rows) { return (rows + 31) / 32 * 32; }
 static int ilu_ring(int rows) { return std::min(12 * rows * kIluRec * 4, 200 << 10); }
 
-// test hook: a grid barrier's arrival (bar[3] = 1), a copy of the ILU sweeps that never come
-enum { kHoldNone, kHoldBarrier, kHoldCopy = 3 };
+// test hook: a grid barrier's arrival (bar[3] = 1), a streamed copy of the final residual
+// pass, a copy of the iterations (streamed passes, ILU sweeps) that never come
+enum { kHoldNone, kHoldBarrier, kHoldLastCopy, kHoldCopy };
 static std::atomic<int> g_fused_test_hold{kHoldNone};
 static int test_hold() { return g_fused_test_hold.load(); }
 
@@ -2027,15 +2030,24 @@ static int cluster_launch(CoopLaunch& c, void (*kern)(P...), int ni, int ctas, i
   return TCAD_OK;
 }
 
+// The flags and the states, in one copy down (they follow each other in Work)
+static int read_states(const Work& w, int ni, unsigned (&hbar)[4], std::vector<KState>& hks,
+                       cudaStream_t s) {
+  const size_t at = reinterpret_cast<char*>(w.ks) - reinterpret_cast<char*>(w.bar);
+  std::vector<char> img(at + sizeof(KState) * ni);
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(img.data(), w.bar, img.size(), cudaMemcpyDeviceToHost, s));
+  TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+  std::memcpy(hbar, img.data(), sizeof(hbar));
+  hks.resize(ni);
+  std::memcpy(hks.data(), img.data() + at, sizeof(KState) * ni);
+  return TCAD_OK;
+}
+
 // Waits for a single-launch solve and reads its result: 1 when a grid
 // barrier gave up (the caller then solves with one launch per step)
 static int coop_result(const Work& w, int ni, std::vector<KState>& hks, cudaStream_t s) {
-  hks.resize(ni);
-  unsigned hbar[4] = {0u, 0u, 0u, 0u};
-  TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState) * ni, cudaMemcpyDeviceToHost,
-                                  s));
-  TCAD_CUDA_CHECK(cudaMemcpyAsync(hbar, w.bar, sizeof(hbar), cudaMemcpyDeviceToHost, s));
-  TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+  unsigned hbar[4];
+  if (int rc = read_states(w, ni, hbar, hks, s)) return rc;
   if (hbar[2] != 0u) {
     g_fused_gave_up.fetch_add(1);
     return 1;
@@ -2176,7 +2188,9 @@ struct RbStreamLauncher {
   template <int PASS>
   int pass(const double* X, bool all, int rearm, unsigned ng, const int32_t* dlist) const {
     return launch(k_rb_stream<DIM, PASS>, ng, rb_stream_smem<DIM>(), pkb, mp, wr.JR, wr.JB, X,
-                  wr.tR, bi, wr.rhs, w.ks, all, wr.partial, w.ticket, rearm, ng, dlist);
+                  wr.tR, bi, wr.rhs, w.ks, all, wr.partial, w.ticket, rearm, ng, dlist, w.bar + 1,
+                  PASS == kRbTrue ? test_hold() == kHoldLastCopy
+                                  : rb_is_red(PASS) && !all && test_hold() == kHoldCopy);
   }
   int iteration(bool formed, unsigned ng, const int32_t* dlist) const {
     int rc = TCAD_OK;
@@ -2238,6 +2252,8 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
   const RbStreamLauncher<3> st3{pkb, L.mp, wr, bi, w, sms, s};
   // colours of b, right-hand side and state of every instance
   TCAD_CUDA_CHECK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned) * ni, s));
+  TCAD_CUDA_CHECK(cudaMemsetAsync(w.bar, 0, 4 * sizeof(unsigned), s));
+  unsigned hbar[4];
   if (d2)
     k_rb_split<2><<<nbb, NT, 0, s>>>(pkb, L.mp, b, wr.bR, wr.bB, wr.bbf, wr.partial, w.ticket);
   else
@@ -2290,14 +2306,10 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
     }
     TCAD_LAUNCH_CHECK();
     done_iters += check;
-    TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState) * ni,
-                                    cudaMemcpyDeviceToHost, s));
-    TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+    if (int rc = read_states(w, ni, hbar, hks, s)) return rc;
+    if (hbar[1] != 0u) return TCAD_ERR_CUDA;   // a streamed pass lost a copy
     bool any = false;
-    for (int i = 0; i < ni; ++i) {
-      if (hks[i].status == TCAD_ERR_CUDA) return TCAD_ERR_CUDA;
-      any = any || hks[i].active;
-    }
+    for (int i = 0; i < ni; ++i) any = any || hks[i].active;
     if (any)
       if (int rc = grid.update(hks, wr.blk, s)) return rc;
     if (!any) {
@@ -2317,9 +2329,8 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
         note_launch(2);
       }
       TCAD_LAUNCH_CHECK();
-      TCAD_CUDA_CHECK(cudaMemcpyAsync(hks.data(), w.ks, sizeof(KState) * ni,
-                                      cudaMemcpyDeviceToHost, s));
-      TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
+      if (int rc = read_states(w, ni, hbar, hks, s)) return rc;
+      if (hbar[1] != 0u) return TCAD_ERR_CUDA;
       for (int i = 0; i < ni; ++i) any = any || hks[i].active;
       ++rechecks;
       if (!any) break;
@@ -2631,9 +2642,9 @@ static int launch_cg_rb(const tcad_pack_t* pk, const RbLayout& L, const WorkEq& 
 using namespace tcad;
 
 extern "C" int tcad_set_krylov_fused_test(int hold) {
-  return g_fused_test_hold.exchange(hold == kHoldCopy ? kHoldCopy
-                                    : hold            ? kHoldBarrier
-                                                      : kHoldNone);
+  return g_fused_test_hold.exchange(hold == kHoldLastCopy || hold == kHoldCopy ? hold
+                                    : hold                                   ? kHoldBarrier
+                                                                             : kHoldNone);
 }
 
 extern "C" uint64_t tcad_krylov_fused_gave_up(void) { return g_fused_gave_up.load(); }

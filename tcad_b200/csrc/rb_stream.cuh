@@ -133,8 +133,8 @@ struct RbStreamer {
   }
 
   // start copying the warp's tile of block q, colour col (every lane has
-  // read the buffer)
-  __device__ __forceinline__ void issue(const RbBlk& q, int col) {
+  // read the buffer); hold: a copy that never comes (test hook)
+  __device__ __forceinline__ void issue(const RbBlk& q, int col, bool hold = false) {
     pend = -1;
     if (warp * 32 >= q.len) return;
     pend = q.id;
@@ -142,7 +142,7 @@ struct RbStreamer {
     if (lane == 0 && !lost) {
       constexpr unsigned n = NE * 32 * sizeof(double);
       mbar_expect(&sh.bar[warp], n);
-      bulk_copy(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32), n, &sh.bar[warp],
+      if (!hold) bulk_copy(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32), n, &sh.bar[warp],
                 policy);
     }
   }
@@ -356,8 +356,9 @@ __device__ __forceinline__ void rb_totals(const tcad_pack_t& pkb, int inst, cons
 
 // ---- one step per launch over nblk blocks (blk: their numbers, null: all) of the
 // instances still iterating (all: of every instance).  A CTA adds its count of
-// blocks to the instance's ticket once; the last CTA takes the totals into ks
-// (status TCAD_ERR_CUDA when a copy did not arrive within its limit).
+// blocks to the instance's ticket once; the last CTA takes the totals into ks.
+// Where a copy did not arrive within its limit a word of its own says so: the launches
+// behind it return at once, and the host gives the solve up.
 struct RbTicket {
   unsigned count = 0u;
   int inst = -1;
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(NTS, 1)
 k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR,
             const double* __restrict__ JB, const double* X, double* Tr, BiVec w,
             const double* rhs, KState* ks, bool all, double* partial, unsigned* ticket,
-            int rearm, int64_t nblk, const int32_t* __restrict__ blk) {
+            int rearm, int64_t nblk, const int32_t* __restrict__ blk, unsigned* lost, bool hold) {
   constexpr int NS = rb_sums(PASS), col = rb_is_red(PASS) ? 0 : 1;
   extern __shared__ __align__(128) double s_tiles[];
   __shared__ RbStreamShared sh;
@@ -421,10 +422,16 @@ k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR
   // J and the tables are older than the kernel before this one; its states and
   // vectors are not
   RbBlk cur = rb_fetch(pkb, nullptr, blockIdx.x, nblk, blk);
-  st.issue(cur, col);
+  st.issue(cur, col, hold && blockIdx.x == 0 && st.warp == 0);
   launch_dependents();
   wait_prior();
-  if (!all && !ks[cur.inst].active) cur.len = 0;
+  const bool off = !all && !ks[cur.inst].active;
+  // (one answer for the CTA: others of this launch may be writing the word)
+  if (__syncthreads_or(*(volatile unsigned*)lost != 0u)) {
+    if (st.pend >= 0) st.arrive();
+    return;
+  }
+  if (off) cur.len = 0;
   for (int64_t i = blockIdx.x; i < nblk; i += gridDim.x) {
     const RbBlk nxt = rb_fetch(pkb, all ? nullptr : ks, i + gridDim.x, nblk, blk);
     if (cur.len > 0) {
@@ -441,10 +448,7 @@ k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR
     cur = nxt;
   }
   if (tk.inst >= 0) rb_flush<NS>(pkb, tk, partial, ticket, fin);
-  if (st.end() && st.lane == 0) {
-    ks[0].status = TCAD_ERR_CUDA;
-    ks[0].active = 0;
-  }
+  if (st.end()) *lost = 1u;
 }
 
 template <int DIM>
