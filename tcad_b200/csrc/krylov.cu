@@ -2067,9 +2067,12 @@ static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double
   const auto kern = k_bicgstab_rb_resident<DIM, K, T, JS, SYNC>;
   const int share = kCluster ? L.share : L.pkb.flat_nodes;
   if (share > T * K) return 1;
-  const size_t smem = JS ? (size_t)share * Stencil<DIM>::NE * 16 : 0;
-  if (JS && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess) {
+  constexpr size_t row = Stencil<DIM>::NE * 16;
+  const size_t smem = JS ? share * row : 0;
+  // (the kernel's limit, not this launch's size: threads share it)
+  constexpr size_t most = std::min(T * K, rb_resident_js_slots(Stencil<DIM>::NE)) * row;
+  if (JS && (smem > most || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)most) != cudaSuccess)) {
     (void)cudaGetLastError();
     return 1;
   }
@@ -2496,9 +2499,12 @@ static int queue_eq_resident_t(const RbLayout& L, const WorkEq& we, const double
   constexpr bool kCluster = std::is_same<SYNC, ClusterSync>::value;
   const auto kern = k_eqrb_resident<DIM, K, T, SYNC>;
   const int share = kCluster ? L.share : L.pkb.flat_nodes;
-  const size_t smem = (size_t)share * (1 + 2 * DIM) * 16;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess) {
+  constexpr size_t row = (1 + 2 * DIM) * 16;
+  const size_t smem = share * row;
+  // (the kernel's limit, not this launch's size: threads share it)
+  constexpr size_t most = T * K * row;
+  if (smem > most || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)most) != cudaSuccess) {
     (void)cudaGetLastError();
     return 1;
   }
