@@ -12,16 +12,20 @@ __device__ __forceinline__ double clip700(double x) {
   return x < -700.0 ? -700.0 : (x > 700.0 ? 700.0 : x);
 }
 
-// a / b from r = 1/b, bit for bit (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990: with r the rounded
-// reciprocal, one residual correction of a r gives the rounded quotient, barring
-// underflow and overflow).
+// a / b from r = 1/b, bit for bit barring underflow and overflow (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990:
+// with r the rounded reciprocal, one residual correction of a quotient within one unit
+// of its last place rounds it correctly).  RN(a r) may be 1.5 units off, but not where
+// that matters: the correction's error is below 2^-51 units, and where a / b is that
+// close to the middle of two numbers RN(a r) is one of the two -- with significands in
+// [1, 2), |r - 1/b| <= 2^-54 moves a r by less than a / 2 units, so only an a within
+// 2^-51 of 2 could get past them, and then a / b lies next to a number.
 __device__ __forceinline__ double div_in_range(double a, double b, double r) {
   const double q = a * r;
   return fma(fma(-q, b, a), r, q);
 }
-// ... of any a: where a or the quotient is zero, infinite, NaN or of a magnitude near
-// the end of the range it is a r.
+// ... of any a and a b whose reciprocal is in range: where a or the quotient is zero,
+// infinite, NaN or of a magnitude near the end of the range it is a r.
 __device__ __forceinline__ double div_by(double a, double b, double r) {
   const double q = a * r;
   const double c = fma(fma(-q, b, a), r, q);
@@ -33,6 +37,20 @@ struct Divisor {
   double b, r;
   static __device__ __forceinline__ Divisor of(double b) { return Divisor{b, 1.0 / b}; }
   __device__ __forceinline__ double divide(double a) const { return div_by(a, b, r); }
+};
+
+// ... and of any b: numerator and divisor are scaled by a power of two where b is far
+// from one, so that neither the reciprocal nor the residual leaves the range.
+struct WideDivisor {
+  Divisor d;
+  double s;
+  static __device__ __forceinline__ WideDivisor of(double b) {
+    // by the exponent: below 2^-700, to 2^700, above
+    const unsigned e = (unsigned)__double2hiint(b) >> 20 & 0x7ffu;
+    const double s = __hiloint2double(e < 323u ? 1623 << 20 : e > 1723u ? 423 << 20 : 1023 << 20, 0);
+    return WideDivisor{Divisor::of(b * s), s};
+  }
+  __device__ __forceinline__ double divide(double a) const { return d.divide(a * s); }
 };
 
 // B(x), B'(x) and those of -x of the series band |x| < 1e-4 (kernels.py:92-96,
@@ -168,7 +186,7 @@ __device__ __forceinline__ void recomb(double n, double p, double nie, double ta
   const double den = taup * (nph + nie) + taun * (pph + nie);
   double R = excess / den;
   const double den2 = den * den;
-  const Divisor by2 = Divisor::of(den2);
+  const WideDivisor by2 = WideDivisor::of(den2);   // (den^2 of a cold semiconductor's carriers)
   double dRdn = by2.divide(pph * den - excess * taup);
   double dRdp = by2.divide(nph * den - excess * taun);
   if (par[TCAD_P_AUGER] != 0.0) {
