@@ -852,7 +852,13 @@ extern "C" size_t tcad_csr_workspace_bytes(int64_t n, int method, int restart) {
   v += 4096 * 4 * sizeof(double) + 64 * sizeof(double) + 256;
   v += (size_t)4096 * (m + 1) * sizeof(double);      // Gram-Schmidt partials
   v += (size_t)(m + 1) * sizeof(double) + vec;       // coefficients, true residual
-  v += (size_t)(m + 1) * (m + 6) * sizeof(double);   // GMRES: H, rotations, sums
+  if (method != 0) {
+    // H, rotations and sums of the min(restart, n) columns that are used lie in what the
+    // partials leave (kGridBlocks of 4096 a column); past 3,500 columns H is larger
+    const int64_t c = std::min<int64_t>(m, n);
+    const int64_t more = (c + 1) * (c + 5) - (4096 - kGridBlocks) * ((int64_t)m + 1);
+    if (more > 0) v += (size_t)more * sizeof(double);
+  }
   return v + (1u << 20);                             // alignment slack
 }
 
@@ -964,6 +970,7 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
     G.R = reinterpret_cast<double*>(take((size_t)m * (m + 1) * 8));
     double** const vec[5] = {&G.h1, &G.h2, &G.cs, &G.sn, &G.g};
     for (double** q : vec) *q = reinterpret_cast<double*>(take((size_t)(m + 1) * 8));
+    if (used > work_bytes) return TCAD_ERR_ARG;
     G.ticket = c.ticket;
     G.st = reinterpret_cast<GState*>(c.scal + 8);
     std::vector<double> R((size_t)m * (m + 1)), g(m + 1), yv(m);
