@@ -174,48 +174,11 @@ __global__ void k_bj_apply(int64_t n, int bs, const double* __restrict__ inv,
   }
 }
 
-// ---- deterministic multi-dot: out[q] = sum_i a_q[i] * b_q[i] -------------
-struct Dots {
-  const double* a[4];
-  const double* b[4];
-  int nd;
-};
-
-__global__ void __launch_bounds__(NT) k_dots(int64_t n, Dots d, double* __restrict__ partial,
-                                             unsigned* ticket, double* __restrict__ out) {
-  __shared__ double sm[32];
-  __shared__ int last;
-  double v[4] = {0, 0, 0, 0};
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
-    for (int q = 0; q < d.nd; ++q) v[q] += d.a[q][i] * d.b[q][i];
-  for (int q = 0; q < d.nd; ++q) {
-    const double r = block_sum<NT>(v[q], sm);
-    if (threadIdx.x == 0) partial[blockIdx.x * 4 + q] = r;
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int q = 0; q < d.nd; ++q) {
-    double s = 0.0;
-    for (unsigned bb = threadIdx.x; bb < gridDim.x; bb += NT) s += __ldcg(&partial[bb * 4 + q]);
-    const double r = block_sum<NT>(s, sm);
-    if (threadIdx.x == 0) out[q] = r;
-  }
-  if (threadIdx.x == 0) *ticket = 0u;
-}
-
-// y = a*x + b*y (+ c*z)
-__global__ void k_axpbypcz(int64_t n, double a, const double* __restrict__ x, double b,
-                           double* __restrict__ y, double c, const double* __restrict__ z) {
+// y = a*x + b*y
+__global__ void k_axpby(int64_t n, double a, const double* __restrict__ x, double b,
+                        double* __restrict__ y) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = a * x[i] + b * y[i];
-  if (z) v += c * z[i];
-  y[i] = v;
+  if (i < n) y[i] = a * x[i] + b * y[i];
 }
 
 // ---- the last block of a grid to finish (ticket), for its totals
@@ -253,6 +216,15 @@ __device__ __forceinline__ bool grid_sums(double (&v)[NS], double* partial, unsi
     tot[q] = block_sum<T>(s, sm);
   }
   return true;
+}
+
+// out = sum_i v[i]^2
+__global__ void __launch_bounds__(NT) k_norm2(int64_t n, const double* __restrict__ v,
+                                              double* partial, unsigned* ticket, double* out) {
+  double s[1] = {0.0}, tot[1];
+  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
+    s[0] += v[i] * v[i];
+  if (grid_sums<1>(s, partial, ticket, tot) && threadIdx.x == 0) out[0] = tot[0];
 }
 
 // z = M^-1 r at one block row (bs = 3, 6), or one row
@@ -698,7 +670,7 @@ __global__ void __launch_bounds__(NT) k_cb_spmv(Sys A, Bicg B) {
   }
   if (!grid_sums<2>(sum, B.partial, B.ticket, tot) || threadIdx.x != 0) return;
   if (T) {
-    // (h[0] = (t, t), h[1] = (s, t) in the reference's naming of the step)
+    // tot[0] = (t, t), tot[1] = (s, t)
     B.st->omega = tot[0] > 0.0 ? tot[1] / tot[0] : 0.0;
   } else if (tot[0] == 0.0 || !isfinite(tot[0])) {
     B.st->done = 1;
@@ -789,18 +761,17 @@ int prec(const Ctx& c, const double* r, double* z) {
   return TCAD_OK;
 }
 
-int dots(const Ctx& c, Dots d, double* host_out) {
-  k_dots<<<c.nblk, NT, 0, c.s>>>(c.A.n, d, c.partial, c.ticket, c.scal);
+int norm(const Ctx& c, const double* v, double& out) {
+  k_norm2<<<c.nblk, NT, 0, c.s>>>(c.A.n, v, c.partial, c.ticket, c.scal);
   note_launch();
-  TCAD_CUDA_CHECK(cudaMemcpyAsync(host_out, c.scal, sizeof(double) * d.nd,
-                                  cudaMemcpyDeviceToHost, c.s));
+  TCAD_CUDA_CHECK(cudaMemcpyAsync(&out, c.scal, sizeof(double), cudaMemcpyDeviceToHost, c.s));
   TCAD_CUDA_CHECK(cudaStreamSynchronize(c.s));
+  out = std::sqrt(out);
   return TCAD_OK;
 }
 
-int axpy(const Ctx& c, double a, const double* x, double b, double* y, double cc = 0.0,
-         const double* z = nullptr) {
-  k_axpbypcz<<<g1(c.A.n), NT, 0, c.s>>>(c.A.n, a, x, b, y, cc, z);
+int axpby(const Ctx& c, double a, const double* x, double b, double* y) {
+  k_axpby<<<g1(c.A.n), NT, 0, c.s>>>(c.A.n, a, x, b, y);
   note_launch();
   return TCAD_OK;
 }
@@ -909,12 +880,9 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
   }
   if (precond_out) *precond_out = c.bs;
   const int64_t N = n;
-  double h[4];
-  // ||b||
-  Dots d0{{b}, {b}, 1};
-  int rc = dots(c, d0, h);
+  double bnorm = 0.0;
+  int rc = norm(c, b, bnorm);
   if (rc) return rc;
-  const double bnorm = std::sqrt(h[0]);
   if (!std::isfinite(bnorm)) return TCAD_ERR_NONFINITE;
   const double tol = std::max(atol, rtol * bnorm);
   int it = 0;
@@ -933,7 +901,7 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
     B.maxit = maxiter;
     // r = b - A x
     spmv(c, x, B.r);
-    axpy(c, 1.0, b, -1.0, B.r);
+    axpby(c, 1.0, b, -1.0, B.r);
     k_cb_start<<<gv, NT, 0, s>>>(B);
     note_launch();
     const unsigned gb = g1(c.bs > 1 ? N / c.bs : N);
@@ -955,7 +923,7 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
       }
       TCAD_LAUNCH_CHECK();
     }
-    if (st.done == 2) axpy(c, st.alpha, B.ph, 1.0, x);
+    if (st.done == 2) axpby(c, st.alpha, B.ph, 1.0, x);
     rn = st.rn;
     it = st.it;
   } else {
@@ -979,10 +947,8 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
     for (int cycle = 0;; ++cycle) {
       // r = b - A x -> V_0
       spmv(c, x, G.w);
-      axpy(c, 1.0, b, -1.0, G.w);
-      Dots dr{{G.w}, {G.w}, 1};
-      if ((rc = dots(c, dr, h))) return rc;
-      rn = std::sqrt(h[0]);
+      axpby(c, 1.0, b, -1.0, G.w);
+      if ((rc = norm(c, G.w, rn))) return rc;
       if (rn <= tol || cycle >= maxiter || !std::isfinite(rn)) break;
       k_gm_start<<<1, NT, 0, s>>>(G, rn);
       k_gm_next<<<gb, NT, 0, s>>>(G, c.bs, c.inv, z);
@@ -1032,7 +998,7 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
       k_lincomb<<<g1(N), NT, 0, s>>>(N, G.V, j, G.h1, y);
       note_launch();
       prec(c, y, z);
-      axpy(c, 1.0, z, 1.0, x);
+      axpby(c, 1.0, z, 1.0, x);
       TCAD_CUDA_CHECK(cudaStreamSynchronize(s));
     }
   }
@@ -1040,11 +1006,11 @@ extern "C" int tcad_csr_krylov(int64_t n, const int32_t* indptr, const int32_t* 
   // pytcad/linsolve.py:973-982)
   double* rt = reinterpret_cast<double*>(take(N * 8));
   spmv(c, x, rt);
-  axpy(c, 1.0, b, -1.0, rt);
-  Dots dt{{rt}, {rt}, 1};
-  if ((rc = dots(c, dt, h))) return rc;
+  axpby(c, 1.0, b, -1.0, rt);
+  double res = 0.0;
+  if ((rc = norm(c, rt, res))) return rc;
   TCAD_LAUNCH_CHECK();
-  const double true_res = std::sqrt(h[0]) / std::max(bnorm, 1e-300);
+  const double true_res = res / std::max(bnorm, 1e-300);
   if (iters_out) *iters_out = it;
   if (resid_out) *resid_out = true_res;
   const bool ok = rn <= tol && std::isfinite(true_res);

@@ -152,8 +152,8 @@ __device__ __forceinline__ void rb_couple(const double* __restrict__ Jc,
 }
 
 // ---- per-block bodies of the per-step kernels; the single-launch solves
-// (rb_resident.cuh, rb_streamed.cuh) and the streamed passes (rb_stream.cuh)
-// run the same arithmetic in the same order
+// (rb_resident.cuh) and the streamed passes (rb_stream.cuh) run the same
+// arithmetic
 
 // bR, bB <- the colours of b at the block's slots; returns the thread's
 // share of (b, b)

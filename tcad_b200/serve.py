@@ -56,7 +56,7 @@ def bytes_per_node(dim):
     work32 = 6 * 3 * 4 + ne * 4 + 2 * 3 * 4
     ilu = (9 + 6) * 8                        # ILU(0) factor and two vectors
     if dim == 2:   # slot-order sweeps: two records of 28 FP32, up to two slots a node
-        ilu += 2 * (27 + 18) * 4 + 2 * 2 * 3 * 8
+        ilu += 2 * 2 * 28 * 4
     eq = (2 * (1 + 2 * dim) + 5) * 8 + 2 * 4 / 256   # equilibrium red-black extension
     return int(np.ceil(doubles * 8 + 1 + work64 + work32 + ilu + eq))
 

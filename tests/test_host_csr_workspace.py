@@ -20,7 +20,7 @@ def _without_h(n, method, m):
 @pytest.mark.parametrize("n,restart", CASES)
 def test_gmres_layout_fits(n, restart):
     m = min(restart, n)
-    parts = [9 * n, 4096 * 4, 64, 32, (m + 1) * n, n, n, n, 592 * (m + 1), m * (m + 1)] \
+    parts = [9 * n, 4096 * 4, 64, 32, (m + 1) * n, n, n, n, n, 592 * (m + 1), m * (m + 1)] \
         + [m + 1] * 5
     assert sum(-(-8 * p // 256) * 256 for p in parts) <= _bytes(n, 1, restart)
 
