@@ -218,9 +218,13 @@ size_t tcad_block_workspace_bytes(const tcad_pack_t* pk, int method, int restart
  * GPU at once (cooperative, bounded grid barriers between the steps) and, on
  * the red-black system, every pack whose instances each fit a thread-block
  * cluster; tcad_csr_krylov's GMRES runs a restart cycle of up to 37,296 rows
- * so -- the same arithmetic in the same order as the launch-per-step
- * kernels, so the result is bit-identical (GMRES: to rounding); on = 0: one launch per step
- * always.  Process-wide; returns the previous setting. */
+ * so; on = 0: one launch per step always.  With one instance the arithmetic and
+ * its order are the launch-per-step kernels', so the result is bit-identical.
+ * With several the two agree to rounding: a cluster sums over its CTAs' shares,
+ * whose size follows from the largest instance and the number of instances, the
+ * launch-per-step kernels over 512-slot blocks.  (So an instance solved in a
+ * batch equals itself solved alone to rounding, not bit for bit.)  GMRES: to
+ * rounding.  Process-wide; returns the previous setting. */
 int tcad_set_krylov_fused(int on);
 
 /* Test hook of the solves' failure paths (no counterpart in the
@@ -400,7 +404,7 @@ typedef struct tcad_newton_opts {
    * eliminated exactly: half the unknowns, the same matrix bytes per
    * product, about half the iterations); the stopping test stays the full
    * system's ||b - A x|| <= eta ||b||.  Small packs are solved in one launch
-   * (tcad_set_krylov_fused; the same arithmetic).  ILU(0) solves, FP32 operators and a workspace sized
+   * (tcad_set_krylov_fused).  ILU(0) solves, FP32 operators and a workspace sized
    * without the red-black extension (tcad_block_workspace_bytes method 0)
    * keep the full system.  tcad_equilibrium_solve: its PCG runs on the
    * red-black Schur complement of the scalar Poisson system (every

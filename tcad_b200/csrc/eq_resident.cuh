@@ -13,7 +13,8 @@
 // each instead (SYNC = ClusterSync): barriers inside a cluster cost a fifth, and a
 // batch's instances run side by side, each to its own convergence.
 // Expressions and the order of the sums are the per-step kernels', so the
-// update is bit-identical to launch_cg_rb's loop over the same blocks.
+// update is bit-identical to launch_cg_rb's loop over the same blocks (of several
+// instances: the CTAs' shares, other blocks than the loop's 512 slots).
 #pragma once
 
 namespace tcad {

@@ -1735,10 +1735,6 @@ static bool fused_fits(unsigned nb) {
   return nb >= 1 && (long long)nb <= (long long)per * sms;
 }
 
-// The whole solve of a single-instance pack in one launch (same arithmetic
-// as the launch-per-step path).  Returns TCAD_OK with hks[0] filled, or 1
-// when the launch was refused or a grid barrier gave up (the caller then
-// solves with one launch per step).
 // Launch grid of a per-step Krylov loop: every flat block, or -- once the
 // instances still iterating cover under 3/4 of them -- only those instances'
 // blocks (a compact list rebuilt whenever the active set changes), so a
@@ -1797,6 +1793,10 @@ struct ActiveGrid {
   }
 };
 
+// The whole solve of a single-instance pack in one launch (same arithmetic
+// as the launch-per-step path).  Returns TCAD_OK with hks[0] filled, or 1
+// when the launch was refused or a grid barrier gave up (the caller then
+// solves with one launch per step).
 static int launch_bicgstab_fused(const tcad_pack_t* pk, const double* J, const double* b,
                                  double* x, double rtol, int maxiter, const BiVec& bi,
                                  const Work& w, const int32_t* pre_status,

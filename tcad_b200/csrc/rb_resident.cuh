@@ -16,7 +16,8 @@
 // result is bit-identical to launch_bicgstab_rb's loop over the same blocks.
 //
 // Instances whose rows fit in the shared memory of one cluster have a cluster
-// each (SYNC = ClusterSync, eq_resident.cuh).
+// each (SYNC = ClusterSync, eq_resident.cuh); their blocks are its CTAs' shares,
+// with several instances other ones than the per-step loop's 512 slots.
 #pragma once
 
 namespace tcad {
