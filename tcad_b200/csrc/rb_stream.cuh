@@ -357,8 +357,8 @@ __device__ __forceinline__ void rb_totals(const tcad_pack_t& pkb, int inst, cons
 // ---- one step per launch over nblk blocks (blk: their numbers, null: all) of the
 // instances still iterating (all: of every instance).  A CTA adds its count of
 // blocks to the instance's ticket once; the last CTA takes the totals into ks.
-// Where a copy did not arrive within its limit a word of its own says so: the launches
-// behind it return at once, and the host gives the solve up.
+// Where a copy did not arrive within its limit a word of its own says so, which the host
+// reads with the states.
 struct RbTicket {
   unsigned count = 0u;
   int inst = -1;
@@ -425,13 +425,7 @@ k_rb_stream(const tcad_pack_t pkb, const RbMap mp, const double* __restrict__ JR
   st.issue(cur, col, hold && blockIdx.x == 0 && st.warp == 0);
   launch_dependents();
   wait_prior();
-  const bool off = !all && !ks[cur.inst].active;
-  // (one answer for the CTA: others of this launch may be writing the word)
-  if (__syncthreads_or(*(volatile unsigned*)lost != 0u)) {
-    if (st.pend >= 0) st.arrive();
-    return;
-  }
-  if (off) cur.len = 0;
+  if (!all && !ks[cur.inst].active) cur.len = 0;
   for (int64_t i = blockIdx.x; i < nblk; i += gridDim.x) {
     const RbBlk nxt = rb_fetch(pkb, all ? nullptr : ks, i + gridDim.x, nblk, blk);
     if (cur.len > 0) {
