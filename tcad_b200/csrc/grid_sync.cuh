@@ -23,7 +23,7 @@
 
 namespace tcad {
 
-constexpr int kSyncMaxCtas = kFlatThreads;                 // one partial per thread
+constexpr int kSyncMaxCtas = 2 * kFlatThreads;             // two partials per thread
 constexpr int kSyncSums = 3;                               // sums per step, at most
 
 // doubles of the partials' two buffers
@@ -126,8 +126,11 @@ struct GridSync {
     if (!ok) return false;
     if constexpr (NQ > 0) {
 #pragma unroll
-      for (int q = 0; q < NQ; ++q)
+      for (int q = 0; q < NQ; ++q) {
         r[q] = 0.0 + (threadIdx.x < G ? __ldcg(&buf[q * kSyncMaxCtas + threadIdx.x]) : 0.0);
+        if (threadIdx.x < NT && threadIdx.x + NT < G)
+          r[q] += __ldcg(&buf[q * kSyncMaxCtas + NT + threadIdx.x]);
+      }
       warps(sb, r);
       __syncthreads();
 #pragma unroll

@@ -674,6 +674,7 @@ k_true_resid(const tcad_pack_t pk, const TJ* __restrict__ J, const T* __restrict
 #include "redblack.cuh"
 #include "grid_sync.cuh"
 #include "rb_resident.cuh"
+#include "rb_wave.cuh"
 #include "rb_stream.cuh"
 namespace tcad {
 
@@ -1440,6 +1441,8 @@ struct WorkRb {
 // kRbResidentCtas blocks of `most` slots) is split over all SMs instead:
 // whole warps of slots, at most one block per SM.
 constexpr int64_t kRbResidentCtas = 148;
+constexpr int64_t kRbWaveSlots2 = 2 * kRbResidentCtas * 512, kRbWaveSlots3 = 106496;   // rb_wave
+constexpr int64_t kRbWaveFull3 = 90112;
 static int64_t rb_cluster_slots(int dim) {
   return std::min(kRbResidentMaxSlots, rb_resident_js_slots(dim == 2 ? TCAD_NE2 : TCAD_NE3));
 }
@@ -1466,10 +1469,13 @@ static int64_t even_share(int64_t slots, int64_t blocks) {
 }
 // slots per flat block of a single instance; `most`, `most_cluster`: what one CTA
 // of the grid's and the cluster's resident solve takes
-static int64_t rb_flat(int64_t slots, int64_t most, int64_t most_cluster) {
+static int64_t rb_flat(int64_t slots, int64_t most, int64_t most_cluster, int dim) {
   const int64_t sms = kRbResidentCtas;
   if (const int c = cluster_ctas(slots, most_cluster, 1)) return even_share(slots, c);
   if (even_share(slots, sms) <= most) return even_share(slots, sms);
+  // (the 3D wave of up to 176 full blocks, in those / evenly over two CTAs an SM: 77k slots
+  // 31.6 / 32.8 us an iteration, 90k 35.9 / 40.7, 95k 46.1 / 41.8)
+  if (dim == 3 && slots <= kRbWaveFull3) return kRbStreamSlots;
   // a larger single instance: as many blocks for every SM, of at most
   // kRbStreamSlots slots
   return even_share(slots, sms * ((slots + sms * kRbStreamSlots - 1) / (sms * kRbStreamSlots)));
@@ -1604,7 +1610,7 @@ static int rb_layout(const tcad_pack_t* pk, const W& wr, RbLayout& L, cudaStream
   const std::vector<int64_t>& noff = at.start;
   std::vector<int64_t> foff(ni + 1, 0);
   int64_t fn = kRbStreamSlots, nflat = 0;
-  if (ni == 1) fn = rb_flat(at.largest, most, most_cluster);
+  if (ni == 1) fn = rb_flat(at.largest, most, most_cluster, pk->dim);
   for (int i = 0; i < ni; ++i) {
     const int64_t hx = (shp[3 * i] + 1) / 2, rows = (int64_t)shp[3 * i + 1] * shp[3 * i + 2];
     sb[3 * i] = (int32_t)hx; sb[3 * i + 1] = (int32_t)rows; sb[3 * i + 2] = 1;
@@ -2095,16 +2101,51 @@ static int queue_rb_resident_t(const RbLayout& L, const WorkRb& wr, const double
   return TCAD_OK;
 }
 
-// whether a resident solve takes the pack (its blocks start on warp tiles), and
-// whether it holds J's rows
+// whether k_bicgstab_rb_wave takes the pack: its blocks are one wave of two CTAs per SM,
+// and in 3D J (66 MB) mostly stays in L2.  Solves of 10 and of 60 iterations and one
+// iteration of many, us, streamed / wave: 2D, 78k slots 562 / 364, 2465 / 1652, 36.8 /
+// 25.8; 113k 585 / 413, 2655 / 1856, 39.7 / 29.0; 150k 685 / 575, 3151 / 2778, 47.2 / 44.0.
+// 3D, 77k 587 / 440, 2664 / 2021, 39.7 / 31.6; 90k 611 / 501, 2788 / 2290, 41.5 / 35.9;
+// 104k 643 / 572, 2910 / 2729, 43.4 / 43.2; 121k 727 / 702, 3376 / 3472, 50.6 / 55.3.
+static bool rb_wave(const tcad_pack_t* pk, const RbLayout& L) {
+  return pk->n_inst == 1 && L.pkb.n_flat > kRbResidentCtas &&
+         L.pkb.n_flat <= 2 * kRbResidentCtas &&
+         L.pkb.n_nodes <= (pk->dim == 2 ? kRbWaveSlots2 : kRbWaveSlots3);
+}
+// whether a single launch takes the pack (its blocks start on warp tiles), and whether
+// it holds J's rows in shared memory
 static bool rb_resident(const tcad_pack_t* pk, const RbLayout& L) {
   return g_fused_mode.load() && L.tiles &&
-         (L.cluster || (pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
-                        L.pkb.flat_nodes <= kRbResidentMaxSlots));
+         (L.cluster || rb_wave(pk, L) ||
+          (pk->n_inst == 1 && L.pkb.n_flat <= kRbResidentCtas &&
+           L.pkb.flat_nodes <= kRbResidentMaxSlots));
 }
 static bool rb_resident_js(const tcad_pack_t* pk, const RbLayout& L) {
   return L.cluster ||
-         L.pkb.flat_nodes <= rb_resident_js_slots(pk->dim == 2 ? TCAD_NE2 : TCAD_NE3);
+         (!rb_wave(pk, L) &&
+          L.pkb.flat_nodes <= rb_resident_js_slots(pk->dim == 2 ? TCAD_NE2 : TCAD_NE3));
+}
+
+// k_bicgstab_rb_wave, queued: 1 when the launch was refused
+template <int DIM>
+static int queue_rb_wave(const RbLayout& L, const WorkRb& wr, const double* b, double* x,
+                         double rtol, int maxiter, const Work& w, const int32_t* pre_status,
+                         bool clear, cudaStream_t s, const double* rtol_inst) {
+  CoopLaunch c;
+  if (int rc = coop_launch(c, (unsigned)L.pkb.n_flat, NT, 0, w.bar, clear, s)) return rc;
+  BiVec bi = w.bi;   // black vectors (stride: the slot count)
+  bi.ph = bi.p;
+  bi.sh = bi.s;
+  const int rechecks = 8;
+  if (cudaLaunchKernelEx(&c.cfg, k_bicgstab_rb_wave<DIM>, L.pkb, L.mp, (const double*)wr.JR,
+                         (const double*)wr.JB, b, x, wr.bR, wr.bB, wr.tR, wr.xb, wr.rhs, bi,
+                         w.ks, wr.sync, w.bar, rtol, maxiter, pre_status, rtol_inst,
+                         rechecks) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  note_launch();
+  return TCAD_OK;
 }
 
 static int queue_rb_resident(const tcad_pack_t* pk, const RbLayout& L, const WorkRb& wr,
@@ -2130,6 +2171,9 @@ static int queue_rb_resident(const tcad_pack_t* pk, const RbLayout& L, const Wor
                          : go(queue_rb_resident_t<3, 1, T3, true, ClusterSync>);
   }
   if (pk->n_inst != 1) return 1;
+  if (rb_wave(pk, L))
+    return (d2 ? queue_rb_wave<2> : queue_rb_wave<3>)(L, wr, b, x, rtol, maxiter, w, pre_status,
+                                                      clear, s, rtol_inst);
   const int fn = L.pkb.flat_nodes;
   if (d2)
     return fn <= NT ? go(queue_rb_resident_t<2, 1, NT, true, GridSync>)
@@ -2245,11 +2289,11 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
                         rtol_inst) == TCAD_OK &&
       coop_result(w, ni, hks, s) == TCAD_OK)
     return TCAD_OK;
-  // J streamed through shared memory where the pack is larger than one wave
-  // of blocks and every block starts on a warp tile
+  // J streamed through shared memory where the pack is larger than the single
+  // launches' and every block starts on a warp tile
   const int sms = sm_count();
   const bool stream = L.tiles && pkb.flat_nodes <= kRbStreamSlots && (int)nbb > sms &&
-                      rb_stream_ready(d2);
+                      !rb_wave(pk, L) && rb_stream_ready(d2);
   const bool formed = pkb.n_nodes <= kRbFormSlots;
   const RbStreamLauncher<2> st2{pkb, L.mp, wr, bi, w, sms, s};
   const RbStreamLauncher<3> st3{pkb, L.mp, wr, bi, w, sms, s};
