@@ -585,10 +585,17 @@ k_bi_init(const tcad_pack_t pk, const T* __restrict__ b, T* __restrict__ x, BiVe
              pre_status ? pre_status[fb.inst] : TCAD_OK);
 }
 
+//
+// early: let the next kernel's CTAs start at once, for the streamed passes, which fetch J
+// while they wait.  Not among these kernels: CTAs that start early fill the SMs unevenly
+// (172k nodes 63 us an iteration against 48, 983k 241.3 against 240.2, an ILU(0) batch of
+// 16 MOSFETs 65.2 ms against 61.6); their chain only hides the launch.
 template <class T>
 __global__ void __launch_bounds__(NT, 4)
-k_bi_p(const tcad_pack_t pk, BiVecT<T> w, const KState* ks, const int32_t* __restrict__ blk) {
-  chain_in();
+k_bi_p(const tcad_pack_t pk, BiVecT<T> w, const KState* ks, const int32_t* __restrict__ blk,
+       bool early) {
+  if (early) launch_dependents();
+  wait_prior();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   const KState s = ks[fb.inst];
@@ -600,7 +607,7 @@ template <int DIM, class T, class TJ = T>
 __global__ void __launch_bounds__(NT)
 k_bi_v(const tcad_pack_t pk, const TJ* __restrict__ J, BiVecT<T> w, KState* ks,
        double* partial, unsigned* ticket, const int32_t* __restrict__ blk) {
-  chain_in();
+  wait_prior();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (!ks[fb.inst].active) return;
@@ -613,8 +620,9 @@ k_bi_v(const tcad_pack_t pk, const TJ* __restrict__ J, BiVecT<T> w, KState* ks,
 template <class T>
 __global__ void __launch_bounds__(NT, 4)
 k_bi_s(const tcad_pack_t pk, BiVecT<T> w, KState* ks, double* partial, unsigned* ticket,
-       const int32_t* __restrict__ blk) {
-  chain_in();
+       const int32_t* __restrict__ blk, bool early) {
+  if (early) launch_dependents();
+  wait_prior();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   const KState s0 = ks[fb.inst];
@@ -629,7 +637,7 @@ template <int DIM, class T, class TJ = T>
 __global__ void __launch_bounds__(NT)
 k_bi_t(const tcad_pack_t pk, const TJ* __restrict__ J, BiVecT<T> w, KState* ks,
        double* partial, unsigned* ticket, const int32_t* __restrict__ blk) {
-  chain_in();
+  wait_prior();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   if (!ks[fb.inst].active) return;
@@ -643,8 +651,9 @@ k_bi_t(const tcad_pack_t pk, const TJ* __restrict__ J, BiVecT<T> w, KState* ks,
 template <class T>
 __global__ void __launch_bounds__(NT, 3)
 k_bi_x(const tcad_pack_t pk, T* x, BiVecT<T> w, KState* ks, double* partial,
-       unsigned* ticket, const int32_t* __restrict__ blk) {
-  chain_in();
+       unsigned* ticket, const int32_t* __restrict__ blk, bool early) {
+  if (early) launch_dependents();
+  wait_prior();
   const int64_t fbi = blk ? (int64_t)blk[blockIdx.x] : (int64_t)blockIdx.x;
   const FlatBlock fb = flat_block(pk, fbi);
   const KState s0 = ks[fb.inst];
@@ -1880,7 +1889,7 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
     const unsigned ng = grid.ng;
     const int32_t* dlist = grid.dlist;
     for (int q = 0; q < check; ++q) {
-      launch_chained(s, ng, NT, 0, k_bi_p<T>, *pk, bi, w.ks, dlist);
+      launch_chained(s, ng, NT, 0, k_bi_p<T>, *pk, bi, w.ks, dlist, false);
       note_launch();
       if (Qilu) {  // ph = M^-1 p
         ilu_apply_t<T>(pk, Jilu, Qilu, bi.p, bi.ph, w, ilu_mask, nzmax, ilc, ng, dlist, s);
@@ -1896,7 +1905,7 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
       // neighbour value instead of one; the single-launch solve of small
       // packs, which is latency-bound, keeps the fused form.)
       {
-        launch_chained(s, ng, NT, 0, k_bi_s<T>, *pk, bi, w.ks, w.partial, w.ticket, dlist);
+        launch_chained(s, ng, NT, 0, k_bi_s<T>, *pk, bi, w.ks, w.partial, w.ticket, dlist, false);
         note_launch();
         if (Qilu) {  // sh = M^-1 s
           ilu_apply_t<T>(pk, Jilu, Qilu, bi.s, bi.sh, w, ilu_mask, nzmax, ilc, ng, dlist, s);
@@ -1907,7 +1916,7 @@ static int launch_bicgstab_t(const tcad_pack_t* pk, const TJ* J, const T* b, T* 
           launch_chained(s, ng, NT, 0, k_bi_t<3, T, TJ>, *pk, J, bi, w.ks, w.partial, w.ticket, dlist);
         note_launch();
       }
-      launch_chained(s, ng, NT, 0, k_bi_x<T>, *pk, x, bi, w.ks, w.partial, w.ticket, dlist);
+      launch_chained(s, ng, NT, 0, k_bi_x<T>, *pk, x, bi, w.ks, w.partial, w.ticket, dlist, false);
       note_launch();
     }
     TCAD_LAUNCH_CHECK();
@@ -2251,13 +2260,13 @@ struct RbStreamLauncher {
                   dlist));
       return rc;
     }
-    k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist);
+    k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist, true);
     then(pass<kRbRed>(bi.p, false, 0, ng, dlist));
     then(pass<kRbVs>(nullptr, false, 0, ng, dlist));
-    k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist);
+    k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist, true);
     then(pass<kRbRed>(bi.s, false, 0, ng, dlist));
     then(pass<kRbTs>(nullptr, false, 0, ng, dlist));
-    k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, wr.partial, w.ticket, dlist);
+    k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, wr.partial, w.ticket, dlist, true);
     note_launch(3);
     return rc;
   }
@@ -2328,7 +2337,7 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
           return rc;
         continue;
       }
-      k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist);
+      k_bi_p<<<ng, NT, 0, s>>>(pkb, bi, w.ks, dlist, false);
       if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.p, wr.tR, w.ks, dlist);
         k_rb_v<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
@@ -2338,7 +2347,7 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
         k_rb_v<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
       }
-      k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist);
+      k_bi_s<<<ng, NT, 0, s>>>(pkb, bi, w.ks, wr.partial, w.ticket, dlist, false);
       if (d2) {
         k_rb_red<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JR, bi.s, wr.tR, w.ks, dlist);
         k_rb_t<2><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
@@ -2348,7 +2357,7 @@ static int launch_bicgstab_rb(const tcad_pack_t* pk, const RbLayout& L, const Wo
         k_rb_t<3><<<ng, NT, 0, s>>>(pkb, L.mp, wr.JB, wr.tR, bi, w.ks, wr.partial, w.ticket,
                                     dlist);
       }
-      k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, wr.partial, w.ticket, dlist);
+      k_bi_x<<<ng, NT, 0, s>>>(pkb, wr.xb, bi, w.ks, wr.partial, w.ticket, dlist, false);
       note_launch(7);
     }
     TCAD_LAUNCH_CHECK();
@@ -3483,17 +3492,17 @@ extern "C" int tcad_block_krylov_noalloc(const tcad_pack_t* pk, const double* J,
   int check = 4, done_iters = 0, rechecks = 0;
   for (;;) {
     for (int q = 0; q < check; ++q) {
-      k_bi_p<<<nb, NT, 0, s>>>(*pk, w.bi, w.ks, nullptr);
+      k_bi_p<<<nb, NT, 0, s>>>(*pk, w.bi, w.ks, nullptr, false);
       if (pk->dim == 2)
         k_bi_v<2><<<nb, NT, 0, s>>>(*pk, J, w.bi, w.ks, w.partial, w.ticket, nullptr);
       else
         k_bi_v<3><<<nb, NT, 0, s>>>(*pk, J, w.bi, w.ks, w.partial, w.ticket, nullptr);
-      k_bi_s<<<nb, NT, 0, s>>>(*pk, w.bi, w.ks, w.partial, w.ticket, nullptr);
+      k_bi_s<<<nb, NT, 0, s>>>(*pk, w.bi, w.ks, w.partial, w.ticket, nullptr, false);
       if (pk->dim == 2)
         k_bi_t<2><<<nb, NT, 0, s>>>(*pk, J, w.bi, w.ks, w.partial, w.ticket, nullptr);
       else
         k_bi_t<3><<<nb, NT, 0, s>>>(*pk, J, w.bi, w.ks, w.partial, w.ticket, nullptr);
-      k_bi_x<<<nb, NT, 0, s>>>(*pk, x, w.bi, w.ks, w.partial, w.ticket, nullptr);
+      k_bi_x<<<nb, NT, 0, s>>>(*pk, x, w.bi, w.ks, w.partial, w.ticket, nullptr, false);
       note_launch(5);
     }
     TCAD_LAUNCH_CHECK();
