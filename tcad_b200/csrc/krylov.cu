@@ -585,7 +585,6 @@ k_bi_init(const tcad_pack_t pk, const T* __restrict__ b, T* __restrict__ x, BiVe
              pre_status ? pre_status[fb.inst] : TCAD_OK);
 }
 
-//
 // early: let the next kernel's CTAs start at once, for the streamed passes, which fetch J
 // while they wait.  Not among these kernels: CTAs that start early fill the SMs unevenly
 // (172k nodes 63 us an iteration against 48, 983k 241.3 against 240.2, an ILU(0) batch of
@@ -1482,6 +1481,9 @@ static int64_t rb_flat(int64_t slots, int64_t most, int64_t most_cluster, int di
   const int64_t sms = kRbResidentCtas;
   if (const int c = cluster_ctas(slots, most_cluster, 1)) return even_share(slots, c);
   if (even_share(slots, sms) <= most) return even_share(slots, sms);
+  // the equilibrium's per-step kernels: full blocks (128 x 96 x 64 tri-gate in 878 of 448
+  // slots 44.9 ms, in 768 of 512 43.5)
+  if (most > kRbResidentMaxSlots) return kRbStreamSlots;
   // (the 3D wave of up to 176 full blocks, in those / evenly over two CTAs an SM: 77k slots
   // 31.6 / 32.8 us an iteration, 90k 35.9 / 40.7, 95k 46.1 / 41.8)
   if (dim == 3 && slots <= kRbWaveFull3) return kRbStreamSlots;
