@@ -20,14 +20,14 @@ namespace tcad {
 void note_launch(uint64_t n = 1);
 
 // ---- programmatic dependent launch
-// A kernel of a chain lets the next one's CTAs start where SMs are free, then waits
-// for the kernels before it (what they wrote is visible then).  Every kernel that
-// launch_chained() starts waits, so a kernel that passed its wait follows all that
-// came before.  What a chained kernel reads before its wait, or through a pointer
+// A kernel of a chain may let the next one's CTAs start where SMs are free (worth it for
+// small grids and for kernels that fetch something while they wait; else the next one
+// starts as this one ends), then waits for the kernels before it (what they wrote is
+// visible then).  Every kernel that launch_chained() starts waits, so a kernel that
+// passed its wait follows all that came before.  What a chained kernel reads before its wait, or through a pointer
 // that lets the compiler move the load there (__restrict__), must be older than the
 // kernel before it.  (Iterations of five to eleven launches of 2 to 10 us each, small
-// systems: GMRES of 13.8k unknowns 37 -> 31 us an iteration; BiCGStab with ILU(0) of 16
-// MOSFETs 207 -> 193.)
+// systems: GMRES of 13.8k unknowns 37 -> 31 us an iteration.)
 __device__ __forceinline__ void launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
