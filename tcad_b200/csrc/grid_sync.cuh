@@ -86,12 +86,13 @@ struct GridSync {
     gb = GridBarrier{b, 0u};
   }
 
-  // tot = the sums over the grid of the first kFlatThreads threads' v, valid in
-  // every thread; NQ = 0: a barrier alone.  Orders all global writes before it, of any
+  // tot = the sums over the grid (of at most PER x kFlatThreads CTAs) of the first
+  // kFlatThreads threads' v, valid in every thread; NQ = 0: a barrier alone.  Orders all global writes before it, of any
   // thread of the grid, before all reads after it.
-  template <int NQ>
+  template <int NQ, int PER = 1>
   __device__ __forceinline__ bool sum(const double* v, double* tot) {
     static_assert(NQ <= kSyncSums, "sums per step");
+    static_assert(PER * kFlatThreads <= kSyncMaxCtas, "partials per thread");
     constexpr int NT = kFlatThreads, NW = NT / 32, NS = NQ > 0 ? NQ : 1;
     __shared__ double sa[NS][NW], sb[NS][NW];
     __shared__ int ok;
@@ -128,7 +129,7 @@ struct GridSync {
 #pragma unroll
       for (int q = 0; q < NQ; ++q) {
         r[q] = 0.0 + (threadIdx.x < G ? __ldcg(&buf[q * kSyncMaxCtas + threadIdx.x]) : 0.0);
-        if (threadIdx.x < NT && threadIdx.x + NT < G)
+        if (PER > 1 && threadIdx.x < NT && threadIdx.x + NT < G)
           r[q] += __ldcg(&buf[q * kSyncMaxCtas + NT + threadIdx.x]);
       }
       warps(sb, r);

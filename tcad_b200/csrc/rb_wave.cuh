@@ -131,10 +131,10 @@ k_bicgstab_rb_wave(const tcad_pack_t pkb, const RbMap mp, const double* __restri
   double tot[3];
   __shared__ KState S;   // thread 0's, read by all after a barrier
   double sum[1] = {rb_split_body<DIM>(pkb, mp, fb, b, bR, bB)};
-  if (!gs.template sum<1>(sum, tot)) return;
+  if (!gs.template sum<1, 2>(sum, tot)) return;
   const double bb = tot[0];
   sum[0] = rb_init_body<DIM>(pkb, mp, fb, JB, bR, bB, rhs, xb, w);
-  if (!gs.template sum<1>(sum, tot)) return;
+  if (!gs.template sum<1, 2>(sum, tot)) return;
   if (threadIdx.x == 0)
     rb_fin_init(S, tot[0], bb, rtol_inst ? rtol_inst[inst] : rtol, maxit,
                 pre_status ? pre_status[inst] : TCAD_OK);
@@ -145,32 +145,32 @@ k_bicgstab_rb_wave(const tcad_pack_t pkb, const RbMap mp, const double* __restri
                        RbFormP{w.r + g.soff, w.p + g.soff, w.v + g.soff, NS, S.beta, S.omega,
                                S.restart},
                        Tr);
-      if (!gs.template sum<0>(nullptr, nullptr)) return;
+      if (!gs.template sum<0, 2>(nullptr, nullptr)) return;
       sum[0] = rb_wave_v<DIM>(g, fb, NS, JB, Tr, w, S.beta, S.omega, S.restart);
-      if (!gs.template sum<1>(sum, tot)) return;
+      if (!gs.template sum<1, 2>(sum, tot)) return;
       if (threadIdx.x == 0) fin_v(S, tot[0]);
       __syncthreads();
       if (!S.active) break;
       rb_wave_red<DIM>(g, fb, NS, JR, RbFormS{w.r + g.soff, w.v + g.soff, NS, S.alpha}, Tr);
-      if (!gs.template sum<0>(nullptr, nullptr)) return;
+      if (!gs.template sum<0, 2>(nullptr, nullptr)) return;
       double s3[3];
       rb_wave_t<DIM>(g, fb, NS, JB, Tr, w, S.alpha, s3);
-      if (!gs.template sum<3>(s3, tot)) return;
+      if (!gs.template sum<3, 2>(s3, tot)) return;
       if (threadIdx.x == 0) {
         fin_s(S, tot[0]);
         fin_t(S, tot[1], tot[2]);
       }
       __syncthreads();
       bi_x_body<double>(pkb, fb, xb, w, S.alpha, S.omega, s3);
-      if (!gs.template sum<3>(s3, tot)) return;
+      if (!gs.template sum<3, 2>(s3, tot)) return;
       if (threadIdx.x == 0) fin_x(S, tot[0], tot[1], tot[2]);
       __syncthreads();
     }
     // true Schur residual r = rhs - S x
     rb_wave_red<DIM>(g, fb, NS, JR, RbVal{xb + g.soff, NS}, Tr);
-    if (!gs.template sum<0>(nullptr, nullptr)) return;
+    if (!gs.template sum<0, 2>(nullptr, nullptr)) return;
     sum[0] = rb_true_body<DIM>(pkb, mp, fb, JB, Tr, rhs, xb, w.r);
-    if (!gs.template sum<1>(sum, tot)) return;
+    if (!gs.template sum<1, 2>(sum, tot)) return;
     if (threadIdx.x == 0) fin_true(S, tot[0], rechecks < max_rechecks ? 1 : 0);
     __syncthreads();
     if (!S.active) break;
