@@ -2,10 +2,10 @@
 // resident but whose slot blocks are all on the GPU at once (one wave: two CTAs of 256
 // threads per SM, a block of at most 512 slots each), in one cooperative launch.
 //
-// Vectors and J stay in global memory and are read through L1, which serves many of a
-// slot's 36 or 54 gathers (the resident kernel's registers do not stretch to two slots a
-// thread at two CTAs an SM: 0.9 KB of spills, 49 us an iteration of a 440 x 480 diode;
-// here 28, streamed 39).  Within a step no CTA reads what another writes, which the
+// Vectors and J stay in global memory and are read through L1 (a fifth of the sectors hit)
+// and L2, 36 or 54 gathers a slot and pass (the resident kernel's registers do not stretch
+// to two slots a thread at two CTAs an SM: 0.9 KB of spills, 49 us an iteration of a 440 x
+// 480 diode; here 28, streamed 39).  Within a step no CTA reads what another writes, which the
 // restrict qualifiers of the steps' bodies tell the compiler, and the solver's state is in
 // shared memory: both slots' gathers then fit in the registers (60 x 56 x 46 tri-gate 40
 // us with the state in every thread, 32).  The five steps of an iteration and their sums
