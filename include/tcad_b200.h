@@ -234,8 +234,9 @@ int tcad_set_krylov_fused(int on);
  * again with one launch per step.  hold = 2, 3: a bulk copy never comes, of a
  * streamed red-black solve's final residual pass (2), of its iterations or of
  * the ILU(0) sweeps (3); the bounded wait for it runs out and the call
- * returns TCAD_ERR_CUDA.  Process-wide; returns the previous setting.  tcad_krylov_fused_gave_up counts the fused launches whose
- * barrier gave up, hook or not. */
+ * returns TCAD_ERR_CUDA.  Process-wide; returns the previous setting.
+ * tcad_krylov_fused_gave_up counts the fused launches whose barrier gave up,
+ * hook or not. */
 int tcad_set_krylov_fused_test(int hold);
 uint64_t tcad_krylov_fused_gave_up(void);
 

@@ -24,10 +24,10 @@ void note_launch(uint64_t n = 1);
 // small grids and for kernels that fetch something while they wait; else the next one
 // starts as this one ends), then waits for the kernels before it (what they wrote is
 // visible then).  Every kernel that launch_chained() starts waits, so a kernel that
-// passed its wait follows all that came before.  What a chained kernel reads before its wait, or through a pointer
-// that lets the compiler move the load there (__restrict__), must be older than the
-// kernel before it.  (Iterations of five to eleven launches of 2 to 10 us each, small
-// systems: GMRES of 13.8k unknowns 37 -> 31 us an iteration.)
+// passed its wait follows all that came before.  What a chained kernel reads before its
+// wait, or through a pointer that lets the compiler move the load there (__restrict__),
+// must be older than the kernel before it.  (Iterations of five to eleven launches of 2 to
+// 10 us each, small systems: GMRES of 13.8k unknowns 37 -> 31 us an iteration.)
 __device__ __forceinline__ void launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -87,8 +87,8 @@ struct GridSync {
   }
 
   // tot = the sums over the grid (of at most PER x kFlatThreads CTAs) of the first
-  // kFlatThreads threads' v, valid in every thread; NQ = 0: a barrier alone.  Orders all global writes before it, of any
-  // thread of the grid, before all reads after it.
+  // kFlatThreads threads' v, valid in every thread; NQ = 0: a barrier alone.  Orders all
+  // global writes before it, of any thread of the grid, before all reads after it.
   template <int NQ, int PER = 1>
   __device__ __forceinline__ bool sum(const double* v, double* tot) {
     static_assert(NQ <= kSyncSums, "sums per step");

@@ -2170,8 +2170,8 @@ static int queue_rb_resident(const tcad_pack_t* pk, const RbLayout& L, const Wor
   // 3D shares above NT slots: a thread for each slot.  Two slots a thread leave no
   // registers for the gathers (54 loads a slot in red(p)): 64 x 48 x 32 tri-gate 32.5 us
   // an iteration, with 352 threads 19.1; 31 x 22 x 16 in a cluster 22.0 and 10.2; 56 x
-  // 48 x 46, rows from L2, 39.0 and with 512 threads 28.5.  2D (36 loads): 512 x 256 MOSFET 16.0 with two slots a thread, 17.7
-  // with 448 threads.
+  // 48 x 46, rows from L2, 39.0 and with 512 threads 28.5.  2D (36 loads): 512 x 256
+  // MOSFET 16.0 with two slots a thread, 17.7 with 448 threads.
   constexpr int T3 = rb_resident_js_slots(TCAD_NE3);
   // (the test hook holds up a grid barrier; clusters have none)
   if (L.cluster && !krylov_fused_hold()) {
@@ -2864,7 +2864,8 @@ extern "C" int tcad_block_krylov(const tcad_pack_t* pk, const double* J, const d
     if (work_bytes < tcad_block_workspace_bytes(pk, 2, 0)) return TCAD_ERR_ARG;
     const WorkRb wrb = carve_rb(pk, reinterpret_cast<char*>(work) + off_rb(pk));
     RbLayout rbl;
-    if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk->dim))) != TCAD_OK) return rc;
+    if ((rc = rb_layout(pk, wrb, rbl, s, kRbResidentMaxSlots, rb_cluster_slots(pk->dim))))
+      return rc;
     rb_pack(pk, rbl, wrb, J, s);
     TCAD_LAUNCH_CHECK();
     rc = launch_bicgstab_rb(pk, rbl, wrb, b, x, rtol, maxiter, w, nullptr, hks, s, nullptr);

@@ -142,8 +142,9 @@ struct RbStreamer {
     if (lane == 0 && !lost) {
       constexpr unsigned n = NE * 32 * sizeof(double);
       mbar_expect(&sh.bar[warp], n);
-      if (!hold) bulk_copy(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32), n, &sh.bar[warp],
-                policy);
+      if (!hold)
+        bulk_copy(tile, (col ? JB : JR) + ((q.begin >> 5) + warp) * (NE * 32), n, &sh.bar[warp],
+                  policy);
     }
   }
   __device__ __forceinline__ void arrive() {

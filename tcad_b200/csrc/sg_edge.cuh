@@ -47,7 +47,8 @@ struct WideDivisor {
   static __device__ __forceinline__ WideDivisor of(double b) {
     // by the exponent: below 2^-700, to 2^700, above
     const unsigned e = (unsigned)__double2hiint(b) >> 20 & 0x7ffu;
-    const double s = __hiloint2double(e < 323u ? 1623 << 20 : e > 1723u ? 423 << 20 : 1023 << 20, 0);
+    const int k = e < 323u ? 1623 : e > 1723u ? 423 : 1023;
+    const double s = __hiloint2double(k << 20, 0);
     return WideDivisor{Divisor::of(b * s), s};
   }
   __device__ __forceinline__ double divide(double a) const { return d.divide(a * s); }
